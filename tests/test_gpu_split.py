@@ -1,0 +1,50 @@
+"""Field items cut by targets and sources (Fields::split): every batch size around a
+warp, a CTA's targets and a tile of sources, against the FP64 oracle.
+
+The oracle's treecode uses the same lists, so FP64 results agree to 1e-12 and
+mixed ones to 1e-6 (relative L2), the bounds of the other convolution tests.
+"""
+import numpy as np
+import pytest
+
+from conftest import rel_l2, to_cuda
+
+pytestmark = pytest.mark.gpu
+
+# leaf: batches of at most that many points; n: total (the last ones are ragged)
+SIZES = [(33, 700), (63, 1500), (64, 1500), (65, 1531), (129, 3000), (257, 5003), (520, 9001)]
+
+
+def cloud(n, seed):
+    rng = np.random.default_rng(seed)
+    p = rng.uniform(-1.0, 1.0, (3, n)) * np.array([[3.0], [2.0], [2.5]])
+    return p[0].copy(), p[1].copy(), p[2].copy(), rng.uniform(0.5, 1.5, n) / n, rng.standard_normal(n)
+
+
+@pytest.mark.parametrize("leaf,n", SIZES)
+@pytest.mark.parametrize("precision,tol", [("mixed", 1e-6), ("fp64", 1e-12)])
+def test_ragged_batches_match_oracle(BT, dev, oracle, leaf, n, precision, tol):
+    x, y, z, w, f = cloud(n, leaf)
+    degree = 2 + leaf % 3
+    plan = dev.TreecodePlan.for_mesh(*to_cuda(x, y, z, w), theta=0.8, degree=degree, source_leaf=leaf, target_leaf=leaf)
+    c = oracle.Plan(x, y, z, x, y, z, w, 0.8, degree, leaf, leaf, 1.0)
+    (ft,) = to_cuda(f)
+    for kernel in (BT.Kernel.YUKAWA, BT.Kernel.COULOMB):
+        for sing in (BT.Singularity.SUBTRACTION, BT.Singularity.SKIPPING):
+            ref = c.convolve(f, f, w, kernel, [1.3], sing)
+            for nt in ((1, 2) if precision == "mixed" else (0,)):
+                got = plan.convolve(ft, ft, kernel, [1.3], sing, precision=precision, targets_per_thread=nt)
+                assert rel_l2(got.cpu().numpy(), ref) <= tol
+    plan.close()
+
+
+def test_targets_that_are_not_sources(BT, dev, oracle):
+    x, y, z, w, f = cloud(4001, 5)
+    tx, ty, tz, _, tv = cloud(611, 6)
+    plan = dev.TreecodePlan(*to_cuda(tx, ty, tz), *to_cuda(x, y, z, w), theta=0.8, degree=3, source_leaf=100,
+                            target_leaf=130)
+    c = oracle.Plan(tx, ty, tz, x, y, z, w, 0.8, 3, 100, 130, 1.0)
+    ref = c.convolve(tv, f, w, BT.Kernel.YUKAWA, [0.9], BT.Singularity.SUBTRACTION)
+    for precision, tol in (("mixed", 1e-6), ("fp64", 1e-12)):
+        got = plan.convolve(*to_cuda(tv, f), BT.Kernel.YUKAWA, [0.9], BT.Singularity.SUBTRACTION, precision=precision)
+        assert rel_l2(got.cpu().numpy(), ref) <= tol

@@ -1,9 +1,14 @@
 // Subsystems (c) far field and (d) near field, plus the per-call glue.
 //
-// One CTA works on one (target batch, orbital) item at a time, pulled from a
-// global counter in heaviest-batch-first order (persistent launch, grid =
-// resident CTAs).  Each target's sum is formed in a fixed order (list order,
-// then source order), so results do not depend on scheduling.
+// One CTA works on one (target chunk of a batch, orbital) item at a time,
+// pulled from a global counter in heaviest-first order (persistent launch,
+// grid = resident CTAs).  In the single-orbital kernels the CTA's eight warps
+// form G groups of targets times S = 8 / G splits of each target's sources
+// (Fields::split, set per plan by field_split).  Each target's sum is formed in
+// a fixed order (list order, then source order), so results do not depend on
+// scheduling; in mixed precision not on the split either: the splits' FP32
+// partials go through shared memory to one thread per target, which adds them
+// in list order.
 //
 // Mixed precision (default fast path):
 //   * coordinates are translated to the batch center in FP64, then rounded to
@@ -40,7 +45,11 @@ namespace tagi {
 namespace {
 
 constexpr int FT = 256;        // threads per field CTA
+constexpr int FW = FT / 32;    // warps per field CTA
 constexpr int NTILE = 512;     // sources per near-field tile
+constexpr int SLOT = 64;       // sources per slot of a tile: one FP32 run per lane pair
+constexpr int SLOTS = NTILE / SLOT;
+static_assert(SLOTS == FW, "warp w stages slot w of a tile");
 constexpr double LOG2E = 1.4426950408889634;
 
 __device__ __forceinline__ float rsqrt_mufu(float x) {
@@ -80,7 +89,7 @@ struct Fields {
     const double *geom;
     const float *qhat32, *what32; // [norb][nslots][P], [nslots][P]
     const double *qhat64, *what64;
-    int nslots, n1, P;
+    int nslots, n1, P, split;     // split: warps that share a target's sources (1, 2, 4 or 8)
     double tn[MAX_DEGREE + 1];
     // per orbital
     const float *ft32;            // [norb][nt] sorted target values
@@ -95,7 +104,7 @@ struct Fields {
 // a CTA reads the fields of its current item's system straight from the
 // parameter bank (dynamic index, no local copy).
 struct Work {
-    const int2 *items;            // {batch, sys << 16 | first orbital}, heaviest first
+    const int4 *items;            // {batch, sys << 16 | first orbital, target begin, end}, heaviest first
     int nitems;
     int *queue;                   // this pass's work counter
     Fields sys[MAX_SYSTEMS];
@@ -107,6 +116,98 @@ __device__ __forceinline__ int next_item(int *queue, int *s_item) {
     if (threadIdx.x == 0) *s_item = atomicAdd(queue, 1);
     __syncthreads();
     return *s_item;
+}
+
+// The place of a warp in its CTA: target group g of G, source split sp of S.
+struct Place {
+    int S, G, g, sp, lane, wid;
+    __device__ __forceinline__ explicit Place(int split)
+        : S(split), G(FW / split), lane(threadIdx.x & 31), wid(threadIdx.x >> 5) {
+        g = wid & (G - 1);
+        sp = wid / G;
+    }
+};
+
+// Adds the S splits' values v of each of a CTA's targets in split order; the
+// result is valid in split 0.  red: FT doubles of shared memory that no warp
+// still reads (the barrier here orders it after the last tile).
+__device__ __forceinline__ double add_splits(double v, const Place &pl, double *red) {
+    if (pl.S == 1) return v;
+    __syncthreads();
+    red[threadIdx.x] = v;   // threadIdx.x = sp * 32 G + (target group, lane)
+    __syncthreads();
+    if (pl.sp) return 0.0;
+    for (int s = 1; s < pl.S; s++) v += red[threadIdx.x + s * 32 * pl.G];
+    return v;
+}
+
+// The near ranges of one pass in list order, up to a CTA's THREADS of them at a
+// time, cut into chunks of SLOT sources: first[i] = chunks before range i.  A
+// tile holds the next chunks whatever ranges they come from (one slot per warp,
+// which stages it), so the warps of a CTA stay evenly loaded where ranges are
+// short or end inside a tile.
+template <int THREADS>
+struct RangeTable {
+    int begin[THREADS], end[THREADS], first[THREADS];
+    int wsum[THREADS / 32], wkeep[THREADS / 32];
+};
+
+// Fills t with the kept ranges of e0 .. e0 + THREADS - 1; returns their number and
+// the number of chunks.  keep(range, dmin) decides; it leaves in range.x the
+// begin, with bit 31 free for its own use.
+template <int THREADS, typename Keep>
+__device__ __forceinline__ int2 load_ranges(const Fields &a, int e0, int r1, RangeTable<THREADS> &t, Keep keep) {
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int e = e0 + threadIdx.x;
+    int2 r = make_int2(0, 0);
+    bool k = false;
+    if (e < r1) {
+        r = a.rng[e];
+        k = keep(r, a.rng_dmin[e]);
+    }
+    const int n = k ? (r.y - (r.x & 0x7fffffff) + SLOT - 1) / SLOT : 0;
+    const unsigned m = __ballot_sync(0xffffffffu, k);
+    int incl = n;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += v;
+    }
+    __syncthreads();   // the table's previous contents are no longer read
+    if (lane == 31) {
+        t.wsum[wid] = incl;
+        t.wkeep[wid] = __popc(m);
+    }
+    __syncthreads();
+    int first = incl - n, pos = __popc(m & ((1u << lane) - 1u)), nr = 0, nch = 0;
+#pragma unroll
+    for (int w = 0; w < THREADS / 32; w++) {
+        if (w < wid) {
+            first += t.wsum[w];
+            pos += t.wkeep[w];
+        }
+        nch += t.wsum[w];
+        nr += t.wkeep[w];
+    }
+    if (k) {
+        t.begin[pos] = r.x;   // keep() may have set bit 31 anew
+        t.end[pos] = r.y;
+        t.first[pos] = first;
+    }
+    __syncthreads();
+    return make_int2(nr, nch);
+}
+
+// The range that holds chunk c (0 <= c < chunks of the table's nr ranges).
+template <int THREADS>
+__device__ __forceinline__ int range_of_chunk(const RangeTable<THREADS> &t, int nr, int c) {
+    int lo = 0, hi = nr - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (t.first[mid] <= c) lo = mid;
+        else hi = mid - 1;
+    }
+    return lo;
 }
 
 // Packed FP32 pairs.  On the sm_100 family one FADD2 / FMUL2 / FFMA2
@@ -163,6 +264,40 @@ __device__ __forceinline__ void kahan_add(float &sum, float &cmp, float part) {
 __device__ __forceinline__ float4 lds4(const float *p) { return *reinterpret_cast<const float4 *>(p); }
 __device__ __forceinline__ float2 lds2(const float *p) { return *reinterpret_cast<const float2 *>(p); }
 
+// Batch-relative source coordinates from the FP32 hi/lo splits (x = h + l to
+// 2^-48 |x|, the batch center c = ch + cl likewise), for two sources at once:
+// the exact difference of the hi parts as a rounded sum and its error (Knuth's
+// two-sum), plus the difference of the lo parts, rounded once.  The value is
+// that of FP64 arithmetic rounded to FP32, except that a difference within about
+// 2^-48 |x| of a rounding tie may fall on the other side.  FP64 subtraction and
+// scaling cost the FP64 pipe (2 lanes per clock and SM) 1,500 clocks per
+// 512-source tile, as long as the pair loops of 64 targets take for half of it.
+__device__ __forceinline__ float2 neg2(float2 a) { return make_float2(-a.x, -a.y); }
+struct Split {
+    float2 h, l;   // a coordinate's hi and lo part in both lanes
+    __device__ __forceinline__ explicit Split(double c) : h(dup2((float)c)), l(dup2((float)(c - (double)(float)c))) {}
+};
+// -(x - c) as rounded difference plus error
+__device__ __forceinline__ void minus_center(float2 xh, float2 xl, const Split &c, float2 &d, float2 &e) {
+    d = add2(c.h, neg2(xh));
+    const float2 b = add2(d, neg2(c.h));
+    e = add2(add2(c.h, neg2(add2(d, neg2(b)))), neg2(add2(xh, b)));
+    e = add2(e, add2(c.l, neg2(xl)));
+}
+__device__ __forceinline__ float2 neg_relative(float2 xh, float2 xl, const Split &c) {
+    float2 d, e;
+    minus_center(xh, xl, c, d, e);
+    return add2(d, e);
+}
+// -(x - c) sc, rounded once
+__device__ __forceinline__ float2 neg_relative(float2 xh, float2 xl, const Split &c, float2 sc) {
+    float2 d, e;
+    minus_center(xh, xl, c, d, e);
+    const float2 p = mul2(d, sc);
+    return add2(p, fma2(e, sc, fma2(d, sc, neg2(p))));
+}
+__device__ __forceinline__ void sts2(float *p, float2 v) { *reinterpret_cast<float2 *>(p) = v; }
+
 // Near-field source tile in shared memory, structure of arrays, NEGATED
 // coordinates so that one FADD2 forms t - s for two sources:
 //   row 0..2  -x, -y, -z   (ordinary tiles: scaled batch-relative FP32;
@@ -173,66 +308,62 @@ __device__ __forceinline__ float2 lds2(const float *p) { return *reinterpret_cas
 // A tile of cnt sources is padded to cnt4 = a multiple of 4 with copies of
 // its first source carrying q = w = 0: their terms are exactly +-0.
 //
-// One tile against NT targets, two sources per packed operation.  Pairs are
-// summed in FP32 per lane over chunks of KCHUNK sources; each chunk's two
-// lane sums are added and the result enters the target's Kahan sum: a long
+// One slot of a tile (n sources from j0, a multiple of 4) against NT targets, two
+// sources per packed operation.  Its pairs are summed in FP32 per lane and the
+// two lane sums are added into out, which enters the target's Kahan sum: a long
 // FP32 run loses ~sqrt(n) u of its total, and singularity subtraction
 // multiplies that loss by |f_i int G| / |phi_i| (often 10-100).
 // PRECISE tiles (close ranges): each difference is (t_hi - s_hi) +
 // (t_lo - s_lo) -- exact hi differences for nearby points -- and the
 // unscaled r^2 is multiplied by sc2 = sc^2, so the shortest pairs keep FP32
 // relative precision in r whatever the batch size.
-constexpr int KCHUNK = 64;
 constexpr int NROWS_PRECISE = 8;
 template <int KERN, bool SS, bool MASK, bool PRECISE, int NT>
-__device__ __forceinline__ void near_tile(const float (*__restrict__ s)[NTILE], int cnt4, const float2 (&tx)[NT],
+__device__ __forceinline__ void near_chunk(const float (*__restrict__ s)[NTILE], int j0, int n, const float2 (&tx)[NT],
                                           const float2 (&ty)[NT], const float2 (&tz)[NT], const float2 (&lx)[NT],
                                           const float2 (&ly)[NT], const float2 (&lz)[NT], float2 sc2,
-                                          const float2 (&nfi)[NT], float (&sum)[NT], float (&cmp)[NT]) {
-    for (int j0 = 0; j0 < cnt4; j0 += KCHUNK) {
-        const int j1 = min(j0 + KCHUNK, cnt4);
-        float2 part[NT];
+                                          const float2 (&nfi)[NT], float (&out)[NT]) {
+    const int j1 = j0 + n;
+    float2 part[NT];
 #pragma unroll
-        for (int k = 0; k < NT; k++) part[k] = make_float2(0.f, 0.f);
+    for (int k = 0; k < NT; k++) part[k] = make_float2(0.f, 0.f);
 #pragma unroll 2
-        for (int j = j0; j < j1; j += 4) {
-            const float4 X = lds4(s[0] + j), Y = lds4(s[1] + j), Z = lds4(s[2] + j);
-            const float4 Q = lds4(s[3] + j), W = lds4(s[4] + j);
-            float4 XL = make_float4(0.f, 0.f, 0.f, 0.f), YL = XL, ZL = XL;
-            if constexpr (PRECISE) {
-                XL = lds4(s[5] + j);
-                YL = lds4(s[6] + j);
-                ZL = lds4(s[7] + j);
-            }
-#pragma unroll
-            for (int h = 0; h < 2; h++) {
-                const float2 sx = h ? make_float2(X.z, X.w) : make_float2(X.x, X.y);
-                const float2 sy = h ? make_float2(Y.z, Y.w) : make_float2(Y.x, Y.y);
-                const float2 sz = h ? make_float2(Z.z, Z.w) : make_float2(Z.x, Z.y);
-                const float2 q = h ? make_float2(Q.z, Q.w) : make_float2(Q.x, Q.y);
-                const float2 w = h ? make_float2(W.z, W.w) : make_float2(W.x, W.y);
-                const float2 sxl = h ? make_float2(XL.z, XL.w) : make_float2(XL.x, XL.y);
-                const float2 syl = h ? make_float2(YL.z, YL.w) : make_float2(YL.x, YL.y);
-                const float2 szl = h ? make_float2(ZL.z, ZL.w) : make_float2(ZL.x, ZL.y);
-#pragma unroll
-                for (int k = 0; k < NT; k++) {
-                    float2 dx = add2(tx[k], sx), dy = add2(ty[k], sy), dz = add2(tz[k], sz);
-                    if (PRECISE) {
-                        dx = add2(dx, add2(lx[k], sxl));
-                        dy = add2(dy, add2(ly[k], syl));
-                        dz = add2(dz, add2(lz[k], szl));
-                    }
-                    float2 r2 = fma2(dx, dx, fma2(dy, dy, mul2(dz, dz)));
-                    if (PRECISE) r2 = mul2(r2, sc2);
-                    part[k] = pair2<KERN, SS, MASK>(r2, q, w, nfi[k], part[k]);
-                }
-            }
+    for (int j = j0; j < j1; j += 4) {
+        const float4 X = lds4(s[0] + j), Y = lds4(s[1] + j), Z = lds4(s[2] + j);
+        const float4 Q = lds4(s[3] + j), W = lds4(s[4] + j);
+        float4 XL = make_float4(0.f, 0.f, 0.f, 0.f), YL = XL, ZL = XL;
+        if constexpr (PRECISE) {
+            XL = lds4(s[5] + j);
+            YL = lds4(s[6] + j);
+            ZL = lds4(s[7] + j);
         }
 #pragma unroll
-        for (int k = 0; k < NT; k++) kahan_add(sum[k], cmp[k], part[k].x + part[k].y);
+        for (int h = 0; h < 2; h++) {
+            const float2 sx = h ? make_float2(X.z, X.w) : make_float2(X.x, X.y);
+            const float2 sy = h ? make_float2(Y.z, Y.w) : make_float2(Y.x, Y.y);
+            const float2 sz = h ? make_float2(Z.z, Z.w) : make_float2(Z.x, Z.y);
+            const float2 q = h ? make_float2(Q.z, Q.w) : make_float2(Q.x, Q.y);
+            const float2 w = h ? make_float2(W.z, W.w) : make_float2(W.x, W.y);
+            const float2 sxl = h ? make_float2(XL.z, XL.w) : make_float2(XL.x, XL.y);
+            const float2 syl = h ? make_float2(YL.z, YL.w) : make_float2(YL.x, YL.y);
+            const float2 szl = h ? make_float2(ZL.z, ZL.w) : make_float2(ZL.x, ZL.y);
+#pragma unroll
+            for (int k = 0; k < NT; k++) {
+                float2 dx = add2(tx[k], sx), dy = add2(ty[k], sy), dz = add2(tz[k], sz);
+                if (PRECISE) {
+                    dx = add2(dx, add2(lx[k], sxl));
+                    dy = add2(dy, add2(ly[k], syl));
+                    dz = add2(dz, add2(lz[k], szl));
+                }
+                float2 r2 = fma2(dx, dx, fma2(dy, dy, mul2(dz, dz)));
+                if (PRECISE) r2 = mul2(r2, sc2);
+                part[k] = pair2<KERN, SS, MASK>(r2, q, w, nfi[k], part[k]);
+            }
+        }
     }
+#pragma unroll
+    for (int k = 0; k < NT; k++) out[k] = part[k].x + part[k].y;
 }
-
 
 // ---------------------------------------------------------------------------
 // Near field, mixed precision.
@@ -247,105 +378,152 @@ template <int KERN, bool SS, int NT, int PASS>
 __global__ void __launch_bounds__(FT, TAGI_NEAR_MINB) near_mixed(const __grid_constant__ Work w) {
     constexpr int NR = PASS == 1 ? NROWS_PRECISE : 5;
     __shared__ __align__(16) float s_src[NR][NTILE];
+    __shared__ RangeTable<FT> s_rng;
+    __shared__ __align__(16) float s_part[SLOTS * FT];   // S > 1: partials [slot][target of the CTA]
+    __shared__ int s_cnt[SLOTS];   // sources of each slot, a multiple of 4; bit 30: leave the Gaussian out
     __shared__ int s_item;
+    constexpr int NOEXP = 1 << 30;
     const int tid = threadIdx.x;
     for (;;) {
         const int item = next_item(w.queue, &s_item);
         if (item >= w.nitems) break;
-        const int2 it = w.items[item];
+        const int4 it = w.items[item];
         const Fields &a = w.sys[it.y >> 16];
+        const Place pl(a.split);
         const int b = it.x, orb = it.y & 0xffff;
         const int bn = a.batch_node[b];
-        const int tb = a.tbegin[bn], te = a.tend[bn];
+        const int te = it.w;
         const double cbx = a.tcenter[3L * bn], cby = a.tcenter[3L * bn + 1],
                      cbz = a.tcenter[3L * bn + 2];
         const float scf = a.kc32[orb];
         const double sc = (double)scf;
         const float2 sc2 = dup2((float)(sc * sc));
+        const Split ccx(cbx), ccy(cby), ccz(cbz);
         const float *q = a.q32 + (long)orb * a.ns;
         const float *ft = a.ft32 + (long)orb * a.nt;
         const int r0 = a.rng_off[b], r1 = a.rng_off[b + 1];
-        for (int base = tb; base < te; base += FT * NT) {
-            // consecutive targets per thread: the threads with targets form a
-            // prefix, so whole warps past it have none and skip the pair loops
-            const bool warp_busy = base + NT * (tid & ~31) < te;
-            float2 tx[NT], ty[NT], tz[NT], lx[NT], ly[NT], lz[NT], nfi[NT];
-            float sum[NT], cmp[NT];
+        // consecutive targets per thread: the threads with targets form a
+        // prefix of the groups, so whole warps past it skip the pair loops
+        const int i0 = it.z + NT * (32 * pl.g + pl.lane);
+        const bool warp_busy = it.z + NT * 32 * pl.g < te;
+        float2 tx[NT], ty[NT], tz[NT], lx[NT], ly[NT], lz[NT], nfi[NT];
+        // S == 1: the Kahan sums of this thread's own targets; S > 1: sum[0], cmp[0]
+        // are those of target it.z + tid
+        float sum[NT], cmp[NT];
+        const int T = 32 * pl.G * NT;
+        int pending = 0;   // slots of the last tile whose partials are still to be added
+        auto add_pending = [&]() {
+            if (tid < T)
+                for (int sl = 0; sl < pending; sl++) kahan_add(sum[0], cmp[0], s_part[sl * T + tid]);
+        };
 #pragma unroll
-            for (int k = 0; k < NT; k++) {
-                const int i = base + NT * tid + k;
-                const bool v = i < te;
-                if (PASS == 1) {
-                    const float4 h = v ? a.thi[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-                    const float4 l = v ? a.tlo[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-                    tx[k] = dup2(h.x);
-                    ty[k] = dup2(h.y);
-                    tz[k] = dup2(h.z);
-                    lx[k] = dup2(l.x);
-                    ly[k] = dup2(l.y);
-                    lz[k] = dup2(l.z);
-                } else {
-                    tx[k] = dup2(v ? (float)((a.tx[i] - cbx) * sc) : 0.f);
-                    ty[k] = dup2(v ? (float)((a.ty[i] - cby) * sc) : 0.f);
-                    tz[k] = dup2(v ? (float)((a.tz[i] - cbz) * sc) : 0.f);
-                    lx[k] = ly[k] = lz[k] = dup2(0.f);
-                }
-                nfi[k] = dup2(v ? -ft[i] : 0.f);
-                sum[k] = 0.f;
-                cmp[k] = 0.f;
+        for (int k = 0; k < NT; k++) {
+            const int i = i0 + k;
+            const bool v = i < te;
+            if (PASS == 1) {
+                const float4 h = v ? a.thi[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+                const float4 l = v ? a.tlo[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+                tx[k] = dup2(h.x);
+                ty[k] = dup2(h.y);
+                tz[k] = dup2(h.z);
+                lx[k] = dup2(l.x);
+                ly[k] = dup2(l.y);
+                lz[k] = dup2(l.z);
+            } else {
+                tx[k] = dup2(v ? (float)((a.tx[i] - cbx) * sc) : 0.f);
+                ty[k] = dup2(v ? (float)((a.ty[i] - cby) * sc) : 0.f);
+                tz[k] = dup2(v ? (float)((a.tz[i] - cbz) * sc) : 0.f);
+                lx[k] = ly[k] = lz[k] = dup2(0.f);
             }
-            for (int e = r0; e < r1; e++) {
-                const int2 r = a.rng[e];
-                const bool close = range_is_close(r);
-                if (close != (PASS == 1)) continue;
-                const int rb = range_begin(r);
-                // Ranges far enough away: Yukawa terms are exactly 0 in FP32
-                // (2^{-r'} with r' > 127 flushes to zero); the Coulomb Gaussian
-                // correction is below 2^-40 of its term and is left out.
-                const float dm = a.rng_dmin[e] * scf;
-                if (KERN == KERNEL_YUKAWA && dm > 127.f) continue;
-                const bool noexp = KERN == KERNEL_COULOMB && SS && dm * dm > 40.f;
-                for (int t0 = rb; t0 < r.y; t0 += NTILE) {
-                    const int cnt = min(NTILE, r.y - t0);
-                    const int cnt4 = (cnt + 3) & ~3;
-                    __syncthreads();
-                    for (int j = tid; j < cnt4; j += FT) {
-                        const bool real = j < cnt;
-                        const int jj = t0 + (real ? j : 0);   // padding: a copy of the first source
+            nfi[k] = dup2(v ? -ft[i] : 0.f);
+            sum[k] = 0.f;
+            cmp[k] = 0.f;
+        }
+        for (int e0 = r0; e0 < r1; e0 += FT) {
+            // Ranges far enough away: Yukawa terms are exactly 0 in FP32
+            // (2^{-r'} with r' > 127 flushes to zero) and the range is left out;
+            // the Coulomb Gaussian correction is below 2^-40 of its term and is
+            // left out (bit 31 of the table's begin, free once the pass is chosen).
+            const int2 n = load_ranges(a, e0, r1, s_rng, [&](int2 &r, float dmin) {
+                if (range_is_close(r) != (PASS == 1)) return false;
+                const float dm = dmin * scf;
+                if (KERN == KERNEL_YUKAWA && dm > 127.f) return false;
+                const bool noexp = KERN == KERNEL_COULOMB && SS && PASS == 0 && dm * dm > 40.f;
+                r.x = range_begin(r) | (noexp ? (int)0x80000000u : 0);
+                return true;
+            });
+            for (int c0 = 0; c0 < n.y; c0 += SLOTS) {
+                __syncthreads();   // the previous tile is no longer read, its partials are written
+                if (pl.S > 1) {
+                    add_pending();
+                    pending = min(SLOTS, n.y - c0);
+                }
+                const int c = c0 + pl.wid;
+                int cnt4 = 0, flag = 0;
+                if (c < n.y) {
+                    const int e = range_of_chunk(s_rng, n.x, c);
+                    const int rb = s_rng.begin[e];
+                    const int t0 = (rb & 0x7fffffff) + (c - s_rng.first[e]) * SLOT;
+                    const int cnt = min(SLOT, s_rng.end[e] - t0);
+                    cnt4 = (cnt + 3) & ~3;
+                    flag = rb < 0 ? NOEXP : 0;
+                    const int j = 2 * pl.lane, d = pl.wid * SLOT + j;
+                    if (j < cnt4) {
+                        const bool real0 = j < cnt, real1 = j + 1 < cnt;
+                        const int j0 = t0 + (real0 ? j : 0), j1 = t0 + (real1 ? j + 1 : 0);   // padding: the first source
+                        const float4 h0 = a.shi[j0], h1 = a.shi[j1], l0 = a.slo[j0], l1 = a.slo[j1];
+                        const float2 hx = make_float2(h0.x, h1.x), hy = make_float2(h0.y, h1.y),
+                                     hz = make_float2(h0.z, h1.z), qx = make_float2(l0.x, l1.x),
+                                     qy = make_float2(l0.y, l1.y), qz = make_float2(l0.z, l1.z);
                         if constexpr (PASS == 1) {
-                            const float4 h = a.shi[jj], l = a.slo[jj];
-                            s_src[0][j] = -h.x;
-                            s_src[1][j] = -h.y;
-                            s_src[2][j] = -h.z;
-                            s_src[5][j] = -l.x;
-                            s_src[6][j] = -l.y;
-                            s_src[7][j] = -l.z;
+                            sts2(&s_src[0][d], neg2(hx));
+                            sts2(&s_src[1][d], neg2(hy));
+                            sts2(&s_src[2][d], neg2(hz));
+                            sts2(&s_src[5][d], neg2(qx));
+                            sts2(&s_src[6][d], neg2(qy));
+                            sts2(&s_src[7][d], neg2(qz));
                         } else {
-                            s_src[0][j] = -(float)((a.sx[jj] - cbx) * sc);
-                            s_src[1][j] = -(float)((a.sy[jj] - cby) * sc);
-                            s_src[2][j] = -(float)((a.sz[jj] - cbz) * sc);
+                            sts2(&s_src[0][d], neg_relative(hx, qx, ccx, dup2(scf)));
+                            sts2(&s_src[1][d], neg_relative(hy, qy, ccy, dup2(scf)));
+                            sts2(&s_src[2][d], neg_relative(hz, qz, ccz, dup2(scf)));
                         }
-                        s_src[3][j] = real ? q[jj] : 0.f;
-                        s_src[4][j] = real ? a.w32[jj] : 0.f;
+                        sts2(&s_src[3][d], make_float2(real0 ? q[j0] : 0.f, real1 ? q[j1] : 0.f));
+                        sts2(&s_src[4][d], make_float2(real0 ? a.w32[j0] : 0.f, real1 ? a.w32[j1] : 0.f));
                     }
-                    __syncthreads();
-                    if (!warp_busy) continue;
-                    if (PASS == 1)
-                        near_tile<KERN, SS, true, true, NT>(s_src, cnt4, tx, ty, tz, lx, ly, lz, sc2, nfi, sum, cmp);
-                    else if (noexp)
-                        near_tile<KERN, false, false, false, NT>(s_src, cnt4, tx, ty, tz, lx, ly, lz, sc2, nfi, sum,
-                                                                 cmp);
-                    else
-                        near_tile<KERN, SS, false, false, NT>(s_src, cnt4, tx, ty, tz, lx, ly, lz, sc2, nfi, sum,
-                                                              cmp);
                 }
-            }
+                if (pl.lane == 0) s_cnt[pl.wid] = cnt4 | flag;
+                __syncthreads();
+                if (!warp_busy) continue;
+                for (int sl = pl.sp; sl < SLOTS; sl += pl.S) {
+                    const int m = s_cnt[sl];
+                    if (m == 0) break;
+                    float part[NT];
+                    if (PASS == 1)
+                        near_chunk<KERN, SS, true, true, NT>(s_src, sl * SLOT, m, tx, ty, tz, lx, ly, lz, sc2, nfi, part);
+                    else if (KERN == KERNEL_COULOMB && SS && (m & NOEXP))
+                        near_chunk<KERN, false, false, false, NT>(s_src, sl * SLOT, m & ~NOEXP, tx, ty, tz, lx, ly,
+                                                                  lz, sc2, nfi, part);
+                    else
+                        near_chunk<KERN, SS, false, false, NT>(s_src, sl * SLOT, m, tx, ty, tz, lx, ly, lz, sc2, nfi,
+                                                               part);
 #pragma unroll
-            for (int k = 0; k < NT; k++) {
-                const int i = base + NT * tid + k;
-                if (i < te) a.out[(long)orb * a.nt + i] = ((double)sum[k] - (double)cmp[k]) * sc;
+                    for (int k = 0; k < NT; k++) {
+                        if (pl.S == 1) kahan_add(sum[k], cmp[k], part[k]);
+                        else s_part[sl * T + NT * (32 * pl.g + pl.lane) + k] = part[k];
+                    }
+                }
             }
         }
+        if (pl.S > 1) {
+            __syncthreads();
+            add_pending();
+            if (tid < T && it.z + tid < te)
+                a.out[(long)orb * a.nt + it.z + tid] = ((double)sum[0] - (double)cmp[0]) * sc;
+            continue;
+        }
+#pragma unroll
+        for (int k = 0; k < NT; k++)
+            if (i0 + k < te) a.out[(long)orb * a.nt + i0 + k] = ((double)sum[k] - (double)cmp[k]) * sc;
     }
 }
 
@@ -359,16 +537,16 @@ __global__ void __launch_bounds__(FT, TAGI_NEAR_MINB) near_mixed(const __grid_co
 // proxy point, the Gaussian term f_i what_k 2^{-r'^2} is below 2^-40 of
 // f_i what_k and is dropped (one MUFU op less per pair); Yukawa clusters
 // with r' > 127 everywhere add exactly 0 in FP32 (2^{-r'} flushes to zero)
-// and are skipped.
+// and are skipped.  add(k1, k, v) takes target k's partial of slab k1.
 // ---------------------------------------------------------------------------
 template <int MAXN1>
 __host__ __device__ constexpr int even_up() { return MAXN1 + (MAXN1 & 1); }
 
-template <int KERN, bool SS, bool EXPTERM, int MAXN1, int NT, bool EXACT = false>
+template <int KERN, bool SS, bool EXPTERM, int MAXN1, int NT, bool EXACT, typename Add>
 __device__ __forceinline__ void far_cluster(const float *__restrict__ s_q, const float *__restrict__ s_w,
-                                            const float (*s_p)[MAXN1], int n1_in, const float (&tx)[NT],
-                                            const float (&ty)[NT], const float (&tz)[NT],
-                                            const float2 (&nfi)[NT], float (&sum)[NT], float (&cmp)[NT]) {
+                                            const float (*s_p)[MAXN1], int n1_in, int slab0, int slab_step,
+                                            const float (&tx)[NT], const float (&ty)[NT], const float (&tz)[NT],
+                                            const float2 (&nfi)[NT], Add add) {
     constexpr int MH = even_up<MAXN1>() / 2;
     constexpr bool PSS = KERN == KERNEL_YUKAWA ? SS : (SS && EXPTERM);
     const int n1 = EXACT ? MAXN1 : n1_in;   // EXACT: every loop bound known at compile time
@@ -382,8 +560,8 @@ __device__ __forceinline__ void far_cluster(const float *__restrict__ s_q, const
             const float d1 = tz[k] - s_p[2][2 * m + 1 < n1 ? 2 * m + 1 : 0];
             dz2[k][m] = make_float2(d0 * d0, d1 * d1);
         }
-    int idx = 0;
-    for (int k1 = 0; k1 < n1; k1++) {  // one (n+1)^2 slab per FP32 partial, then Kahan
+    for (int k1 = slab0; k1 < n1; k1 += slab_step) {  // one (n+1)^2 slab per FP32 partial, then Kahan
+        int idx = k1 * n1 * n1p;
         float2 part[NT];
         float dx2[NT];
 #pragma unroll
@@ -411,96 +589,156 @@ __device__ __forceinline__ void far_cluster(const float *__restrict__ s_q, const
             idx += n1p;
         }
 #pragma unroll
-        for (int k = 0; k < NT; k++) kahan_add(sum[k], cmp[k], part[k].x + part[k].y);
+        for (int k = 0; k < NT; k++) add(k1, k, part[k].x + part[k].y);
     }
 }
 
+// The slabs of cluster number cl of a tile that split sp of S takes start here
+// and go on in steps of S: slabs are dealt to the splits in turn over the
+// whole tile.
+__device__ __forceinline__ int first_slab(int cl, int n1, const Place &pl) { return (pl.sp - cl * n1) & (pl.S - 1); }
+
 // EXACT: every system of the launch has n + 1 = MAXN1 (the loops over the
-// proxy grid are then fully known at compile time).
+// proxy grid are then fully known at compile time).  FAR_CL clusters are
+// staged per pair of barriers.
+template <int MAXN1>
+__host__ __device__ constexpr int far_clusters() { return MAXN1 <= 4 ? 8 : (MAXN1 <= 8 ? 4 : 2); }
+constexpr int FAR_PART = 4096;   // partials of a far tile where a target's slabs are split (16 KB); 11 slabs of 256 targets fit
+static_assert(FAR_PART >= (MAX_DEGREE + 1) * FT, "one cluster's slabs of a CTA's targets");
+
 template <int KERN, bool SS, int MAXN1, int NT, bool EXACT = false>
 __global__ void __launch_bounds__(FT, 2) far_mixed(const __grid_constant__ Work w) {
     constexpr int MAXPP = MAXN1 * MAXN1 * even_up<MAXN1>();
-    __shared__ __align__(16) float s_q[MAXPP];
-    __shared__ __align__(16) float s_w[MAXPP];
-    __shared__ float s_p[3][MAXN1];
-    __shared__ int s_item, s_mode;
+    constexpr int FAR_CL = far_clusters<MAXN1>();
+    __shared__ __align__(16) float s_q[FAR_CL][MAXPP];
+    __shared__ __align__(16) float s_w[FAR_CL][MAXPP];
+    __shared__ float s_p[FAR_CL][3][MAXN1];
+    __shared__ int s_slot[FT];   // the item's next clusters that count: slot << 1 | leave the Gaussian out
+    __shared__ int s_kept[FW];
+    __shared__ float s_part[FAR_PART];   // S > 1: partials [cluster of the tile, slab][target of the CTA]
+    __shared__ int s_item;
     const int tid = threadIdx.x;
     for (;;) {
         const int item = next_item(w.queue, &s_item);
         if (item >= w.nitems) break;
-        const int2 it = w.items[item];
+        const int4 it = w.items[item];
         const Fields &a = w.sys[it.y >> 16];
+        const Place pl(a.split);
         const int b = it.x, orb = it.y & 0xffff;
         const int n1 = EXACT ? MAXN1 : a.n1, P = EXACT ? MAXN1 * MAXN1 * MAXN1 : a.P;
         const int n1p = n1 + (n1 & 1), Pp = n1 * n1 * n1p;
         const int f0 = a.far_off[b], f1 = a.far_off[b + 1];
-        if (f0 == f1) continue;
         const int bn = a.batch_node[b];
-        const int tb = a.tbegin[bn], te = a.tend[bn];
+        const int te = it.w;
         const double cb[3] = {a.tcenter[3L * bn], a.tcenter[3L * bn + 1], a.tcenter[3L * bn + 2]};
         const double rb = a.tradius[bn];
         const float scf = a.kc32[orb];
         const double sc = (double)scf;
         const float *ft = a.ft32 + (long)orb * a.nt;
         const float *qh = a.qhat32 + (long)orb * a.nslots * P;
-        for (int base = tb; base < te; base += FT * NT) {
-            const bool warp_busy = base + NT * (tid & ~31) < te;
-            float tx[NT], ty[NT], tz[NT], sum[NT], cmp[NT];
-            float2 nfi[NT];
+        const int i0 = it.z + NT * (32 * pl.g + pl.lane);
+        const bool warp_busy = it.z + NT * 32 * pl.g < te;
+        float tx[NT], ty[NT], tz[NT];
+        // S == 1: the Kahan sums of this thread's own targets; S > 1: sum[0], cmp[0]
+        // are those of target it.z + tid
+        float sum[NT], cmp[NT];
+        const int T = 32 * pl.G * NT;
+        const int tile = pl.S == 1 ? FAR_CL : min(FAR_CL, max(1, FAR_PART / (T * n1)));
+        int pending = 0;   // slabs of the last tile whose partials are still to be added
+        auto add_pending = [&]() {
+            if (tid < T)
+                for (int u = 0; u < pending; u++) kahan_add(sum[0], cmp[0], s_part[u * T + tid]);
+        };
+        float2 nfi[NT];
 #pragma unroll
-            for (int k = 0; k < NT; k++) {
-                const int i = base + NT * tid + k;
-                const bool v = i < te;
-                tx[k] = v ? (float)(a.tx[i] - cb[0]) * scf : 0.f;
-                ty[k] = v ? (float)(a.ty[i] - cb[1]) * scf : 0.f;
-                tz[k] = v ? (float)(a.tz[i] - cb[2]) * scf : 0.f;
-                nfi[k] = dup2(v ? -ft[i] : 0.f);
-                sum[k] = 0.f;
-                cmp[k] = 0.f;
-            }
-            for (int e = f0; e < f1; e++) {
-                const int slot = a.node_slot[a.far_list[e]];
+        for (int k = 0; k < NT; k++) {
+            const int i = i0 + k;
+            const bool v = i < te;
+            tx[k] = v ? (float)(a.tx[i] - cb[0]) * scf : 0.f;
+            ty[k] = v ? (float)(a.ty[i] - cb[1]) * scf : 0.f;
+            tz[k] = v ? (float)(a.tz[i] - cb[2]) * scf : 0.f;
+            nfi[k] = dup2(v ? -ft[i] : 0.f);
+            sum[k] = 0.f;
+            cmp[k] = 0.f;
+        }
+        for (int e0 = f0; e0 < f1; e0 += FT) {
+            int slot = 0, mode = 2;
+            if (e0 + tid < f1) {
+                slot = a.node_slot[a.far_list[e0 + tid]];
                 const double *g = a.geom + 6L * slot;
-                __syncthreads();
-                const float *qs = qh + (long)slot * P;
-                const float *ws = a.what32 + (long)slot * P;
-                for (int k = tid; k < Pp; k += FT) {
-                    const int row = k / n1p, k3 = k - row * n1p;
-                    const bool real = k3 < n1;
-                    const int src = row * n1 + (real ? k3 : 0);
-                    s_q[k] = real ? qs[src] : 0.f;
-                    s_w[k] = real ? ws[src] : 0.f;
-                }
-                if (tid < 3 * n1) {
-                    const int d = tid / n1, m = tid - d * n1;
-                    const double cbd = d == 0 ? cb[0] : (d == 1 ? cb[1] : cb[2]);
-                    s_p[d][m] = (float)((g[d] + g[3 + d] * a.tn[m]) - cbd) * scf;
-                }
-                if (tid == 0) {
-                    // smallest scaled distance from the batch to the proxy box (conservative)
-                    const double dx = cb[0] - g[0], dy = cb[1] - g[1], dz = cb[2] - g[2];
-                    const double rc = sqrt(g[3] * g[3] + g[4] * g[4] + g[5] * g[5]);
-                    const double dmin = (sqrt(dx * dx + dy * dy + dz * dz) - rb - rc) * sc * (1.0 - 1e-6);
-                    int mode = 0;
-                    if (KERN == KERNEL_YUKAWA && dmin > 127.0) mode = 2;  // 2^{-r'} flushes to 0: adds exactly 0
-                    // Gaussian correction below 2^-40 of its own term everywhere: dropped
-                    if (KERN == KERNEL_COULOMB && SS && dmin > 0.0 && dmin * dmin > 40.0) mode = 1;
-                    s_mode = mode;
-                }
-                __syncthreads();
-                const int mode = s_mode;
-                if (mode == 2 || !warp_busy) continue;
-                if (mode == 1)
-                    far_cluster<KERN, SS, false, MAXN1, NT, EXACT>(s_q, s_w, s_p, n1, tx, ty, tz, nfi, sum, cmp);
-                else
-                    far_cluster<KERN, SS, true, MAXN1, NT, EXACT>(s_q, s_w, s_p, n1, tx, ty, tz, nfi, sum, cmp);
+                // smallest scaled distance from the batch to the proxy box (conservative)
+                const double dx = cb[0] - g[0], dy = cb[1] - g[1], dz = cb[2] - g[2];
+                const double rc = sqrt(g[3] * g[3] + g[4] * g[4] + g[5] * g[5]);
+                const double dmin = (sqrt(dx * dx + dy * dy + dz * dz) - rb - rc) * sc * (1.0 - 1e-6);
+                mode = 0;
+                if (KERN == KERNEL_YUKAWA && dmin > 127.0) mode = 2;  // 2^{-r'} flushes to 0: adds exactly 0
+                // Gaussian correction below 2^-40 of its own term everywhere: dropped
+                if (KERN == KERNEL_COULOMB && SS && dmin > 0.0 && dmin * dmin > 40.0) mode = 1;
             }
+            const unsigned kept = __ballot_sync(0xffffffffu, mode != 2);
+            __syncthreads();   // the previous clusters' slots are no longer read
+            if (pl.lane == 0) s_kept[pl.wid] = __popc(kept);
+            __syncthreads();
+            int pos = __popc(kept & ((1u << pl.lane) - 1u)), ne = 0;
 #pragma unroll
-            for (int k = 0; k < NT; k++) {
-                const int i = base + NT * tid + k;
-                if (i < te) a.out[(long)orb * a.nt + i] = ((double)sum[k] - (double)cmp[k]) * sc;
+            for (int v = 0; v < FW; v++) {
+                if (v < pl.wid) pos += s_kept[v];
+                ne += s_kept[v];
+            }
+            if (mode != 2) s_slot[pos] = (slot << 1) | mode;
+            for (int c0 = 0; c0 < ne; c0 += tile) {
+                const int nc = min(tile, ne - c0);
+                __syncthreads();   // slots written; the previous tile is no longer read, its partials are written
+                if (pl.S > 1) {
+                    add_pending();
+                    pending = nc * n1;
+                }
+                for (int cl = 0; cl < nc; cl++) {
+                    const int sl = s_slot[c0 + cl] >> 1;
+                    const float *qs = qh + (long)sl * P;
+                    const float *ws = a.what32 + (long)sl * P;
+                    for (int k = tid; k < Pp; k += FT) {
+                        const int row = k / n1p, k3 = k - row * n1p;
+                        const bool real = k3 < n1;
+                        const int src = row * n1 + (real ? k3 : 0);
+                        s_q[cl][k] = real ? qs[src] : 0.f;
+                        s_w[cl][k] = real ? ws[src] : 0.f;
+                    }
+                }
+                for (int u = tid; u < 3 * n1 * nc; u += FT) {
+                    const int cl = u / (3 * n1), v = u - cl * 3 * n1;
+                    const int d = v / n1, m = v - d * n1;
+                    const double *g = a.geom + 6L * (s_slot[c0 + cl] >> 1);
+                    const double cbd = d == 0 ? cb[0] : (d == 1 ? cb[1] : cb[2]);
+                    s_p[cl][d][m] = (float)((g[d] + g[3 + d] * a.tn[m]) - cbd) * scf;
+                }
+                __syncthreads();
+                if (!warp_busy) continue;
+                for (int cl = 0; cl < nc; cl++) {
+                    auto add = [&](int k1, int k, float part) {
+                        if (pl.S == 1) kahan_add(sum[k], cmp[k], part);
+                        else s_part[(cl * n1 + k1) * T + NT * (32 * pl.g + pl.lane) + k] = part;
+                    };
+                    const int slab = first_slab(cl, n1, pl);
+                    if (s_slot[c0 + cl] & 1)
+                        far_cluster<KERN, SS, false, MAXN1, NT, EXACT>(s_q[cl], s_w[cl], s_p[cl], n1, slab, pl.S, tx,
+                                                                       ty, tz, nfi, add);
+                    else
+                        far_cluster<KERN, SS, true, MAXN1, NT, EXACT>(s_q[cl], s_w[cl], s_p[cl], n1, slab, pl.S, tx,
+                                                                      ty, tz, nfi, add);
+                }
             }
         }
+        if (pl.S > 1) {
+            __syncthreads();
+            add_pending();
+            if (tid < T && it.z + tid < te)
+                a.out[(long)orb * a.nt + it.z + tid] = ((double)sum[0] - (double)cmp[0]) * sc;
+            continue;
+        }
+#pragma unroll
+        for (int k = 0; k < NT; k++)
+            if (i0 + k < te) a.out[(long)orb * a.nt + i0 + k] = ((double)sum[k] - (double)cmp[k]) * sc;
     }
 }
 
@@ -519,7 +757,9 @@ __global__ void __launch_bounds__(FT, 2) far_mixed(const __grid_constant__ Work 
 // Orbitals past the last one of the request have zero charges and are not
 // written.
 // ---------------------------------------------------------------------------
-constexpr int GTILE = 512;   // sources per group tile
+constexpr int GT = 128;            // threads (targets) per CTA
+constexpr int GW = GT / 32;
+constexpr int GTILE = GW * SLOT;   // sources per group tile, one slot per warp
 
 __device__ __forceinline__ int q4_pos(int j, int o, int og) {   // float index of q(o, j) in the staged layout
     return (((j >> 1) * (og >> 1) + (o >> 1)) << 2) + ((o & 1) << 1) + (j & 1);
@@ -528,68 +768,68 @@ __device__ __forceinline__ int q4_pos(int j, int o, int og) {   // float index o
 // Group tile rows: 0..2 negated coordinates (batch-relative, or hi parts of
 // the absolute splits), 3 weight, 4..6 negated lo parts (PRECISE).
 template <bool SS, bool MASK, bool PRECISE, int OG>
-__device__ __forceinline__ void group_tile(const float (*__restrict__ s)[GTILE], const float4 *__restrict__ s_q4,
-                                           int cnt2, float2 tx, float2 ty, float2 tz, float2 lx, float2 ly,
+__device__ __forceinline__ void group_chunk(const float (*__restrict__ s)[GTILE], const float4 *__restrict__ s_q4,
+                                           int j0, int n, float2 tx, float2 ty, float2 tz, float2 lx, float2 ly,
                                            float2 lz, const float2 (&nfi)[OG], const float2 (&kc)[OG],
                                            float (&sum)[OG], float (&cmp)[OG]) {
-    for (int j0 = 0; j0 < cnt2; j0 += KCHUNK) {
-        const int j1 = min(j0 + KCHUNK, cnt2);
-        float2 part[OG];
+    const int j1 = j0 + n;
+    float2 part[OG];
 #pragma unroll
-        for (int o = 0; o < OG; o++) part[o] = make_float2(0.f, 0.f);
+    for (int o = 0; o < OG; o++) part[o] = make_float2(0.f, 0.f);
 #pragma unroll 1   // measured: unrolling the source loop slows the group kernels
-        for (int j = j0; j < j1; j += 2) {
-            float2 dx = add2(tx, lds2(s[0] + j)), dy = add2(ty, lds2(s[1] + j)), dz = add2(tz, lds2(s[2] + j));
-            if constexpr (PRECISE) {
-                dx = add2(dx, add2(lx, lds2(s[4] + j)));
-                dy = add2(dy, add2(ly, lds2(s[5] + j)));
-                dz = add2(dz, add2(lz, lds2(s[6] + j)));
-            }
-            const float2 wv = lds2(s[3] + j);
-            const float2 r2 = fma2(dx, dx, fma2(dy, dy, mul2(dz, dz)));
-            float2 rinv = rsqrt2(r2);
-            float2 nl = nlog2r2(r2);
-            if (MASK) {   // r = 0: r = 0 and 2^{-inf} = 0, so the pair adds exactly 0
-                rinv.x = r2.x > 0.f ? rinv.x : 0.f;
-                rinv.y = r2.y > 0.f ? rinv.y : 0.f;
-                nl.x = r2.x > 0.f ? nl.x : -INFINITY;
-                nl.y = r2.y > 0.f ? nl.y : -INFINITY;
-            }
-            const float2 r = mul2(r2, rinv);
+    for (int j = j0; j < j1; j += 2) {
+        float2 dx = add2(tx, lds2(s[0] + j)), dy = add2(ty, lds2(s[1] + j)), dz = add2(tz, lds2(s[2] + j));
+        if constexpr (PRECISE) {
+            dx = add2(dx, add2(lx, lds2(s[4] + j)));
+            dy = add2(dy, add2(ly, lds2(s[5] + j)));
+            dz = add2(dz, add2(lz, lds2(s[6] + j)));
+        }
+        const float2 wv = lds2(s[3] + j);
+        const float2 r2 = fma2(dx, dx, fma2(dy, dy, mul2(dz, dz)));
+        float2 rinv = rsqrt2(r2);
+        float2 nl = nlog2r2(r2);
+        if (MASK) {   // r = 0: r = 0 and 2^{-inf} = 0, so the pair adds exactly 0
+            rinv.x = r2.x > 0.f ? rinv.x : 0.f;
+            rinv.y = r2.y > 0.f ? rinv.y : 0.f;
+            nl.x = r2.x > 0.f ? nl.x : -INFINITY;
+            nl.y = r2.y > 0.f ? nl.y : -INFINITY;
+        }
+        const float2 r = mul2(r2, rinv);
 #pragma unroll
-            for (int o2 = 0; o2 < OG / 2; o2++) {
-                const float4 q4 = s_q4[(j >> 1) * (OG / 2) + o2];
+        for (int o2 = 0; o2 < OG / 2; o2++) {
+            const float4 q4 = s_q4[(j >> 1) * (OG / 2) + o2];
 #pragma unroll
-                for (int u = 0; u < 2; u++) {
-                    const int o = 2 * o2 + u;
-                    const float2 q = u ? make_float2(q4.z, q4.w) : make_float2(q4.x, q4.y);
-                    // e^{-k r} / r = 2^{-k log2(e) r - log2 r}
-                    const float2 g = ex2pos2(fma2(kc[o], r, nl));
-                    part[o] = fma2(g, SS ? fma2(nfi[o], wv, q) : q, part[o]);
-                }
+            for (int u = 0; u < 2; u++) {
+                const int o = 2 * o2 + u;
+                const float2 q = u ? make_float2(q4.z, q4.w) : make_float2(q4.x, q4.y);
+                // e^{-k r} / r = 2^{-k log2(e) r - log2 r}
+                const float2 g = ex2pos2(fma2(kc[o], r, nl));
+                part[o] = fma2(g, SS ? fma2(nfi[o], wv, q) : q, part[o]);
             }
         }
-#pragma unroll
-        for (int o = 0; o < OG; o++) kahan_add(sum[o], cmp[o], part[o].x + part[o].y);
     }
+#pragma unroll
+    for (int o = 0; o < OG; o++) kahan_add(sum[o], cmp[o], part[o].x + part[o].y);
 }
 
 template <bool SS, int OG, int PASS>
-__global__ void __launch_bounds__(FT, 2) near_group(const __grid_constant__ Work w) {
+__global__ void __launch_bounds__(GT, 4) near_group(const __grid_constant__ Work w) {
     constexpr int NR = PASS == 1 ? 7 : 4;
     __shared__ __align__(16) float s_src[NR][GTILE];
     __shared__ float4 s_q4[GTILE * OG / 4];
+    __shared__ RangeTable<GT> s_rng;
+    __shared__ int s_cnt[GW];
     __shared__ int s_item;
-    const int tid = threadIdx.x;
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     for (;;) {
         const int item = next_item(w.queue, &s_item);
         if (item >= w.nitems) break;
-        const int2 it = w.items[item];
+        const int4 it = w.items[item];
         const Fields &a = w.sys[it.y >> 16];
         const int b = it.x, g0 = it.y & 0xffff;
         const int bn = a.batch_node[b];
-        const int tb = a.tbegin[bn], te = a.tend[bn];
         const double cbx = a.tcenter[3L * bn], cby = a.tcenter[3L * bn + 1], cbz = a.tcenter[3L * bn + 2];
+        const Split ccx(cbx), ccy(cby), ccz(cbz);
         float2 kc[OG];
         float kmin = 3.4e38f;
 #pragma unroll
@@ -599,83 +839,93 @@ __global__ void __launch_bounds__(FT, 2) near_group(const __grid_constant__ Work
             if (orb < a.norb) kmin = fminf(kmin, a.kc32[orb]);
         }
         const int r0 = a.rng_off[b], r1 = a.rng_off[b + 1];
-        for (int base = tb; base < te; base += FT) {
-            const int i = base + tid;
-            const bool v = i < te;
-            const bool warp_busy = base + (tid & ~31) < te;
-            float2 tx, ty, tz, lx = dup2(0.f), ly = dup2(0.f), lz = dup2(0.f);
-            if (PASS == 1) {  // absolute hi/lo splits (see near_tile)
-                const float4 h = v ? a.thi[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-                const float4 l = v ? a.tlo[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-                tx = dup2(h.x);
-                ty = dup2(h.y);
-                tz = dup2(h.z);
-                lx = dup2(l.x);
-                ly = dup2(l.y);
-                lz = dup2(l.z);
-            } else {
-                tx = dup2(v ? (float)(a.tx[i] - cbx) : 0.f);
-                ty = dup2(v ? (float)(a.ty[i] - cby) : 0.f);
-                tz = dup2(v ? (float)(a.tz[i] - cbz) : 0.f);
-            }
-            float2 nfi[OG];
-            float sum[OG], cmp[OG];
+        const int i = it.z + tid;
+        const bool v = i < it.w;
+        const bool warp_busy = it.z + (tid & ~31) < it.w;
+        float2 tx, ty, tz, lx = dup2(0.f), ly = dup2(0.f), lz = dup2(0.f);
+        if (PASS == 1) {  // absolute hi/lo splits (see near_chunk)
+            const float4 h = v ? a.thi[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+            const float4 l = v ? a.tlo[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+            tx = dup2(h.x);
+            ty = dup2(h.y);
+            tz = dup2(h.z);
+            lx = dup2(l.x);
+            ly = dup2(l.y);
+            lz = dup2(l.z);
+        } else {
+            tx = dup2(v ? (float)(a.tx[i] - cbx) : 0.f);
+            ty = dup2(v ? (float)(a.ty[i] - cby) : 0.f);
+            tz = dup2(v ? (float)(a.tz[i] - cbz) : 0.f);
+        }
+        float2 nfi[OG];
+        float sum[OG], cmp[OG];
 #pragma unroll
-            for (int o = 0; o < OG; o++) {
-                const int orb = g0 + o;
-                nfi[o] = dup2((v && orb < a.norb) ? -a.ft32[(long)orb * a.nt + i] : 0.f);
-                sum[o] = 0.f;
-                cmp[o] = 0.f;
-            }
-            for (int e = r0; e < r1; e++) {
-                const int2 r = a.rng[e];
-                if (a.rng_dmin[e] * kmin > 127.f) continue;  // every orbital's term is exactly 0
-                const bool close = range_is_close(r);
-                if (close != (PASS == 1)) continue;
-                const int rb = range_begin(r);
-                for (int t0 = rb; t0 < r.y; t0 += GTILE) {
-                    const int cnt = min(GTILE, r.y - t0);
-                    const int cnt2 = (cnt + 1) & ~1;
-                    __syncthreads();
-                    for (int j = tid; j < cnt2; j += FT) {
-                        const bool real = j < cnt;
-                        const int jj = t0 + (real ? j : 0);   // padding: a copy of the first source
+        for (int o = 0; o < OG; o++) {
+            const int orb = g0 + o;
+            nfi[o] = dup2((v && orb < a.norb) ? -a.ft32[(long)orb * a.nt + i] : 0.f);
+            sum[o] = 0.f;
+            cmp[o] = 0.f;
+        }
+        for (int e0 = r0; e0 < r1; e0 += GT) {
+            const int2 n = load_ranges(a, e0, r1, s_rng, [&](int2 &r, float dmin) {
+                if (range_is_close(r) != (PASS == 1)) return false;
+                r.x = range_begin(r);
+                return !(dmin * kmin > 127.f);   // beyond: every orbital's term is exactly 0
+            });
+            for (int c0 = 0; c0 < n.y; c0 += GW) {
+                __syncthreads();   // the previous tile is no longer read
+                const int c = c0 + wid;
+                int cnt2 = 0;
+                if (c < n.y) {
+                    const int e = range_of_chunk(s_rng, n.x, c);
+                    const int t0 = s_rng.begin[e] + (c - s_rng.first[e]) * SLOT;
+                    const int cnt = min(SLOT, s_rng.end[e] - t0);
+                    cnt2 = (cnt + 1) & ~1;
+                    const int j = 2 * lane, d = wid * SLOT + j;
+                    if (j < cnt2) {
+                        const bool real0 = j < cnt, real1 = j + 1 < cnt;
+                        const int j0 = t0 + (real0 ? j : 0), j1 = t0 + (real1 ? j + 1 : 0);   // padding: the first source
+                        const float4 h0 = a.shi[j0], h1 = a.shi[j1], l0 = a.slo[j0], l1 = a.slo[j1];
+                        const float2 hx = make_float2(h0.x, h1.x), hy = make_float2(h0.y, h1.y),
+                                     hz = make_float2(h0.z, h1.z), qx = make_float2(l0.x, l1.x),
+                                     qy = make_float2(l0.y, l1.y), qz = make_float2(l0.z, l1.z);
                         if constexpr (PASS == 1) {
-                            const float4 h = a.shi[jj], l = a.slo[jj];
-                            s_src[0][j] = -h.x;
-                            s_src[1][j] = -h.y;
-                            s_src[2][j] = -h.z;
-                            s_src[4][j] = -l.x;
-                            s_src[5][j] = -l.y;
-                            s_src[6][j] = -l.z;
+                            sts2(&s_src[0][d], neg2(hx));
+                            sts2(&s_src[1][d], neg2(hy));
+                            sts2(&s_src[2][d], neg2(hz));
+                            sts2(&s_src[4][d], neg2(qx));
+                            sts2(&s_src[5][d], neg2(qy));
+                            sts2(&s_src[6][d], neg2(qz));
                         } else {
-                            s_src[0][j] = -(float)(a.sx[jj] - cbx);
-                            s_src[1][j] = -(float)(a.sy[jj] - cby);
-                            s_src[2][j] = -(float)(a.sz[jj] - cbz);
+                            sts2(&s_src[0][d], neg_relative(hx, qx, ccx));
+                            sts2(&s_src[1][d], neg_relative(hy, qy, ccy));
+                            sts2(&s_src[2][d], neg_relative(hz, qz, ccz));
                         }
-                        s_src[3][j] = real ? a.w32[jj] : 0.f;
+                        sts2(&s_src[3][d], make_float2(real0 ? a.w32[j0] : 0.f, real1 ? a.w32[j1] : 0.f));
+#pragma unroll
+                        for (int o = 0; o < OG; o++) {
+                            const float *qo = a.q32 + (long)(g0 + o) * a.ns;
+                            const bool has = g0 + o < a.norb;
+                            sts2(reinterpret_cast<float *>(s_q4) + q4_pos(d, o, OG),
+                                 make_float2(has && real0 ? qo[j0] : 0.f, has && real1 ? qo[j1] : 0.f));
+                        }
                     }
-                    for (int k = tid; k < cnt2 * OG; k += FT) {   // orbital-major: coalesced global reads
-                        const int o = k / cnt2, j = k - o * cnt2;
-                        const int orb = g0 + o;
-                        reinterpret_cast<float *>(s_q4)[q4_pos(j, o, OG)] =
-                            (j < cnt && orb < a.norb) ? a.q32[(long)orb * a.ns + t0 + j] : 0.f;
-                    }
-                    __syncthreads();
-                    if (!warp_busy) continue;
-                    if (PASS == 1)
-                        group_tile<SS, true, true, OG>(s_src, s_q4, cnt2, tx, ty, tz, lx, ly, lz, nfi, kc, sum,
-                                                       cmp);
-                    else
-                        group_tile<SS, false, false, OG>(s_src, s_q4, cnt2, tx, ty, tz, lx, ly, lz, nfi, kc, sum,
-                                                         cmp);
+                }
+                if (lane == 0) s_cnt[wid] = cnt2;
+                __syncthreads();
+                if (!warp_busy) continue;
+                for (int sl = 0; sl < GW; sl++) {
+                    const int m = s_cnt[sl];
+                    if (m == 0) break;
+                    group_chunk<SS, PASS == 1, PASS == 1, OG>(s_src, s_q4, sl * SLOT, m, tx, ty, tz, lx, ly, lz, nfi,
+                                                              kc, sum, cmp);
                 }
             }
-            if (v) {
+        }
+        if (v) {
 #pragma unroll
-                for (int o = 0; o < OG; o++)
-                    if (g0 + o < a.norb) a.out[(long)(g0 + o) * a.nt + i] = (double)sum[o] - (double)cmp[o];
-            }
+            for (int o = 0; o < OG; o++)
+                if (g0 + o < a.norb) a.out[(long)(g0 + o) * a.nt + i] = (double)sum[o] - (double)cmp[o];
         }
     }
 }
@@ -684,9 +934,9 @@ __global__ void __launch_bounds__(FT, 2) near_group(const __grid_constant__ Work
 // far_cluster for the padded innermost axis).
 template <bool SS, int MAXN1, int OG, bool EXACT = false>
 __device__ __forceinline__ void far_group_cluster(const float4 *__restrict__ s_q4, const float *__restrict__ s_w,
-                                                  const float (*s_p)[MAXN1], int n1_in, float tx, float ty, float tz,
-                                                  const float2 (&nfi)[OG], const float2 (&kc)[OG],
-                                                  float (&sum)[OG], float (&cmp)[OG]) {
+                                                  const float (*s_p)[MAXN1], int n1_in,
+                                                  float tx, float ty, float tz, const float2 (&nfi)[OG],
+                                                  const float2 (&kc)[OG], float (&sum)[OG], float (&cmp)[OG]) {
     constexpr int MH = even_up<MAXN1>() / 2;
     const int n1 = EXACT ? MAXN1 : n1_in;
     const int n1p = n1 + (n1 & 1);
@@ -742,7 +992,7 @@ __host__ __device__ constexpr size_t far_group_smem(int n1, int og) {
 }
 
 template <bool SS, int MAXN1, int OG, bool EXACT = false>
-__global__ void __launch_bounds__(FT, 2) far_group(const __grid_constant__ Work w) {
+__global__ void __launch_bounds__(GT, 4) far_group(const __grid_constant__ Work w) {
     extern __shared__ __align__(16) float s_dyn[];
     __shared__ float s_p[3][MAXN1];
     __shared__ int s_item;
@@ -751,65 +1001,62 @@ __global__ void __launch_bounds__(FT, 2) far_group(const __grid_constant__ Work 
     for (;;) {
         const int item = next_item(w.queue, &s_item);
         if (item >= w.nitems) break;
-        const int2 it = w.items[item];
+        const int4 it = w.items[item];
         const Fields &a = w.sys[it.y >> 16];
         const int b = it.x, g0 = it.y & 0xffff;
         const int n1 = EXACT ? MAXN1 : a.n1, P = EXACT ? MAXN1 * MAXN1 * MAXN1 : a.P;
         const int n1p = n1 + (n1 & 1), Pp = n1 * n1 * n1p;
         const float *s_w = s_dyn + (size_t)Pp * OG;   // Pp * OG is a multiple of 4: float4 aligned
         const int f0 = a.far_off[b], f1 = a.far_off[b + 1];
-        if (f0 == f1) continue;
         const int bn = a.batch_node[b];
-        const int tb = a.tbegin[bn], te = a.tend[bn];
         const double cb[3] = {a.tcenter[3L * bn], a.tcenter[3L * bn + 1], a.tcenter[3L * bn + 2]};
         float2 kc[OG];
 #pragma unroll
         for (int o = 0; o < OG; o++) kc[o] = dup2((g0 + o) < a.norb ? -a.kc32[g0 + o] : 0.f);
-        for (int base = tb; base < te; base += FT) {
-            const int i = base + tid;
-            const bool v = i < te;
-            const bool warp_busy = base + (tid & ~31) < te;
-            const float tx = v ? (float)(a.tx[i] - cb[0]) : 0.f;
-            const float ty = v ? (float)(a.ty[i] - cb[1]) : 0.f;
-            const float tz = v ? (float)(a.tz[i] - cb[2]) : 0.f;
-            float2 nfi[OG];
-            float sum[OG], cmp[OG];
+        const int i = it.z + tid;
+        const bool v = i < it.w;
+        const bool warp_busy = it.z + (tid & ~31) < it.w;
+        const float tx = v ? (float)(a.tx[i] - cb[0]) : 0.f;
+        const float ty = v ? (float)(a.ty[i] - cb[1]) : 0.f;
+        const float tz = v ? (float)(a.tz[i] - cb[2]) : 0.f;
+        float2 nfi[OG];
+        float sum[OG], cmp[OG];
 #pragma unroll
-            for (int o = 0; o < OG; o++) {
+        for (int o = 0; o < OG; o++) {
+            const int orb = g0 + o;
+            nfi[o] = dup2((v && orb < a.norb) ? -a.ft32[(long)orb * a.nt + i] : 0.f);
+            sum[o] = 0.f;
+            cmp[o] = 0.f;
+        }
+        for (int e = f0; e < f1; e++) {
+            const int slot = a.node_slot[a.far_list[e]];
+            const double *gm = a.geom + 6L * slot;
+            __syncthreads();
+            for (int k = tid; k < Pp * OG; k += GT) {   // orbital-major: coalesced global reads
+                const int o = k / Pp, kk = k - o * Pp;
+                const int row = kk / n1p, k3 = kk - row * n1p;
                 const int orb = g0 + o;
-                nfi[o] = dup2((v && orb < a.norb) ? -a.ft32[(long)orb * a.nt + i] : 0.f);
-                sum[o] = 0.f;
-                cmp[o] = 0.f;
+                reinterpret_cast<float *>(s_q4)[q4_pos(kk, o, OG)] =
+                    (k3 < n1 && orb < a.norb) ? a.qhat32[((long)orb * a.nslots + slot) * P + row * n1 + k3] : 0.f;
             }
-            for (int e = f0; e < f1; e++) {
-                const int slot = a.node_slot[a.far_list[e]];
-                const double *gm = a.geom + 6L * slot;
-                __syncthreads();
-                for (int k = tid; k < Pp * OG; k += FT) {   // orbital-major: coalesced global reads
-                    const int o = k / Pp, kk = k - o * Pp;
-                    const int row = kk / n1p, k3 = kk - row * n1p;
-                    const int orb = g0 + o;
-                    reinterpret_cast<float *>(s_q4)[q4_pos(kk, o, OG)] =
-                        (k3 < n1 && orb < a.norb) ? a.qhat32[((long)orb * a.nslots + slot) * P + row * n1 + k3] : 0.f;
-                }
-                for (int k = tid; k < Pp; k += FT) {
-                    const int row = k / n1p, k3 = k - row * n1p;
-                    s_dyn[(size_t)Pp * OG + k] = k3 < n1 ? a.what32[(long)slot * P + row * n1 + k3] : 0.f;
-                }
-                if (tid < 3 * n1) {
-                    const int d = tid / n1, m = tid - d * n1;
-                    const double cbd = d == 0 ? cb[0] : (d == 1 ? cb[1] : cb[2]);
-                    s_p[d][m] = (float)((gm[d] + gm[3 + d] * a.tn[m]) - cbd);
-                }
-                __syncthreads();
-                if (!warp_busy) continue;
-                far_group_cluster<SS, MAXN1, OG, EXACT>(s_q4, s_w, s_p, n1, tx, ty, tz, nfi, kc, sum, cmp);
+            for (int k = tid; k < Pp; k += GT) {
+                const int row = k / n1p, k3 = k - row * n1p;
+                s_dyn[(size_t)Pp * OG + k] = k3 < n1 ? a.what32[(long)slot * P + row * n1 + k3] : 0.f;
             }
-            if (v) {
+            if (tid < 3 * n1) {
+                const int d = tid / n1, m = tid - d * n1;
+                const double cbd = d == 0 ? cb[0] : (d == 1 ? cb[1] : cb[2]);
+                s_p[d][m] = (float)((gm[d] + gm[3 + d] * a.tn[m]) - cbd);
+            }
+            __syncthreads();
+            if (!warp_busy) continue;
+            far_group_cluster<SS, MAXN1, OG, EXACT>(s_q4, s_w, s_p, n1, tx, ty, tz,
+                                                    nfi, kc, sum, cmp);
+        }
+        if (v) {
 #pragma unroll
-                for (int o = 0; o < OG; o++)
-                    if (g0 + o < a.norb) a.out[(long)(g0 + o) * a.nt + i] = (double)sum[o] - (double)cmp[o];
-            }
+            for (int o = 0; o < OG; o++)
+                if (g0 + o < a.norb) a.out[(long)(g0 + o) * a.nt + i] = (double)sum[o] - (double)cmp[o];
         }
     }
 }
@@ -838,7 +1085,7 @@ constexpr int DB_N1 = 8, DB_P = DB_N1 * DB_N1 * DB_N1;   // degree 7
 __host__ __device__ constexpr size_t far_group_db_smem(int og) { return sizeof(float) * 2 * (size_t)DB_P * (og + 1); }
 
 template <bool SS, int OG>
-__global__ void __launch_bounds__(FT, 2) far_group_db(const __grid_constant__ Work w) {
+__global__ void __launch_bounds__(GT, 4) far_group_db(const __grid_constant__ Work w) {
     constexpr int BUF = DB_P * OG + DB_P;   // floats per buffer: charges, then weight charges
     extern __shared__ __align__(16) float s_dyn[];
     __shared__ float s_p[2][3][DB_N1];
@@ -847,29 +1094,28 @@ __global__ void __launch_bounds__(FT, 2) far_group_db(const __grid_constant__ Wo
     for (;;) {
         const int item = next_item(w.queue, &s_item);
         if (item >= w.nitems) break;
-        const int2 it = w.items[item];
+        const int4 it = w.items[item];
         const Fields &a = w.sys[it.y >> 16];
         const int b = it.x, g0 = it.y & 0xffff;
         const int f0 = a.far_off[b], f1 = a.far_off[b + 1];
-        if (f0 == f1) continue;
         const int bn = a.batch_node[b];
-        const int tb = a.tbegin[bn], te = a.tend[bn];
         const double cb[3] = {a.tcenter[3L * bn], a.tcenter[3L * bn + 1], a.tcenter[3L * bn + 2]};
         float2 kc[OG];
 #pragma unroll
         for (int o = 0; o < OG; o++) kc[o] = dup2((g0 + o) < a.norb ? -a.kc32[g0 + o] : 0.f);
+        if (f0 == f1) continue;
         // issue the copies of far cluster e into buffer buf (completes at the next wait + barrier)
         auto stage = [&](int e, int buf) {
             const int slot = a.node_slot[a.far_list[e]];
             float *q = s_dyn + (size_t)buf * BUF;
-            for (int k = tid; k < DB_P * OG / 2; k += FT) {
+            for (int k = tid; k < DB_P * OG / 2; k += GT) {
                 const int o = k / (DB_P / 2), kk = 2 * (k - o * (DB_P / 2));
                 const int orb = g0 + o;
                 const bool valid = orb < a.norb;
                 const float *src = a.qhat32 + ((long)(valid ? orb : g0) * a.nslots + slot) * DB_P + kk;
                 cp_async8(q + q4_pos(kk, o, OG), src, valid);
             }
-            for (int k = tid; k < DB_P / 4; k += FT) cp_async16(q + DB_P * OG + 4 * k, a.what32 + (long)slot * DB_P + 4 * k);
+            for (int k = tid; k < DB_P / 4; k += GT) cp_async16(q + DB_P * OG + 4 * k, a.what32 + (long)slot * DB_P + 4 * k);
             cp_async_commit();
             if (tid < 3 * DB_N1) {
                 const double *gm = a.geom + 6L * slot;
@@ -878,39 +1124,37 @@ __global__ void __launch_bounds__(FT, 2) far_group_db(const __grid_constant__ Wo
                 s_p[buf][d][m] = (float)((gm[d] + gm[3 + d] * a.tn[m]) - cbd);
             }
         };
-        for (int base = tb; base < te; base += FT) {
-            const int i = base + tid;
-            const bool v = i < te;
-            const bool warp_busy = base + (tid & ~31) < te;
-            const float tx = v ? (float)(a.tx[i] - cb[0]) : 0.f;
-            const float ty = v ? (float)(a.ty[i] - cb[1]) : 0.f;
-            const float tz = v ? (float)(a.tz[i] - cb[2]) : 0.f;
-            float2 nfi[OG];
-            float sum[OG], cmp[OG];
+        const int i = it.z + tid;
+        const bool v = i < it.w;
+        const bool warp_busy = it.z + (tid & ~31) < it.w;
+        const float tx = v ? (float)(a.tx[i] - cb[0]) : 0.f;
+        const float ty = v ? (float)(a.ty[i] - cb[1]) : 0.f;
+        const float tz = v ? (float)(a.tz[i] - cb[2]) : 0.f;
+        float2 nfi[OG];
+        float sum[OG], cmp[OG];
 #pragma unroll
-            for (int o = 0; o < OG; o++) {
-                const int orb = g0 + o;
-                nfi[o] = dup2((v && orb < a.norb) ? -a.ft32[(long)orb * a.nt + i] : 0.f);
-                sum[o] = 0.f;
-                cmp[o] = 0.f;
-            }
-            __syncthreads();   // every thread is done with both buffers of the previous target chunk
-            stage(f0, 0);
-            for (int e = f0; e < f1; e++) {
-                const int cur = (e - f0) & 1;
-                cp_async_wait_all();   // this thread's copies of cluster e
-                __syncthreads();       // everyone's copies visible; everyone done reading the other buffer
-                if (e + 1 < f1) stage(e + 1, cur ^ 1);
-                if (!warp_busy) continue;
-                const float *q = s_dyn + (size_t)cur * BUF;
-                far_group_cluster<SS, DB_N1, OG, true>(reinterpret_cast<const float4 *>(q), q + DB_P * OG, s_p[cur],
-                                                       DB_N1, tx, ty, tz, nfi, kc, sum, cmp);
-            }
-            if (v) {
+        for (int o = 0; o < OG; o++) {
+            const int orb = g0 + o;
+            nfi[o] = dup2((v && orb < a.norb) ? -a.ft32[(long)orb * a.nt + i] : 0.f);
+            sum[o] = 0.f;
+            cmp[o] = 0.f;
+        }
+        __syncthreads();   // every thread is done with both buffers of the previous target chunk
+        stage(f0, 0);
+        for (int e = f0; e < f1; e++) {
+            const int cur = (e - f0) & 1;
+            cp_async_wait_all();   // this thread's copies of cluster e
+            __syncthreads();       // everyone's copies visible; everyone done reading the other buffer
+            if (e + 1 < f1) stage(e + 1, cur ^ 1);
+            if (!warp_busy) continue;
+            const float *q = s_dyn + (size_t)cur * BUF;
+            far_group_cluster<SS, DB_N1, OG, true>(reinterpret_cast<const float4 *>(q), q + DB_P * OG, s_p[cur],
+                                                   DB_N1, tx, ty, tz, nfi, kc, sum, cmp);
+        }
+        if (v) {
 #pragma unroll
-                for (int o = 0; o < OG; o++)
-                    if (g0 + o < a.norb) a.out[(long)(g0 + o) * a.nt + i] = (double)sum[o] - (double)cmp[o];
-            }
+            for (int o = 0; o < OG; o++)
+                if (g0 + o < a.norb) a.out[(long)(g0 + o) * a.nt + i] = (double)sum[o] - (double)cmp[o];
         }
     }
 }
@@ -934,20 +1178,22 @@ __global__ void __launch_bounds__(FT, 2) far_group_db(const __grid_constant__ Wo
 constexpr int QS16 = 20;
 constexpr int KCHUNK16 = 32;
 
-// One tile of cnt4 sources (a multiple of 4) for 16 orbitals.  Four sources
+// The slots of a tile for 16 orbitals (cnt: sources of each slot, a
+// multiple of 4; the slots with sources come first).  A full slot runs on into
+// the next one, so the pipeline drains only where a range ends.  Four sources
 // per iteration (two packed pairs), software pipelined: the next four
 // sources' geometry (loads, rsqrt, lg2) is issued before this iteration's
 // 64 orbital-pair updates, which hides its latency.  The per-orbital Kahan
-// sums live in shared memory (s_k[o][FT] sums, s_k[16 + o][FT]
+// sums live in shared memory (s_k[o][GT] sums, s_k[16 + o][GT]
 // compensations, touched once per KCHUNK16 sources), which leaves the
 // registers for the pipelined geometry.  NP: orbital pairs of the item that
 // hold orbitals (the last group of a request may be partly filled); the
 // pairs past NP are not computed.
 template <bool SS, bool MASK, bool PRECISE, int NP = 8>
 __device__ __forceinline__ void group16_tile(const float (*__restrict__ s)[GTILE], const float *__restrict__ s_q,
-                                             int cnt4, float2 tx, float2 ty, float2 tz, float2 lx, float2 ly,
-                                             float2 lz, const float2 (&nfi)[8], const float2 (&kc)[8],
-                                             float *__restrict__ s_k) {
+                                             const int *__restrict__ cnt, float2 tx, float2 ty,
+                                             float2 tz, float2 lx, float2 ly, float2 lz, const float2 (&nfi)[8],
+                                             const float2 (&kc)[8], float *__restrict__ s_k) {
     // r, -log2 r and w of the source pair at j (packed over the two sources)
     auto geometry = [&](int j, float2 &r, float2 &nl, float2 &wv) {
         float2 dx = add2(tx, lds2(s[0] + j)), dy = add2(ty, lds2(s[1] + j)), dz = add2(tz, lds2(s[2] + j));
@@ -973,54 +1219,63 @@ __device__ __forceinline__ void group16_tile(const float (*__restrict__ s)[GTILE
 #pragma unroll
     for (int p = 0; p < 8; p++) part[p] = make_float2(0.f, 0.f);
     float2 rc[2], nc[2], wc[2];
-    geometry(0, rc[0], nc[0], wc[0]);
-    geometry(2, rc[1], nc[1], wc[1]);
+    for (int sl = 0; sl < GW;) {
+        const int j0 = sl * SLOT;
+        int n = cnt[sl++], j1 = j0 + n;
+        if (n == 0) return;
+        while (n == SLOT && sl < GW) {
+            n = cnt[sl++];
+            j1 += n;
+        }
+        geometry(j0, rc[0], nc[0], wc[0]);
+        geometry(j0 + 2, rc[1], nc[1], wc[1]);
 #pragma unroll 1
-    for (int j = 0; j < cnt4; j += 4) {
-        const int jn = j + 4 < cnt4 ? j + 4 : j;
-        float2 rn[2], nn[2], wn[2];
-        geometry(jn, rn[0], nn[0], wn[0]);
-        geometry(jn + 2, rn[1], nn[1], wn[1]);
+        for (int j = j0; j < j1; j += 4) {
+            const int jn = j + 4 < j1 ? j + 4 : j;
+            float2 rn[2], nn[2], wn[2];
+            geometry(jn, rn[0], nn[0], wn[0]);
+            geometry(jn + 2, rn[1], nn[1], wn[1]);
 #pragma unroll
-        for (int u = 0; u < 4; u++) {
-            const float ru = (u & 1) ? rc[u >> 1].y : rc[u >> 1].x;
-            const float nu = (u & 1) ? nc[u >> 1].y : nc[u >> 1].x;
-            const float wu = (u & 1) ? wc[u >> 1].y : wc[u >> 1].x;
-            const float2 rd = dup2(ru), nd = dup2(nu), wd = dup2(wu);
-            const float *qj = s_q + (j + u) * QS16;
+            for (int u = 0; u < 4; u++) {
+                const float ru = (u & 1) ? rc[u >> 1].y : rc[u >> 1].x;
+                const float nu = (u & 1) ? nc[u >> 1].y : nc[u >> 1].x;
+                const float wu = (u & 1) ? wc[u >> 1].y : wc[u >> 1].x;
+                const float2 rd = dup2(ru), nd = dup2(nu), wd = dup2(wu);
+                const float *qj = s_q + (j + u) * QS16;
 #pragma unroll
-            for (int o4 = 0; o4 < (NP + 1) / 2; o4++) {
-                const float4 q4 = lds4(qj + 4 * o4);
+                for (int o4 = 0; o4 < (NP + 1) / 2; o4++) {
+                    const float4 q4 = lds4(qj + 4 * o4);
 #pragma unroll
-                for (int h = 0; h < 2; h++) {
-                    const int p = 2 * o4 + h;   // orbitals 2p, 2p+1
-                    if (p < NP) {
-                        const float2 q = h ? make_float2(q4.z, q4.w) : make_float2(q4.x, q4.y);
-                        const float2 g = ex2pos2(fma2(kc[p], rd, nd));
-                        part[p] = fma2(g, SS ? fma2(nfi[p], wd, q) : q, part[p]);
+                    for (int h = 0; h < 2; h++) {
+                        const int p = 2 * o4 + h;   // orbitals 2p, 2p+1
+                        if (p < NP) {
+                            const float2 q = h ? make_float2(q4.z, q4.w) : make_float2(q4.x, q4.y);
+                            const float2 g = ex2pos2(fma2(kc[p], rd, nd));
+                            part[p] = fma2(g, SS ? fma2(nfi[p], wd, q) : q, part[p]);
+                        }
                     }
                 }
             }
-        }
-        if ((j + 4) % KCHUNK16 == 0 || j + 4 >= cnt4) {   // end of a run of KCHUNK16 sources
+            if ((j + 4) % KCHUNK16 == 0 || j + 4 >= j1) {   // end of a run of KCHUNK16 sources
 #pragma unroll
-            for (int p = 0; p < NP; p++) {
+                for (int p = 0; p < NP; p++) {
 #pragma unroll
-                for (int h = 0; h < 2; h++) {
-                    const int o = 2 * p + h;
-                    float sm = s_k[o * FT + tid], cm = s_k[(16 + o) * FT + tid];
-                    kahan_add(sm, cm, h ? part[p].y : part[p].x);
-                    s_k[o * FT + tid] = sm;
-                    s_k[(16 + o) * FT + tid] = cm;
+                    for (int h = 0; h < 2; h++) {
+                        const int o = 2 * p + h;
+                        float sm = s_k[o * GT + tid], cm = s_k[(16 + o) * GT + tid];
+                        kahan_add(sm, cm, h ? part[p].y : part[p].x);
+                        s_k[o * GT + tid] = sm;
+                        s_k[(16 + o) * GT + tid] = cm;
+                    }
+                    part[p] = make_float2(0.f, 0.f);
                 }
-                part[p] = make_float2(0.f, 0.f);
             }
-        }
 #pragma unroll
-        for (int v = 0; v < 2; v++) {
-            rc[v] = rn[v];
-            nc[v] = nn[v];
-            wc[v] = wn[v];
+            for (int v = 0; v < 2; v++) {
+                rc[v] = rn[v];
+                nc[v] = nn[v];
+                wc[v] = wn[v];
+            }
         }
     }
 }
@@ -1028,10 +1283,10 @@ __device__ __forceinline__ void group16_tile(const float (*__restrict__ s)[GTILE
 // group16_tile for the item's np filled orbital pairs (1..8).
 template <bool SS, bool MASK, bool PRECISE>
 __device__ __forceinline__ void group16_tile_np(int np, const float (*__restrict__ s)[GTILE],
-                                                const float *__restrict__ s_q, int cnt4, float2 tx, float2 ty,
-                                                float2 tz, float2 lx, float2 ly, float2 lz, const float2 (&nfi)[8],
-                                                const float2 (&kc)[8], float *__restrict__ s_k) {
-#define TAGI_G16(N) group16_tile<SS, MASK, PRECISE, N>(s, s_q, cnt4, tx, ty, tz, lx, ly, lz, nfi, kc, s_k)
+                                                const float *__restrict__ s_q, const int *__restrict__ cnt, float2 tx, float2 ty, float2 tz, float2 lx, float2 ly,
+                                                float2 lz, const float2 (&nfi)[8], const float2 (&kc)[8],
+                                                float *__restrict__ s_k) {
+#define TAGI_G16(N) group16_tile<SS, MASK, PRECISE, N>(s, s_q, cnt, tx, ty, tz, lx, ly, lz, nfi, kc, s_k)
     switch (np) {
     case 1: TAGI_G16(1); break;
     case 2: TAGI_G16(2); break;
@@ -1064,112 +1319,121 @@ __device__ __forceinline__ void group16_constants(const Fields &a, int g0, float
 // Dynamic shared memory of near_group16: the source rows, the charges, then
 // the per-thread Kahan sums and compensations of 16 orbitals.
 __host__ __device__ constexpr size_t near_group16_smem(int pass) {
-    return sizeof(float) * ((size_t)GTILE * ((pass == 1 ? 7 : 4) + QS16) + 32 * FT);
+    return sizeof(float) * ((size_t)GTILE * ((pass == 1 ? 7 : 4) + QS16) + 32 * GT);
 }
 
 template <bool SS, int PASS>
-__global__ void __launch_bounds__(FT, 2) near_group16(const __grid_constant__ Work w) {
+__global__ void __launch_bounds__(GT, 4) near_group16(const __grid_constant__ Work w) {
     constexpr int NR = PASS == 1 ? 7 : 4;
     extern __shared__ __align__(16) float s_dyn[];
     float(*s_src)[GTILE] = reinterpret_cast<float(*)[GTILE]>(s_dyn);
     float *s_q = s_dyn + NR * GTILE;
     float *s_k = s_q + GTILE * QS16;
+    __shared__ RangeTable<GT> s_rng;
+    __shared__ int s_cnt[GW];
     __shared__ int s_item;
-    const int tid = threadIdx.x;
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     for (;;) {
         const int item = next_item(w.queue, &s_item);
         if (item >= w.nitems) break;
-        const int2 it = w.items[item];
+        const int4 it = w.items[item];
         const Fields &a = w.sys[it.y >> 16];
         const int b = it.x, g0 = it.y & 0xffff;
         const int bn = a.batch_node[b];
-        const int tb = a.tbegin[bn], te = a.tend[bn];
         const double cbx = a.tcenter[3L * bn], cby = a.tcenter[3L * bn + 1], cbz = a.tcenter[3L * bn + 2];
+        const Split ccx(cbx), ccy(cby), ccz(cbz);
         float2 kc[8];
         float kmin;
         group16_constants(a, g0, kc, &kmin);
         const int r0 = a.rng_off[b], r1 = a.rng_off[b + 1];
-        for (int base = tb; base < te; base += FT) {
-            const int i = base + tid;
-            const bool v = i < te;
-            const bool warp_busy = base + (tid & ~31) < te;
-            float2 tx, ty, tz, lx = dup2(0.f), ly = dup2(0.f), lz = dup2(0.f);
-            if (PASS == 1) {  // absolute hi/lo splits (see near_tile)
-                const float4 h = v ? a.thi[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-                const float4 l = v ? a.tlo[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-                tx = dup2(h.x);
-                ty = dup2(h.y);
-                tz = dup2(h.z);
-                lx = dup2(l.x);
-                ly = dup2(l.y);
-                lz = dup2(l.z);
-            } else {
-                tx = dup2(v ? (float)(a.tx[i] - cbx) : 0.f);
-                ty = dup2(v ? (float)(a.ty[i] - cby) : 0.f);
-                tz = dup2(v ? (float)(a.tz[i] - cbz) : 0.f);
-            }
-            float2 nfi[8];
+        const int i = it.z + tid;
+        const bool v = i < it.w;
+        const bool warp_busy = it.z + (tid & ~31) < it.w;
+        float2 tx, ty, tz, lx = dup2(0.f), ly = dup2(0.f), lz = dup2(0.f);
+        if (PASS == 1) {  // absolute hi/lo splits (see near_chunk)
+            const float4 h = v ? a.thi[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+            const float4 l = v ? a.tlo[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+            tx = dup2(h.x);
+            ty = dup2(h.y);
+            tz = dup2(h.z);
+            lx = dup2(l.x);
+            ly = dup2(l.y);
+            lz = dup2(l.z);
+        } else {
+            tx = dup2(v ? (float)(a.tx[i] - cbx) : 0.f);
+            ty = dup2(v ? (float)(a.ty[i] - cby) : 0.f);
+            tz = dup2(v ? (float)(a.tz[i] - cbz) : 0.f);
+        }
+        float2 nfi[8];
 #pragma unroll
-            for (int p = 0; p < 8; p++) {
-                const int o0 = g0 + 2 * p, o1 = o0 + 1;
-                nfi[p] = make_float2((v && o0 < a.norb) ? -a.ft32[(long)o0 * a.nt + i] : 0.f,
-                                     (v && o1 < a.norb) ? -a.ft32[(long)o1 * a.nt + i] : 0.f);
-            }
+        for (int p = 0; p < 8; p++) {
+            const int o0 = g0 + 2 * p, o1 = o0 + 1;
+            nfi[p] = make_float2((v && o0 < a.norb) ? -a.ft32[(long)o0 * a.nt + i] : 0.f,
+                                 (v && o1 < a.norb) ? -a.ft32[(long)o1 * a.nt + i] : 0.f);
+        }
 #pragma unroll
-            for (int o = 0; o < 32; o++) s_k[o * FT + tid] = 0.f;   // this thread's own sums
-            for (int e = r0; e < r1; e++) {
-                const int2 r = a.rng[e];
-                if (a.rng_dmin[e] * kmin > 127.f) continue;  // every orbital's term is exactly 0
-                const bool close = range_is_close(r);
-                if (close != (PASS == 1)) continue;
-                const int rb = range_begin(r);
-                for (int t0 = rb; t0 < r.y; t0 += GTILE) {
-                    const int cnt = min(GTILE, r.y - t0);
-                    const int cnt4 = (cnt + 3) & ~3;
-                    __syncthreads();
-                    for (int j = tid; j < cnt4; j += FT) {
-                        const bool real = j < cnt;
-                        const int jj = t0 + (real ? j : 0);   // padding: a copy of the first source
+        for (int o = 0; o < 32; o++) s_k[o * GT + tid] = 0.f;   // this thread's own sums
+        for (int e0 = r0; e0 < r1; e0 += GT) {
+            const int2 n = load_ranges(a, e0, r1, s_rng, [&](int2 &r, float dmin) {
+                if (range_is_close(r) != (PASS == 1)) return false;
+                r.x = range_begin(r);
+                return !(dmin * kmin > 127.f);   // beyond: every orbital's term is exactly 0
+            });
+            for (int c0 = 0; c0 < n.y; c0 += GW) {
+                __syncthreads();   // the previous tile is no longer read
+                const int c = c0 + wid;
+                int cnt4 = 0;
+                if (c < n.y) {
+                    const int e = range_of_chunk(s_rng, n.x, c);
+                    const int t0 = s_rng.begin[e] + (c - s_rng.first[e]) * SLOT;
+                    const int cnt = min(SLOT, s_rng.end[e] - t0);
+                    cnt4 = (cnt + 3) & ~3;
+                    const int j = 2 * lane, d = wid * SLOT + j;
+                    if (j < cnt4) {
+                        const bool real0 = j < cnt, real1 = j + 1 < cnt;
+                        const int j0 = t0 + (real0 ? j : 0), j1 = t0 + (real1 ? j + 1 : 0);   // padding: the first source
+                        const float4 h0 = a.shi[j0], h1 = a.shi[j1], l0 = a.slo[j0], l1 = a.slo[j1];
+                        const float2 hx = make_float2(h0.x, h1.x), hy = make_float2(h0.y, h1.y),
+                                     hz = make_float2(h0.z, h1.z), qx = make_float2(l0.x, l1.x),
+                                     qy = make_float2(l0.y, l1.y), qz = make_float2(l0.z, l1.z);
                         if constexpr (PASS == 1) {
-                            const float4 h = a.shi[jj], l = a.slo[jj];
-                            s_src[0][j] = -h.x;
-                            s_src[1][j] = -h.y;
-                            s_src[2][j] = -h.z;
-                            s_src[4][j] = -l.x;
-                            s_src[5][j] = -l.y;
-                            s_src[6][j] = -l.z;
+                            sts2(&s_src[0][d], neg2(hx));
+                            sts2(&s_src[1][d], neg2(hy));
+                            sts2(&s_src[2][d], neg2(hz));
+                            sts2(&s_src[4][d], neg2(qx));
+                            sts2(&s_src[5][d], neg2(qy));
+                            sts2(&s_src[6][d], neg2(qz));
                         } else {
-                            s_src[0][j] = -(float)(a.sx[jj] - cbx);
-                            s_src[1][j] = -(float)(a.sy[jj] - cby);
-                            s_src[2][j] = -(float)(a.sz[jj] - cbz);
+                            sts2(&s_src[0][d], neg_relative(hx, qx, ccx));
+                            sts2(&s_src[1][d], neg_relative(hy, qy, ccy));
+                            sts2(&s_src[2][d], neg_relative(hz, qz, ccz));
                         }
-                        s_src[3][j] = real ? a.w32[jj] : 0.f;
+                        sts2(&s_src[3][d], make_float2(real0 ? a.w32[j0] : 0.f, real1 ? a.w32[j1] : 0.f));
                     }
-                    // a warp stages 8 sources x 4 orbitals: 32-byte global segments,
-                    // conflict-free shared writes with the QS16 stride
-                    for (int k = tid; k < ((cnt4 + 7) & ~7) * 16; k += FT) {
-                        const int jb = k >> 7, rem = k & 127;
-                        const int o = rem >> 3, j = (jb << 3) + (rem & 7);
-                        if (j >= cnt4) continue;
-                        const int orb = g0 + o;
-                        s_q[j * QS16 + o] = (j < cnt && orb < a.norb) ? a.q32[(long)orb * a.ns + t0 + j] : 0.f;
-                    }
-                    __syncthreads();
-                    if (!warp_busy) continue;
-                    const int np = group16_pairs(a.norb, g0);
-                    if (PASS == 1)
-                        group16_tile_np<SS, true, true>(np, s_src, s_q, cnt4, tx, ty, tz, lx, ly, lz, nfi, kc, s_k);
-                    else
-                        group16_tile_np<SS, false, false>(np, s_src, s_q, cnt4, tx, ty, tz, lx, ly, lz, nfi, kc,
-                                                          s_k);
-                }
-            }
-            if (v) {
+                    // a warp stages 8 sources x 4 orbitals at a time: 32-byte global
+                    // segments, conflict-free shared writes with the QS16 stride
+                    const int o4 = lane >> 3, j8 = lane & 7;
+                    for (int j = j8; j < cnt4; j += 8) {
 #pragma unroll
-                for (int o = 0; o < 16; o++)
-                    if (g0 + o < a.norb)
-                        a.out[(long)(g0 + o) * a.nt + i] = (double)s_k[o * FT + tid] - (double)s_k[(16 + o) * FT + tid];
+                        for (int o = o4; o < 16; o += 4) {
+                            const int orb = g0 + o;
+                            s_q[(wid * SLOT + j) * QS16 + o] =
+                                (j < cnt && orb < a.norb) ? a.q32[(long)orb * a.ns + t0 + j] : 0.f;
+                        }
+                    }
+                }
+                if (lane == 0) s_cnt[wid] = cnt4;
+                __syncthreads();
+                if (!warp_busy) continue;
+                group16_tile_np<SS, PASS == 1, PASS == 1>(group16_pairs(a.norb, g0), s_src, s_q, s_cnt, tx, ty, tz, lx, ly,
+                                                          lz, nfi, kc, s_k);
             }
+        }
+        if (v) {
+#pragma unroll
+            for (int o = 0; o < 16; o++)
+                if (g0 + o < a.norb)
+                    a.out[(long)(g0 + o) * a.nt + i] = (double)s_k[o * GT + tid] - (double)s_k[(16 + o) * GT + tid];
         }
     }
 }
@@ -1179,9 +1443,9 @@ __global__ void __launch_bounds__(FT, 2) near_group16(const __grid_constant__ Wo
 // NP: filled orbital pairs, as in group16_tile.
 template <bool SS, int MAXN1, bool EXACT, int NP = 8>
 __device__ __forceinline__ void far_group16_cluster(const float *__restrict__ s_q, const float *__restrict__ s_w,
-                                                    const float (*s_p)[MAXN1], int n1_in, float tx, float ty,
-                                                    float tz, const float2 (&nfi)[8], const float2 (&kc)[8],
-                                                    float (&sum)[16], float (&cmp)[16]) {
+                                                    const float (*s_p)[MAXN1], int n1_in,
+                                                    float tx, float ty, float tz, const float2 (&nfi)[8],
+                                                    const float2 (&kc)[8], float (&sum)[16], float (&cmp)[16]) {
     constexpr int MH = even_up<MAXN1>() / 2;
     const int n1 = EXACT ? MAXN1 : n1_in;
     const int n1p = n1 + (n1 & 1);
@@ -1243,10 +1507,11 @@ __device__ __forceinline__ void far_group16_cluster(const float *__restrict__ s_
 template <bool SS, int MAXN1, bool EXACT>
 __device__ __forceinline__ void far_group16_cluster_np(int np, const float *__restrict__ s_q,
                                                        const float *__restrict__ s_w, const float (*s_p)[MAXN1],
-                                                       int n1, float tx, float ty, float tz, const float2 (&nfi)[8],
-                                                       const float2 (&kc)[8], float (&sum)[16],
-                                                       float (&cmp)[16]) {
-#define TAGI_F16(N) far_group16_cluster<SS, MAXN1, EXACT, N>(s_q, s_w, s_p, n1, tx, ty, tz, nfi, kc, sum, cmp)
+                                                       int n1, float tx, float ty,
+                                                       float tz, const float2 (&nfi)[8], const float2 (&kc)[8],
+                                                       float (&sum)[16], float (&cmp)[16]) {
+#define TAGI_F16(N) \
+    far_group16_cluster<SS, MAXN1, EXACT, N>(s_q, s_w, s_p, n1, tx, ty, tz, nfi, kc, sum, cmp)
     switch (np) {
     case 1: TAGI_F16(1); break;
     case 2: TAGI_F16(2); break;
@@ -1267,7 +1532,7 @@ __host__ __device__ constexpr size_t far_group16_smem(int n1) {
 }
 
 template <bool SS, int MAXN1, bool EXACT>
-__global__ void __launch_bounds__(FT, 2) far_group16(const __grid_constant__ Work w) {
+__global__ void __launch_bounds__(GT, 4) far_group16(const __grid_constant__ Work w) {
     extern __shared__ __align__(16) float s_dyn[];
     __shared__ float s_p[3][MAXN1];
     __shared__ int s_item;
@@ -1275,7 +1540,7 @@ __global__ void __launch_bounds__(FT, 2) far_group16(const __grid_constant__ Wor
     for (;;) {
         const int item = next_item(w.queue, &s_item);
         if (item >= w.nitems) break;
-        const int2 it = w.items[item];
+        const int4 it = w.items[item];
         const Fields &a = w.sys[it.y >> 16];
         const int b = it.x, g0 = it.y & 0xffff;
         const int n1 = EXACT ? MAXN1 : a.n1, P = EXACT ? MAXN1 * MAXN1 * MAXN1 : a.P;
@@ -1283,65 +1548,61 @@ __global__ void __launch_bounds__(FT, 2) far_group16(const __grid_constant__ Wor
         float *s_q = s_dyn;
         float *s_w = s_dyn + (size_t)Pp * QS16;
         const int f0 = a.far_off[b], f1 = a.far_off[b + 1];
-        if (f0 == f1) continue;
         const int bn = a.batch_node[b];
-        const int tb = a.tbegin[bn], te = a.tend[bn];
         const double cb[3] = {a.tcenter[3L * bn], a.tcenter[3L * bn + 1], a.tcenter[3L * bn + 2]};
         float2 kc[8];
         group16_constants(a, g0, kc, nullptr);
-        for (int base = tb; base < te; base += FT) {
-            const int i = base + tid;
-            const bool v = i < te;
-            const bool warp_busy = base + (tid & ~31) < te;
-            const float tx = v ? (float)(a.tx[i] - cb[0]) : 0.f;
-            const float ty = v ? (float)(a.ty[i] - cb[1]) : 0.f;
-            const float tz = v ? (float)(a.tz[i] - cb[2]) : 0.f;
-            float2 nfi[8];
-            float sum[16], cmp[16];
+        const int i = it.z + tid;
+        const bool v = i < it.w;
+        const bool warp_busy = it.z + (tid & ~31) < it.w;
+        const float tx = v ? (float)(a.tx[i] - cb[0]) : 0.f;
+        const float ty = v ? (float)(a.ty[i] - cb[1]) : 0.f;
+        const float tz = v ? (float)(a.tz[i] - cb[2]) : 0.f;
+        float2 nfi[8];
+        float sum[16], cmp[16];
 #pragma unroll
-            for (int p = 0; p < 8; p++) {
-                const int o0 = g0 + 2 * p, o1 = o0 + 1;
-                nfi[p] = make_float2((v && o0 < a.norb) ? -a.ft32[(long)o0 * a.nt + i] : 0.f,
-                                     (v && o1 < a.norb) ? -a.ft32[(long)o1 * a.nt + i] : 0.f);
-            }
+        for (int p = 0; p < 8; p++) {
+            const int o0 = g0 + 2 * p, o1 = o0 + 1;
+            nfi[p] = make_float2((v && o0 < a.norb) ? -a.ft32[(long)o0 * a.nt + i] : 0.f,
+                                 (v && o1 < a.norb) ? -a.ft32[(long)o1 * a.nt + i] : 0.f);
+        }
 #pragma unroll
-            for (int o = 0; o < 16; o++) {
-                sum[o] = 0.f;
-                cmp[o] = 0.f;
+        for (int o = 0; o < 16; o++) {
+            sum[o] = 0.f;
+            cmp[o] = 0.f;
+        }
+        for (int e = f0; e < f1; e++) {
+            const int slot = a.node_slot[a.far_list[e]];
+            const double *gm = a.geom + 6L * slot;
+            __syncthreads();
+            // a warp stages 8 proxy points x 4 orbitals (see near_group16)
+            for (int k = tid; k < ((Pp + 7) & ~7) * 16; k += GT) {
+                const int kb = k >> 7, rem = k & 127;
+                const int o = rem >> 3, kk = (kb << 3) + (rem & 7);
+                if (kk >= Pp) continue;
+                const int row = kk / n1p, k3 = kk - row * n1p;
+                const int orb = g0 + o;
+                s_q[kk * QS16 + o] =
+                    (k3 < n1 && orb < a.norb) ? a.qhat32[((long)orb * a.nslots + slot) * P + row * n1 + k3] : 0.f;
             }
-            for (int e = f0; e < f1; e++) {
-                const int slot = a.node_slot[a.far_list[e]];
-                const double *gm = a.geom + 6L * slot;
-                __syncthreads();
-                // a warp stages 8 proxy points x 4 orbitals (see near_group16)
-                for (int k = tid; k < ((Pp + 7) & ~7) * 16; k += FT) {
-                    const int kb = k >> 7, rem = k & 127;
-                    const int o = rem >> 3, kk = (kb << 3) + (rem & 7);
-                    if (kk >= Pp) continue;
-                    const int row = kk / n1p, k3 = kk - row * n1p;
-                    const int orb = g0 + o;
-                    s_q[kk * QS16 + o] =
-                        (k3 < n1 && orb < a.norb) ? a.qhat32[((long)orb * a.nslots + slot) * P + row * n1 + k3] : 0.f;
-                }
-                for (int k = tid; k < Pp; k += FT) {
-                    const int row = k / n1p, k3 = k - row * n1p;
-                    s_w[k] = k3 < n1 ? a.what32[(long)slot * P + row * n1 + k3] : 0.f;
-                }
-                if (tid < 3 * n1) {
-                    const int d = tid / n1, m = tid - d * n1;
-                    const double cbd = d == 0 ? cb[0] : (d == 1 ? cb[1] : cb[2]);
-                    s_p[d][m] = (float)((gm[d] + gm[3 + d] * a.tn[m]) - cbd);
-                }
-                __syncthreads();
-                if (!warp_busy) continue;
-                far_group16_cluster_np<SS, MAXN1, EXACT>(group16_pairs(a.norb, g0), s_q, s_w, s_p, n1, tx, ty, tz,
-                                                         nfi, kc, sum, cmp);
+            for (int k = tid; k < Pp; k += GT) {
+                const int row = k / n1p, k3 = k - row * n1p;
+                s_w[k] = k3 < n1 ? a.what32[(long)slot * P + row * n1 + k3] : 0.f;
             }
-            if (v) {
+            if (tid < 3 * n1) {
+                const int d = tid / n1, m = tid - d * n1;
+                const double cbd = d == 0 ? cb[0] : (d == 1 ? cb[1] : cb[2]);
+                s_p[d][m] = (float)((gm[d] + gm[3 + d] * a.tn[m]) - cbd);
+            }
+            __syncthreads();
+            if (!warp_busy) continue;
+            far_group16_cluster_np<SS, MAXN1, EXACT>(group16_pairs(a.norb, g0), s_q, s_w, s_p, n1,
+                                                     tx, ty, tz,                                                      nfi, kc, sum, cmp);
+        }
+        if (v) {
 #pragma unroll
-                for (int o = 0; o < 16; o++)
-                    if (g0 + o < a.norb) a.out[(long)(g0 + o) * a.nt + i] = (double)sum[o] - (double)cmp[o];
-            }
+            for (int o = 0; o < 16; o++)
+                if (g0 + o < a.norb) a.out[(long)(g0 + o) * a.nt + i] = (double)sum[o] - (double)cmp[o];
         }
     }
 }
@@ -1373,42 +1634,40 @@ __global__ void __launch_bounds__(FT) near_f64(const __grid_constant__ Work w) {
     for (;;) {
         const int item = next_item(w.queue, &s_item);
         if (item >= w.nitems) break;
-        const int2 it = w.items[item];
+        const int4 it = w.items[item];
         const Fields &a = w.sys[it.y >> 16];
+        const Place pl(a.split);
         const int b = it.x, orb = it.y & 0xffff;
-        const int bn = a.batch_node[b];
-        const int tb = a.tbegin[bn], te = a.tend[bn];
         const double kp = a.kp64[orb];
         const double *f = a.f64 + (long)orb * a.ns;
         const double *ft = a.ft64 + (long)orb * a.nt;
         const int r0 = a.rng_off[b], r1 = a.rng_off[b + 1];
-        for (int base = tb; base < te; base += FT) {
-            const int i = base + tid;
-            const bool v = i < te;
-            const double xi = v ? a.tx[i] : 0.0, yi = v ? a.ty[i] : 0.0, zi = v ? a.tz[i] : 0.0;
-            const double fi = v ? ft[i] : 0.0;
-            double acc = 0.0;
-            for (int e = r0; e < r1; e++) {
-                const int2 r = a.rng[e];
-                for (int t0 = range_begin(r); t0 < r.y; t0 += T64) {
-                    const int cnt = min(T64, r.y - t0);
-                    __syncthreads();
-                    if (tid < cnt) {
-                        int jj = t0 + tid;
-                        s_x[tid] = a.sx[jj];
-                        s_y[tid] = a.sy[jj];
-                        s_z[tid] = a.sz[jj];
-                        s_f[tid] = f[jj];
-                        s_w[tid] = a.w64[jj];
-                    }
-                    __syncthreads();
-                    for (int j = 0; j < cnt; j++)
-                        acc += pair_f64<KERN, SS>(xi - s_x[j], yi - s_y[j], zi - s_z[j], s_f[j],
-                                                  s_w[j], fi, kp);
+        const int i = it.z + 32 * pl.g + pl.lane;
+        const bool v = i < it.w;
+        const double xi = v ? a.tx[i] : 0.0, yi = v ? a.ty[i] : 0.0, zi = v ? a.tz[i] : 0.0;
+        const double fi = v ? ft[i] : 0.0;
+        double acc = 0.0;
+        for (int e = r0; e < r1; e++) {
+            const int2 r = a.rng[e];
+            for (int t0 = range_begin(r); t0 < r.y; t0 += T64) {
+                const int cnt = min(T64, r.y - t0);
+                __syncthreads();
+                if (tid < cnt) {
+                    int jj = t0 + tid;
+                    s_x[tid] = a.sx[jj];
+                    s_y[tid] = a.sy[jj];
+                    s_z[tid] = a.sz[jj];
+                    s_f[tid] = f[jj];
+                    s_w[tid] = a.w64[jj];
                 }
+                __syncthreads();
+                for (int j = pl.sp; j < cnt; j += pl.S)
+                    acc += pair_f64<KERN, SS>(xi - s_x[j], yi - s_y[j], zi - s_z[j], s_f[j],
+                                              s_w[j], fi, kp);
             }
-            if (v) a.out[(long)orb * a.nt + i] = acc;
         }
+        acc = add_splits(acc, pl, s_x);
+        if (v && pl.sp == 0) a.out[(long)orb * a.nt + i] = acc;
     }
 }
 
@@ -1416,66 +1675,63 @@ template <int KERN, bool SS, int MAXN1>
 __global__ void __launch_bounds__(FT) far_f64(const __grid_constant__ Work w) {
     constexpr int MAXP = MAXN1 * MAXN1 * MAXN1;
     __shared__ double s_q[MAXP], s_wh[MAXP];
-    __shared__ double s_p[3][MAXN1];
+    __shared__ double s_p[3][MAXN1], s_red[FT];
     __shared__ int s_item;
     const int tid = threadIdx.x;
     for (;;) {
         const int item = next_item(w.queue, &s_item);
         if (item >= w.nitems) break;
-        const int2 it = w.items[item];
+        const int4 it = w.items[item];
         const Fields &a = w.sys[it.y >> 16];
+        const Place pl(a.split);
         const int b = it.x, orb = it.y & 0xffff;
         const int n1 = a.n1, P = a.P;
         const int f0 = a.far_off[b], f1 = a.far_off[b + 1];
-        if (f0 == f1) continue;
-        const int bn = a.batch_node[b];
-        const int tb = a.tbegin[bn], te = a.tend[bn];
         const double kp = a.kp64[orb];
         const double *ft = a.ft64 + (long)orb * a.nt;
         const double *qh = a.qhat64 + (long)orb * a.nslots * P;
-        for (int base = tb; base < te; base += FT) {
-            const int i = base + tid;
-            const bool v = i < te;
-            const double xi = v ? a.tx[i] : 0.0, yi = v ? a.ty[i] : 0.0, zi = v ? a.tz[i] : 0.0;
-            const double fi = v ? ft[i] : 0.0;
-            double acc = 0.0;
-            for (int e = f0; e < f1; e++) {
-                const int slot = a.node_slot[a.far_list[e]];
-                __syncthreads();
-                for (int k = tid; k < P; k += FT) {
-                    s_q[k] = qh[(long)slot * P + k];
-                    s_wh[k] = a.what64[(long)slot * P + k];
-                }
-                if (tid < 3 * n1) {
-                    int d = tid / n1, m = tid - d * n1;
-                    const double *g = a.geom + 6L * slot;
-                    s_p[d][m] = g[d] + g[3 + d] * a.tn[m];
-                }
-                __syncthreads();
-                int idx = 0;
-                for (int k1 = 0; k1 < n1; k1++) {
-                    const double dx = xi - s_p[0][k1];
-                    for (int k2 = 0; k2 < n1; k2++) {
-                        const double dy = yi - s_p[1][k2];
-                        for (int k3 = 0; k3 < n1; k3++) {
-                            const double dz = zi - s_p[2][k3];
-                            const double r2 = dx * dx + dy * dy + dz * dz;
-                            const double r = sqrt(r2);
-                            const double qk = s_q[idx + k3], wk = s_wh[idx + k3];
-                            if (KERN == KERNEL_YUKAWA) {
-                                acc += exp(-kp * r) / r * (SS ? (qk - fi * wk) : qk);
-                            } else if (SS) {
-                                acc += (qk - fi * wk * exp(-kp * kp * r2)) / r;
-                            } else {
-                                acc += qk / r;
-                            }
+        const int i = it.z + 32 * pl.g + pl.lane;
+        const bool v = i < it.w;
+        const double xi = v ? a.tx[i] : 0.0, yi = v ? a.ty[i] : 0.0, zi = v ? a.tz[i] : 0.0;
+        const double fi = v ? ft[i] : 0.0;
+        double acc = 0.0;
+        for (int e = f0; e < f1; e++) {
+            const int slot = a.node_slot[a.far_list[e]];
+            __syncthreads();
+            for (int k = tid; k < P; k += FT) {
+                s_q[k] = qh[(long)slot * P + k];
+                s_wh[k] = a.what64[(long)slot * P + k];
+            }
+            if (tid < 3 * n1) {
+                int d = tid / n1, m = tid - d * n1;
+                const double *g = a.geom + 6L * slot;
+                s_p[d][m] = g[d] + g[3 + d] * a.tn[m];
+            }
+            __syncthreads();
+            for (int k1 = first_slab(e - f0, n1, pl); k1 < n1; k1 += pl.S) {
+                int idx = k1 * n1 * n1;
+                const double dx = xi - s_p[0][k1];
+                for (int k2 = 0; k2 < n1; k2++) {
+                    const double dy = yi - s_p[1][k2];
+                    for (int k3 = 0; k3 < n1; k3++) {
+                        const double dz = zi - s_p[2][k3];
+                        const double r2 = dx * dx + dy * dy + dz * dz;
+                        const double r = sqrt(r2);
+                        const double qk = s_q[idx + k3], wk = s_wh[idx + k3];
+                        if (KERN == KERNEL_YUKAWA) {
+                            acc += exp(-kp * r) / r * (SS ? (qk - fi * wk) : qk);
+                        } else if (SS) {
+                            acc += (qk - fi * wk * exp(-kp * kp * r2)) / r;
+                        } else {
+                            acc += qk / r;
                         }
-                        idx += n1;
                     }
+                    idx += n1;
                 }
             }
-            if (v) a.out[(long)orb * a.nt + i] = acc;
         }
+        acc = add_splits(acc, pl, s_red);
+        if (v && pl.sp == 0) a.out[(long)orb * a.nt + i] = acc;
     }
 }
 
@@ -1524,11 +1780,11 @@ __global__ void epilogue(const double *__restrict__ nearv, const double *__restr
 }
 
 template <typename K>
-int occupancy_grid(K kern, int *grid, size_t smem = 0) {
+int occupancy_grid(K kern, int *grid, size_t smem = 0, int threads = FT) {
     int dev = 0, sms = 0, per = 0;
     TAGI_CUDA(cudaGetDevice(&dev));
     TAGI_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    TAGI_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, FT, smem));
+    TAGI_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, threads, smem));
     *grid = sms * (per > 0 ? per : 1);
     return TAGI_OK;
 }
@@ -1537,15 +1793,15 @@ int occupancy_grid(K kern, int *grid, size_t smem = 0) {
 // bytes of dynamic shared memory; for large requests the kernel's limit is
 // raised first.
 template <typename K>
-int launch_persistent(K kern, const Work &w, cudaStream_t s, size_t smem = 0) {
+int launch_persistent(K kern, const Work &w, cudaStream_t s, size_t smem = 0, int threads = FT) {
     if (w.nitems == 0) return TAGI_OK;
     if (smem > 32 * 1024)   // dynamic + static above the 48 KB default needs the opt-in
         TAGI_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int grid = 0;
-    TAGI_TRY(occupancy_grid(kern, &grid, smem));
+    TAGI_TRY(occupancy_grid(kern, &grid, smem, threads));
     if (grid > w.nitems) grid = w.nitems;
     if (grid < 1) grid = 1;
-    launch(kern, grid, FT, smem, s, w);
+    launch(kern, grid, threads, smem, s, w);
     TAGI_LAUNCH_CHECK();
     return TAGI_OK;
 }
@@ -1579,7 +1835,11 @@ __global__ void __launch_bounds__(FT) pair_peak_near(int reps, float *out) {
         nfi[k] = dup2(-0.3f);
     }
     for (int r = 0; r < reps; r++)
-        near_tile<KERN, SS, false, false, 2>(s, NTILE, tx, ty, tz, z2, z2, z2, dup2(1.f), nfi, sum, cmp);
+        for (int j0 = 0; j0 < NTILE; j0 += SLOT) {
+            float part[2];
+            near_chunk<KERN, SS, false, false, 2>(s, j0, SLOT, tx, ty, tz, z2, z2, z2, dup2(1.f), nfi, part);
+            for (int k = 0; k < 2; k++) kahan_add(sum[k], cmp[k], part[k]);
+        }
     out[blockIdx.x * FT + threadIdx.x] = sum[0] + sum[1] - cmp[0] - cmp[1];
 }
 
@@ -1604,24 +1864,25 @@ __global__ void __launch_bounds__(FT) pair_peak_far(int reps, float *out) {
         nfi[k] = dup2(-0.3f);
     }
     for (int r = 0; r < reps; r++)
-        far_cluster<KERN, SS, true, N1, 2, true>(s_q, s_w, s_p, N1, tx, ty, tz, nfi, sum, cmp);
+        far_cluster<KERN, SS, true, N1, 2, true>(s_q, s_w, s_p, N1, 0, 1, tx, ty, tz, nfi,
+                                                 [&](int, int k, float part) { kahan_add(sum[k], cmp[k], part); });
     out[blockIdx.x * FT + threadIdx.x] = sum[0] + sum[1] - cmp[0] - cmp[1];
 }
 
 // Yukawa orbital groups, 8 orbitals per pair geometry; counted per (pair, orbital).
 template <bool SS>
-__global__ void __launch_bounds__(FT, 2) pair_peak_near_group(int reps, float *out) {
+__global__ void __launch_bounds__(GT, 4) pair_peak_near_group(int reps, float *out) {
     constexpr int OG = 8;
     __shared__ __align__(16) float s[4][GTILE];
     __shared__ float4 s_q4[GTILE * OG / 4];
-    for (int j = threadIdx.x; j < GTILE; j += FT) {
+    for (int j = threadIdx.x; j < GTILE; j += GT) {
         const float v = (float)((j * 37) % 101) * 0.01f - 0.5f;
         s[0][j] = -v;
         s[1][j] = -(0.3f * v + 0.1f);
         s[2][j] = -(0.7f - v);
         s[3][j] = 0.25f;
     }
-    for (int k = threadIdx.x; k < GTILE * OG; k += FT) reinterpret_cast<float *>(s_q4)[k] = 0.5f + 0.001f * k;
+    for (int k = threadIdx.x; k < GTILE * OG; k += GT) reinterpret_cast<float *>(s_q4)[k] = 0.5f + 0.001f * k;
     __syncthreads();
     const float2 tx = dup2(0.01f * (threadIdx.x & 31)), ty = dup2(0.02f), tz = dup2(-0.03f * (threadIdx.x >> 5));
     float2 nfi[OG], kc[OG];
@@ -1634,22 +1895,23 @@ __global__ void __launch_bounds__(FT, 2) pair_peak_near_group(int reps, float *o
     }
     const float2 z = dup2(0.f);
     for (int r = 0; r < reps; r++)
-        group_tile<SS, false, false, OG>(s, s_q4, GTILE, tx, ty, tz, z, z, z, nfi, kc, sum, cmp);
+        for (int j0 = 0; j0 < GTILE; j0 += SLOT)
+            group_chunk<SS, false, false, OG>(s, s_q4, j0, SLOT, tx, ty, tz, z, z, z, nfi, kc, sum, cmp);
     float acc = 0.f;
 #pragma unroll
     for (int o = 0; o < OG; o++) acc += sum[o] - cmp[o];
-    out[blockIdx.x * FT + threadIdx.x] = acc;
+    out[blockIdx.x * GT + threadIdx.x] = acc;
 }
 
 // Yukawa orbital groups in the far field: one degree-7 proxy grid, 8 orbitals.
 template <bool SS>
-__global__ void __launch_bounds__(FT, 2) pair_peak_far_group(int reps, float *out) {
+__global__ void __launch_bounds__(GT, 4) pair_peak_far_group(int reps, float *out) {
     constexpr int OG = 8, N1 = 8, PP = N1 * N1 * N1;
     __shared__ float4 s_q4[PP * OG / 4];
     __shared__ __align__(16) float s_w[PP];
     __shared__ float s_p[3][N1];
-    for (int k = threadIdx.x; k < PP * OG; k += FT) reinterpret_cast<float *>(s_q4)[k] = 0.5f + 0.001f * k;
-    for (int k = threadIdx.x; k < PP; k += FT) s_w[k] = 0.25f;
+    for (int k = threadIdx.x; k < PP * OG; k += GT) reinterpret_cast<float *>(s_q4)[k] = 0.5f + 0.001f * k;
+    for (int k = threadIdx.x; k < PP; k += GT) s_w[k] = 0.25f;
     if (threadIdx.x < 3 * N1) s_p[threadIdx.x / N1][threadIdx.x % N1] = 1.0f + 0.1f * threadIdx.x;
     __syncthreads();
     const float tx = 0.01f * (threadIdx.x & 31), ty = 0.02f, tz = -0.03f * (threadIdx.x >> 5);
@@ -1666,26 +1928,28 @@ __global__ void __launch_bounds__(FT, 2) pair_peak_far_group(int reps, float *ou
     float acc = 0.f;
 #pragma unroll
     for (int o = 0; o < OG; o++) acc += sum[o] - cmp[o];
-    out[blockIdx.x * FT + threadIdx.x] = acc;
+    out[blockIdx.x * GT + threadIdx.x] = acc;
 }
 
 // The same two loops with 16 orbitals packed by orbital (near: shared memory
 // laid out as near_group16's, dynamic).
 constexpr int PEAK16_TILE = GTILE;
 template <bool SS>
-__global__ void __launch_bounds__(FT, 2) pair_peak_near_group16(int reps, float *out) {
+__global__ void __launch_bounds__(GT, 4) pair_peak_near_group16(int reps, float *out) {
     extern __shared__ __align__(16) float s_dyn[];
     float(*s)[GTILE] = reinterpret_cast<float(*)[GTILE]>(s_dyn);
     float *s_q = s_dyn + 4 * GTILE;
     float *s_k = s_q + GTILE * QS16;
-    for (int j = threadIdx.x; j < PEAK16_TILE; j += FT) {
+    for (int j = threadIdx.x; j < PEAK16_TILE; j += GT) {
         const float v = (float)((j * 37) % 101) * 0.01f - 0.5f;
         s[0][j] = -v;
         s[1][j] = -(0.3f * v + 0.1f);
         s[2][j] = -(0.7f - v);
         s[3][j] = 0.25f;
     }
-    for (int k = threadIdx.x; k < PEAK16_TILE * QS16; k += FT) s_q[k] = 0.5f + 0.001f * k;
+    __shared__ int s_cnt[GW];
+    if (threadIdx.x < GW) s_cnt[threadIdx.x] = SLOT;
+    for (int k = threadIdx.x; k < PEAK16_TILE * QS16; k += GT) s_q[k] = 0.5f + 0.001f * k;
     __syncthreads();
     const float2 tx = dup2(0.01f * (threadIdx.x & 31)), ty = dup2(0.02f), tz = dup2(-0.03f * (threadIdx.x >> 5));
     float2 nfi[8], kc[8];
@@ -1694,23 +1958,23 @@ __global__ void __launch_bounds__(FT, 2) pair_peak_near_group16(int reps, float 
         kc[p] = make_float2((float)(-(0.5 + 0.3 * (2 * p)) * LOG2E), (float)(-(0.5 + 0.3 * (2 * p + 1)) * LOG2E));
         nfi[p] = dup2(-0.3f);
     }
-    for (int o = 0; o < 32; o++) s_k[o * FT + threadIdx.x] = 0.f;
+    for (int o = 0; o < 32; o++) s_k[o * GT + threadIdx.x] = 0.f;
     const float2 z = dup2(0.f);
     for (int r = 0; r < reps; r++)
-        group16_tile<SS, false, false>(s, s_q, PEAK16_TILE, tx, ty, tz, z, z, z, nfi, kc, s_k);
+        group16_tile<SS, false, false>(s, s_q, s_cnt, tx, ty, tz, z, z, z, nfi, kc, s_k);
     float acc = 0.f;
-    for (int o = 0; o < 16; o++) acc += s_k[o * FT + threadIdx.x] - s_k[(16 + o) * FT + threadIdx.x];
-    out[blockIdx.x * FT + threadIdx.x] = acc;
+    for (int o = 0; o < 16; o++) acc += s_k[o * GT + threadIdx.x] - s_k[(16 + o) * GT + threadIdx.x];
+    out[blockIdx.x * GT + threadIdx.x] = acc;
 }
 
 template <bool SS>
-__global__ void __launch_bounds__(FT, 2) pair_peak_far_group16(int reps, float *out) {
+__global__ void __launch_bounds__(GT, 4) pair_peak_far_group16(int reps, float *out) {
     constexpr int N1 = 8, PP = N1 * N1 * N1;
     __shared__ __align__(16) float s_q[PP * QS16];
     __shared__ __align__(16) float s_w[PP];
     __shared__ float s_p[3][N1];
-    for (int k = threadIdx.x; k < PP * QS16; k += FT) s_q[k] = 0.5f + 0.001f * k;
-    for (int k = threadIdx.x; k < PP; k += FT) s_w[k] = 0.25f;
+    for (int k = threadIdx.x; k < PP * QS16; k += GT) s_q[k] = 0.5f + 0.001f * k;
+    for (int k = threadIdx.x; k < PP; k += GT) s_w[k] = 0.25f;
     if (threadIdx.x < 3 * N1) s_p[threadIdx.x / N1][threadIdx.x % N1] = 1.0f + 0.1f * threadIdx.x;
     __syncthreads();
     const float tx = 0.01f * (threadIdx.x & 31), ty = 0.02f, tz = -0.03f * (threadIdx.x >> 5);
@@ -1728,17 +1992,17 @@ __global__ void __launch_bounds__(FT, 2) pair_peak_far_group16(int reps, float *
     float acc = 0.f;
 #pragma unroll
     for (int o = 0; o < 16; o++) acc += sum[o] - cmp[o];
-    out[blockIdx.x * FT + threadIdx.x] = acc;
+    out[blockIdx.x * GT + threadIdx.x] = acc;
 }
 
 template <int KERN, bool SS>
 int launch_pair_peak(int variant, int grid, int reps, float *out, cudaStream_t s) {
     if (variant == 0) launch(pair_peak_near<KERN, SS>, grid, FT, 0, s, reps, out);
     else if (variant == 1) launch(pair_peak_far<KERN, SS>, grid, FT, 0, s, reps, out);
-    else if (variant == 2) launch(pair_peak_near_group<SS>, grid, FT, 0, s, reps, out);
-    else if (variant == 3) launch(pair_peak_far_group<SS>, grid, FT, 0, s, reps, out);
-    else if (variant == 4) launch(pair_peak_near_group16<SS>, grid, FT, near_group16_smem(0), s, reps, out);
-    else launch(pair_peak_far_group16<SS>, grid, FT, 0, s, reps, out);
+    else if (variant == 2) launch(pair_peak_near_group<SS>, grid, GT, 0, s, reps, out);
+    else if (variant == 3) launch(pair_peak_far_group<SS>, grid, GT, 0, s, reps, out);
+    else if (variant == 4) launch(pair_peak_near_group16<SS>, grid, GT, near_group16_smem(0), s, reps, out);
+    else launch(pair_peak_far_group16<SS>, grid, GT, 0, s, reps, out);
     TAGI_LAUNCH_CHECK();
     return TAGI_OK;
 }
@@ -1754,14 +2018,14 @@ int run_pair_peak(int variant, double *pairs_per_s, cudaStream_t s) {
     int grid = 0;
     if (variant == 0) TAGI_TRY(occupancy_grid(pair_peak_near<KERN, SS>, &grid));
     else if (variant == 1) TAGI_TRY(occupancy_grid(pair_peak_far<KERN, SS>, &grid));
-    else if (variant == 2) TAGI_TRY(occupancy_grid(pair_peak_near_group<SS>, &grid));
-    else if (variant == 3) TAGI_TRY(occupancy_grid(pair_peak_far_group<SS>, &grid));
+    else if (variant == 2) TAGI_TRY(occupancy_grid(pair_peak_near_group<SS>, &grid, 0, GT));
+    else if (variant == 3) TAGI_TRY(occupancy_grid(pair_peak_far_group<SS>, &grid, 0, GT));
     else if (variant == 4) {
         TAGI_CUDA(cudaFuncSetAttribute(pair_peak_near_group16<SS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)near_group16_smem(0)));
-        TAGI_TRY(occupancy_grid(pair_peak_near_group16<SS>, &grid, near_group16_smem(0)));
+        TAGI_TRY(occupancy_grid(pair_peak_near_group16<SS>, &grid, near_group16_smem(0), GT));
     }
-    else TAGI_TRY(occupancy_grid(pair_peak_far_group16<SS>, &grid));
+    else TAGI_TRY(occupancy_grid(pair_peak_far_group16<SS>, &grid, 0, GT));
     Arena tmp;
     tmp.stream = s;
     float *out = nullptr;
@@ -1789,14 +2053,14 @@ int run_pair_peak(int variant, double *pairs_per_s, cudaStream_t s) {
     cudaEventDestroy(b);
     tmp.release();
     if (rc) return rc;
-    *pairs_per_s = (double)grid * FT * per_rep * reps / (ms * 1e-3);
+    *pairs_per_s = (double)grid * (variant < 2 ? FT : GT) * per_rep * reps / (ms * 1e-3);
     return TAGI_OK;
 }
 
 // Kernel shape shared by every system of one field launch.
 struct LaunchShape {
     int og = 1;     // orbitals per item (orbital-group kernels) or 1
-    int nt = 1;     // targets per thread: 2 when some batch holds more than FT targets
+    int nt = 1;     // targets per thread (single-orbital mixed kernels)
     int maxn1 = 1;        // largest proxy-grid edge n + 1
     int minn1 = 1 << 20;  // smallest proxy-grid edge n + 1
 };
@@ -1824,47 +2088,47 @@ int launch_fields(const SysCall *calls, const Fields *f, int nsys, const Schedul
     const bool one = sh.nt == 1;
     phase_mark(PH_NEAR, true, s);
     if (precision == PREC_MIXED && KERN == KERNEL_YUKAWA && sh.og == 16) {
-        TAGI_TRY(launch_persistent(near_group16<SS, 0>, wn, s, near_group16_smem(0)));
+        TAGI_TRY(launch_persistent(near_group16<SS, 0>, wn, s, near_group16_smem(0), GT));
         phase_mark(PH_NEAR, false, s);
         phase_mark(PH_NEAR_CLOSE, true, s);
-        TAGI_TRY(launch_persistent(near_group16<SS, 1>, wc, s, near_group16_smem(1)));
+        TAGI_TRY(launch_persistent(near_group16<SS, 1>, wc, s, near_group16_smem(1), GT));
         phase_mark(PH_NEAR_CLOSE, false, s);
         phase_mark(PH_FAR, true, s);
         if (sh.maxn1 <= 4)
-            TAGI_TRY(launch_persistent(far_group16<SS, 4, false>, wf, s, far_group16_smem(sh.maxn1)));
+            TAGI_TRY(launch_persistent(far_group16<SS, 4, false>, wf, s, far_group16_smem(sh.maxn1), GT));
         else if (sh.maxn1 == 8 && sh.minn1 == 8)   // degree 7 everywhere: fixed loops
-            TAGI_TRY(launch_persistent(far_group16<SS, 8, true>, wf, s, far_group16_smem(8)));
+            TAGI_TRY(launch_persistent(far_group16<SS, 8, true>, wf, s, far_group16_smem(8), GT));
         else if (sh.maxn1 <= 8)
-            TAGI_TRY(launch_persistent(far_group16<SS, 8, false>, wf, s, far_group16_smem(sh.maxn1)));
+            TAGI_TRY(launch_persistent(far_group16<SS, 8, false>, wf, s, far_group16_smem(sh.maxn1), GT));
         else
-            TAGI_TRY(launch_persistent(far_group16<SS, MAX_DEGREE + 1, false>, wf, s, far_group16_smem(sh.maxn1)));
+            TAGI_TRY(launch_persistent(far_group16<SS, MAX_DEGREE + 1, false>, wf, s, far_group16_smem(sh.maxn1), GT));
         phase_mark(PH_FAR, false, s);
         return TAGI_OK;
     }
     if (precision == PREC_MIXED && KERN == KERNEL_YUKAWA && sh.og > 1) {
         // orbital groups share the geometry of each pair across og orbitals
         const bool g8 = sh.og == 8;
-        if (g8) TAGI_TRY(launch_persistent(near_group<SS, 8, 0>, wn, s));
-        else TAGI_TRY(launch_persistent(near_group<SS, 4, 0>, wn, s));
+        if (g8) TAGI_TRY(launch_persistent(near_group<SS, 8, 0>, wn, s, 0, GT));
+        else TAGI_TRY(launch_persistent(near_group<SS, 4, 0>, wn, s, 0, GT));
         phase_mark(PH_NEAR, false, s);
         phase_mark(PH_NEAR_CLOSE, true, s);
-        if (g8) TAGI_TRY(launch_persistent(near_group<SS, 8, 1>, wc, s));
-        else TAGI_TRY(launch_persistent(near_group<SS, 4, 1>, wc, s));
+        if (g8) TAGI_TRY(launch_persistent(near_group<SS, 8, 1>, wc, s, 0, GT));
+        else TAGI_TRY(launch_persistent(near_group<SS, 4, 1>, wc, s, 0, GT));
         phase_mark(PH_NEAR_CLOSE, false, s);
         phase_mark(PH_FAR, true, s);
         const size_t fsm = far_group_smem(sh.maxn1, sh.og);
         if (sh.maxn1 <= 4) {
-            if (g8) TAGI_TRY(launch_persistent(far_group<SS, 4, 8>, wf, s, fsm));
-            else TAGI_TRY(launch_persistent(far_group<SS, 4, 4>, wf, s, fsm));
+            if (g8) TAGI_TRY(launch_persistent(far_group<SS, 4, 8>, wf, s, fsm, GT));
+            else TAGI_TRY(launch_persistent(far_group<SS, 4, 4>, wf, s, fsm, GT));
         } else if (sh.maxn1 == 8 && sh.minn1 == 8) {   // degree 7 everywhere: pipelined staging, fixed loops
-            if (g8) TAGI_TRY(launch_persistent(far_group_db<SS, 8>, wf, s, far_group_db_smem(8)));
-            else TAGI_TRY(launch_persistent(far_group_db<SS, 4>, wf, s, far_group_db_smem(4)));
+            if (g8) TAGI_TRY(launch_persistent(far_group_db<SS, 8>, wf, s, far_group_db_smem(8), GT));
+            else TAGI_TRY(launch_persistent(far_group_db<SS, 4>, wf, s, far_group_db_smem(4), GT));
         } else if (sh.maxn1 <= 8) {
-            if (g8) TAGI_TRY(launch_persistent(far_group<SS, 8, 8>, wf, s, fsm));
-            else TAGI_TRY(launch_persistent(far_group<SS, 8, 4>, wf, s, fsm));
+            if (g8) TAGI_TRY(launch_persistent(far_group<SS, 8, 8>, wf, s, fsm, GT));
+            else TAGI_TRY(launch_persistent(far_group<SS, 8, 4>, wf, s, fsm, GT));
         } else {
-            if (g8) TAGI_TRY(launch_persistent(far_group<SS, MAX_DEGREE + 1, 8>, wf, s, fsm));
-            else TAGI_TRY(launch_persistent(far_group<SS, MAX_DEGREE + 1, 4>, wf, s, fsm));
+            if (g8) TAGI_TRY(launch_persistent(far_group<SS, MAX_DEGREE + 1, 8>, wf, s, fsm, GT));
+            else TAGI_TRY(launch_persistent(far_group<SS, MAX_DEGREE + 1, 4>, wf, s, fsm, GT));
         }
         phase_mark(PH_FAR, false, s);
         return TAGI_OK;
@@ -2072,55 +2336,94 @@ int orbitals_per_item(int kernel, int precision, const int *norb, const double *
     return best;
 }
 
-bool schedule_matches(const Schedule &sc, const int *norb, int nsys, int og) {
-    if (sc.og != og || (int)sc.norb.size() != nsys) return false;
+bool schedule_matches(const Schedule &sc, const int *norb, int nsys, int og, int nt, int precision) {
+    if (sc.og != og || sc.nt != nt || sc.precision != precision || (int)sc.norb.size() != nsys) return false;
     for (int i = 0; i < nsys; i++)
         if (sc.norb[i] != norb[i]) return false;
     return true;
 }
 
+// Warps that share a target's sources in the single-orbital kernels, by the
+// plan's targets: a CTA then holds 256 / split threads' targets, and a small
+// mesh still has items for every SM, while a large one stages each tile for as
+// many targets as fit.  Set by the plan and the precision, not by the launch, so
+// an FP64 sum's last bits are the same however calls are batched (mixed sums do
+// not depend on the split).
+// Measured, ms per call at split 1, 2, 4, 8 (the targets and sources in one piece
+// before: first figure): Yukawa, 50k points, plan kept 4.1 -> 4.2, 3.1, 2.0, 1.5;
+// FP64, 50k points, one shot 636 -> 333, 325, 204, 180; one shot, mixed: Coulomb, 913k
+// points, degree 6, 63.6 -> 60.3, 55.0, 45.9; 1.13M, degree 5, 61.0 -> 61.4, 68.0,
+// 60.3; 1.5M, degree 7, 114.4 -> 119.1, 115.1, 117.4, 121.2.
+int field_split(int nt, int precision) {
+    if (nt <= 131072) return 8;
+    return precision == PREC_FP64 || nt <= 1200000 ? 4 : 2;
+}
+
+// Targets that a CTA of the field kernels holds.
+int cta_targets(int nt, int og, int nt_per_thread, int precision) {
+    return og > 1 ? GT : FT / field_split(nt, precision) * nt_per_thread;
+}
+
+// Targets per thread: the caller's request, else 2 where a batch holds more
+// than FT targets (single-orbital mixed kernels only).
+int targets_per_thread(Plan *const *plans, int nsys, int precision, int og, int requested) {
+    if (precision != PREC_MIXED || og != 1) return 1;
+    if (requested == 1 || requested == 2) return requested;
+    for (int i = 0; i < nsys; i++)
+        if (plans[i]->max_batch > FT) return 2;
+    return 1;
+}
+
 // Work lists for one launch over nsys systems: one item per (system, batch,
-// group of og orbitals), ordered by pair count times orbitals in the item,
-// heaviest first (ties in system, batch, group order).  Passes that have
-// nothing to do for a batch (no close ranges, no far entries) get no item:
-// their outputs are cleared before the launch.
-int build_schedule(Plan *const *plans, const int *norb, int nsys, int og, Schedule &sc, cudaStream_t s) {
+// chunk of its targets, group of og orbitals), ordered by pair count, heaviest
+// first (ties in system, batch, chunk, group order).  A batch's targets are cut
+// evenly, in whole warps, into chunks of at most what a CTA holds (nt per thread).
+// Passes that have nothing to do for a batch (no close ranges, no far entries)
+// get no item: their outputs are cleared before the launch.
+int build_schedule(Plan *const *plans, const int *norb, int nsys, int og, int nt, int precision, Schedule &sc,
+                   cudaStream_t s) {
     if (nsys < 1 || nsys > MAX_SYSTEMS) return set_error(TAGI_ERR_ARG, "%d systems (1..%d per launch)", nsys, MAX_SYSTEMS);
-    struct It {
-        long long cost;
-        int2 v;
+    struct Batch {
+        long long cost;   // pairs of one chunk
+        int sys, b, begin, end, chunk;
     };
-    std::vector<It> lists[3];
+    std::vector<Batch> lists[3];
     for (int i = 0; i < nsys; i++) {
         const Plan &p = *plans[i];
         if (norb[i] < 1 || norb[i] > 0xffff) return set_error(TAGI_ERR_ARG, "system %d: %d orbitals", i, norb[i]);
         if ((int)p.cost_near.size() != p.nbatch) return set_error(TAGI_ERR_STATE, "plan without batch costs");
-        for (int b = 0; b < p.nbatch; b++)
-            for (int g0 = 0; g0 < norb[i]; g0 += og) {
-                const long long lanes = og;
-                const int2 v = make_int2(b, (i << 16) | g0);
-                lists[0].push_back({p.cost_near[b] * lanes, v});
-                if (p.cost_close[b] > 0) lists[1].push_back({p.cost_close[b] * lanes, v});
-                if (p.cost_far[b] > 0) lists[2].push_back({p.cost_far[b] * lanes, v});
-            }
+        const int warp = 32 * nt, most = cta_targets(p.tgt.n, og, nt, precision);
+        for (int b = 0, at = 0; b < p.nbatch; at += p.batch_size[b++]) {
+            const int n = p.batch_size[b], chunks = (n + most - 1) / most;
+            const int chunk = ((n + chunks - 1) / chunks + warp - 1) / warp * warp;
+            const long long *cost[3] = {&p.cost_near[b], &p.cost_close[b], &p.cost_far[b]};
+            for (int k = 0; k < 3; k++)
+                if (k == 0 || *cost[k] > 0) lists[k].push_back({*cost[k] / n * std::min(n, chunk), i, b, at, at + n, chunk});
+        }
     }
-    std::vector<int2> all;
+    std::vector<int4> all;
     for (int k = 0; k < 3; k++) {
-        std::stable_sort(lists[k].begin(), lists[k].end(), [](const It &a, const It &b) { return a.cost > b.cost; });
+        std::stable_sort(lists[k].begin(), lists[k].end(),
+                         [](const Batch &a, const Batch &b) { return a.cost > b.cost; });
         sc.off[k] = (long)all.size();
-        sc.count[k] = (int)lists[k].size();
-        for (const It &it : lists[k]) all.push_back(it.v);
+        for (const Batch &v : lists[k])
+            for (int t = v.begin; t < v.end; t += v.chunk)
+                for (int g0 = 0; g0 < norb[v.sys]; g0 += og)
+                    all.push_back(make_int4(v.b, (v.sys << 16) | g0, t, std::min(t + v.chunk, v.end)));
+        sc.count[k] = (int)((long)all.size() - sc.off[k]);
     }
     // the old list may be in use on any stream: wait, then replace it
     TAGI_CUDA(cudaDeviceSynchronize());
     sc.release();
-    if (all.empty()) all.push_back(make_int2(0, 0));
+    if (all.empty()) all.push_back(make_int4(0, 0, 0, 0));
     void *v = nullptr;
-    TAGI_CUDA(cudaMalloc(&v, sizeof(int2) * all.size()));
-    sc.items = static_cast<int2 *>(v);
+    TAGI_CUDA(cudaMalloc(&v, sizeof(int4) * all.size()));
+    sc.items = static_cast<int4 *>(v);
     // pageable source: the copy has read it when the call returns
-    TAGI_CUDA(cudaMemcpyAsync(sc.items, all.data(), sizeof(int2) * all.size(), cudaMemcpyHostToDevice, s));
+    TAGI_CUDA(cudaMemcpyAsync(sc.items, all.data(), sizeof(int4) * all.size(), cudaMemcpyHostToDevice, s));
     sc.og = og;
+    sc.nt = nt;
+    sc.precision = precision;
     sc.norb.assign(norb, norb + nsys);
     return TAGI_OK;
 }
@@ -2149,7 +2452,7 @@ static int orbital_setup(Plan &p, const SysCall &c, int kernel, int singularity,
 // memory: scratch, schedule and FP64 weight charges must exist already, and
 // kernel parameters must be on the device.
 int convolve_systems(SysCall *calls, int nsys, int kernel, int singularity, int precision, const Schedule &sc,
-                     int *queue, cudaStream_t s, int nt_request) {
+                     int *queue, cudaStream_t s) {
     if (nsys < 1 || nsys > MAX_SYSTEMS) return set_error(TAGI_ERR_ARG, "%d systems (1..%d per launch)", nsys, MAX_SYSTEMS);
     const bool mixed = precision == PREC_MIXED;
     const bool ss = singularity == SING_SUBTRACTION;
@@ -2157,6 +2460,7 @@ int convolve_systems(SysCall *calls, int nsys, int kernel, int singularity, int 
     Fields f[MAX_SYSTEMS];
     LaunchShape sh;
     sh.og = sc.og;
+    sh.nt = sc.nt;
     for (int i = 0; i < nsys; i++) {
         SysCall &c = calls[i];
         Plan &p = *c.p;
@@ -2181,14 +2485,13 @@ int convolve_systems(SysCall *calls, int nsys, int kernel, int singularity, int 
         phase_mark(PH_UPWARD, false, s);
         if (!mixed && p.nslots && !p.what64) return set_error(TAGI_ERR_DEVICE, "FP64 weight charges missing");
         f[i] = make_fields(p, c.norb);
-        if (p.max_batch > FT) sh.nt = 2;  // automatic: two targets per thread for batches above FT
+        f[i].split = field_split(p.tgt.n, precision);
         if (p.n1 > sh.maxn1) sh.maxn1 = p.n1;
         if (p.n1 < sh.minn1) sh.minn1 = p.n1;
         // the far and close-range passes write only the batches they visit
         TAGI_CUDA(cudaMemsetAsync(p.far_out, 0, sizeof(double) * (size_t)c.norb * nt, s));
         TAGI_CUDA(cudaMemsetAsync(p.near2_out, 0, sizeof(double) * (size_t)c.norb * nt, s));
     }
-    if (nt_request == 1 || nt_request == 2) sh.nt = nt_request;
     TAGI_CUDA(cudaMemsetAsync(queue, 0, 3 * sizeof(int), s));
     if (kernel == KERNEL_YUKAWA) {
         if (ss) TAGI_TRY((launch_fields<KERNEL_YUKAWA, true>(calls, f, nsys, sc, sh, precision, queue, s)));
@@ -2221,9 +2524,11 @@ int convolve(Plan &p, const double *tv, const double *sv, double *out, int norb,
              const double *kparams, int nkp, int singularity, int precision, cudaStream_t s, bool kp_device,
              int og_request, int nt_request) {
     const int og = orbitals_per_item(kernel, precision, &norb, nullptr, 1, og_request, p.n1);
+    Plan *pp = &p;
+    const int nt = targets_per_thread(&pp, 1, precision, og, nt_request);
     const Schedule *sc = nullptr;
     for (const Schedule &c : p.scheds)
-        if (schedule_matches(c, &norb, 1, og)) sc = &c;
+        if (schedule_matches(c, &norb, 1, og, nt, precision)) sc = &c;
     if (!sc) {
         if (stream_capturing(s))
             return set_error(TAGI_ERR_STATE, "graph capture needs a prior uncaptured call with the same orbital count");
@@ -2234,8 +2539,7 @@ int convolve(Plan &p, const double *tv, const double *sv, double *out, int norb,
             p.scheds.erase(p.scheds.begin());
         }
         p.scheds.emplace_back();
-        Plan *pp = &p;
-        const int rc = build_schedule(&pp, &norb, 1, og, p.scheds.back(), s);
+        const int rc = build_schedule(&pp, &norb, 1, og, nt, precision, p.scheds.back(), s);
         if (rc) {
             p.scheds.back().release();
             p.scheds.pop_back();
@@ -2252,7 +2556,7 @@ int convolve(Plan &p, const double *tv, const double *sv, double *out, int norb,
     c.kp = kparams;
     c.nkp = nkp;
     c.kp_device = kp_device;
-    return convolve_systems(&c, 1, kernel, singularity, precision, *sc, p.queue, s, nt_request);
+    return convolve_systems(&c, 1, kernel, singularity, precision, *sc, p.queue, s);
 }
 
 int pair_peak(int kernel, int singularity, int variant, double kp, double *pairs_per_s, cudaStream_t s) {

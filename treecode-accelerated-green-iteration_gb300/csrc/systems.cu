@@ -20,7 +20,6 @@ struct Systems {
     std::vector<Plan *> plans;  // borrowed
     std::vector<int> norb;
     int kernel = KERNEL_YUKAWA, precision = PREC_MIXED;
-    int nt_request = 0;  // targets per thread: 0 automatic, 1 or 2
     Schedule sched;
     int *queue = nullptr;  // 3 work counters
     cudaStream_t stream = nullptr;
@@ -113,7 +112,6 @@ int tagi_systems_create(tagi_systems **systems, int numSystems, tagi_plan *const
     y->stream = (cudaStream_t)stream;
     y->kernel = kernel;
     y->precision = precision;
-    y->nt_request = targetsPerThread;
     for (int i = 0; i < numSystems; i++) {
         y->plans.push_back(reinterpret_cast<Plan *>(plans[i]));
         y->norb.push_back(numOrbitals[i]);
@@ -125,7 +123,9 @@ int tagi_systems_create(tagi_systems **systems, int numSystems, tagi_plan *const
         wt.push_back((double)q->src.n);
     }
     const int og = orbitals_per_item(kernel, precision, y->norb.data(), wt.data(), numSystems, orbitalsPerItem, maxn1);
-    int rc = build_schedule(y->plans.data(), y->norb.data(), numSystems, og, y->sched, y->stream);
+    const int nt = targets_per_thread(y->plans.data(), numSystems, precision, og, targetsPerThread);
+    int rc = build_schedule(y->plans.data(), y->norb.data(), numSystems, og, nt, precision, y->sched,
+                            y->stream);
     if (!rc) {
         void *v = nullptr;
         if (cudaMalloc(&v, 3 * sizeof(int)) != cudaSuccess)
@@ -185,8 +185,7 @@ int tagi_systems_convolve(tagi_systems *systems, const double *const *targetValu
         calls[i].nkp = numberOfKernelParameters;
         calls[i].kp_device = kernelParametersOnDevice != 0;
     }
-    return convolve_systems(calls, n, y.kernel, singularity, y.precision, y.sched, y.queue, (cudaStream_t)stream,
-                            y.nt_request);
+    return convolve_systems(calls, n, y.kernel, singularity, y.precision, y.sched, y.queue, (cudaStream_t)stream);
 }
 
 int tagi_systems_destroy(tagi_systems *systems) {

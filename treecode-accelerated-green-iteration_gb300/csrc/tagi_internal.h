@@ -116,14 +116,18 @@ struct Tree {
     double *center = nullptr, *half = nullptr, *radius = nullptr;
 };
 
-// Work list of one field launch: items {batch, sys << 16 | first orbital},
-// heaviest first, in three segments: near pass 0 (every batch), near close
-// pass (batches with close ranges), far field (batches with far entries).
-// og orbitals per item (orbital-group kernels) or 1.
+// Work list of one field launch: items {batch, sys << 16 | first orbital,
+// target begin, target end}, heaviest first, in three segments: near pass 0
+// (every batch), near close pass (batches with close ranges), far field
+// (batches with far entries).  og orbitals per item (orbital-group kernels) or
+// 1; nt targets per thread.  Chunks of a batch's targets depend on og, nt and
+// precision (field_split).
 struct Schedule {
     int og = 0;                 // 0 = not built
+    int nt = 1;
+    int precision = PREC_MIXED;
     std::vector<int> norb;      // orbitals per system the schedule was built for
-    int2 *items = nullptr;      // device, owned
+    int4 *items = nullptr;      // device, owned
     int count[3] = {0, 0, 0};
     long off[3] = {0, 0, 0};
     void release() {  // caller makes sure no launch still reads the list
@@ -190,6 +194,7 @@ struct Plan {
     // per-batch pair counts (host) for work ordering: ordinary near ranges,
     // close ranges, far field
     std::vector<long long> cost_near, cost_close, cost_far;
+    std::vector<int> batch_size;           // targets of each batch (batches follow one another)
     std::vector<Schedule> scheds;          // single-plan work lists by (orbitals, group), cached
 };
 
@@ -229,10 +234,12 @@ constexpr int MAX_SYSTEMS = 8;  // systems per field launch
 int ensure_scratch(Plan &p, int norb);
 int orbitals_per_item(int kernel, int precision, const int *norb, const double *weight, int nsys, int requested,
                       int max_n1);
-int build_schedule(Plan *const *plans, const int *norb, int nsys, int og, Schedule &sc, cudaStream_t s);
-bool schedule_matches(const Schedule &sc, const int *norb, int nsys, int og);
+int targets_per_thread(Plan *const *plans, int nsys, int precision, int og, int requested);
+int build_schedule(Plan *const *plans, const int *norb, int nsys, int og, int nt, int precision, Schedule &sc,
+                   cudaStream_t s);
+bool schedule_matches(const Schedule &sc, const int *norb, int nsys, int og, int nt, int precision);
 int convolve_systems(SysCall *calls, int nsys, int kernel, int singularity, int precision,
-                     const Schedule &sc, int *queue, cudaStream_t s, int nt_request = 0);
+                     const Schedule &sc, int *queue, cudaStream_t s);
 int convolve(Plan &p, const double *tv, const double *sv, double *out, int norb, int kernel,
              const double *kparams, int nkp, int singularity, int precision, cudaStream_t s,
              bool kp_device = false, int og_request = 0, int nt_request = 0);

@@ -741,6 +741,7 @@ int build_lists(Plan &p, cudaStream_t s) {
             p.cost_close[b] = hcc[b];
             p.cost_far[b] = hcf[b] * (long long)p.P;
         }
+        p.batch_size = std::move(hsz);
         if (cudaGetLastError() != cudaSuccess) { rc = set_error(TAGI_ERR_CUDA, "list kernels failed"); break; }
     } while (0);
     tmp.release();
