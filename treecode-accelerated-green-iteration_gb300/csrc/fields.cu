@@ -118,6 +118,18 @@ __device__ __forceinline__ int next_item(int *queue, int *s_item) {
     return *s_item;
 }
 
+// The field passes of a call (near, close, far) only read what earlier kernels
+// wrote and write separate outputs, so each pass may start on the SMs that the
+// one before has run out of items for: programmatic dependent launch.  A pass
+// lets its successor start as soon as it runs (pass_begin), and one CTA of each
+// pass ends only after the pass before has ended (pass_end), so that whatever
+// follows the last pass in the stream follows all of them.  Both are no-ops
+// where the launches are not programmatic.
+__device__ __forceinline__ void pass_begin() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pass_end() {
+    if (blockIdx.x == 0) asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 // The place of a warp in its CTA: target group g of G, source split sp of S.
 struct Place {
     int S, G, g, sp, lane, wid;
@@ -384,6 +396,7 @@ __global__ void __launch_bounds__(FT, TAGI_NEAR_MINB) near_mixed(const __grid_co
     __shared__ int s_item;
     constexpr int NOEXP = 1 << 30;
     const int tid = threadIdx.x;
+    pass_begin();
     for (;;) {
         const int item = next_item(w.queue, &s_item);
         if (item >= w.nitems) break;
@@ -525,6 +538,7 @@ __global__ void __launch_bounds__(FT, TAGI_NEAR_MINB) near_mixed(const __grid_co
         for (int k = 0; k < NT; k++)
             if (i0 + k < te) a.out[(long)orb * a.nt + i0 + k] = ((double)sum[k] - (double)cmp[k]) * sc;
     }
+    pass_end();
 }
 
 // ---------------------------------------------------------------------------
@@ -618,6 +632,7 @@ __global__ void __launch_bounds__(FT, 2) far_mixed(const __grid_constant__ Work 
     __shared__ float s_part[FAR_PART];   // S > 1: partials [cluster of the tile, slab][target of the CTA]
     __shared__ int s_item;
     const int tid = threadIdx.x;
+    pass_begin();
     for (;;) {
         const int item = next_item(w.queue, &s_item);
         if (item >= w.nitems) break;
@@ -740,6 +755,7 @@ __global__ void __launch_bounds__(FT, 2) far_mixed(const __grid_constant__ Work 
         for (int k = 0; k < NT; k++)
             if (i0 + k < te) a.out[(long)orb * a.nt + i0 + k] = ((double)sum[k] - (double)cmp[k]) * sc;
     }
+    pass_end();
 }
 
 // ---------------------------------------------------------------------------
@@ -821,6 +837,7 @@ __global__ void __launch_bounds__(GT, 4) near_group(const __grid_constant__ Work
     __shared__ int s_cnt[GW];
     __shared__ int s_item;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    pass_begin();
     for (;;) {
         const int item = next_item(w.queue, &s_item);
         if (item >= w.nitems) break;
@@ -928,6 +945,7 @@ __global__ void __launch_bounds__(GT, 4) near_group(const __grid_constant__ Work
                 if (g0 + o < a.norb) a.out[(long)(g0 + o) * a.nt + i] = (double)sum[o] - (double)cmp[o];
         }
     }
+    pass_end();
 }
 
 // One staged proxy grid against one target for a group of orbitals (see
@@ -998,6 +1016,7 @@ __global__ void __launch_bounds__(GT, 4) far_group(const __grid_constant__ Work 
     __shared__ int s_item;
     float4 *s_q4 = reinterpret_cast<float4 *>(s_dyn);
     const int tid = threadIdx.x;
+    pass_begin();
     for (;;) {
         const int item = next_item(w.queue, &s_item);
         if (item >= w.nitems) break;
@@ -1059,6 +1078,7 @@ __global__ void __launch_bounds__(GT, 4) far_group(const __grid_constant__ Work 
                 if (g0 + o < a.norb) a.out[(long)(g0 + o) * a.nt + i] = (double)sum[o] - (double)cmp[o];
         }
     }
+    pass_end();
 }
 
 // ---------------------------------------------------------------------------
@@ -1091,6 +1111,7 @@ __global__ void __launch_bounds__(GT, 4) far_group_db(const __grid_constant__ Wo
     __shared__ float s_p[2][3][DB_N1];
     __shared__ int s_item;
     const int tid = threadIdx.x;
+    pass_begin();
     for (;;) {
         const int item = next_item(w.queue, &s_item);
         if (item >= w.nitems) break;
@@ -1157,6 +1178,7 @@ __global__ void __launch_bounds__(GT, 4) far_group_db(const __grid_constant__ Wo
                 if (g0 + o < a.norb) a.out[(long)(g0 + o) * a.nt + i] = (double)sum[o] - (double)cmp[o];
         }
     }
+    pass_end();
 }
 
 // ---------------------------------------------------------------------------
@@ -1333,6 +1355,7 @@ __global__ void __launch_bounds__(GT, 4) near_group16(const __grid_constant__ Wo
     __shared__ int s_cnt[GW];
     __shared__ int s_item;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    pass_begin();
     for (;;) {
         const int item = next_item(w.queue, &s_item);
         if (item >= w.nitems) break;
@@ -1436,6 +1459,7 @@ __global__ void __launch_bounds__(GT, 4) near_group16(const __grid_constant__ Wo
                     a.out[(long)(g0 + o) * a.nt + i] = (double)s_k[o * GT + tid] - (double)s_k[(16 + o) * GT + tid];
         }
     }
+    pass_end();
 }
 
 // One staged proxy grid against one target for 16 orbitals (see far_cluster
@@ -1537,6 +1561,7 @@ __global__ void __launch_bounds__(GT, 4) far_group16(const __grid_constant__ Wor
     __shared__ float s_p[3][MAXN1];
     __shared__ int s_item;
     const int tid = threadIdx.x;
+    pass_begin();
     for (;;) {
         const int item = next_item(w.queue, &s_item);
         if (item >= w.nitems) break;
@@ -1605,6 +1630,7 @@ __global__ void __launch_bounds__(GT, 4) far_group16(const __grid_constant__ Wor
                 if (g0 + o < a.norb) a.out[(long)(g0 + o) * a.nt + i] = (double)sum[o] - (double)cmp[o];
         }
     }
+    pass_end();
 }
 
 // ---------------------------------------------------------------------------
@@ -1631,6 +1657,7 @@ __global__ void __launch_bounds__(FT) near_f64(const __grid_constant__ Work w) {
     __shared__ double s_x[T64], s_y[T64], s_z[T64], s_f[T64], s_w[T64];
     __shared__ int s_item;
     const int tid = threadIdx.x;
+    pass_begin();
     for (;;) {
         const int item = next_item(w.queue, &s_item);
         if (item >= w.nitems) break;
@@ -1669,6 +1696,7 @@ __global__ void __launch_bounds__(FT) near_f64(const __grid_constant__ Work w) {
         acc = add_splits(acc, pl, s_x);
         if (v && pl.sp == 0) a.out[(long)orb * a.nt + i] = acc;
     }
+    pass_end();
 }
 
 template <int KERN, bool SS, int MAXN1>
@@ -1678,6 +1706,7 @@ __global__ void __launch_bounds__(FT) far_f64(const __grid_constant__ Work w) {
     __shared__ double s_p[3][MAXN1], s_red[FT];
     __shared__ int s_item;
     const int tid = threadIdx.x;
+    pass_begin();
     for (;;) {
         const int item = next_item(w.queue, &s_item);
         if (item >= w.nitems) break;
@@ -1733,6 +1762,7 @@ __global__ void __launch_bounds__(FT) far_f64(const __grid_constant__ Work w) {
         acc = add_splits(acc, pl, s_red);
         if (v && pl.sp == 0) a.out[(long)orb * a.nt + i] = acc;
     }
+    pass_end();
 }
 
 // ---------------------------------------------------------------------------
@@ -1791,9 +1821,11 @@ int occupancy_grid(K kern, int *grid, size_t smem = 0, int threads = FT) {
 
 // Persistent launch: grid = resident CTAs (at most one per work item).  smem
 // bytes of dynamic shared memory; for large requests the kernel's limit is
-// raised first.
+// raised first.  follows: whether the launch before it in the stream was another
+// field pass of this call (set to true by a launch).
 template <typename K>
-int launch_persistent(K kern, const Work &w, cudaStream_t s, size_t smem = 0, int threads = FT) {
+int launch_persistent(K kern, const Work &w, cudaStream_t s, size_t smem = 0, int threads = FT,
+                      bool *follows = nullptr) {
     if (w.nitems == 0) return TAGI_OK;
     if (smem > 32 * 1024)   // dynamic + static above the 48 KB default needs the opt-in
         TAGI_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -1801,8 +1833,19 @@ int launch_persistent(K kern, const Work &w, cudaStream_t s, size_t smem = 0, in
     TAGI_TRY(occupancy_grid(kern, &grid, smem, threads));
     if (grid > w.nitems) grid = w.nitems;
     if (grid < 1) grid = 1;
-    launch(kern, grid, threads, smem, s, w);
-    TAGI_LAUNCH_CHECK();
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = &at;
+    cfg.numAttrs = follows && *follows ? 1 : 0;
+    count_launch();
+    TAGI_CUDA(cudaLaunchKernelEx(&cfg, kern, w));
+    if (follows) *follows = true;
     return TAGI_OK;
 }
 
@@ -2087,83 +2130,84 @@ int launch_fields(const SysCall *calls, const Fields *f, int nsys, const Schedul
     wf.queue = queue + 1;
     const bool one = sh.nt == 1;
     phase_mark(PH_NEAR, true, s);
+    bool pdl = false;   // no field pass of this call launched yet
     if (precision == PREC_MIXED && KERN == KERNEL_YUKAWA && sh.og == 16) {
-        TAGI_TRY(launch_persistent(near_group16<SS, 0>, wn, s, near_group16_smem(0), GT));
+        TAGI_TRY(launch_persistent(near_group16<SS, 0>, wn, s, near_group16_smem(0), GT, &pdl));
         phase_mark(PH_NEAR, false, s);
         phase_mark(PH_NEAR_CLOSE, true, s);
-        TAGI_TRY(launch_persistent(near_group16<SS, 1>, wc, s, near_group16_smem(1), GT));
+        TAGI_TRY(launch_persistent(near_group16<SS, 1>, wc, s, near_group16_smem(1), GT, &pdl));
         phase_mark(PH_NEAR_CLOSE, false, s);
         phase_mark(PH_FAR, true, s);
         if (sh.maxn1 <= 4)
-            TAGI_TRY(launch_persistent(far_group16<SS, 4, false>, wf, s, far_group16_smem(sh.maxn1), GT));
+            TAGI_TRY(launch_persistent(far_group16<SS, 4, false>, wf, s, far_group16_smem(sh.maxn1), GT, &pdl));
         else if (sh.maxn1 == 8 && sh.minn1 == 8)   // degree 7 everywhere: fixed loops
-            TAGI_TRY(launch_persistent(far_group16<SS, 8, true>, wf, s, far_group16_smem(8), GT));
+            TAGI_TRY(launch_persistent(far_group16<SS, 8, true>, wf, s, far_group16_smem(8), GT, &pdl));
         else if (sh.maxn1 <= 8)
-            TAGI_TRY(launch_persistent(far_group16<SS, 8, false>, wf, s, far_group16_smem(sh.maxn1), GT));
+            TAGI_TRY(launch_persistent(far_group16<SS, 8, false>, wf, s, far_group16_smem(sh.maxn1), GT, &pdl));
         else
-            TAGI_TRY(launch_persistent(far_group16<SS, MAX_DEGREE + 1, false>, wf, s, far_group16_smem(sh.maxn1), GT));
+            TAGI_TRY(launch_persistent(far_group16<SS, MAX_DEGREE + 1, false>, wf, s, far_group16_smem(sh.maxn1), GT, &pdl));
         phase_mark(PH_FAR, false, s);
         return TAGI_OK;
     }
     if (precision == PREC_MIXED && KERN == KERNEL_YUKAWA && sh.og > 1) {
         // orbital groups share the geometry of each pair across og orbitals
         const bool g8 = sh.og == 8;
-        if (g8) TAGI_TRY(launch_persistent(near_group<SS, 8, 0>, wn, s, 0, GT));
-        else TAGI_TRY(launch_persistent(near_group<SS, 4, 0>, wn, s, 0, GT));
+        if (g8) TAGI_TRY(launch_persistent(near_group<SS, 8, 0>, wn, s, 0, GT, &pdl));
+        else TAGI_TRY(launch_persistent(near_group<SS, 4, 0>, wn, s, 0, GT, &pdl));
         phase_mark(PH_NEAR, false, s);
         phase_mark(PH_NEAR_CLOSE, true, s);
-        if (g8) TAGI_TRY(launch_persistent(near_group<SS, 8, 1>, wc, s, 0, GT));
-        else TAGI_TRY(launch_persistent(near_group<SS, 4, 1>, wc, s, 0, GT));
+        if (g8) TAGI_TRY(launch_persistent(near_group<SS, 8, 1>, wc, s, 0, GT, &pdl));
+        else TAGI_TRY(launch_persistent(near_group<SS, 4, 1>, wc, s, 0, GT, &pdl));
         phase_mark(PH_NEAR_CLOSE, false, s);
         phase_mark(PH_FAR, true, s);
         const size_t fsm = far_group_smem(sh.maxn1, sh.og);
         if (sh.maxn1 <= 4) {
-            if (g8) TAGI_TRY(launch_persistent(far_group<SS, 4, 8>, wf, s, fsm, GT));
-            else TAGI_TRY(launch_persistent(far_group<SS, 4, 4>, wf, s, fsm, GT));
+            if (g8) TAGI_TRY(launch_persistent(far_group<SS, 4, 8>, wf, s, fsm, GT, &pdl));
+            else TAGI_TRY(launch_persistent(far_group<SS, 4, 4>, wf, s, fsm, GT, &pdl));
         } else if (sh.maxn1 == 8 && sh.minn1 == 8) {   // degree 7 everywhere: pipelined staging, fixed loops
-            if (g8) TAGI_TRY(launch_persistent(far_group_db<SS, 8>, wf, s, far_group_db_smem(8), GT));
-            else TAGI_TRY(launch_persistent(far_group_db<SS, 4>, wf, s, far_group_db_smem(4), GT));
+            if (g8) TAGI_TRY(launch_persistent(far_group_db<SS, 8>, wf, s, far_group_db_smem(8), GT, &pdl));
+            else TAGI_TRY(launch_persistent(far_group_db<SS, 4>, wf, s, far_group_db_smem(4), GT, &pdl));
         } else if (sh.maxn1 <= 8) {
-            if (g8) TAGI_TRY(launch_persistent(far_group<SS, 8, 8>, wf, s, fsm, GT));
-            else TAGI_TRY(launch_persistent(far_group<SS, 8, 4>, wf, s, fsm, GT));
+            if (g8) TAGI_TRY(launch_persistent(far_group<SS, 8, 8>, wf, s, fsm, GT, &pdl));
+            else TAGI_TRY(launch_persistent(far_group<SS, 8, 4>, wf, s, fsm, GT, &pdl));
         } else {
-            if (g8) TAGI_TRY(launch_persistent(far_group<SS, MAX_DEGREE + 1, 8>, wf, s, fsm, GT));
-            else TAGI_TRY(launch_persistent(far_group<SS, MAX_DEGREE + 1, 4>, wf, s, fsm, GT));
+            if (g8) TAGI_TRY(launch_persistent(far_group<SS, MAX_DEGREE + 1, 8>, wf, s, fsm, GT, &pdl));
+            else TAGI_TRY(launch_persistent(far_group<SS, MAX_DEGREE + 1, 4>, wf, s, fsm, GT, &pdl));
         }
         phase_mark(PH_FAR, false, s);
         return TAGI_OK;
     }
     if (precision == PREC_MIXED) {
-        if (one) TAGI_TRY(launch_persistent(near_mixed<KERN, SS, 1, 0>, wn, s));
-        else TAGI_TRY(launch_persistent(near_mixed<KERN, SS, 2, 0>, wn, s));
+        if (one) TAGI_TRY(launch_persistent(near_mixed<KERN, SS, 1, 0>, wn, s, 0, FT, &pdl));
+        else TAGI_TRY(launch_persistent(near_mixed<KERN, SS, 2, 0>, wn, s, 0, FT, &pdl));
         phase_mark(PH_NEAR, false, s);
         phase_mark(PH_NEAR_CLOSE, true, s);
-        if (one) TAGI_TRY(launch_persistent(near_mixed<KERN, SS, 1, 1>, wc, s));
-        else TAGI_TRY(launch_persistent(near_mixed<KERN, SS, 2, 1>, wc, s));
+        if (one) TAGI_TRY(launch_persistent(near_mixed<KERN, SS, 1, 1>, wc, s, 0, FT, &pdl));
+        else TAGI_TRY(launch_persistent(near_mixed<KERN, SS, 2, 1>, wc, s, 0, FT, &pdl));
         phase_mark(PH_NEAR_CLOSE, false, s);
     } else {
         // one FP64 pass over all near ranges, close ones included
-        TAGI_TRY(launch_persistent(near_f64<KERN, SS>, wn, s));
+        TAGI_TRY(launch_persistent(near_f64<KERN, SS>, wn, s, 0, FT, &pdl));
         phase_mark(PH_NEAR, false, s);
     }
     phase_mark(PH_FAR, true, s);
     if (precision == PREC_MIXED) {
         const bool deg7 = sh.maxn1 == 8 && sh.minn1 == 8;
         if (one) {
-            if (sh.maxn1 <= 4) TAGI_TRY(launch_persistent(far_mixed<KERN, SS, 4, 1>, wf, s));
-            else if (deg7) TAGI_TRY(launch_persistent(far_mixed<KERN, SS, 8, 1, true>, wf, s));
-            else if (sh.maxn1 <= 8) TAGI_TRY(launch_persistent(far_mixed<KERN, SS, 8, 1>, wf, s));
-            else TAGI_TRY(launch_persistent(far_mixed<KERN, SS, MAX_DEGREE + 1, 1>, wf, s));
+            if (sh.maxn1 <= 4) TAGI_TRY(launch_persistent(far_mixed<KERN, SS, 4, 1>, wf, s, 0, FT, &pdl));
+            else if (deg7) TAGI_TRY(launch_persistent(far_mixed<KERN, SS, 8, 1, true>, wf, s, 0, FT, &pdl));
+            else if (sh.maxn1 <= 8) TAGI_TRY(launch_persistent(far_mixed<KERN, SS, 8, 1>, wf, s, 0, FT, &pdl));
+            else TAGI_TRY(launch_persistent(far_mixed<KERN, SS, MAX_DEGREE + 1, 1>, wf, s, 0, FT, &pdl));
         } else {
-            if (sh.maxn1 <= 4) TAGI_TRY(launch_persistent(far_mixed<KERN, SS, 4, 2>, wf, s));
-            else if (deg7) TAGI_TRY(launch_persistent(far_mixed<KERN, SS, 8, 2, true>, wf, s));
-            else if (sh.maxn1 <= 8) TAGI_TRY(launch_persistent(far_mixed<KERN, SS, 8, 2>, wf, s));
-            else TAGI_TRY(launch_persistent(far_mixed<KERN, SS, MAX_DEGREE + 1, 2>, wf, s));
+            if (sh.maxn1 <= 4) TAGI_TRY(launch_persistent(far_mixed<KERN, SS, 4, 2>, wf, s, 0, FT, &pdl));
+            else if (deg7) TAGI_TRY(launch_persistent(far_mixed<KERN, SS, 8, 2, true>, wf, s, 0, FT, &pdl));
+            else if (sh.maxn1 <= 8) TAGI_TRY(launch_persistent(far_mixed<KERN, SS, 8, 2>, wf, s, 0, FT, &pdl));
+            else TAGI_TRY(launch_persistent(far_mixed<KERN, SS, MAX_DEGREE + 1, 2>, wf, s, 0, FT, &pdl));
         }
     } else {
-        if (sh.maxn1 <= 4) TAGI_TRY(launch_persistent(far_f64<KERN, SS, 4>, wf, s));
-        else if (sh.maxn1 <= 8) TAGI_TRY(launch_persistent(far_f64<KERN, SS, 8>, wf, s));
-        else TAGI_TRY(launch_persistent(far_f64<KERN, SS, MAX_DEGREE + 1>, wf, s));
+        if (sh.maxn1 <= 4) TAGI_TRY(launch_persistent(far_f64<KERN, SS, 4>, wf, s, 0, FT, &pdl));
+        else if (sh.maxn1 <= 8) TAGI_TRY(launch_persistent(far_f64<KERN, SS, 8>, wf, s, 0, FT, &pdl));
+        else TAGI_TRY(launch_persistent(far_f64<KERN, SS, MAX_DEGREE + 1>, wf, s, 0, FT, &pdl));
     }
     phase_mark(PH_FAR, false, s);
     return TAGI_OK;
