@@ -453,6 +453,11 @@ int tagi_pipe_rates(double *rates, void *stream);
 int tagi_profile(int enable);
 int tagi_profile_read(double *ms, long long *count, int nphase);
 
+/* Device memory that the library keeps for its next calls on the current device
+ * (work arrays of plans and one-shot calls, at most 1 GiB once nothing is in
+ * use) goes back to the driver. */
+int tagi_release_memory(void);
+
 int tagi_last_error(void);
 const char *tagi_last_error_message(void);
 void tagi_clear_error(void);

@@ -98,6 +98,7 @@ SIGNATURES = {
     "tagi_pipe_rates": (_i, [_dp, _vp]),
     "tagi_profile": (_i, [_i]),
     "tagi_profile_read": (_i, [_dp, ctypes.POINTER(ctypes.c_longlong), _i]),
+    "tagi_release_memory": (_i, []),
     "tagi_last_error": (_i, []),
     "tagi_last_error_message": (ctypes.c_char_p, []),
     "tagi_clear_error": (None, []),

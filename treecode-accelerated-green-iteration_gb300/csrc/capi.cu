@@ -49,6 +49,42 @@ int set_error(int code, const char *fmt, ...) {
 
 int last_error() { return g_err; }
 
+namespace {
+std::mutex g_pool_mu;
+cudaMemPool_t g_pools[64] = {};
+
+// The library's pool of a device, made on first use; nullptr where none can be
+// made (the default pool then serves).
+cudaMemPool_t pool_of(int dev) {
+    if (dev < 0 || dev >= 64) return nullptr;
+    std::lock_guard<std::mutex> lk(g_pool_mu);
+    if (!g_pools[dev]) {
+        cudaMemPoolProps props{};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = dev;
+        cudaMemPool_t p = nullptr;
+        if (cudaMemPoolCreate(&p, &props) != cudaSuccess) {
+            cudaGetLastError();
+            return nullptr;
+        }
+        uint64_t keep = POOL_KEEP;
+        cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep);
+        g_pools[dev] = p;
+    }
+    return g_pools[dev];
+}
+}  // namespace
+
+// Under stream capture the allocation becomes a node of the caller's graph, which
+// the default pool's call does.
+cudaError_t pool_alloc(void **p, size_t bytes, cudaStream_t s) {
+    int dev = -1;
+    cudaMemPool_t pool = nullptr;
+    if (!stream_capturing(s) && cudaGetDevice(&dev) == cudaSuccess) pool = pool_of(dev);
+    return pool ? cudaMallocFromPoolAsync(p, bytes, pool, s) : cudaMallocAsync(p, bytes, s);
+}
+
 int validate(int nt, int ns, int kernel, int nkp, const double *kp, int sing, int approx,
              int ctype, double theta, int degree, int sl, int tl, double size_check, int precision) {
     if (nt < 0 || ns < 0) return set_error(TAGI_ERR_ARG, "negative point count (%d targets, %d sources)", nt, ns);
@@ -139,7 +175,7 @@ double ss_constant(int kernel, int sing, double k) {
 
 int plan_create(Plan **out, int nt, const double *tx, const double *ty, const double *tz, int ns,
                 const double *sx, const double *sy, const double *sz, const double *sw,
-                double theta, int degree, int sl, int tl, double size_check, cudaStream_t s) {
+                double theta, int degree, int sl, int tl, double size_check, cudaStream_t s, bool one_shot) {
     *out = nullptr;
     if (nt < 1 || ns < 1) return set_error(TAGI_ERR_ARG, "a plan needs >= 1 target and source (%d, %d)", nt, ns);
     if (!tx || !ty || !tz || !sx || !sy || !sz || !sw) return set_error(TAGI_ERR_ARG, "null device pointer");
@@ -151,6 +187,7 @@ int plan_create(Plan **out, int nt, const double *tx, const double *ty, const do
     Plan *p = new Plan();
     cudaGetDevice(&p->device);
     p->arena.stream = s;
+    p->one_shot = one_shot;
     p->degree = degree;
     p->n1 = degree + 1;
     p->P = p->n1 * p->n1 * p->n1;
@@ -187,6 +224,7 @@ int plan_create(Plan **out, int nt, const double *tx, const double *ty, const do
         if ((rc = build_lists(*p, s))) break;
         if ((rc = build_weight_charges(*p, s))) break;
         phase_mark(PH_LISTS, false, s);
+        if (one_shot) break;   // the convolution follows on the same stream
         cudaError_t e = cudaStreamSynchronize(s);
         if (e != cudaSuccess) { rc = set_error(TAGI_ERR_CUDA, "plan build: %s", cudaGetErrorString(e)); break; }
     } while (0);
@@ -203,6 +241,11 @@ int plan_create(Plan **out, int nt, const double *tx, const double *ty, const do
 
 void plan_destroy(Plan *p) {
     if (!p) return;
+    if (p->one_shot) {   // everything ran on one stream: freed in its order
+        p->arena.release();
+        delete p;
+        return;
+    }
     cudaDeviceSynchronize();
     for (void *v : p->scratch) cudaFree(v);
     for (Schedule &sc : p->scheds) sc.release();
@@ -229,7 +272,7 @@ int treecode_device(int nt, int ns, const double *tx, const double *ty, const do
     }
     double t0 = now_s();
     Plan *p = nullptr;
-    TAGI_TRY(plan_create(&p, nt, tx, ty, tz, ns, sx, sy, sz, sw, theta, degree, sl, tl, size_check, s));
+    TAGI_TRY(plan_create(&p, nt, tx, ty, tz, ns, sx, sy, sz, sw, theta, degree, sl, tl, size_check, s, true));
     double t1 = now_s();
     int rc = convolve(*p, tv, sv, out, 1, kernel, kp, nkp, sing, precision, s);
     if (!rc && verbosity > 0) {
@@ -242,6 +285,8 @@ int treecode_device(int nt, int ns, const double *tx, const double *ty, const do
                 p->far_pairs, precision == PREC_MIXED ? "mixed" : "fp64");
     }
     plan_destroy(p);
+    const cudaError_t e = cudaStreamSynchronize(s);
+    if (!rc && e != cudaSuccess) rc = set_error(TAGI_ERR_CUDA, "convolution: %s", cudaGetErrorString(e));
     return rc;
 }
 
@@ -278,6 +323,11 @@ int treecode_host(int nt, int ns, const double *tx, const double *ty, const doub
         const double *h[9] = {tx, ty, tz, tv, sx, sy, sz, sv, sw};
         const int n[9] = {nt, nt, nt, nt, ns, ns, ns, ns, ns};
         for (int i = 0; i < 9 && !rc; i++) {
+            // an array passed twice (targets that are the sources) is copied once, and
+            // the plan then sees one point set
+            for (int j = 0; j < i; j++)
+                if (h[j] == h[i] && n[j] == n[i]) d[i] = d[j];
+            if (d[i]) continue;
             rc = ar.alloc(&d[i], n[i] > 0 ? n[i] : 1);
             if (!rc && n[i] > 0 &&
                 cudaMemcpyAsync(d[i], h[i], sizeof(double) * n[i], cudaMemcpyHostToDevice, s) != cudaSuccess)
@@ -304,6 +354,13 @@ int treecode_host(int nt, int ns, const double *tx, const double *ty, const doub
 extern "C" {
 
 int tagi_version(void) { return 100; }
+
+int tagi_release_memory(void) {
+    int dev = 0;
+    TAGI_CUDA(cudaGetDevice(&dev));
+    if (cudaMemPool_t p = pool_of(dev)) TAGI_CUDA(cudaMemPoolTrimTo(p, 0));
+    return TAGI_OK;
+}
 int tagi_last_error(void) { return g_err; }
 const char *tagi_last_error_message(void) { return g_msg; }
 void tagi_clear_error(void) {

@@ -1768,29 +1768,33 @@ __global__ void __launch_bounds__(FT) far_f64(const __grid_constant__ Work w) {
 // ---------------------------------------------------------------------------
 // Per-call glue: sorted charges, epilogue.
 // ---------------------------------------------------------------------------
+template <bool MIXED>
 __global__ void prep_sources(const double *__restrict__ sv, const int *__restrict__ perm,
-                             const double *__restrict__ w, int ns, int norb,
-                             float *__restrict__ q32, double *__restrict__ q64,
-                             double *__restrict__ f64) {
+                             const double *__restrict__ w, int ns, float *__restrict__ q32,
+                             double *__restrict__ q64, double *__restrict__ f64) {
     long j = (long)blockIdx.x * blockDim.x + threadIdx.x;
     int orb = blockIdx.y;
     if (j >= ns) return;
     long o = (long)orb * ns + j;
     double f = sv[(long)orb * ns + perm[j]];
     double q = f * w[j];
-    q32[o] = (float)q;
-    q64[o] = q;
-    f64[o] = f;
+    if (MIXED) {
+        q32[o] = (float)q;
+    } else {
+        q64[o] = q;
+        f64[o] = f;
+    }
 }
 
+template <bool MIXED>
 __global__ void prep_targets(const double *__restrict__ tv, const int *__restrict__ perm, int nt,
                              float *__restrict__ f32, double *__restrict__ f64) {
     long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
     int orb = blockIdx.y;
     if (i >= nt) return;
     double f = tv[(long)orb * nt + perm[i]];
-    f32[(long)orb * nt + i] = (float)f;
-    f64[(long)orb * nt + i] = f;
+    if (MIXED) f32[(long)orb * nt + i] = (float)f;
+    else f64[(long)orb * nt + i] = f;
 }
 
 // phi_i = near + far + f_i * SS factor, scattered back to caller order.  The
@@ -2301,41 +2305,53 @@ bool stream_capturing(cudaStream_t s) {
     return st == cudaStreamCaptureStatusActive;
 }
 
-// Per-call scratch for norb orbitals.  Growing it is rare (a larger orbital
-// count than any earlier call) and synchronizes the device first: the old
-// buffers may still be in use by calls on any stream.  Plain cudaMalloc keeps
-// the new buffers valid on every stream.
-int ensure_scratch(Plan &p, int norb) {
+// Per-call scratch for norb orbitals, one block.  Growing it is rare (a larger
+// orbital count than any earlier call) and synchronizes the device first: the
+// old block may still be in use by calls on any stream.  Plain cudaMalloc keeps
+// the new one valid on every stream.  A one-shot plan's scratch serves one call
+// of one precision on the plan's stream and comes from its arena.
+int ensure_scratch(Plan &p, int norb, int precision) {
     if ((size_t)norb <= p.scratch_orbitals) return TAGI_OK;
-    TAGI_CUDA(cudaDeviceSynchronize());
-    for (void *v : p.scratch) cudaFree(v);
-    p.scratch.clear();
-    p.scratch_orbitals = 0;
     const size_t ns = p.src.n, nt = p.tgt.n, no = norb;
-    auto alloc = [&](auto **ptr, size_t count) -> int {
-        void *v = nullptr;
-        const size_t bytes = (count ? count : 1) * sizeof(**ptr);
-        cudaError_t e = cudaMalloc(&v, bytes);
+    const bool mixed = !p.one_shot || precision == PREC_MIXED, fp64 = !p.one_shot || precision == PREC_FP64;
+    auto carve = [&](char *base) {   // the block's size; sets the pointers if base is given
+        size_t at = 0;
+        auto take = [&](auto **ptr, size_t count, bool wanted = true) {
+            if (!wanted) return;
+            if (base) *ptr = reinterpret_cast<std::remove_reference_t<decltype(*ptr)>>(base + at);
+            at += ((count ? count : 1) * sizeof(**ptr) + 255) / 256 * 256;
+        };
+        take(&p.q32, no * ns, mixed);
+        take(&p.ft32, no * nt, mixed);
+        take(&p.q64, no * ns, fp64);
+        take(&p.f64s, no * ns, fp64);
+        take(&p.ft64, no * nt, fp64);
+        take(&p.part, no * p.nitems * p.P);
+        take(&p.qhat32, no * p.nslots * p.P, mixed);
+        take(&p.qhat64, no * p.nslots * p.P, fp64);
+        take(&p.near_out, no * nt);
+        take(&p.near2_out, no * nt);
+        take(&p.far_out, no * nt);
+        take(&p.d_kc, no);
+        take(&p.d_kp, no);
+        take(&p.d_ss, no);
+        return at;
+    };
+    const size_t bytes = carve(nullptr);
+    char *block = nullptr;
+    if (p.one_shot) {
+        TAGI_TRY(p.arena.alloc(&block, bytes));
+    } else {
+        TAGI_CUDA(cudaDeviceSynchronize());
+        for (void *v : p.scratch) cudaFree(v);
+        p.scratch.clear();
+        p.scratch_orbitals = 0;
+        const cudaError_t e = cudaMalloc(reinterpret_cast<void **>(&block), bytes);
         if (e != cudaSuccess)
             return set_error(TAGI_ERR_CUDA, "device allocation of %zu bytes failed: %s", bytes, cudaGetErrorString(e));
-        p.scratch.push_back(v);
-        *ptr = static_cast<std::remove_reference_t<decltype(**ptr)> *>(v);
-        return TAGI_OK;
-    };
-    TAGI_TRY(alloc(&p.q32, no * ns));
-    TAGI_TRY(alloc(&p.ft32, no * nt));
-    TAGI_TRY(alloc(&p.q64, no * ns));
-    TAGI_TRY(alloc(&p.f64s, no * ns));
-    TAGI_TRY(alloc(&p.ft64, no * nt));
-    TAGI_TRY(alloc(&p.part, no * p.nitems * p.P));
-    TAGI_TRY(alloc(&p.qhat32, no * p.nslots * p.P));
-    TAGI_TRY(alloc(&p.qhat64, no * p.nslots * p.P));
-    TAGI_TRY(alloc(&p.near_out, no * nt));
-    TAGI_TRY(alloc(&p.near2_out, no * nt));
-    TAGI_TRY(alloc(&p.far_out, no * nt));
-    TAGI_TRY(alloc(&p.d_kc, no));
-    TAGI_TRY(alloc(&p.d_kp, no));
-    TAGI_TRY(alloc(&p.d_ss, no));
+        p.scratch.push_back(block);
+    }
+    carve(block);
     p.scratch_orbitals = no;
     return TAGI_OK;
 }
@@ -2456,13 +2472,18 @@ int build_schedule(Plan *const *plans, const int *norb, int nsys, int og, int nt
                     all.push_back(make_int4(v.b, (v.sys << 16) | g0, t, std::min(t + v.chunk, v.end)));
         sc.count[k] = (int)((long)all.size() - sc.off[k]);
     }
-    // the old list may be in use on any stream: wait, then replace it
-    TAGI_CUDA(cudaDeviceSynchronize());
-    sc.release();
     if (all.empty()) all.push_back(make_int4(0, 0, 0, 0));
-    void *v = nullptr;
-    TAGI_CUDA(cudaMalloc(&v, sizeof(int4) * all.size()));
-    sc.items = static_cast<int4 *>(v);
+    if (nsys == 1 && plans[0]->one_shot) {
+        TAGI_TRY(plans[0]->arena.alloc(&sc.items, all.size()));
+        sc.borrowed = true;
+    } else {
+        // the old list may be in use on any stream: wait, then replace it
+        TAGI_CUDA(cudaDeviceSynchronize());
+        sc.release();
+        void *v = nullptr;
+        TAGI_CUDA(cudaMalloc(&v, sizeof(int4) * all.size()));
+        sc.items = static_cast<int4 *>(v);
+    }
     // pageable source: the copy has read it when the call returns
     TAGI_CUDA(cudaMemcpyAsync(sc.items, all.data(), sizeof(int4) * all.size(), cudaMemcpyHostToDevice, s));
     sc.og = og;
@@ -2514,13 +2535,14 @@ int convolve_systems(SysCall *calls, int nsys, int kernel, int singularity, int 
                                  "graph capture needs a prior uncaptured call with the same orbital counts and "
                                  "precision, and kernel parameters on the device");
         }
-        TAGI_TRY(ensure_scratch(p, c.norb));
+        TAGI_TRY(ensure_scratch(p, c.norb, precision));
         TAGI_TRY(orbital_setup(p, c, kernel, singularity, mixed ? 1 : 0, s));
         const int ns = p.src.n, nt = p.tgt.n;
         dim3 gs((ns + 255) / 256, c.norb), gt((nt + 255) / 256, c.norb);
         phase_mark(PH_GLUE, true, s);
-        launch(prep_sources, gs, 256, 0, s, c.sv, p.src.perm, p.sw64, ns, c.norb, p.q32, p.q64, p.f64s);
-        launch(prep_targets, gt, 256, 0, s, c.tv, p.tgt.perm, nt, p.ft32, p.ft64);
+        launch(mixed ? prep_sources<true> : prep_sources<false>, gs, 256, 0, s, c.sv, p.src.perm, p.sw64, ns, p.q32,
+               p.q64, p.f64s);
+        launch(mixed ? prep_targets<true> : prep_targets<false>, gt, 256, 0, s, c.tv, p.tgt.perm, nt, p.ft32, p.ft64);
         phase_mark(PH_GLUE, false, s);
         TAGI_LAUNCH_CHECK();
         phase_mark(PH_UPWARD, true, s);

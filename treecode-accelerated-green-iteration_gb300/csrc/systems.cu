@@ -133,7 +133,7 @@ int tagi_systems_create(tagi_systems **systems, int numSystems, tagi_plan *const
         y->queue = static_cast<int *>(v);
     }
     // scratch for every system now, so later calls can be captured
-    for (int i = 0; !rc && i < numSystems; i++) rc = ensure_scratch(*y->plans[i], y->norb[i]);
+    for (int i = 0; !rc && i < numSystems; i++) rc = ensure_scratch(*y->plans[i], y->norb[i], precision);
     if (!rc && cudaStreamSynchronize(y->stream) != cudaSuccess) rc = set_error(TAGI_ERR_CUDA, "systems setup failed");
     if (rc) {
         cudaStreamSynchronize(y->stream);

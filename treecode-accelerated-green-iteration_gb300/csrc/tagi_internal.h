@@ -80,6 +80,14 @@ constexpr double CLOSE_RANGE_FRACTION = 0.1;
 enum Phase { PH_TREE = 0, PH_LISTS, PH_UPWARD, PH_NEAR, PH_FAR, PH_GLUE, PH_NEAR_CLOSE, PH_COUNT };
 void phase_mark(int phase, bool begin, cudaStream_t s);
 
+// Stream-ordered device memory from the library's own pool of the current
+// device (capi.cu): the default pool returns its memory to the driver at every
+// synchronization, and a call that builds a plan allocates some sixty arrays and
+// synchronizes several times.  The pool keeps at most POOL_KEEP bytes between
+// calls (0.4% of this GPU's memory); tagi_release_memory gives those back too.
+constexpr unsigned long long POOL_KEEP = 1ULL << 30;
+cudaError_t pool_alloc(void **p, size_t bytes, cudaStream_t s);
+
 // Stream-ordered device allocations owned by a plan (freed on destroy).
 struct Arena {
     std::vector<void *> ptrs;
@@ -89,7 +97,7 @@ struct Arena {
         void *v = nullptr;
         size_t bytes = count * sizeof(T);
         if (bytes == 0) bytes = 16;
-        cudaError_t e = cudaMallocAsync(&v, bytes, stream);
+        cudaError_t e = pool_alloc(&v, bytes, stream);
         if (e != cudaSuccess)
             return set_error(TAGI_ERR_CUDA, "device allocation of %zu bytes failed: %s", bytes,
                              cudaGetErrorString(e));
@@ -127,11 +135,12 @@ struct Schedule {
     int nt = 1;
     int precision = PREC_MIXED;
     std::vector<int> norb;      // orbitals per system the schedule was built for
-    int4 *items = nullptr;      // device, owned
+    int4 *items = nullptr;      // device, owned unless borrowed
+    bool borrowed = false;      // items belong to the plan's arena (one-shot calls)
     int count[3] = {0, 0, 0};
     long off[3] = {0, 0, 0};
     void release() {  // caller makes sure no launch still reads the list
-        if (items) cudaFree(items);
+        if (items && !borrowed) cudaFree(items);
         items = nullptr;
         og = 0;
         norb.clear();
@@ -141,6 +150,7 @@ struct Schedule {
 struct Plan {
     int device = 0;
     Arena arena;
+    bool one_shot = false;                 // built, used once and freed on arena.stream alone
     Tree src, tgt;
     int degree = 7, n1 = 8, P = 512;
     double theta = 0.7, size_check = 1.0;
@@ -212,7 +222,7 @@ struct SysCall {
 struct Plan;
 int plan_create(Plan **out, int nt, const double *tx, const double *ty, const double *tz, int ns,
                 const double *sx, const double *sy, const double *sz, const double *sw, double theta, int degree,
-                int sl, int tl, double size_check, cudaStream_t s);
+                int sl, int tl, double size_check, cudaStream_t s, bool one_shot = false);
 void plan_destroy(Plan *p);
 
 // scan_sort.cu
@@ -231,7 +241,7 @@ int modified_charges(Plan &p, int precision, int norb, cudaStream_t s);
 
 // fields.cu
 constexpr int MAX_SYSTEMS = 8;  // systems per field launch
-int ensure_scratch(Plan &p, int norb);
+int ensure_scratch(Plan &p, int norb, int precision);
 int orbitals_per_item(int kernel, int precision, const int *norb, const double *weight, int nsys, int requested,
                       int max_n1);
 int targets_per_thread(Plan *const *plans, int nsys, int precision, int og, int requested);
