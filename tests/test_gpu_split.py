@@ -48,3 +48,28 @@ def test_targets_that_are_not_sources(BT, dev, oracle):
     for precision, tol in (("mixed", 1e-6), ("fp64", 1e-12)):
         got = plan.convolve(*to_cuda(tv, f), BT.Kernel.YUKAWA, [0.9], BT.Singularity.SUBTRACTION, precision=precision)
         assert rel_l2(got.cpu().numpy(), ref) <= tol
+
+
+@pytest.mark.parametrize("scale", [1e-22, 1e-3, 1.0, 60.0, 1e4, 1e21])
+@pytest.mark.parametrize("name,k", [("YUKAWA", 0.7), ("COULOMB", 1.1)])
+@pytest.mark.parametrize("sing", ["SUBTRACTION", "SKIPPING"])
+def test_fp64_pairs_over_the_distance_range(BT, dev, scale, name, k, sing):
+    """Distances from far below to far above FP32's squared range, exponents past
+    underflow, coincident points: the sums of numpy's FP64 functions to 1e-12 of
+    the sum of the terms' magnitudes."""
+    rng = np.random.default_rng(3)
+    p = rng.uniform(-1.0, 1.0, (3, 150)) * scale
+    p[:, 70:75] = p[:, 10:15]                      # coincident pairs are left out
+    w, f = rng.uniform(0.5, 1.5, 150), rng.standard_normal(150)
+    d2 = ((p[:, :, None] - p[:, None, :]) ** 2).sum(0)
+    with np.errstate(divide="ignore", invalid="ignore", over="ignore", under="ignore"):
+        r = np.sqrt(d2)
+        if name == "YUKAWA":
+            t = (f[None, :] - (f[:, None] if sing == "SUBTRACTION" else 0.0)) * w[None, :] * np.exp(-k * r) / r
+        else:
+            t = w[None, :] * (f[None, :] - (f[:, None] * np.exp(-k * k * d2) if sing == "SUBTRACTION" else 0.0)) / r
+    t[d2 == 0.0] = 0.0
+    own = f * (4.0 if name == "YUKAWA" else 2.0) * np.pi / k ** 2 if sing == "SUBTRACTION" else 0.0 * f
+    got = dev.TreecodePlan.for_mesh(*to_cuda(*p, w), theta=0.7, degree=2, source_leaf=200, target_leaf=200).convolve(
+        *to_cuda(f, f), getattr(BT.Kernel, name), [k], getattr(BT.Singularity, sing), precision="fp64").cpu().numpy()
+    assert np.all(np.abs(got - (t.sum(1) + own)) <= 1e-12 * (np.abs(t).sum(1) + np.abs(own)) + 1e-300)

@@ -107,6 +107,7 @@ struct Work {
     const int4 *items;            // {batch, sys << 16 | first orbital, target begin, end}, heaviest first
     int nitems;
     int *queue;                   // this pass's work counter
+    const double *exp_table;      // FP64 passes: 2^{i / EXP_N}
     Fields sys[MAX_SYSTEMS];
 };
 static_assert(sizeof(Work) <= 4096, "field-kernel parameter block above 4 KB");
@@ -1635,29 +1636,183 @@ __global__ void __launch_bounds__(GT, 4) far_group16(const __grid_constant__ Wor
 
 // ---------------------------------------------------------------------------
 // FP64 near and far fields (the plain path).
+//
+// Bound: the FP64 pipe.  It issues 1/64 of the FP32 rate (measured 527 G DFMA/s
+// against 3.9e13 FFMA/s), so one FP64 instruction costs as much as some seventy
+// FP32 or integer ones.  sqrt, exp and the division of a Yukawa pair are about
+// 35 FP64 instructions; here a pair is 22 in all (Coulomb with subtraction 18):
+//   * 1/r from the FP32 rsqrt estimate y of r2 by one cubic Newton step:
+//     z = r2 y, e = 1 - z y, 1/r = y (1 + d), r = z (1 + d), d = e/2 + 3 e^2/8;
+//     e^2 < 2^-43 leaves its term to FP32;
+//   * 2^{-t/EXP_N} with t = K r, K = k EXP_N / ln 2 in two doubles: n = rint(t)
+//     from FP32, the remainder f = n - t by fused multiply-adds on z and z d (r
+//     itself is not rounded), and a table of 2^{i/EXP_N}, i < EXP_N, times a cubic
+//     in f, |f| < 0.6 (table lookup and short polynomial: P. T. P. Tang, ACM TOMS
+//     15, 1989); the cubic's upper terms are below 2^-30 and go to FP32;
+//   * conversions between FP32 and FP64 are shifts of the bit patterns.
+// Against 128-bit arithmetic e^{-kr}/r is off by 0.45 ulp rms at kr <= 1 and 1.2
+// at kr <= 16 (sqrt, exp and a division: 0.45 and 2.8).  A squared distance
+// outside FP32's range (zero: a coincident pair; NaN) takes the library
+// functions; e^{-kr} below 2^-1021 counts as 0.
+// Near field, 50k points, split 8: 167 -> 79 ms; the whole one-shot call 177 -> 84 ms.
 // ---------------------------------------------------------------------------
-template <int KERN, bool SS>
-__device__ __forceinline__ double pair_f64(double dx, double dy, double dz, double f, double w,
-                                           double fi, double kp) {
-    double r2 = dx * dx + dy * dy + dz * dz;
-    if (!(r2 > 0.0)) return 0.0;
-    double r = sqrt(r2);
-    if (KERN == KERNEL_YUKAWA) {
-        double g = exp(-kp * r) / r;
-        return SS ? w * (f - fi) * g : w * f * g;
-    } else {
-        if (SS) return w * (f - fi * exp(-kp * kp * r2)) / r;
-        return w * f / r;
+constexpr int EXP_BITS = 13, EXP_N = 1 << EXP_BITS;
+
+// 2^{2^b / EXP_N} as hi + lo
+__constant__ double2 c_exp_step[EXP_BITS] = {
+    {0x1.00058ba01fba0p+0, -0x1.a4a4d4cad39fep-54}, {0x1.000b175effdc7p+0, 0x1.ae8e38c59c72ap-54},
+    {0x1.00162f3904052p+0, -0x1.7b5d0d58ea8f4p-58}, {0x1.002c605e2e8cfp+0, -0x1.d7c96f201bb2fp-55},
+    {0x1.0058c86da1c0ap+0, -0x1.5e00e62d6b30dp-56}, {0x1.00b1afa5abcbfp+0, -0x1.4f6b2a7609f71p-55},
+    {0x1.0163da9fb3335p+0, 0x1.b61299ab8cdb7p-54},  {0x1.02c9a3e778061p+0, -0x1.19083535b085dp-56},
+    {0x1.059b0d3158574p+0, 0x1.d73e2a475b465p-55},  {0x1.0b5586cf9890fp+0, 0x1.8a62e4adc610bp-54},
+    {0x1.172b83c7d517bp+0, -0x1.19041b9d78a76p-55}, {0x1.306fe0a31b715p+0, 0x1.6f46ad23182e4p-55},
+    {0x1.6a09e667f3bcdp+0, -0x1.bdd3413b26456p-54}};
+
+// table[i] = 2^{i / EXP_N}, the product of the steps of i's bits in double-double
+__global__ void exp_table(double *__restrict__ table) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    double h = 1.0, l = 0.0;
+#pragma unroll 1
+    for (int b = 0; b < EXP_BITS; b++) {
+        if (!((i >> b) & 1)) continue;
+        const double2 c = c_exp_step[b];
+        const double p = __dmul_rn(h, c.x);
+        const double e = __fma_rn(l, c.x, __fma_rn(h, c.y, __fma_rn(h, c.x, -p)));
+        h = __dadd_rn(p, e);
+        l = __dadd_rn(e, -__dadd_rn(h, -p));
     }
+    table[i] = h;
+}
+
+// A positive float as a double, by its bits (zero becomes 2^-127).
+__device__ __forceinline__ double bits_f2d(float x) {
+    const unsigned b = __float_as_uint(x);
+    return __hiloint2double((int)((b >> 3) + 0x38000000u), (int)(b << 29));
+}
+// A double in FP32's normal range as a float, truncated (zero becomes +-2).
+__device__ __forceinline__ float bits_d2f(double x) {
+    const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+    const unsigned m = __funnelshift_l(lo, hi & 0x7fffffffu, 3) + 0x40000000u;
+    return __uint_as_float((m & 0x7fffffffu) | (hi & 0x80000000u));
+}
+
+// Parameters of 2^{-t / EXP_N}, t = K x: K = kh + kl.
+struct ExpScale {
+    double kh, kl;
+    float kf;
+};
+// x^e with e = -a x (Yukawa: a = k) or -a^2 x (Coulomb subtraction)
+__device__ __forceinline__ ExpScale exp_scale(double a, bool square) {
+    constexpr double CH = 0x1.71547652b82fep+13, CL = 0x1.777d0ffda0d24p-43;   // EXP_N / ln 2
+    ExpScale s;
+    const double b = square ? __dmul_rn(a, a) : a, be = square ? __fma_rn(a, a, -b) : 0.0;
+    s.kh = __dmul_rn(b, CH);
+    s.kl = __dadd_rn(__fma_rn(b, CH, -s.kh), __fma_rn(b, CL, be * CH));
+    s.kf = (float)s.kh;
+    return s;
+}
+
+struct InvRoot {
+    double z, y, d;   // r = z (1 + d), 1/r = y (1 + d)
+    float zf;         // r in FP32
+};
+__device__ __forceinline__ bool in_fp32_range(double r2) {
+    return (unsigned)__double2hiint(r2) - 0x38100000u < 0x0fd00000u;   // [2^-126, 2^127)
+}
+__device__ __forceinline__ InvRoot inv_root(double r2) {
+    InvRoot q;
+    const float rf = bits_d2f(r2), yf = rsqrt_mufu(rf);
+    q.zf = rf * yf;
+    q.y = bits_f2d(yf);
+    q.z = __dmul_rn(r2, q.y);
+    const double e = __fma_rn(-q.z, q.y, 1.0);
+    const float ef = ((unsigned)__double2hiint(e) << 1) ? bits_d2f(e) : 0.f;
+    q.d = __fma_rn(0.5, e, bits_f2d(0.375f * ef * ef));
+    return q;
+}
+
+constexpr float EXP_LIMIT = 1021.f * EXP_N;
+// 2^{(n - t)/EXP_N} 2^{-n/EXP_N}: tf = t in FP32; the caller forms f = n - t from nd = n.
+__device__ __forceinline__ double exp_n(float tf, int &n) {
+    n = __float2int_rn(fminf(tf, EXP_LIMIT));
+    return bits_f2d((float)n);
+}
+__device__ __forceinline__ double exp_finish(double f, int n, float tf, const double *__restrict__ tab) {
+    constexpr double C1 = 0x1.62e42fefa39efp-14;                       // ln 2 / EXP_N
+    constexpr float C2 = 0x1.ebfbdff82c58fp-29, C3 = 0x1.c6b08d704a0c0p-44;   // C1^2 / 2, C1^3 / 6
+    const double q = __fma_rn(f, bits_f2d(__fmaf_rn(bits_d2f(f), C3, C2)), C1);
+    const double t = tab[-n & (EXP_N - 1)];
+    const double ts = __hiloint2double(__double2hiint(t) + (((-n) >> EXP_BITS) << 20), __double2loint(t));
+    const double v = __fma_rn(ts, __dmul_rn(f, q), ts);
+    return tf < EXP_LIMIT ? v : 0.0;
+}
+// e^{-k r}
+__device__ __forceinline__ double exp_root(const InvRoot &q, const ExpScale &s, const double *__restrict__ tab) {
+    const float tf = q.zf * s.kf;
+    int n;
+    double f = __fma_rn(-s.kh, q.z, exp_n(tf, n));
+    f = __fma_rn(-s.kh, __dmul_rn(q.z, q.d), f);
+    f = __fma_rn(-s.kl, q.z, f);
+    return exp_finish(f, n, tf, tab);
+}
+// e^{-a^2 x}
+__device__ __forceinline__ double exp_square(double x, const ExpScale &s, const double *__restrict__ tab) {
+    const float tf = bits_d2f(x) * s.kf;
+    int n;
+    double f = __fma_rn(-s.kh, x, exp_n(tf, n));
+    f = __fma_rn(-s.kl, x, f);
+    return exp_finish(f, n, tf, tab);
+}
+
+// One pair with the library's functions: r2 outside FP32's range.  q and w are the
+// charge f w and the weight; the near field passes f and w (near: true).
+template <int KERN, bool SS, bool NEAR>
+__device__ __noinline__ double pair_f64_any(double r2, double q, double w, double fi, double kp) {
+    if (NEAR && !(r2 > 0.0)) return 0.0;
+    const double r = sqrt(r2);
+    if (KERN == KERNEL_YUKAWA) {
+        const double g = exp(-kp * r) / r;
+        return SS ? (NEAR ? w * (q - fi) : q - fi * w) * g : q * g;
+    }
+    if (SS) return (NEAR ? w * (q - fi * exp(-kp * kp * r2)) : q - fi * w * exp(-kp * kp * r2)) / r;
+    return q / r;
+}
+template <int KERN, bool SS, bool NEAR>
+__device__ __forceinline__ double pair_f64(double r2, double q, double w, double fi, double kp, const ExpScale &es,
+                                           const double *__restrict__ tab, double acc) {
+    if (!in_fp32_range(r2)) return acc + pair_f64_any<KERN, SS, NEAR>(r2, q, w, fi, kp);
+    const InvRoot v = inv_root(r2);
+    const double rinv = __fma_rn(v.y, v.d, v.y);
+    if (KERN == KERNEL_YUKAWA) {
+        const double c = SS ? (NEAR ? w * (q - fi) : __fma_rn(-fi, w, q)) : q;
+        return __fma_rn(c, __dmul_rn(exp_root(v, es, tab), rinv), acc);
+    }
+    if (SS) {
+        const double e = exp_square(r2, es, tab);
+        const double c = NEAR ? w * __fma_rn(-fi, e, q) : __fma_rn(-fi * w, e, q);
+        return __fma_rn(c, rinv, acc);
+    }
+    return __fma_rn(q, rinv, acc);
+}
+
+// Dynamic shared memory of the FP64 kernels: the exponential table, where used.
+template <int KERN, bool SS>
+constexpr size_t f64_smem() { return KERN == KERNEL_YUKAWA || SS ? sizeof(double) * EXP_N : 0; }
+template <int KERN, bool SS>
+__device__ __forceinline__ void load_exp_table(double *s_tab, const double *__restrict__ table) {
+    if constexpr (KERN == KERNEL_YUKAWA || SS)
+        for (int i = threadIdx.x; i < EXP_N; i += FT) s_tab[i] = table[i];   // read after the item barriers
 }
 
 template <int KERN, bool SS>
 __global__ void __launch_bounds__(FT) near_f64(const __grid_constant__ Work w) {
     constexpr int T64 = 256;
+    extern __shared__ double s_tab[];
     __shared__ double s_x[T64], s_y[T64], s_z[T64], s_f[T64], s_w[T64];
     __shared__ int s_item;
     const int tid = threadIdx.x;
     pass_begin();
+    load_exp_table<KERN, SS>(s_tab, w.exp_table);
     for (;;) {
         const int item = next_item(w.queue, &s_item);
         if (item >= w.nitems) break;
@@ -1666,11 +1821,13 @@ __global__ void __launch_bounds__(FT) near_f64(const __grid_constant__ Work w) {
         const Place pl(a.split);
         const int b = it.x, orb = it.y & 0xffff;
         const double kp = a.kp64[orb];
+        const ExpScale es = exp_scale(kp, KERN == KERNEL_COULOMB);
         const double *f = a.f64 + (long)orb * a.ns;
         const double *ft = a.ft64 + (long)orb * a.nt;
         const int r0 = a.rng_off[b], r1 = a.rng_off[b + 1];
         const int i = it.z + 32 * pl.g + pl.lane;
         const bool v = i < it.w;
+        const bool warp_busy = it.z + 32 * pl.g < it.w;
         const double xi = v ? a.tx[i] : 0.0, yi = v ? a.ty[i] : 0.0, zi = v ? a.tz[i] : 0.0;
         const double fi = v ? ft[i] : 0.0;
         double acc = 0.0;
@@ -1684,13 +1841,16 @@ __global__ void __launch_bounds__(FT) near_f64(const __grid_constant__ Work w) {
                     s_x[tid] = a.sx[jj];
                     s_y[tid] = a.sy[jj];
                     s_z[tid] = a.sz[jj];
-                    s_f[tid] = f[jj];
+                    s_f[tid] = SS ? f[jj] : a.w64[jj] * f[jj];
                     s_w[tid] = a.w64[jj];
                 }
                 __syncthreads();
-                for (int j = pl.sp; j < cnt; j += pl.S)
-                    acc += pair_f64<KERN, SS>(xi - s_x[j], yi - s_y[j], zi - s_z[j], s_f[j],
-                                              s_w[j], fi, kp);
+                if (!warp_busy) continue;
+                for (int j = pl.sp; j < cnt; j += pl.S) {
+                    const double dx = xi - s_x[j], dy = yi - s_y[j], dz = zi - s_z[j];
+                    acc = pair_f64<KERN, SS, true>(dx * dx + dy * dy + dz * dz, s_f[j], s_w[j], fi, kp, es, s_tab,
+                                                   acc);
+                }
             }
         }
         acc = add_splits(acc, pl, s_x);
@@ -1702,11 +1862,13 @@ __global__ void __launch_bounds__(FT) near_f64(const __grid_constant__ Work w) {
 template <int KERN, bool SS, int MAXN1>
 __global__ void __launch_bounds__(FT) far_f64(const __grid_constant__ Work w) {
     constexpr int MAXP = MAXN1 * MAXN1 * MAXN1;
+    extern __shared__ double s_tab[];
     __shared__ double s_q[MAXP], s_wh[MAXP];
     __shared__ double s_p[3][MAXN1], s_red[FT];
     __shared__ int s_item;
     const int tid = threadIdx.x;
     pass_begin();
+    load_exp_table<KERN, SS>(s_tab, w.exp_table);
     for (;;) {
         const int item = next_item(w.queue, &s_item);
         if (item >= w.nitems) break;
@@ -1717,10 +1879,12 @@ __global__ void __launch_bounds__(FT) far_f64(const __grid_constant__ Work w) {
         const int n1 = a.n1, P = a.P;
         const int f0 = a.far_off[b], f1 = a.far_off[b + 1];
         const double kp = a.kp64[orb];
+        const ExpScale es = exp_scale(kp, KERN == KERNEL_COULOMB);
         const double *ft = a.ft64 + (long)orb * a.nt;
         const double *qh = a.qhat64 + (long)orb * a.nslots * P;
         const int i = it.z + 32 * pl.g + pl.lane;
         const bool v = i < it.w;
+        const bool warp_busy = it.z + 32 * pl.g < it.w;
         const double xi = v ? a.tx[i] : 0.0, yi = v ? a.ty[i] : 0.0, zi = v ? a.tz[i] : 0.0;
         const double fi = v ? ft[i] : 0.0;
         double acc = 0.0;
@@ -1737,26 +1901,24 @@ __global__ void __launch_bounds__(FT) far_f64(const __grid_constant__ Work w) {
                 s_p[d][m] = g[d] + g[3 + d] * a.tn[m];
             }
             __syncthreads();
-            for (int k1 = first_slab(e - f0, n1, pl); k1 < n1; k1 += pl.S) {
-                int idx = k1 * n1 * n1;
-                const double dx = xi - s_p[0][k1];
-                for (int k2 = 0; k2 < n1; k2++) {
-                    const double dy = yi - s_p[1][k2];
-                    for (int k3 = 0; k3 < n1; k3++) {
-                        const double dz = zi - s_p[2][k3];
-                        const double r2 = dx * dx + dy * dy + dz * dz;
-                        const double r = sqrt(r2);
-                        const double qk = s_q[idx + k3], wk = s_wh[idx + k3];
-                        if (KERN == KERNEL_YUKAWA) {
-                            acc += exp(-kp * r) / r * (SS ? (qk - fi * wk) : qk);
-                        } else if (SS) {
-                            acc += (qk - fi * wk * exp(-kp * kp * r2)) / r;
-                        } else {
-                            acc += qk / r;
-                        }
-                    }
-                    idx += n1;
-                }
+            if (!warp_busy) continue;
+            // rows (k1, k2) of the grid are dealt to the splits in turn over the clusters
+            const int rows = n1 * n1;
+            double dz2[MAXN1];
+#pragma unroll
+            for (int m = 0; m < MAXN1; m++) {
+                const double dz = zi - s_p[2][m < n1 ? m : 0];
+                dz2[m] = dz * dz;
+            }
+            for (int row = first_slab(e - f0, rows, pl); row < rows; row += pl.S) {
+                const int k1 = row / n1, k2 = row - k1 * n1;
+                const double dx = xi - s_p[0][k1], dy = yi - s_p[1][k2];
+                const double rxy = dx * dx + dy * dy;
+                const double *qr = s_q + row * n1, *wr = s_wh + row * n1;
+#pragma unroll
+                for (int m = 0; m < MAXN1; m++)
+                    if (m < n1)
+                        acc = pair_f64<KERN, SS, false>(rxy + dz2[m], qr[m], wr[m], fi, kp, es, s_tab, acc);
             }
         }
         acc = add_splits(acc, pl, s_red);
@@ -2117,6 +2279,10 @@ int launch_fields(const SysCall *calls, const Fields *f, int nsys, const Schedul
                   int precision, int *queue, cudaStream_t s) {
     Work wn{};
     wn.queue = queue;
+    if (precision != PREC_MIXED && f64_smem<KERN, SS>()) {
+        launch(exp_table, EXP_N / 64, 64, 0, s, calls[0].p->exp_table);
+        wn.exp_table = calls[0].p->exp_table;
+    }
     for (int i = 0; i < nsys; i++) wn.sys[i] = f[i];
     Work wc = wn, wf = wn;
     for (int i = 0; i < nsys; i++) {
@@ -2191,7 +2357,7 @@ int launch_fields(const SysCall *calls, const Fields *f, int nsys, const Schedul
         phase_mark(PH_NEAR_CLOSE, false, s);
     } else {
         // one FP64 pass over all near ranges, close ones included
-        TAGI_TRY(launch_persistent(near_f64<KERN, SS>, wn, s, 0, FT, &pdl));
+        TAGI_TRY(launch_persistent(near_f64<KERN, SS>, wn, s, f64_smem<KERN, SS>(), FT, &pdl));
         phase_mark(PH_NEAR, false, s);
     }
     phase_mark(PH_FAR, true, s);
@@ -2209,9 +2375,9 @@ int launch_fields(const SysCall *calls, const Fields *f, int nsys, const Schedul
             else TAGI_TRY(launch_persistent(far_mixed<KERN, SS, MAX_DEGREE + 1, 2>, wf, s, 0, FT, &pdl));
         }
     } else {
-        if (sh.maxn1 <= 4) TAGI_TRY(launch_persistent(far_f64<KERN, SS, 4>, wf, s, 0, FT, &pdl));
-        else if (sh.maxn1 <= 8) TAGI_TRY(launch_persistent(far_f64<KERN, SS, 8>, wf, s, 0, FT, &pdl));
-        else TAGI_TRY(launch_persistent(far_f64<KERN, SS, MAX_DEGREE + 1>, wf, s, 0, FT, &pdl));
+        if (sh.maxn1 <= 4) TAGI_TRY(launch_persistent(far_f64<KERN, SS, 4>, wf, s, f64_smem<KERN, SS>(), FT, &pdl));
+        else if (sh.maxn1 <= 8) TAGI_TRY(launch_persistent(far_f64<KERN, SS, 8>, wf, s, f64_smem<KERN, SS>(), FT, &pdl));
+        else TAGI_TRY(launch_persistent(far_f64<KERN, SS, MAX_DEGREE + 1>, wf, s, f64_smem<KERN, SS>(), FT, &pdl));
     }
     phase_mark(PH_FAR, false, s);
     return TAGI_OK;
@@ -2329,6 +2495,7 @@ int ensure_scratch(Plan &p, int norb, int precision) {
         take(&p.part, no * p.nitems * p.P);
         take(&p.qhat32, no * p.nslots * p.P, mixed);
         take(&p.qhat64, no * p.nslots * p.P, fp64);
+        take(&p.exp_table, EXP_N, fp64);
         take(&p.near_out, no * nt);
         take(&p.near2_out, no * nt);
         take(&p.far_out, no * nt);

@@ -191,6 +191,7 @@ struct Plan {
     double *part = nullptr;                // upward-pass partials [norb][nitems][P]
     float *qhat32 = nullptr;               // [norb][nslots][P]
     double *qhat64 = nullptr;
+    double *exp_table = nullptr;           // FP64 kernels' 2^{i / N}, written by every FP64 call
     double *near_out = nullptr, *far_out = nullptr;  // [norb][nt] sorted order
     double *near2_out = nullptr;           // close-range pass of the near field
     float *d_kc = nullptr;                 // [norb] exp2 constants
