@@ -146,3 +146,39 @@ def test_training_learns_a_linear_update_map(pkg):
     Y = net.forward(Xt, rows)
     pred = float(net.params["alpha"].item()) * dnt + Y
     assert float(torch.linalg.norm(pred - Tt) / torch.linalg.norm(Tt)) < 0.1
+
+
+# Operands that TMA can read: tiles of 128 x 128 x 64, their edges and remainders, every
+# combination of majors, one and several ranges of K.
+@pytest.mark.parametrize("M,N,K", [(8, 8, 8), (128, 128, 64), (136, 120, 72), (264, 136, 200), (128, 256, 1056),
+                                   (72, 520, 328)])
+@pytest.mark.parametrize("ta,tb", [(False, False), (True, False), (False, True), (True, True)])
+def test_tma_gemm_matches_numpy(L, native, mo, M, N, K, ta, tb):
+    rng = np.random.default_rng(M + N + K)
+    A = mo.bf16(rng.standard_normal((M, K)).astype(np.float32))
+    B = mo.bf16(rng.standard_normal((K, N)).astype(np.float32))
+    At, Bt = _bf(A.T if ta else A), _bf(B.T if tb else B)
+    (sAm, sAk), (sBk, sBn) = (1, M) if ta else (K, 1), (1, K) if tb else (N, 1)
+    ref = A.astype(np.float64) @ B.astype(np.float64)
+    C = torch.zeros(M, N, dtype=torch.float32, device="cuda")
+    native.check(L.tagi_mlp_gemm(_p(At), sAm, sAk, _p(Bt), sBk, sBn, M, N, K, 0, _p(C), None, N, None, None, None))
+    assert rel_l2(C.cpu().numpy(), ref) <= 1e-5
+    for splits in (2, 5):
+        part = torch.full((splits * M * N,), float("nan"), dtype=torch.float32, device="cuda")
+        C2 = torch.zeros_like(C)
+        native.check(L.tagi_mlp_gemm_splitk(_p(At), sAm, sAk, _p(Bt), sBk, sBn, M, N, K, splits, _p(part), _p(C2), None))
+        assert rel_l2(C2.cpu().numpy(), ref) <= 1e-5
+    bias = torch.as_tensor(rng.standard_normal(N).astype(np.float32), device="cuda")
+    ldc = N + 3                                     # rows of C that no vector store can take
+    H = torch.full((M, ldc), 7.0, dtype=torch.bfloat16, device="cuda")
+    native.check(L.tagi_mlp_gemm(_p(At), sAm, sAk, _p(Bt), sBk, sBn, M, N, K, 1, None, _p(H), ldc, _p(bias), None, None))
+    refh = np.maximum(ref + bias.cpu().numpy(), 0)
+    assert rel_l2(H[:, :N].float().cpu().numpy(), refh) <= 1e-2
+    assert torch.all(H[:, N:] == 7.0)
+    Y = torch.zeros(M, N, dtype=torch.float32, device="cuda")
+    native.check(L.tagi_mlp_gemm(_p(At), sAm, sAk, _p(Bt), sBk, sBn, M, N, K, 3, _p(Y), None, N, _p(bias), None, None))
+    assert rel_l2(Y.cpu().numpy(), ref + bias.cpu().numpy()) <= 1e-5
+    mask = torch.as_tensor(rng.standard_normal((M, N)).astype(np.float32)).to(torch.bfloat16).cuda()
+    D = torch.zeros(M, N, dtype=torch.bfloat16, device="cuda")
+    native.check(L.tagi_mlp_gemm(_p(At), sAm, sAk, _p(Bt), sBk, sBn, M, N, K, 2, None, _p(D), N, None, _p(mask), None))
+    assert rel_l2(D.float().cpu().numpy(), ref * (mask.float().cpu().numpy() > 0)) <= 1e-2

@@ -13,13 +13,17 @@
 // MLP: Linear(Din -> H) ReLU Linear(H -> H) ReLU Linear(H -> P), weights BF16
 // (FP32 master copies for Adam), every product accumulated in FP32.
 //
-// GEMMs run on the tensor cores with warp-level mma.sync (m16n8k16, BF16
-// in, FP32 accumulate): C[M x N] = A[M x K] B[K x N] with arbitrary strides,
-// so the transposes of the backward pass need no copies.  Weight gradients
-// split K across blocks into partial sums that a second kernel adds in a
-// fixed order: results do not depend on scheduling.
+// GEMMs run on the tensor cores, BF16 in, FP32 accumulate: C[M x N] =
+// A[M x K] B[K x N] with strides, so the transposes of the backward pass need
+// no copies.  Operands that TMA can read (one unit stride, the other a multiple
+// of 16 bytes, base 16-byte aligned) take gemm_tc (tcgen05, accumulators in
+// TMEM); others, such as rows of 125 or 343 patch points, take gemm_bf16
+// (warp-level mma.sync, element-wise staging).  Weight gradients split K across
+// blocks into partial sums that a second kernel adds in a fixed order: results
+// do not depend on scheduling.
 #include "tagi_internal.h"
 
+#include <cuda.h>
 #include <cuda_bf16.h>
 
 namespace tagi {
@@ -138,6 +142,284 @@ __global__ void __launch_bounds__(GEMM_THREADS) gemm_bf16(const GemmArgs g) {
             }
 }
 
+// ---------------------------------------------------------------------------
+// gemm_tc: one 128 x 128 tile of C per CTA on the 5th-generation tensor cores.
+// Bound: at the extrapolator's sizes (10,752 rows, 256 wide) reading the
+// activations; a K step of 64 moves 32 KB into shared memory for 128 clocks of
+// tcgen05.mma.  So: 128-byte-swizzled TMA tiles in a three-stage ring (96 KB, two
+// CTAs per SM: one's epilogue runs beside the other's loads), one thread issuing
+// the copies, one the MMAs, the accumulator in 128 TMEM columns, and an epilogue
+// through shared memory so that rows of C are written in whole sectors.  A tile
+// of either operand may lie K-major (rows of 64 k) or MN-major (rows of 64 m or n:
+// the weight gradients' transposes); TMA fills elements outside the matrix with 0.
+// 10,752 rows of 512-point patches, hidden width 256: five GEMMs and a column sum
+// 872 -> 157 us (mma.sync with element-wise staging before).
+// ---------------------------------------------------------------------------
+constexpr int TC_M = 128, TC_N = 128, TC_K = 64, TC_STAGES = 3, TC_THREADS = 128;
+constexpr int TC_TILE = 128 * TC_K * 2;                 // bytes of one operand's tile
+constexpr int TC_PITCH = TC_N + 4;                      // floats per staged row of C
+constexpr size_t TC_SMEM = 1024 + (size_t)TC_STAGES * 2 * TC_TILE;
+static_assert((size_t)TC_M * TC_PITCH * 4 <= (size_t)TC_STAGES * 2 * TC_TILE, "C tile in the ring's memory");
+constexpr int TC_SPINS = 1 << 20;                       // tries of a barrier wait before it gives up
+
+__device__ __forceinline__ unsigned smem_u32(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void mbar_init(uint64_t *b, unsigned n) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(b)), "r"(n) : "memory");
+}
+__device__ __forceinline__ void mbar_expect(uint64_t *b, unsigned bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(b)), "r"(bytes) : "memory");
+}
+// false if the phase did not complete within TC_SPINS tries
+__device__ __forceinline__ bool mbar_wait(uint64_t *b, unsigned parity) {
+    for (int i = 0; i < TC_SPINS; i++) {
+        unsigned ok;
+        asm volatile(
+            "{\n.reg .pred p;\n"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+            "selp.u32 %0, 1, 0, p;\n}\n"
+            : "=r"(ok)
+            : "r"(smem_u32(b)), "r"(parity)
+            : "memory");
+        if (ok) return true;
+    }
+    return false;
+}
+__device__ __forceinline__ void tma_load(void *dst, const CUtensorMap *map, int x, int y, uint64_t *bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
+            smem_u32(dst)),
+        "l"(map), "r"(x), "r"(y), "r"(smem_u32(bar))
+        : "memory");
+}
+// Shared-memory matrix descriptor, 128-byte swizzle.  K-major: rows of 64 k,
+// groups of 8 rows 1024 bytes apart.  MN-major: 64 m (or n) per row of one k, 8 k
+// per 1024 bytes, the next 64 m 8192 bytes on.
+__device__ __forceinline__ uint64_t smem_desc(unsigned addr, bool k_major) {
+    const uint64_t lbo = k_major ? 1 : 8192 >> 4, sbo = 1024 >> 4;
+    return (uint64_t)((addr >> 4) & 0x3fff) | lbo << 16 | sbo << 32 | 1ULL << 46 | 2ULL << 61;
+}
+
+struct TcArgs {
+    GemmArgs g;
+    int a_kmajor, b_kmajor;
+};
+
+__device__ int g_tc_timeout;   // set by a CTA whose barrier wait gave up (its tile of C is NaN)
+
+__global__ void __launch_bounds__(TC_THREADS) gemm_tc(const __grid_constant__ CUtensorMap mapA,
+                                                      const __grid_constant__ CUtensorMap mapB,
+                                                      const __grid_constant__ TcArgs t) {
+    extern __shared__ char s_raw[];
+    __shared__ __align__(8) uint64_t s_full[TC_STAGES], s_empty[TC_STAGES], s_done;
+    __shared__ unsigned s_tmem;
+    __shared__ int s_fail;
+    const GemmArgs &g = t.g;
+    char *ring = s_raw + (1024 - (smem_u32(s_raw) & 1023)) % 1024;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int m0 = blockIdx.y * TC_M, n0 = blockIdx.x * TC_N;
+    const int kb = blockIdx.z * g.k_per_split, ke = min(g.K, kb + g.k_per_split);
+    const int steps = (ke - kb + TC_K - 1) / TC_K;
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 128;" ::"r"(smem_u32(&s_tmem))
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    }
+    if (tid == 0) {
+        for (int i = 0; i < TC_STAGES; i++) {
+            mbar_init(&s_full[i], 1);
+            mbar_init(&s_empty[i], 1);
+        }
+        mbar_init(&s_done, 1);
+        s_fail = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const unsigned tmem = s_tmem;
+    if (tid == 0) {   // copies
+        for (int i = 0; i < steps; i++) {
+            const int st = i % TC_STAGES;
+            char *a = ring + st * 2 * TC_TILE, *b = a + TC_TILE;
+            if (i >= TC_STAGES && !mbar_wait(&s_empty[st], (i / TC_STAGES - 1) & 1)) {
+                s_fail = 1;
+                break;
+            }
+            const int k = kb + i * TC_K;
+            mbar_expect(&s_full[st], 2 * TC_TILE);
+            if (t.a_kmajor) {
+                tma_load(a, &mapA, k, m0, &s_full[st]);
+            } else {
+                tma_load(a, &mapA, m0, k, &s_full[st]);
+                tma_load(a + TC_TILE / 2, &mapA, m0 + 64, k, &s_full[st]);
+            }
+            if (t.b_kmajor) {
+                tma_load(b, &mapB, k, n0, &s_full[st]);
+            } else {
+                tma_load(b, &mapB, n0, k, &s_full[st]);
+                tma_load(b + TC_TILE / 2, &mapB, n0 + 64, k, &s_full[st]);
+            }
+        }
+    } else if (tid == 32) {   // MMAs
+        // f32 accumulator, bf16 operands, their majors, N / 8, M / 16
+        const unsigned idesc = 1u << 4 | 1u << 7 | 1u << 10 | (t.a_kmajor ? 0u : 1u << 15) |
+                               (t.b_kmajor ? 0u : 1u << 16) | (unsigned)(TC_N / 8) << 17 | (unsigned)(TC_M / 16) << 24;
+        const unsigned stepA = t.a_kmajor ? 32 >> 4 : 2048 >> 4, stepB = t.b_kmajor ? 32 >> 4 : 2048 >> 4;
+        for (int i = 0; i < steps; i++) {
+            const int st = i % TC_STAGES;
+            if (!mbar_wait(&s_full[st], (i / TC_STAGES) & 1)) {
+                s_fail = 1;
+                break;
+            }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const unsigned a = smem_u32(ring + st * 2 * TC_TILE);
+            uint64_t da = smem_desc(a, t.a_kmajor), db = smem_desc(a + TC_TILE, t.b_kmajor);
+#pragma unroll
+            for (int kk = 0; kk < TC_K / 16; kk++) {
+                const unsigned acc = i > 0 || kk > 0;
+                asm volatile(
+                    "{\n.reg .pred p;\nsetp.ne.u32 p, %4, 0;\n"
+                    "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem),
+                    "l"(da), "l"(db), "r"(idesc), "r"(acc)
+                    : "memory");
+                da += stepA;
+                db += stepB;
+            }
+            asm volatile(
+                "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(&s_empty[st]))
+                : "memory");
+        }
+        asm volatile(
+            "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(&s_done))
+            : "memory");
+    }
+    __syncwarp();
+    bool ok = mbar_wait(&s_done, 0);
+    __syncthreads();
+    ok = ok && !s_fail;
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    if (!ok) {   // give the copies in flight time to land before the memory is reused or left
+        if (tid == 0) {
+            g_tc_timeout = 1;
+            for (int st = 0; st < TC_STAGES; st++) mbar_wait(&s_full[st], 0), mbar_wait(&s_full[st], 1);
+        }
+        __syncthreads();
+    }
+    // accumulator: lane 32 warp + lane of TMEM is row m0 + 32 warp + lane
+    float *crow = reinterpret_cast<float *>(ring) + (32 * warp + lane) * TC_PITCH;
+#pragma unroll
+    for (int c = 0; c < TC_N; c += 32) {
+        unsigned v[32];
+        asm volatile(
+            "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+            "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,"
+            "%29,%30,%31}, [%32];"
+            : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
+              "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]),
+              "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]),
+              "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
+            : "r"(tmem + ((unsigned)(32 * warp) << 16) + c));
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+        for (int q = 0; q < 32; q += 4)
+            *reinterpret_cast<float4 *>(crow + c + q) = make_float4(__uint_as_float(v[q]), __uint_as_float(v[q + 1]),
+                                                                    __uint_as_float(v[q + 2]), __uint_as_float(v[q + 3]));
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 128;" ::"r"(tmem));
+    const float bad = ok ? 0.f : __int_as_float(0x7fffffff);
+    const float *ct = reinterpret_cast<const float *>(ring);
+    const int rows = min(TC_M, g.M - m0), cols = min(TC_N, g.N - n0);
+    if (g.epi == EPI_F32 || g.epi == EPI_BIAS_F32) {   // a warp writes 128 bytes of a row at a time
+        float *C = g.C32 + (long)blockIdx.z * g.M * g.sCm + (long)m0 * g.sCm + n0;
+        for (int c = lane; c < cols; c += 32) {
+            const float bias = (g.epi == EPI_BIAS_F32 ? g.bias[n0 + c] : 0.f) + bad;
+            for (int r = warp; r < rows; r += TC_THREADS / 32) {
+                const float v = ct[r * TC_PITCH + c];
+                C[(long)r * g.sCm + c] = g.epi == EPI_BIAS_F32 ? v + bias : v + bad;
+            }
+        }
+        return;
+    }
+    __nv_bfloat16 *C = g.C16 + (long)m0 * g.sCm + n0;
+    const __nv_bfloat16 *mask = g.epi == EPI_MASK_BF16 ? g.mask + (long)m0 * g.sCm + n0 : nullptr;
+    auto value = [&](int r, int c) {
+        float v = ct[r * TC_PITCH + c] + bad;
+        if (mask) return __float2bfloat16_rn(v * (__bfloat162float(mask[(long)r * g.sCm + c]) > 0.f ? 1.f : 0.f));
+        v += g.bias[n0 + c];
+        return __float2bfloat16_rn(v > 0.f ? v : (v != v ? v : 0.f));
+    };
+    const bool pairs = !(g.sCm & 1) && !(reinterpret_cast<uintptr_t>(C) & 3);
+    for (int r = warp; r < rows; r += TC_THREADS / 32) {
+        if (pairs) {
+            for (int c = 2 * lane; c < cols; c += 64) {
+                if (c + 1 < cols)
+                    *reinterpret_cast<unsigned *>(C + (long)r * g.sCm + c) = pack2(value(r, c), value(r, c + 1));
+                else
+                    C[(long)r * g.sCm + c] = value(r, c);
+            }
+        } else {
+            for (int c = lane; c < cols; c += 32) C[(long)r * g.sCm + c] = value(r, c);
+        }
+    }
+}
+
+typedef CUresult (*EncodeTiled)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
+                                const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
+                                CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+EncodeTiled encode_tiled() {
+    static const EncodeTiled fn = [] {
+        void *p = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &q) != cudaSuccess) {
+            cudaGetLastError();
+            return static_cast<EncodeTiled>(nullptr);
+        }
+        return reinterpret_cast<EncodeTiled>(p);
+    }();
+    return fn;
+}
+
+// Map of an operand with mn rows (or columns) and K: element (i, k) at
+// base[i smn + k sk].  false if TMA cannot read it.
+bool tc_map(CUtensorMap *map, const void *base, long smn, long sk, int mn, int K, int *k_major) {
+    const bool km = sk == 1 && (smn > 1 || mn == 1), mm = !km && smn == 1;
+    if (!km && !mm) return false;
+    const long ld = km ? smn : sk;
+    const int inner = km ? K : mn, outer = km ? mn : K;
+    if (ld < inner || (ld * 2) % 16 || reinterpret_cast<uintptr_t>(base) % 16 || !encode_tiled()) return false;
+    const cuuint64_t dims[2] = {(cuuint64_t)inner, (cuuint64_t)outer}, strides[1] = {(cuuint64_t)ld * 2};
+    const cuuint32_t box[2] = {64, (cuuint32_t)(km ? 128 : 64)}, one[2] = {1, 1};
+    *k_major = km;
+    return encode_tiled()(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void *>(base), dims, strides, box, one,
+                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// One GEMM over `splits` ranges of K (g.k_per_split is set here).
+int run_gemm(GemmArgs g, int splits, int *used, cudaStream_t s) {
+    CUtensorMap ma, mb;
+    TcArgs t;
+    const bool tc = tc_map(&ma, g.A, g.sAm, g.sAk, g.M, g.K, &t.a_kmajor) &&
+                    tc_map(&mb, g.B, g.sBn, g.sBk, g.N, g.K, &t.b_kmajor);
+    const int step = tc ? TC_K : BK;
+    const int kps = ((g.K + splits - 1) / splits + step - 1) / step * step;
+    g.k_per_split = kps;
+    *used = (g.K + kps - 1) / kps;
+    if (tc) {
+        t.g = g;
+        TAGI_CUDA(cudaFuncSetAttribute(gemm_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM));
+        dim3 grid((g.N + TC_N - 1) / TC_N, (g.M + TC_M - 1) / TC_M, *used);
+        launch(gemm_tc, grid, TC_THREADS, TC_SMEM, s, ma, mb, t);
+    } else {
+        dim3 grid((g.N + BN - 1) / BN, (g.M + BM - 1) / BM, *used);
+        launch(gemm_bf16, grid, GEMM_THREADS, 0, s, g);
+    }
+    TAGI_LAUNCH_CHECK();
+    return TAGI_OK;
+}
+
 // out[m][n] = sum over splits of part[s][m][n] (fixed order)
 __global__ void splitk_reduce(const float *__restrict__ part, int splits, long mn, float *__restrict__ out) {
     const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -235,8 +517,10 @@ __global__ void __launch_bounds__(PT) mse_grad(const float *__restrict__ Y, cons
 
 // Column sums of a [rows x N] matrix (bias gradients; f32, or bf16 for the
 // hidden layers' gradients): chunk b of COL_ROWS rows -> part[b][N], then the
-// chunks are added in order.
-constexpr int COL_ROWS = 1024;
+// chunks are added in order.  A block holds 32 columns and COL_GROUPS row
+// groups, whose sums are added in order: one thread per column and 1024 rows was
+// a chain of loads 62 us long at 10,752 rows, 256 columns; the six calls of a step went from 157 to 124 us.
+constexpr int COL_ROWS = 256, COL_GROUPS = 8;
 
 template <typename T>
 __device__ __forceinline__ float to_f(T v);
@@ -245,22 +529,37 @@ __device__ __forceinline__ float to_f<float>(float v) { return v; }
 template <>
 __device__ __forceinline__ float to_f<__nv_bfloat16>(__nv_bfloat16 v) { return __bfloat162float(v); }
 
+// Sums rows r0 + g, r0 + g + COL_GROUPS, ... of column j for this thread's group g,
+// then the groups; valid in group 0.
 template <typename T>
-__global__ void colsum_partial(const T *__restrict__ G, long rows, int N, float *__restrict__ part) {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= N) return;
-    const long r0 = (long)blockIdx.y * COL_ROWS, r1 = min(rows, r0 + COL_ROWS);
+__device__ __forceinline__ float column_sum(const T *__restrict__ G, long r0, long r1, int N, int j) {
+    __shared__ float sh[COL_GROUPS][33];
     float s = 0.f;
-    for (long r = r0; r < r1; r++) s += to_f(G[r * N + j]);
-    part[(long)blockIdx.y * N + j] = s;
+    if (j < N) {
+#pragma unroll 8
+        for (long r = r0 + threadIdx.y; r < r1; r += COL_GROUPS) s += to_f(G[r * N + j]);
+    }
+    sh[threadIdx.y][threadIdx.x] = s;
+    __syncthreads();
+    if (threadIdx.y == 0)
+        for (int g = 1; g < COL_GROUPS; g++) s += sh[g][threadIdx.x];
+    return s;
 }
 
-__global__ void colsum_final(const float *__restrict__ part, int chunks, int N, float *__restrict__ out) {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= N) return;
-    float s = 0.f;
-    for (int b = 0; b < chunks; b++) s += part[(long)b * N + j];
-    out[j] = s;
+template <typename T>
+__global__ void __launch_bounds__(32 * COL_GROUPS) colsum_partial(const T *__restrict__ G, long rows, int N,
+                                                                  float *__restrict__ part) {
+    const int j = blockIdx.y * 32 + threadIdx.x;
+    const long r0 = (long)blockIdx.x * COL_ROWS;
+    const float s = column_sum(G, r0, min(rows, r0 + COL_ROWS), N, j);
+    if (threadIdx.y == 0 && j < N) part[(long)blockIdx.x * N + j] = s;
+}
+
+__global__ void __launch_bounds__(32 * COL_GROUPS) colsum_final(const float *__restrict__ part, int chunks, int N,
+                                                                float *__restrict__ out) {
+    const int j = blockIdx.x * 32 + threadIdx.x;
+    const float s = column_sum(part, 0, chunks, N, j);
+    if (threadIdx.y == 0 && j < N) out[j] = s;
 }
 
 // loss and dalpha from the per-row partials: thread t adds rows t, t + 256,
@@ -359,17 +658,14 @@ int tagi_mlp_gemm(const void *A, long long sAm, long long sAk, const void *B, lo
     g.M = M;
     g.N = N;
     g.K = K;
-    g.k_per_split = ((K + BK - 1) / BK) * BK;
     g.C32 = C32;
     g.C16 = static_cast<__nv_bfloat16 *>(C16);
     g.sCm = ldc;
     g.bias = bias;
     g.mask = static_cast<const __nv_bfloat16 *>(mask);
     g.epi = epilogue;
-    dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM, 1);
-    launch(gemm_bf16, grid, GEMM_THREADS, 0, (cudaStream_t)stream, g);
-    TAGI_LAUNCH_CHECK();
-    return TAGI_OK;
+    int used = 1;
+    return run_gemm(g, 1, &used, (cudaStream_t)stream);
 }
 
 // f32 C = A B with K split over `splits` blocks; `partial` holds
@@ -388,10 +684,6 @@ int tagi_mlp_gemm_splitk(const void *A, long long sAm, long long sAk, const void
     g.M = M;
     g.N = N;
     g.K = K;
-    int kps = (K + splits - 1) / splits;
-    kps = ((kps + BK - 1) / BK) * BK;
-    splits = (K + kps - 1) / kps;
-    g.k_per_split = kps;
     g.C32 = partial;
     g.C16 = nullptr;
     g.sCm = N;
@@ -399,8 +691,7 @@ int tagi_mlp_gemm_splitk(const void *A, long long sAm, long long sAk, const void
     g.mask = nullptr;
     g.epi = EPI_F32;
     cudaStream_t s = (cudaStream_t)stream;
-    dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM, splits);
-    launch(gemm_bf16, grid, GEMM_THREADS, 0, s, g);
+    TAGI_TRY(run_gemm(g, splits, &splits, s));
     const long mn = (long)M * N;
     launch(splitk_reduce, (unsigned)((mn + 255) / 256), 256, 0, s, partial, splits, mn, C);
     TAGI_LAUNCH_CHECK();
@@ -450,13 +741,12 @@ int tagi_mlp_colsum(const void *G, int isBf16, long long rows, int N, float *out
     if (workFloats < tagi_mlp_colsum_workspace(rows, N)) return set_error(TAGI_ERR_ARG, "workspace too small");
     cudaStream_t s = (cudaStream_t)stream;
     const int chunks = (int)((rows + COL_ROWS - 1) / COL_ROWS);
-    dim3 g((N + 127) / 128, chunks);
+    const dim3 g(chunks, (N + 31) / 32), t(32, COL_GROUPS);
     if (isBf16)
-        launch(colsum_partial<__nv_bfloat16>, g, 128, 0, s, static_cast<const __nv_bfloat16 *>(G), (long)rows, N,
-               work);
+        launch(colsum_partial<__nv_bfloat16>, g, t, 0, s, static_cast<const __nv_bfloat16 *>(G), (long)rows, N, work);
     else
-        launch(colsum_partial<float>, g, 128, 0, s, static_cast<const float *>(G), (long)rows, N, work);
-    launch(colsum_final, (N + 127) / 128, 128, 0, s, work, chunks, N, out);
+        launch(colsum_partial<float>, g, t, 0, s, static_cast<const float *>(G), (long)rows, N, work);
+    launch(colsum_final, (N + 31) / 32, t, 0, s, work, chunks, N, out);
     TAGI_LAUNCH_CHECK();
     return TAGI_OK;
 }

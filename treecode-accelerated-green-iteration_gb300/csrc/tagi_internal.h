@@ -65,6 +65,32 @@ inline void launch(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, c
     kern<<<grid, block, smem, s>>>(std::forward<Args>(args)...);
 }
 
+// launch() of a kernel that may start before the kernel ahead of it in the stream
+// has ended (programmatic dependent launch): it calls chain_begin() before it
+// touches anything an earlier kernel wrote or reads, which waits for that kernel
+// and its writes, so only its launch latency overlaps.
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_chained(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
+                                  Args &&...args) {
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    count_launch();
+    return cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
+}
+#ifdef __CUDACC__
+__device__ __forceinline__ void chain_begin() {
+    asm volatile("griddepcontrol.launch_dependents;\ngriddepcontrol.wait;" ::: "memory");
+}
+#endif
+
 // Merged near ranges are int2 {begin, end} in sorted source order; bit 31 of
 // begin marks a CLOSE range: its box lies within 0.1 batch radii of the
 // batch's box (touching included).  Close ranges hold the short pairs whose
