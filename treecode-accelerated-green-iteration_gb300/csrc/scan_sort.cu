@@ -66,7 +66,42 @@ __global__ void add_tile_offsets(int *__restrict__ out, int n, const int *__rest
     }
 }
 
-__global__ void copy_one(const int *src, int *dst) { *dst = *src; }
+// Exclusive scan by one block, a tile at a time, total included: up to SCAN_SMALL
+// elements one launch is quicker than tiles, their sums and the offsets (5,104
+// cells: 4 launches of 2-3 us each before).
+constexpr int SCAN_SMALL = 4 * SCAN_TILE;
+__global__ void __launch_bounds__(SCAN_THREADS) scan_small(const int *__restrict__ in, int *__restrict__ out, int n,
+                                                           int *__restrict__ total) {
+    __shared__ int warp_tot[SCAN_THREADS / 32];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    int carry = 0;
+    for (int base = 0; base < n; base += SCAN_TILE) {
+        int v[SCAN_ITEMS], tsum = 0;
+#pragma unroll
+        for (int k = 0; k < SCAN_ITEMS; k++) {
+            const int i = base + threadIdx.x * SCAN_ITEMS + k;
+            v[k] = i < n ? in[i] : 0;
+            tsum += v[k];
+        }
+        const int incl = warp_incl_scan(tsum);
+        __syncthreads();   // the previous tile's warp totals are no longer read
+        if (lane == 31) warp_tot[wid] = incl;
+        __syncthreads();
+        int before = 0, all = 0;
+        const int wt = warp_tot[lane], ws = warp_incl_scan(wt);
+        all = __shfl_sync(0xffffffffu, ws, 31);
+        before = __shfl_sync(0xffffffffu, ws - wt, wid);
+        int run = carry + before + incl - tsum;
+#pragma unroll
+        for (int k = 0; k < SCAN_ITEMS; k++) {
+            const int i = base + threadIdx.x * SCAN_ITEMS + k;
+            if (i < n) out[i] = run;
+            run += v[k];
+        }
+        carry += all;
+    }
+    if (total && threadIdx.x == 0) *total = carry;
+}
 
 }  // namespace
 
@@ -75,16 +110,16 @@ int exclusive_scan(const int *in, int *out, int n, int *d_total, Arena &ar, cuda
         if (d_total) TAGI_CUDA(cudaMemsetAsync(d_total, 0, sizeof(int), s));
         return TAGI_OK;
     }
+    if (n <= SCAN_SMALL) {
+        launch(scan_small, 1, SCAN_THREADS, 0, s, in, out, n, d_total);
+        TAGI_LAUNCH_CHECK();
+        return TAGI_OK;
+    }
     int nb = (n + SCAN_TILE - 1) / SCAN_TILE;
     int *sums = nullptr;
     TAGI_TRY(ar.alloc(&sums, nb + 1));
     launch(scan_tiles, nb, SCAN_THREADS, 0, s, in, out, n, sums);
     TAGI_LAUNCH_CHECK();
-    if (nb == 1) {
-        if (d_total) launch(copy_one, 1, 1, 0, s, sums, d_total);
-        TAGI_LAUNCH_CHECK();
-        return TAGI_OK;
-    }
     int *offs = nullptr;
     TAGI_TRY(ar.alloc(&offs, nb));
     TAGI_TRY(exclusive_scan(sums, offs, nb, d_total, ar, s));
@@ -164,10 +199,59 @@ __global__ void __launch_bounds__(RS_THREADS) rs_scatter(const uint64_t *__restr
     }
 }
 
+// Up to SORT_SMALL pairs in one block's shared memory: a bitonic network on (key,
+// position), so equal keys keep their order.  One launch of about 10 us where the
+// radix passes are 40 launches.
+constexpr int SORT_SMALL = 8192, SORT_THREADS = 1024;
+__global__ void __launch_bounds__(SORT_THREADS) sort_small(uint64_t *__restrict__ keys, int *__restrict__ vals, int n,
+                                                           int m) {   // m: power of two >= n
+    extern __shared__ uint64_t s_key[];
+    int *s_val = reinterpret_cast<int *>(s_key + m);
+    short *s_pos = reinterpret_cast<short *>(s_val + m);
+    for (int i = threadIdx.x; i < m; i += SORT_THREADS) {
+        s_key[i] = i < n ? keys[i] : ~0ULL;
+        s_val[i] = i < n ? vals[i] : 0;
+        s_pos[i] = (short)i;   // padding sorts after every pair: its positions are the last
+    }
+    for (int k = 2; k <= m; k <<= 1)
+        for (int j = k >> 1; j > 0; j >>= 1) {
+            __syncthreads();
+            for (int t = threadIdx.x; t < m / 2; t += SORT_THREADS) {
+                const int a = 2 * t - (t & (j - 1)), b = a + j;
+                const uint64_t ka = s_key[a], kb = s_key[b];
+                const short pa = s_pos[a], pb = s_pos[b];
+                const bool up = (a & k) == 0, greater = ka > kb || (ka == kb && pa > pb);
+                if (greater == up) {
+                    const int va = s_val[a];
+                    s_key[a] = kb;
+                    s_key[b] = ka;
+                    s_pos[a] = pb;
+                    s_pos[b] = pa;
+                    s_val[a] = s_val[b];
+                    s_val[b] = va;
+                }
+            }
+        }
+    __syncthreads();
+    for (int i = threadIdx.x; i < n; i += SORT_THREADS) {
+        keys[i] = s_key[i];
+        vals[i] = s_val[i];
+    }
+}
+
 }  // namespace
 
 int radix_sort_u64(uint64_t *keys, int *vals, int n, Arena &ar, cudaStream_t s) {
     if (n <= 1) return TAGI_OK;
+    if (n <= SORT_SMALL) {
+        int m = 2;
+        while (m < n) m <<= 1;
+        const size_t smem = (size_t)m * (sizeof(uint64_t) + sizeof(int) + sizeof(short));
+        TAGI_CUDA(cudaFuncSetAttribute(sort_small, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        launch(sort_small, 1, SORT_THREADS, smem, s, keys, vals, n, m);
+        TAGI_LAUNCH_CHECK();
+        return TAGI_OK;
+    }
     int nb = (n + RS_TILE - 1) / RS_TILE;
     uint64_t *k2 = nullptr;
     int *v2 = nullptr, *hist = nullptr, *offs = nullptr;

@@ -100,22 +100,25 @@ def refine_cells(base, atoms, order, h, H, r, level, min_depth=0, max_depth=16, 
     atoms_d = torch.as_tensor(np.asarray(atoms, np.float64).reshape(-1, 3) if not torch.is_tensor(atoms) else atoms,
                               dtype=torch.float64, device=device).contiguous()
     nb, na = base_d.shape[0], atoms_d.shape[0]
-    if stream is not None:
-        stream.wait_stream(torch.cuda.current_stream())  # base_d / atoms_d were made there
     ncell, ncp, nfp = ctypes.c_int(0), ctypes.c_longlong(0), ctypes.c_longlong(0)
     args = (_dev(base_d, "base"), nb, _dev(atoms_d, "atoms") if na else ctypes.c_void_p(0), na, int(order),
             float(h), float(H), float(r), float(level), int(min_depth), int(max_depth))
     s = _stream(stream)
-    null = [ctypes.c_void_p(0)] * 8
-    _native.check(L.tagi_mesh_refine(*args, *null, 0, ctypes.byref(ncell), ctypes.byref(ncp), ctypes.byref(nfp), s))
-    n = ncell.value
-    f64 = dict(dtype=torch.float64, device=device)
-    cells = [torch.empty(n, **f64) for _ in range(6)]
-    ppc_c = torch.empty(n, dtype=torch.int32, device=device)
-    ppc_f = torch.empty(n, dtype=torch.int32, device=device)
-    outs = [_dev(c, "cell") for c in cells] + [_dev(ppc_c, "ppc_c", torch.int32), _dev(ppc_f, "ppc_f", torch.int32)]
-    _native.check(L.tagi_mesh_refine(*args, *outs, n, ctypes.byref(ncell), ctypes.byref(ncp), ctypes.byref(nfp), s))
-    return cells, ppc_c, ppc_f, int(nfp.value)
+    # room for the usual cell count first; a mesh with more cells says how many and runs again
+    room = max(16384, 16 * nb)
+    while True:
+        f64 = torch.empty((6, room), dtype=torch.float64, device=device)
+        i32 = torch.empty((2, room), dtype=torch.int32, device=device)
+        if stream is not None:
+            stream.wait_stream(torch.cuda.current_stream())  # the table's memory was given out there
+        outs = [ctypes.c_void_p(t.data_ptr()) for t in (*f64, *i32)]
+        rc = L.tagi_mesh_refine(*args, *outs, room, ctypes.byref(ncell), ctypes.byref(ncp), ctypes.byref(nfp), s)
+        n = ncell.value
+        if rc and n > room:
+            room = n
+            continue
+        _native.check(rc)
+        return [t[:n] for t in f64], i32[0][:n], i32[1][:n], int(nfp.value)
 
 
 def mesh_points(cells, ppc_f, order, num_fine=None, tables=None, device="cuda", stream=None):
