@@ -30,7 +30,6 @@ enum { COMPUTE_PARTICLE_CLUSTER = 1 };
 enum { PREC_MIXED = 0, PREC_FP64 = 1 };
 
 constexpr int MAX_DEGREE = 10;        // far-field kernels are instantiated for 1..10
-constexpr int TRAVERSAL_STACK = 256;  // DFS stack entries per target batch
 
 int set_error(int code, const char *fmt, ...);
 int last_error();
@@ -137,6 +136,13 @@ struct Arena {
     }
 };
 
+// A tree node in pre-order: center, radius, the index after its subtree, its
+// points, whether it is a leaf, and its number.
+struct PreNode {
+    double x, y, z, r;
+    int stop, count, leaf, node;
+};
+
 struct Tree {
     int n = 0;
     int nnodes = 0;
@@ -148,6 +154,9 @@ struct Tree {
     int *begin = nullptr, *end = nullptr, *parent = nullptr, *first_child = nullptr,
         *nchild = nullptr;
     double *center = nullptr, *half = nullptr, *radius = nullptr;
+    PreNode *pre = nullptr;        // nodes in pre-order
+    int *leaf_node = nullptr;      // leaves in Morton order
+    int nleaves = 0;
 };
 
 // Work list of one field launch: items {batch, sys << 16 | first orbital,

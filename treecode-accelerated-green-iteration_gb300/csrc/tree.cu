@@ -210,57 +210,198 @@ __global__ void fill_children(const uint64_t *__restrict__ codes, int *__restric
     }
 }
 
-// One warp per node of a level; children (deeper level) are already done.
-__global__ void node_boxes(int ls, int le, const int *__restrict__ begin,
-                           const int *__restrict__ end, const int *__restrict__ first_child,
-                           const int *__restrict__ nchild, const double *__restrict__ x,
-                           const double *__restrict__ y, const double *__restrict__ z,
-                           double *__restrict__ box, double *__restrict__ center,
-                           double *__restrict__ half, double *__restrict__ radius) {
-    int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    int lane = threadIdx.x & 31;
-    int v = ls + warp;
-    if (v >= le) return;
-    double l[3] = {INFINITY, INFINITY, INFINITY}, h[3] = {-INFINITY, -INFINITY, -INFINITY};
-    int nc = nchild[v];
-    if (nc == 0) {
-        for (int i = begin[v] + lane; i < end[v]; i += 32) {
-            double p[3] = {x[i], y[i], z[i]};
+// Node header on the device: [0] nodes, [1] levels, [2 + l] first node of level l
+// (and, after the last level, the node count).
+constexpr int MAX_LEVELS = 23;   // 21 digits split at most
+constexpr int HDR = MAX_LEVELS + 3;
+
+// The whole octree by one block, a level at a time: eight threads per node find
+// the starts of its eight digits by binary search, so a round of 128 nodes is one
+// search deep, and nothing waits for the host between levels.  Meshes have a few
+// thousand nodes: 1.5M points, leaves of 2000: 8 levels, count + fill + scan
+// launches and a synchronisation each, 1.35 -> 0.78 ms for the tree and its sort.  Above
+// SMALL_TREE leaves' worth of points one launch per level is quicker.
+constexpr int SMALL_TREE = 4096;
+constexpr int BUILD_THREADS = 1024;
+__global__ void __launch_bounds__(BUILD_THREADS) build_nodes(const uint64_t *__restrict__ codes, int n, int leaf,
+                                                             int *__restrict__ begin, int *__restrict__ end,
+                                                             int *__restrict__ parent, int *__restrict__ first_child,
+                                                             int *__restrict__ nchild, int *__restrict__ hdr) {
+    __shared__ int s_cnt[BUILD_THREADS / 32];
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, digit = tid & 7;
+    if (tid == 0) {
+        begin[0] = 0;
+        end[0] = n;
+        parent[0] = -1;
+    }
+    __syncthreads();
+    int ls = 0, le = 1, level = 0;
+    for (;; level++) {
+        if (tid == 0) hdr[2 + level] = ls;
+        int next = le;
+        for (int base = ls; base < le; base += BUILD_THREADS / 8) {
+            const int v = base + (tid >> 3);
+            int b = 0, e = 0, sh = -1, lo = 0;
+            if (v < le) {
+                b = begin[v];
+                e = end[v];
+                if (e - b > leaf) sh = split_shift(codes, b, e);
+            }
+            if (sh >= 0) {   // first index in [b, e) whose digit is >= this thread's
+                const uint64_t key = ((codes[b] >> (sh + 3)) << 3) | (uint64_t)digit;
+                int hi = e;
+                lo = b;
+                while (lo < hi) {
+                    const int mid = lo + ((hi - lo) >> 1);
+                    if ((codes[mid] >> sh) >= key) hi = mid;
+                    else lo = mid + 1;
+                }
+            }
+            int to = __shfl_down_sync(0xffffffffu, lo, 1, 8);
+            if (digit == 7) to = e;
+            const bool child = sh >= 0 && to > lo;
+            const unsigned m = __ballot_sync(0xffffffffu, child);
+            __syncthreads();   // s_cnt of the previous round is no longer read
+            if (lane == 0) s_cnt[wid] = __popc(m);
+            __syncthreads();
+            int before = 0, all = 0;
+            for (int w = 0; w < BUILD_THREADS / 32; w++) {
+                if (w < wid) before += s_cnt[w];
+                all += s_cnt[w];
+            }
+            const int at = next + before + __popc(m & ((1u << lane) - 1u));
+            if (child) {
+                begin[at] = lo;
+                end[at] = to;
+                parent[at] = v;
+            }
+            if (digit == 0 && v < le) {
+                const int c = __popc((m >> lane) & 0xffu);
+                nchild[v] = c;
+                first_child[v] = c ? at : -1;
+            }
+            next += all;
+        }
+        __syncthreads();   // the new level's begin, end are written
+        if (next == le) break;
+        ls = le;
+        le = next;
+    }
+    if (tid == 0) {
+        hdr[3 + level] = le;
+        hdr[0] = le;
+        hdr[1] = level + 1;
+    }
+}
+
+__global__ void write_header(int *hdr, int nnodes) { hdr[0] = nnodes; }
+
+// Boxes of all nodes in one launch, with the nodes and leaves of each subtree: a
+// warp does a leaf, and the warp that finishes a node's last child goes on with
+// the node.
+__global__ void __launch_bounds__(256) node_boxes(const int *__restrict__ hdr, const int *__restrict__ begin,
+                                                  const int *__restrict__ end, const int *__restrict__ parent,
+                                                  const int *__restrict__ first_child, const int *__restrict__ nchild,
+                                                  const double *__restrict__ x, const double *__restrict__ y,
+                                                  const double *__restrict__ z, double *box, double *__restrict__ center,
+                                                  double *__restrict__ half, double *__restrict__ radius, int *size,
+                                                  int *leaves, int *done) {
+    const int nn = hdr[0], lane = threadIdx.x & 31;
+    for (int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < nn; w += (gridDim.x * blockDim.x) >> 5) {
+        if (nchild[w]) continue;
+        double l[3] = {INFINITY, INFINITY, INFINITY}, h[3] = {-INFINITY, -INFINITY, -INFINITY};
+        int sz = 0, lv = 0;   // of the children (lane 0's own start below)
+        for (int i = begin[w] + lane; i < end[w]; i += 32) {
+            const double p[3] = {x[i], y[i], z[i]};
 #pragma unroll
             for (int d = 0; d < 3; d++) {
                 l[d] = dmin(l[d], p[d]);
                 h[d] = dmax(h[d], p[d]);
             }
         }
-    } else if (lane < nc) {
-        const double *cb = box + 6L * (first_child[v] + lane);
+        for (int v = w;;) {
 #pragma unroll
-        for (int d = 0; d < 3; d++) {
-            l[d] = cb[d];
-            h[d] = cb[3 + d];
+            for (int o = 16; o > 0; o >>= 1) {
+#pragma unroll
+                for (int d = 0; d < 3; d++) {
+                    l[d] = dmin(l[d], __shfl_xor_sync(0xffffffffu, l[d], o));
+                    h[d] = dmax(h[d], __shfl_xor_sync(0xffffffffu, h[d], o));
+                }
+                sz += __shfl_xor_sync(0xffffffffu, sz, o);
+                lv += __shfl_xor_sync(0xffffffffu, lv, o);
+            }
+            int last = 0;
+            const int pv = parent[v];
+            if (lane == 0) {
+                double hh[3];
+#pragma unroll
+                for (int d = 0; d < 3; d++) {
+                    __stcg(box + 6L * v + d, l[d]);
+                    __stcg(box + 6L * v + 3 + d, h[d]);
+                    center[3L * v + d] = __dmul_rn(__dadd_rn(l[d], h[d]), 0.5);
+                    hh[d] = __dmul_rn(__dsub_rn(h[d], l[d]), 0.5);
+                    half[3L * v + d] = hh[d];
+                }
+                double s = __dmul_rn(hh[0], hh[0]);
+                s = __dadd_rn(s, __dmul_rn(hh[1], hh[1]));
+                s = __dadd_rn(s, __dmul_rn(hh[2], hh[2]));
+                radius[v] = __dsqrt_rn(s);
+                __stcg(size + v, sz + 1);
+                __stcg(leaves + v, v == w ? 1 : lv);
+                if (pv >= 0) {
+                    __threadfence();
+                    last = atomicAdd(done + pv, 1) == nchild[pv] - 1;
+                    __threadfence();
+                }
+            }
+            if (!__shfl_sync(0xffffffffu, last, 0)) break;
+            __syncwarp();   // the other lanes' reads come after lane 0's fence
+            v = pv;
+            const int c = first_child[v] + lane;
+            const bool has = lane < nchild[v];
+#pragma unroll
+            for (int d = 0; d < 3; d++) {
+                l[d] = has ? __ldcg(box + 6L * c + d) : INFINITY;
+                h[d] = has ? __ldcg(box + 6L * c + 3 + d) : -INFINITY;
+            }
+            sz = has ? __ldcg(size + c) : 0;
+            lv = has ? __ldcg(leaves + c) : 0;
         }
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-        for (int d = 0; d < 3; d++) {
-            l[d] = dmin(l[d], __shfl_xor_sync(0xffffffffu, l[d], o));
-            h[d] = dmax(h[d], __shfl_xor_sync(0xffffffffu, h[d], o));
+}
+
+// Each node's place in pre-order (children in digit order) and each leaf's among
+// the leaves, from the subtrees passed on the way to the root.
+__global__ void preorder(const int *__restrict__ hdr, const int *__restrict__ begin, const int *__restrict__ end,
+                         const int *__restrict__ parent, const int *__restrict__ first_child,
+                         const int *__restrict__ nchild, const double *__restrict__ center,
+                         const double *__restrict__ radius, const int *__restrict__ size,
+                         const int *__restrict__ leaves, PreNode *__restrict__ pre, int *__restrict__ leaf_node,
+                         int *__restrict__ nleaves) {
+    const int nn = hdr[0];
+    for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < nn; v += gridDim.x * blockDim.x) {
+        int pos = 0, rank = 0;
+        for (int c = v; c != 0;) {
+            const int p = parent[c];
+            pos++;
+            for (int k = first_child[p]; k < c; k++) {
+                pos += size[k];
+                rank += leaves[k];
+            }
+            c = p;
         }
-    if (lane == 0) {
-        double hh[3];
-#pragma unroll
-        for (int d = 0; d < 3; d++) {
-            box[6L * v + d] = l[d];
-            box[6L * v + 3 + d] = h[d];
-            center[3L * v + d] = __dmul_rn(__dadd_rn(l[d], h[d]), 0.5);
-            hh[d] = __dmul_rn(__dsub_rn(h[d], l[d]), 0.5);
-            half[3L * v + d] = hh[d];
-        }
-        double s = __dmul_rn(hh[0], hh[0]);
-        s = __dadd_rn(s, __dmul_rn(hh[1], hh[1]));
-        s = __dadd_rn(s, __dmul_rn(hh[2], hh[2]));
-        radius[v] = __dsqrt_rn(s);
+        PreNode q;
+        q.x = center[3L * v];
+        q.y = center[3L * v + 1];
+        q.z = center[3L * v + 2];
+        q.r = radius[v];
+        q.node = v;
+        q.stop = pos + size[v];
+        q.count = end[v] - begin[v];
+        q.leaf = nchild[v] == 0;
+        pre[pos] = q;
+        if (q.leaf) leaf_node[rank] = v;
+        if (v == 0) *nleaves = leaves[0];
     }
 }
 
@@ -294,51 +435,76 @@ int build_tree(Tree &t, const double *x, const double *y, const double *z, int n
         if ((rc = ar.alloc(&t.x, n)) || (rc = ar.alloc(&t.y, n)) || (rc = ar.alloc(&t.z, n))) break;
         launch(gather3, (n + 255) / 256, 256, 0, s, x, y, z, t.perm, n, t.x, t.y, t.z);
 
-        const long cap = 2L * n + 1;
+        // internal nodes hold more than leaf points, n / leaf of them per level at most
+        const bool small = n / leaf <= SMALL_TREE;
+        const long cap = std::min(2L * n + 1, small ? 8L * 21 * (n / leaf) + 9 : 2L * n + 1);
         if ((rc = ar.alloc(&t.begin, cap)) || (rc = ar.alloc(&t.end, cap)) ||
             (rc = ar.alloc(&t.parent, cap)) || (rc = ar.alloc(&t.first_child, cap)) ||
             (rc = ar.alloc(&t.nchild, cap)))
             break;
-        int *cc = nullptr, *off = nullptr, *total = nullptr;
-        if ((rc = tmp.alloc(&cc, cap)) || (rc = tmp.alloc(&off, cap)) || (rc = tmp.alloc(&total, 1)))
-            break;
-        launch(init_root, 1, 1, 0, s, t.begin, t.end, t.parent, n);
+        int *hdr = nullptr, *nleaves = nullptr;
+        if ((rc = tmp.alloc(&hdr, HDR + 1))) break;
+        nleaves = hdr + HDR;
         t.level_start.assign(1, 0);
-        int ls = 0, le = 1;
-        while (ls < le) {
-            int m = le - ls;
-            launch(count_children, (m + 127) / 128, 128, 0, s, t.codes, t.begin, t.end, ls, le, leaf, cc);
-            if ((rc = exclusive_scan(cc, off, m, total, tmp, s))) break;
-            launch(fill_children, (m + 127) / 128, 128, 0, s, t.codes, t.begin, t.end, t.parent,
-                                                          t.first_child, t.nchild, ls, le, cc, off);
-            int h_total = 0;
-            if (cudaMemcpyAsync(&h_total, total, sizeof(int), cudaMemcpyDeviceToHost, s) !=
-                    cudaSuccess ||
-                cudaStreamSynchronize(s) != cudaSuccess) {
-                rc = set_error(TAGI_ERR_CUDA, "tree level build: %s",
-                               cudaGetErrorString(cudaGetLastError()));
+        if (small) {
+            launch(build_nodes, 1, BUILD_THREADS, 0, s, t.codes, n, leaf, t.begin, t.end, t.parent, t.first_child,
+                   t.nchild, hdr);
+        } else {
+            int *cc = nullptr, *off = nullptr, *total = nullptr;
+            if ((rc = tmp.alloc(&cc, cap)) || (rc = tmp.alloc(&off, cap)) || (rc = tmp.alloc(&total, 1)))
                 break;
+            launch(init_root, 1, 1, 0, s, t.begin, t.end, t.parent, n);
+            int ls = 0, le = 1;
+            while (ls < le) {
+                int m = le - ls;
+                launch(count_children, (m + 127) / 128, 128, 0, s, t.codes, t.begin, t.end, ls, le, leaf, cc);
+                if ((rc = exclusive_scan(cc, off, m, total, tmp, s))) break;
+                launch(fill_children, (m + 127) / 128, 128, 0, s, t.codes, t.begin, t.end, t.parent, t.first_child,
+                       t.nchild, ls, le, cc, off);
+                int h_total = 0;
+                if (cudaMemcpyAsync(&h_total, total, sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+                    cudaStreamSynchronize(s) != cudaSuccess) {
+                    rc = set_error(TAGI_ERR_CUDA, "tree level build: %s", cudaGetErrorString(cudaGetLastError()));
+                    break;
+                }
+                if (le + (long)h_total > cap) { rc = set_error(TAGI_ERR_DEVICE, "tree node capacity exceeded"); break; }
+                ls = le;
+                le += h_total;
+                t.level_start.push_back(ls);
             }
-            if (le + (long)h_total > cap) { rc = set_error(TAGI_ERR_DEVICE, "tree node capacity exceeded"); break; }
-            ls = le;
-            le += h_total;
-            t.level_start.push_back(ls);
+            if (rc) break;
+            t.nnodes = le;
+            launch(write_header, 1, 1, 0, s, hdr, t.nnodes);
         }
-        if (rc) break;
-        t.nnodes = le;
-        t.nlevels = (int)t.level_start.size() - 1;
+        const long nodes = small ? cap : t.nnodes;
         double *box = nullptr;
-        if ((rc = tmp.alloc(&box, 6L * t.nnodes))) break;
-        if ((rc = ar.alloc(&t.center, 3L * t.nnodes)) || (rc = ar.alloc(&t.half, 3L * t.nnodes)) ||
-            (rc = ar.alloc(&t.radius, t.nnodes)))
+        int *work = nullptr;
+        if ((rc = tmp.alloc(&box, 6 * nodes)) || (rc = tmp.alloc(&work, 3 * nodes)) ||
+            (rc = ar.alloc(&t.center, 3 * nodes)) || (rc = ar.alloc(&t.half, 3 * nodes)) ||
+            (rc = ar.alloc(&t.radius, nodes)) || (rc = ar.alloc(&t.pre, nodes)) || (rc = ar.alloc(&t.leaf_node, nodes)))
             break;
-        for (int lv = t.nlevels - 1; lv >= 0; lv--) {
-            int a = t.level_start[lv], b = t.level_start[lv + 1];
-            int warps = b - a;
-            launch(node_boxes, (warps * 32 + 255) / 256, 256, 0, s, a, b, t.begin, t.end, t.first_child,
-                                                                t.nchild, t.x, t.y, t.z, box,
-                                                                t.center, t.half, t.radius);
+        int *size = work, *leaves = work + nodes, *done = work + 2 * nodes;
+        if (cudaMemsetAsync(done, 0, sizeof(int) * nodes, s) != cudaSuccess) {
+            rc = set_error(TAGI_ERR_CUDA, "tree memset failed");
+            break;
         }
+        const unsigned bw = (unsigned)std::min(152L * 8, (nodes + 7) / 8), bt = (unsigned)std::min(152L * 8, (nodes + 255) / 256);
+        launch(node_boxes, bw, 256, 0, s, hdr, t.begin, t.end, t.parent, t.first_child, t.nchild, t.x, t.y, t.z, box,
+               t.center, t.half, t.radius, size, leaves, done);
+        launch(preorder, bt, 256, 0, s, hdr, t.begin, t.end, t.parent, t.first_child, t.nchild, t.center, t.radius, size,
+               leaves, t.pre, t.leaf_node, nleaves);
+        int h[HDR + 1] = {};
+        if (cudaMemcpyAsync(h, hdr, sizeof(h), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+            cudaStreamSynchronize(s) != cudaSuccess) {
+            rc = set_error(TAGI_ERR_CUDA, "tree build: %s", cudaGetErrorString(cudaGetLastError()));
+            break;
+        }
+        t.nleaves = h[HDR];
+        if (small) {
+            t.nnodes = h[0];
+            t.level_start.assign(h + 2, h + 3 + h[1]);
+        }
+        t.nlevels = (int)t.level_start.size() - 1;
         if (cudaGetLastError() != cudaSuccess) { rc = set_error(TAGI_ERR_CUDA, "node box launch"); break; }
     } while (0);
     tmp.release();
@@ -350,99 +516,77 @@ int build_tree(Tree &t, const double *x, const double *y, const double *z, int n
 // ---------------------------------------------------------------------------
 namespace {
 
-__global__ void mark_leaves(int nn, const int *__restrict__ nchild, const int *__restrict__ begin,
-                            int *__restrict__ mark) {
-    int v = blockIdx.x * blockDim.x + threadIdx.x;
-    if (v < nn && nchild[v] == 0) mark[begin[v]] = v + 1;
-}
-
-__global__ void nonzero_flags(const int *__restrict__ a, int n, int *__restrict__ f) {
-    long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) f[i] = a[i] != 0;
-}
-
-__global__ void compact_leaves(const int *__restrict__ mark, const int *__restrict__ idx, int n,
-                               int *__restrict__ batch_node) {
-    long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n && mark[i]) batch_node[idx[i]] = mark[i] - 1;
-}
-
 struct TravArgs {
-    int nbatch;
+    int nbatch, nn;
     const int *batch_node;
     const double *tc, *tr;                 // target centers / radii
-    const double *sc, *sr;                 // source centers / radii
-    const int *sbegin, *send, *snchild, *sfirst;
+    const PreNode *pre;                    // source nodes in pre-order
     double theta, thresh;
     int *near_cnt, *far_cnt;
     const int *near_off, *far_off;
     int *near_list, *far_list;
     int *node_flag;
-    int *err;
 };
 
+// The depth-first walk of one batch by one warp, 32 nodes of the pre-order at a
+// time: a node that meets the criterion covers its subtree (the indices up to its
+// stop), and a node is visited if no node before it covers it.  One thread per
+// batch with a stack took 1 ms for 2,900 batches, a chain of dependent loads.
 template <bool FILL>
-__global__ void traverse(TravArgs a) {
-    int b = blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(256) traverse(TravArgs a) {
+    const int b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (b >= a.nbatch) return;
-    int bn = a.batch_node[b];
+    const int bn = a.batch_node[b];
     const double cbx = a.tc[3L * bn], cby = a.tc[3L * bn + 1], cbz = a.tc[3L * bn + 2];
     const double rb = a.tr[bn];
-    int stack[TRAVERSAL_STACK];
-    int sp = 0;
-    stack[sp++] = 0;
     int cn = 0, cf = 0;
     int *nl = FILL ? a.near_list + a.near_off[b] : nullptr;
     int *fl = FILL ? a.far_list + a.far_off[b] : nullptr;
-    while (sp > 0) {
-        int c = stack[--sp];
-        double dx = __dsub_rn(cbx, a.sc[3L * c]);
-        double dy = __dsub_rn(cby, a.sc[3L * c + 1]);
-        double dz = __dsub_rn(cbz, a.sc[3L * c + 2]);
-        double d2 = __dmul_rn(dx, dx);
-        d2 = __dadd_rn(d2, __dmul_rn(dy, dy));
-        d2 = __dadd_rn(d2, __dmul_rn(dz, dz));
-        double dist = __dsqrt_rn(d2);
-        bool mac = __dadd_rn(rb, a.sr[c]) < __dmul_rn(a.theta, dist);
-        int nc = a.snchild[c];
-        if (mac) {
-            if ((double)(a.send[c] - a.sbegin[c]) > a.thresh) {
-                if (FILL) {
-                    fl[cf] = c;
-                    a.node_flag[c] = 1;
-                }
-                cf++;
-            } else {
-                if (FILL) nl[cn] = c;
-                cn++;
-            }
-        } else if (nc == 0) {
-            if (FILL) nl[cn] = c;
-            cn++;
-        } else {
-            if (sp + nc > TRAVERSAL_STACK) {
-                atomicOr(a.err, 1);
-                break;
-            }
-            int f = a.sfirst[c];
-            for (int k = nc - 1; k >= 0; k--) stack[sp++] = f + k;
+    int skip = 0;   // nodes below this index are covered
+    for (int base = 0; base < a.nn; base = max(base + 32, skip)) {
+        const int i = base + lane;
+        bool mac = false, leaf = false, big = false;
+        int stop = 0, node = 0;
+        if (i < a.nn) {
+            const PreNode q = a.pre[i];
+            const double dx = __dsub_rn(cbx, q.x), dy = __dsub_rn(cby, q.y), dz = __dsub_rn(cbz, q.z);
+            double d2 = __dmul_rn(dx, dx);
+            d2 = __dadd_rn(d2, __dmul_rn(dy, dy));
+            d2 = __dadd_rn(d2, __dmul_rn(dz, dz));
+            const double dist = __dsqrt_rn(d2);
+            mac = __dadd_rn(rb, q.r) < __dmul_rn(a.theta, dist);
+            leaf = q.leaf;
+            big = (double)q.count > a.thresh;
+            stop = mac ? q.stop : 0;
+            node = q.node;
         }
+        int reach = stop;   // the furthest stop among this lane and those before it
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, reach, o);
+            if (lane >= o) reach = max(reach, v);
+        }
+        int before = __shfl_up_sync(0xffffffffu, reach, 1);
+        if (lane == 0) before = 0;
+        const bool emit = i < a.nn && max(before, skip) <= i && (mac || leaf);
+        const bool far = emit && mac && big;
+        const unsigned mf = __ballot_sync(0xffffffffu, far), mn = __ballot_sync(0xffffffffu, emit && !far);
+        if (FILL) {
+            const unsigned lt = (1u << lane) - 1u;
+            if (far) {
+                fl[cf + __popc(mf & lt)] = node;
+                a.node_flag[node] = 1;
+            } else if (emit) {
+                nl[cn + __popc(mn & lt)] = node;
+            }
+        }
+        cf += __popc(mf);
+        cn += __popc(mn);
+        skip = max(skip, __shfl_sync(0xffffffffu, reach, 31));
     }
-    if (!FILL) {
+    if (!FILL && lane == 0) {
         a.near_cnt[b] = cn;
         a.far_cnt[b] = cf;
-    }
-}
-
-__global__ void assign_slots(int nn, const int *__restrict__ flag, const int *__restrict__ idx,
-                             int *__restrict__ node_slot, int *__restrict__ slot_node) {
-    int v = blockIdx.x * blockDim.x + threadIdx.x;
-    if (v >= nn) return;
-    if (flag[v]) {
-        node_slot[v] = idx[v];
-        slot_node[idx[v]] = v;
-    } else {
-        node_slot[v] = -1;
     }
 }
 
@@ -466,124 +610,161 @@ __device__ __forceinline__ double box_gap(const double *cb, const double *hb, co
 // CLOSE_RANGE_FRACTION batch radii of the batch's box (touching included).
 // Close ranges are stored with bit 31 of their begin set (range_is_close).
 // rng_dmin = smallest node gap of the range, rounded down: a lower bound of
-// every pair distance in it.
+// every pair distance in it.  One warp per batch, 32 entries at a time; the fill
+// also writes the batch's pair counts: near, far (clusters), size, close.
 template <bool FILL>
-__global__ void merge_ranges(int nbatch, const int *__restrict__ near_off,
-                             const int *__restrict__ near_list, const int *__restrict__ sbegin,
-                             const int *__restrict__ send, const double *__restrict__ scenter,
-                             const double *__restrict__ shalf, const int *__restrict__ batch_node,
-                             const double *__restrict__ tcenter, const double *__restrict__ thalf,
-                             const double *__restrict__ tradius,
-                             int *__restrict__ cnt, const int *__restrict__ rng_off,
-                             int2 *__restrict__ rng, float *__restrict__ rng_dmin) {
-    int b = blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(256) merge_ranges(int nbatch, const int *__restrict__ near_off,
+                                                    const int *__restrict__ near_list, const int *__restrict__ sbegin,
+                                                    const int *__restrict__ send, const double *__restrict__ scenter,
+                                                    const double *__restrict__ shalf,
+                                                    const int *__restrict__ batch_node,
+                                                    const double *__restrict__ tcenter,
+                                                    const double *__restrict__ thalf,
+                                                    const double *__restrict__ tradius, int *__restrict__ cnt,
+                                                    const int *__restrict__ rng_off, int2 *rng, float *rng_dmin,
+                                                    const int *__restrict__ tbegin, const int *__restrict__ tend,
+                                                    const int *__restrict__ far_off, long long *__restrict__ costs) {
+    const int b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (b >= nbatch) return;
     const int bn = batch_node[b];
     const double cb[3] = {tcenter[3L * bn], tcenter[3L * bn + 1], tcenter[3L * bn + 2]};
     const double hb[3] = {thalf[3L * bn], thalf[3L * bn + 1], thalf[3L * bn + 2]};
     const double close_gap = CLOSE_RANGE_FRACTION * tradius[bn];
-    int k = 0;
-    int cb0 = -1, ce = -1;
-    bool cclose = false;
-    double cmin = INFINITY;
-    for (int e = near_off[b]; e <= near_off[b + 1]; e++) {
-        int c = -1, nb = -1, ne = -1;
-        bool nclose = false;
-        double gap = 0.0;
-        if (e < near_off[b + 1]) {
-            c = near_list[e];
+    const int e0 = near_off[b], e1 = near_off[b + 1];
+    int k = 0, prev_end = -1, prev_close = 0;   // ranges begun; the last entry's end and class
+    double carry = INFINITY;                    // smallest gap of the range in progress
+    long long all = 0, close_all = 0;
+    for (int base = e0; base < e1; base += 32) {
+        const int e = base + lane;
+        const bool valid = e < e1;
+        int nb = 0, ne = 0, nclose = 0;
+        double gap = INFINITY;
+        if (valid) {
+            const int c = near_list[e];
             nb = sbegin[c];
             ne = send[c];
             const double cc[3] = {scenter[3L * c], scenter[3L * c + 1], scenter[3L * c + 2]};
             const double hc[3] = {shalf[3L * c], shalf[3L * c + 1], shalf[3L * c + 2]};
             gap = box_gap(cb, hb, cc, hc);
             nclose = gap <= close_gap;
+            all += ne - nb;
+            if (nclose) close_all += ne - nb;
         }
-        if (c >= 0 && cb0 >= 0 && nb == ce && nclose == cclose) {
-            ce = ne;
-            cmin = fmin(cmin, gap);
-            continue;
+        int pe = __shfl_up_sync(0xffffffffu, ne, 1), pc = __shfl_up_sync(0xffffffffu, nclose, 1);
+        if (lane == 0) {
+            pe = prev_end;
+            pc = prev_close;
         }
-        if (cb0 >= 0) {
-            if (FILL) {
-                rng[rng_off[b] + k] = make_int2(cb0 | (cclose ? (int)0x80000000u : 0), ce);
-                rng_dmin[rng_off[b] + k] = (float)(cmin * (1.0 - 1e-6));
-            }
-            k++;
-        }
-        if (c < 0) break;
-        cb0 = nb;
-        ce = ne;
-        cclose = nclose;
-        cmin = gap;
-    }
-    if (!FILL) cnt[b] = k;
-}
-
-__global__ void batch_costs(int nbatch, const int *__restrict__ batch_node,
-                            const int *__restrict__ tbegin, const int *__restrict__ tend,
-                            const int *__restrict__ rng_off, const int2 *__restrict__ rng,
-                            const int *__restrict__ far_off, long long *__restrict__ cost_near,
-                            long long *__restrict__ cost_far, int *__restrict__ bsize,
-                            long long *__restrict__ cost_close) {
-    int b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= nbatch) return;
-    int bn = batch_node[b];
-    long long nb = tend[bn] - tbegin[bn];
-    long long s = 0, sc = 0;
-    for (int e = rng_off[b]; e < rng_off[b + 1]; e++) {
-        const long long len = rng[e].y - range_begin(rng[e]);
-        s += len;
-        if (range_is_close(rng[e])) sc += len;
-    }
-    cost_near[b] = nb * s;
-    cost_close[b] = nb * sc;
-    cost_far[b] = nb * (long long)(far_off[b + 1] - far_off[b]);
-    bsize[b] = (int)nb;
-}
-
-__global__ void slot_chunks(int nslots, const int *__restrict__ slot_node,
-                            const int *__restrict__ sbegin, const int *__restrict__ send,
-                            int chunk, int *__restrict__ nch) {
-    int sl = blockIdx.x * blockDim.x + threadIdx.x;
-    if (sl >= nslots) return;
-    int c = slot_node[sl];
-    int cnt = send[c] - sbegin[c];
-    nch[sl] = (cnt + chunk - 1) / chunk;
-}
-
-__global__ void fill_items(int nslots, const int *__restrict__ slot_node,
-                           const int *__restrict__ sbegin, const int *__restrict__ send,
-                           int chunk, const int *__restrict__ off, int *__restrict__ item_slot,
-                           int *__restrict__ item_begin, int *__restrict__ item_end) {
-    int sl = blockIdx.x * blockDim.x + threadIdx.x;
-    if (sl >= nslots) return;
-    int c = slot_node[sl];
-    int b = sbegin[c], e = send[c];
-    int k = off[sl];
-    for (int p = b; p < e; p += chunk, k++) {
-        item_slot[k] = sl;
-        item_begin[k] = p;
-        item_end[k] = min(p + chunk, e);
-    }
-}
-
-// Proxy box of each slot: node center and half widths; a zero width gets a
-// small one (1e-3 of the largest, or 1) so the barycentric map stays finite.
-__global__ void slot_geometry(int nslots, const int *__restrict__ slot_node,
-                              const double *__restrict__ center, const double *__restrict__ half,
-                              double *__restrict__ geom) {
-    int sl = blockIdx.x * blockDim.x + threadIdx.x;
-    if (sl >= nslots) return;
-    int c = slot_node[sl];
-    double h[3] = {half[3L * c], half[3L * c + 1], half[3L * c + 2]};
-    double hm = dmax(dmax(h[0], h[1]), h[2]);
+        const bool start = valid && (e == e0 || nb != pe || nclose != pc);
+        const unsigned m = __ballot_sync(0xffffffffu, start), mv = __ballot_sync(0xffffffffu, valid);
+        const unsigned le = 0xffffffffu >> (31 - lane);
+        if (FILL) {
+            const int first = (m & le) ? 31 - __clz(m & le) : 0;   // this entry's range begins here (or earlier)
+            double v = gap;
 #pragma unroll
-    for (int d = 0; d < 3; d++) {
-        geom[6L * sl + d] = center[3L * c + d];
-        double v = h[d];
-        if (!(v > 0.0)) v = hm > 0.0 ? hm * 1.0e-3 : 1.0;
-        geom[6L * sl + 3 + d] = v;
+            for (int o = 1; o < 32; o <<= 1) {
+                const double u = __shfl_up_sync(0xffffffffu, v, o);
+                if (lane - o >= first) v = fmin(v, u);
+            }
+            if (!(m & le)) v = fmin(v, carry);
+            const int r = rng_off[b] + k + __popc(m & le) - 1;
+            if (start) rng[r].x = nb | (nclose ? (int)0x80000000u : 0);
+            const unsigned after = lane == 31 ? 0u : (mv & ~m) >> (lane + 1) & 1u;   // the next entry goes on with the range
+            if (valid && !after) {   // a later round writes these again if the range goes on there
+                rng[r].y = ne;
+                rng_dmin[r] = (float)(v * (1.0 - 1e-6));
+            }
+            carry = __shfl_sync(0xffffffffu, v, 31 - __clz(mv));
+            __syncwarp();
+        }
+        prev_end = __shfl_sync(0xffffffffu, ne, 31 - __clz(mv));
+        prev_close = __shfl_sync(0xffffffffu, nclose, 31 - __clz(mv));
+        k += __popc(m);
+    }
+    if constexpr (FILL) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            all += __shfl_xor_sync(0xffffffffu, all, o);
+            close_all += __shfl_xor_sync(0xffffffffu, close_all, o);
+        }
+        if (lane == 0) {
+            const long long nt = tend[bn] - tbegin[bn];
+            costs[4L * b] = nt * all;
+            costs[4L * b + 1] = nt * close_all;
+            costs[4L * b + 2] = nt * (long long)(far_off[b + 1] - far_off[b]);
+            costs[4L * b + 3] = nt;
+        }
+    } else if (lane == 0) {
+        cnt[b] = k;
+    }
+}
+
+// Slots (far nodes in ascending node order), their proxy boxes and the upward
+// pass's work items, by one block: node_slot, slot_node, geometry (node center and
+// half widths; a zero width gets a small one, 1e-3 of the largest or 1, so the
+// barycentric map stays finite), slot_item_off and the items of at most `chunk`
+// sources.  total[0], total[1]: slots, items.
+constexpr int SLOT_THREADS = 1024;
+__global__ void __launch_bounds__(SLOT_THREADS) build_slots(int nn, const int *__restrict__ flag,
+                                                            const int *__restrict__ sbegin, const int *__restrict__ send,
+                                                            const double *__restrict__ center,
+                                                            const double *__restrict__ half, int chunk,
+                                                            int *__restrict__ node_slot, int *__restrict__ slot_node,
+                                                            double *__restrict__ geom, int *__restrict__ slot_item_off,
+                                                            int *__restrict__ item_slot, int *__restrict__ item_begin,
+                                                            int *__restrict__ item_end, int *__restrict__ total) {
+    __shared__ long long s_sum[SLOT_THREADS / 32];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    long long carry = 0;   // slots << 32 | items
+    for (int base = 0; base < nn; base += SLOT_THREADS) {
+        const int v = base + threadIdx.x;
+        const bool is = v < nn && flag[v];
+        int b = 0, e = 0;
+        if (is) {
+            b = sbegin[v];
+            e = send[v];
+        }
+        const long long mine = is ? (1LL << 32) + (e - b + chunk - 1) / chunk : 0;
+        long long incl = mine;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const long long u = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += u;
+        }
+        __syncthreads();   // the previous round's sums are no longer read
+        if (lane == 31) s_sum[wid] = incl;
+        __syncthreads();
+        long long at = carry + incl - mine;
+        for (int w = 0; w < SLOT_THREADS / 32; w++) {
+            if (w < wid) at += s_sum[w];
+            carry += s_sum[w];
+        }
+        if (v < nn) node_slot[v] = is ? (int)(at >> 32) : -1;
+        if (is) {
+            const int sl = (int)(at >> 32);
+            int k = (int)(at & 0xffffffffLL);
+            slot_node[sl] = v;
+            slot_item_off[sl] = k;
+            const double h[3] = {half[3L * v], half[3L * v + 1], half[3L * v + 2]};
+            const double hm = dmax(dmax(h[0], h[1]), h[2]);
+#pragma unroll
+            for (int d = 0; d < 3; d++) {
+                geom[6L * sl + d] = center[3L * v + d];
+                double u = h[d];
+                if (!(u > 0.0)) u = hm > 0.0 ? hm * 1.0e-3 : 1.0;
+                geom[6L * sl + 3 + d] = u;
+            }
+            for (int p = b; p < e; p += chunk, k++) {
+                item_slot[k] = sl;
+                item_begin[k] = p;
+                item_end[k] = min(p + chunk, e);
+            }
+        }
+    }
+    if (threadIdx.x == 0) {
+        total[0] = (int)(carry >> 32);
+        total[1] = (int)(carry & 0xffffffffLL);
+        slot_item_off[carry >> 32] = total[1];
     }
 }
 
@@ -596,27 +777,10 @@ int build_lists(Plan &p, cudaStream_t s) {
     tmp.stream = s;
     Arena &ar = p.arena;
     int rc = TAGI_OK;
-    auto sync_int = [&](const int *d, int *h) -> int {
-        if (cudaMemcpyAsync(h, d, sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
-            cudaStreamSynchronize(s) != cudaSuccess)
-            return set_error(TAGI_ERR_CUDA, "list build sync: %s",
-                             cudaGetErrorString(cudaGetLastError()));
-        return TAGI_OK;
-    };
     do {
-        const int nt = p.tgt.n, nns = p.src.nnodes, nnt = p.tgt.nnodes;
-        int *mark = nullptr, *flags = nullptr, *idx = nullptr, *total = nullptr;
-        if ((rc = tmp.alloc(&mark, nt)) || (rc = tmp.alloc(&flags, nt)) ||
-            (rc = tmp.alloc(&idx, nt)) || (rc = tmp.alloc(&total, 1)))
-            break;
-        cudaMemsetAsync(mark, 0, sizeof(int) * nt, s);
-        launch(mark_leaves, (nnt + 255) / 256, 256, 0, s, nnt, p.tgt.nchild, p.tgt.begin, mark);
-        launch(nonzero_flags, (nt + 255) / 256, 256, 0, s, mark, nt, flags);
-        if ((rc = exclusive_scan(flags, idx, nt, total, tmp, s))) break;
-        if ((rc = sync_int(total, &p.nbatch))) break;
-        if ((rc = ar.alloc(&p.batch_node, p.nbatch))) break;
-        launch(compact_leaves, (nt + 255) / 256, 256, 0, s, mark, idx, nt, p.batch_node);
-
+        const int nns = p.src.nnodes;
+        p.nbatch = p.tgt.nleaves;
+        p.batch_node = p.tgt.leaf_node;
         const int nb = p.nbatch;
         int *ncnt = nullptr, *fcnt = nullptr;
         if ((rc = tmp.alloc(&ncnt, nb)) || (rc = tmp.alloc(&fcnt, nb))) break;
@@ -626,15 +790,11 @@ int build_lists(Plan &p, cudaStream_t s) {
         cudaMemsetAsync(node_flag, 0, sizeof(int) * nns, s);
         TravArgs ta;
         ta.nbatch = nb;
+        ta.nn = nns;
         ta.batch_node = p.batch_node;
         ta.tc = p.tgt.center;
         ta.tr = p.tgt.radius;
-        ta.sc = p.src.center;
-        ta.sr = p.src.radius;
-        ta.sbegin = p.src.begin;
-        ta.send = p.src.end;
-        ta.snchild = p.src.nchild;
-        ta.sfirst = p.src.first_child;
+        ta.pre = p.src.pre;
         ta.theta = p.theta;
         ta.thresh = p.size_check * (double)p.P;
         ta.near_cnt = ncnt;
@@ -644,87 +804,53 @@ int build_lists(Plan &p, cudaStream_t s) {
         ta.near_list = nullptr;
         ta.far_list = nullptr;
         ta.node_flag = node_flag;
-        ta.err = p.err_flag;
-        launch(traverse<false>, (nb + 63) / 64, 64, 0, s, ta);
+        const unsigned bw = (unsigned)((nb + 7) / 8);   // a warp per batch
+        launch(traverse<false>, bw, 256, 0, s, ta);
         if ((rc = exclusive_scan(ncnt, p.near_off, nb, p.near_off + nb, tmp, s))) break;
         if ((rc = exclusive_scan(fcnt, p.far_off, nb, p.far_off + nb, tmp, s))) break;
-        if ((rc = sync_int(p.near_off + nb, &p.near_total))) break;
-        if ((rc = sync_int(p.far_off + nb, &p.far_total))) break;
-        if ((rc = ar.alloc(&p.near_list, p.near_total)) || (rc = ar.alloc(&p.far_list, p.far_total)))
+        if (cudaMemcpyAsync(&p.near_total, p.near_off + nb, sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+            cudaMemcpyAsync(&p.far_total, p.far_off + nb, sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+            cudaStreamSynchronize(s) != cudaSuccess) {
+            rc = set_error(TAGI_ERR_CUDA, "list build: %s", cudaGetErrorString(cudaGetLastError()));
             break;
+        }
+        // at most near_total ranges and nns slots; items: a slot's last chunk is partial
+        const long most = nns + (long)p.src.nlevels * (p.src.n / P2M_CHUNK + 1);
+        long long *costs = nullptr;   // 4 per batch, then the range, slot and item counts
+        if ((rc = ar.alloc(&p.near_list, p.near_total)) || (rc = ar.alloc(&p.far_list, p.far_total)) ||
+            (rc = ar.alloc(&p.rng_off, nb + 1)) || (rc = ar.alloc(&p.rng, p.near_total)) ||
+            (rc = ar.alloc(&p.rng_dmin, p.near_total)) || (rc = ar.alloc(&p.node_slot, nns)) ||
+            (rc = ar.alloc(&p.slot_node, nns)) || (rc = ar.alloc(&p.slot_geom, 6L * nns)) ||
+            (rc = ar.alloc(&p.slot_item_off, nns + 1)) || (rc = ar.alloc(&p.item_slot, most)) ||
+            (rc = ar.alloc(&p.item_begin, most)) || (rc = ar.alloc(&p.item_end, most)) ||
+            (rc = tmp.alloc(&costs, 4L * nb + 2)))
+            break;
+        int *counts = reinterpret_cast<int *>(costs + 4L * nb);
         ta.near_list = p.near_list;
         ta.far_list = p.far_list;
-        launch(traverse<true>, (nb + 63) / 64, 64, 0, s, ta);
-        int h_err = 0;
-        if ((rc = sync_int(p.err_flag, &h_err))) break;
-        if (h_err) { rc = set_error(TAGI_ERR_DEVICE, "source tree deeper than the traversal stack"); break; }
-
-        // Slots (far nodes, ascending node index).
-        int *sidx = nullptr;
-        if ((rc = tmp.alloc(&sidx, nns))) break;
-        if ((rc = exclusive_scan(node_flag, sidx, nns, total, tmp, s))) break;
-        if ((rc = sync_int(total, &p.nslots))) break;
-        if ((rc = ar.alloc(&p.node_slot, nns)) || (rc = ar.alloc(&p.slot_node, p.nslots))) break;
-        launch(assign_slots, (nns + 255) / 256, 256, 0, s, nns, node_flag, sidx, p.node_slot, p.slot_node);
-        if ((rc = ar.alloc(&p.slot_geom, 6L * p.nslots))) break;
-        if (p.nslots)
-            launch(slot_geometry, (p.nslots + 127) / 128, 128, 0, s, p.nslots, p.slot_node, p.src.center,
-                                                                 p.src.half, p.slot_geom);
-
-        // Merged near ranges.
-        int *rcnt = nullptr;
-        if ((rc = tmp.alloc(&rcnt, nb))) break;
-        if ((rc = ar.alloc(&p.rng_off, nb + 1))) break;
-        launch(merge_ranges<false>, (nb + 127) / 128, 128, 0, s, nb, p.near_off, p.near_list, p.src.begin,
-               p.src.end, p.src.center, p.src.half, p.batch_node, p.tgt.center, p.tgt.half, p.tgt.radius, rcnt,
-               nullptr, nullptr, nullptr);
-        if ((rc = exclusive_scan(rcnt, p.rng_off, nb, p.rng_off + nb, tmp, s))) break;
-        if ((rc = sync_int(p.rng_off + nb, &p.rng_total))) break;
-        if ((rc = ar.alloc(&p.rng, p.rng_total)) || (rc = ar.alloc(&p.rng_dmin, p.rng_total))) break;
-        launch(merge_ranges<true>, (nb + 127) / 128, 128, 0, s, nb, p.near_off, p.near_list, p.src.begin,
-               p.src.end, p.src.center, p.src.half, p.batch_node, p.tgt.center, p.tgt.half, p.tgt.radius, nullptr,
-               p.rng_off, p.rng, p.rng_dmin);
-
-        // Upward-pass work items.
-        if ((rc = ar.alloc(&p.slot_item_off, p.nslots + 1))) break;
-        if (p.nslots) {
-            int *nch = nullptr;
-            if ((rc = tmp.alloc(&nch, p.nslots))) break;
-            launch(slot_chunks, (p.nslots + 127) / 128, 128, 0, s, p.nslots, p.slot_node, p.src.begin,
-                                                               p.src.end, P2M_CHUNK, nch);
-            if ((rc = exclusive_scan(nch, p.slot_item_off, p.nslots, p.slot_item_off + p.nslots, tmp, s)))
-                break;
-            if ((rc = sync_int(p.slot_item_off + p.nslots, &p.nitems))) break;
-        } else {
-            cudaMemsetAsync(p.slot_item_off, 0, sizeof(int), s);
-            p.nitems = 0;
-        }
-        if ((rc = ar.alloc(&p.item_slot, p.nitems)) || (rc = ar.alloc(&p.item_begin, p.nitems)) ||
-            (rc = ar.alloc(&p.item_end, p.nitems)))
-            break;
-        if (p.nslots)
-            launch(fill_items, (p.nslots + 127) / 128, 128, 0, s, p.nslots, p.slot_node, p.src.begin,
-                                                              p.src.end, P2M_CHUNK, p.slot_item_off,
-                                                              p.item_slot, p.item_begin, p.item_end);
-
-        // Per-batch pair counts: the field kernels' work lists go heaviest first.
-        long long *cn = nullptr, *cf = nullptr, *cc2 = nullptr;
-        int *bsz = nullptr;
-        if ((rc = tmp.alloc(&cn, nb)) || (rc = tmp.alloc(&cf, nb)) || (rc = tmp.alloc(&bsz, nb)) ||
-            (rc = tmp.alloc(&cc2, nb)))
-            break;
-        launch(batch_costs, (nb + 127) / 128, 128, 0, s, nb, p.batch_node, p.tgt.begin, p.tgt.end,
-                                                     p.rng_off, p.rng, p.far_off, cn, cf, bsz, cc2);
-        std::vector<long long> hcn(nb), hcf(nb), hcc(nb);
-        std::vector<int> hsz(nb);
-        if (cudaMemcpyAsync(hcn.data(), cn, sizeof(long long) * nb, cudaMemcpyDeviceToHost, s) ||
-            cudaMemcpyAsync(hcf.data(), cf, sizeof(long long) * nb, cudaMemcpyDeviceToHost, s) ||
-            cudaMemcpyAsync(hsz.data(), bsz, sizeof(int) * nb, cudaMemcpyDeviceToHost, s) ||
-            cudaMemcpyAsync(hcc.data(), cc2, sizeof(long long) * nb, cudaMemcpyDeviceToHost, s) ||
-            cudaStreamSynchronize(s)) {
-            rc = set_error(TAGI_ERR_CUDA, "batch cost copy failed");
+        launch(traverse<true>, bw, 256, 0, s, ta);
+        launch(build_slots, 1, SLOT_THREADS, 0, s, nns, node_flag, p.src.begin, p.src.end, p.src.center, p.src.half,
+               P2M_CHUNK, p.node_slot, p.slot_node, p.slot_geom, p.slot_item_off, p.item_slot, p.item_begin, p.item_end,
+               counts + 1);
+        launch(merge_ranges<false>, bw, 256, 0, s, nb, p.near_off, p.near_list, p.src.begin, p.src.end, p.src.center,
+               p.src.half, p.batch_node, p.tgt.center, p.tgt.half, p.tgt.radius, ncnt, nullptr, nullptr, nullptr,
+               p.tgt.begin, p.tgt.end, p.far_off, nullptr);
+        if ((rc = exclusive_scan(ncnt, p.rng_off, nb, p.rng_off + nb, tmp, s))) break;
+        launch(merge_ranges<true>, bw, 256, 0, s, nb, p.near_off, p.near_list, p.src.begin, p.src.end, p.src.center,
+               p.src.half, p.batch_node, p.tgt.center, p.tgt.half, p.tgt.radius, nullptr, p.rng_off, p.rng,
+               p.rng_dmin, p.tgt.begin, p.tgt.end, p.far_off, costs);
+        // Pair counts of each batch: the field kernels' work lists go heaviest first.
+        std::vector<long long> h(4L * nb + 2);
+        if (cudaMemcpyAsync(counts, p.rng_off + nb, sizeof(int), cudaMemcpyDeviceToDevice, s) != cudaSuccess ||
+            cudaMemcpyAsync(h.data(), costs, sizeof(long long) * h.size(), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+            cudaStreamSynchronize(s) != cudaSuccess) {
+            rc = set_error(TAGI_ERR_CUDA, "list build: %s", cudaGetErrorString(cudaGetLastError()));
             break;
         }
+        const int *hc = reinterpret_cast<const int *>(h.data() + 4L * nb);
+        p.rng_total = hc[0];
+        p.nslots = hc[1];
+        p.nitems = hc[2];
         p.near_pairs = 0;
         p.near_close_pairs = 0;
         p.far_pairs = 0;
@@ -732,16 +858,18 @@ int build_lists(Plan &p, cudaStream_t s) {
         p.cost_near.resize(nb);
         p.cost_close.resize(nb);
         p.cost_far.resize(nb);
+        p.batch_size.resize(nb);
         for (int b = 0; b < nb; b++) {
-            p.near_pairs += (double)hcn[b];
-            p.near_close_pairs += (double)hcc[b];
-            p.far_pairs += (double)hcf[b] * p.P;
-            p.max_batch = std::max(p.max_batch, hsz[b]);
-            p.cost_near[b] = hcn[b] - hcc[b];
-            p.cost_close[b] = hcc[b];
-            p.cost_far[b] = hcf[b] * (long long)p.P;
+            const long long *c = &h[4L * b];
+            p.near_pairs += (double)c[0];
+            p.near_close_pairs += (double)c[1];
+            p.far_pairs += (double)c[2] * p.P;
+            p.batch_size[b] = (int)c[3];
+            p.max_batch = std::max(p.max_batch, p.batch_size[b]);
+            p.cost_near[b] = c[0] - c[1];
+            p.cost_close[b] = c[1];
+            p.cost_far[b] = c[2] * (long long)p.P;
         }
-        p.batch_size = std::move(hsz);
         if (cudaGetLastError() != cudaSuccess) { rc = set_error(TAGI_ERR_CUDA, "list kernels failed"); break; }
     } while (0);
     tmp.release();
