@@ -768,7 +768,9 @@ __global__ void __launch_bounds__(SLOT_THREADS) build_slots(int nn, const int *_
     }
 }
 
-constexpr int P2M_CHUNK = 2048;
+// Sources per upward-pass item: small meshes need items for every SM, large ones
+// few partial sums.
+int p2m_chunk(int n) { return n <= 65536 ? 256 : (n <= 262144 ? 512 : 2048); }
 
 }  // namespace
 
@@ -815,7 +817,7 @@ int build_lists(Plan &p, cudaStream_t s) {
             break;
         }
         // at most near_total ranges and nns slots; items: a slot's last chunk is partial
-        const long most = nns + (long)p.src.nlevels * (p.src.n / P2M_CHUNK + 1);
+        const long most = nns + (long)p.src.nlevels * (p.src.n / p2m_chunk(p.src.n) + 1);
         long long *costs = nullptr;   // 4 per batch, then the range, slot and item counts
         if ((rc = ar.alloc(&p.near_list, p.near_total)) || (rc = ar.alloc(&p.far_list, p.far_total)) ||
             (rc = ar.alloc(&p.rng_off, nb + 1)) || (rc = ar.alloc(&p.rng, p.near_total)) ||
@@ -830,7 +832,7 @@ int build_lists(Plan &p, cudaStream_t s) {
         ta.far_list = p.far_list;
         launch(traverse<true>, bw, 256, 0, s, ta);
         launch(build_slots, 1, SLOT_THREADS, 0, s, nns, node_flag, p.src.begin, p.src.end, p.src.center, p.src.half,
-               P2M_CHUNK, p.node_slot, p.slot_node, p.slot_geom, p.slot_item_off, p.item_slot, p.item_begin, p.item_end,
+               p2m_chunk(p.src.n), p.node_slot, p.slot_node, p.slot_geom, p.slot_item_off, p.item_slot, p.item_begin, p.item_end,
                counts + 1);
         launch(merge_ranges<false>, bw, 256, 0, s, nb, p.near_off, p.near_list, p.src.begin, p.src.end, p.src.center,
                p.src.half, p.batch_node, p.tgt.center, p.tgt.half, p.tgt.radius, ncnt, nullptr, nullptr, nullptr,

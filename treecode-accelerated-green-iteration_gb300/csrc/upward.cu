@@ -5,11 +5,19 @@
 // (-1)^m (halved at both ends), u = (y - c) / h in the slot's proxy box.
 // k = (k1 * (n+1) + k2) * (n+1) + k3, x-major like the reference's cells.
 //
-// Work items are (slot, chunk of <= 2048 sorted sources); each item writes
-// FP64 partial sums and a second kernel adds the partials of a slot in item
-// order, so results do not depend on scheduling.  The weight charges (q = w)
-// are built once per plan in FP64; charge vectors are done per call, in FP32
-// products with FP64 accumulation across tiles (mixed) or all in FP64.
+// Work items are (slot, chunk of sorted sources); each item writes FP64 partial
+// sums and a second kernel adds the partials of a slot in item order, so results
+// do not depend on scheduling.  The weight charges (q = w) are built once per plan;
+// charge vectors are done per call, in FP32 products summed over a tile of 64
+// sources, the tiles' sums then accumulated without error (mixed), or all in
+// FP64.
+//
+// Bound (mixed): FP32 issue.  A tile's sums were added in FP64, whose pipe (1/64 of
+// the FP32 rate) took three quarters of the kernel; they now go into three FP32
+// words by two-sums (72 bits, 13 FP32 operations, two at a time in packed form,
+// in place of one FP64 addition), and a CTA shares a tile's basis values between
+// P2M_OB orbitals.  32 orbitals x 1M points 29.3 -> 14.8 ms; 6k points, one charge
+// vector, chunks of 256 sources instead of 2048 157 -> 28 us.
 #include "tagi_internal.h"
 
 namespace tagi {
@@ -28,7 +36,7 @@ struct P2MArgs {
     const T *q;                  // [norb][ns] sorted charges
     long q_stride;
     double *part;                // [norb][nitems][P]
-    int n1, P;
+    int n1, P, norb;
     T tn[MAX_DEGREE + 1];
 };
 
@@ -39,11 +47,129 @@ __device__ __forceinline__ T bary_weight(int m, int n1) {
     return w;
 }
 
-template <typename T, int MAXN1>
-__global__ void __launch_bounds__(P2M_THREADS) p2m_kernel(P2MArgs<T> a) {
+// A sum of floats in three words, each the rounding error of the one before.
+struct Sum3 {
+    float2 hi, mid, lo;
+};
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __fadd2_rn(a, make_float2(-b.x, -b.y)); }
+__device__ __forceinline__ float2 two_sum(float2 &s, float2 v) {   // s += v; returns the error (Knuth)
+    const float2 t = __fadd2_rn(s, v), w = sub2(t, s);
+    const float2 e = __fadd2_rn(sub2(s, sub2(t, w)), sub2(v, w));
+    s = t;
+    return e;
+}
+__device__ __forceinline__ void add(Sum3 &a, float2 v) {
+    a.lo = __fadd2_rn(a.lo, two_sum(a.mid, two_sum(a.hi, v)));
+}
+
+// Barycentric basis values of coordinate src in the slot's box along one axis, into
+// L[0..n1-1].
+template <typename T>
+__device__ __forceinline__ void basis(double src, double c, double h, const T *tn, int n1, T *L) {
+    // FP32 basis: the FP64 quotient is only rounded to FP32, so a product serves
+    const T u = sizeof(T) == 4 ? (T)((src - c) * h) : (T)((src - c) / h);
+    int exact = -1;
+    for (int m = 0; m < n1; m++)
+        if (u - tn[m] == T(0)) exact = m;
+    if (exact >= 0) {
+        for (int m = 0; m < n1; m++) L[m] = (m == exact) ? T(1) : T(0);
+    } else {
+        T s = T(0);
+        for (int m = 0; m < n1; m++) {
+            T l = bary_weight<T>(m, n1) / (u - tn[m]);
+            L[m] = l;
+            s += l;
+        }
+        for (int m = 0; m < n1; m++) L[m] = L[m] / s;
+    }
+}
+
+// Mixed: OB orbitals of one item.  Thread (g, k1, k2) sums the sources g, g + G, ...
+// of each tile for its row of the grid.
+constexpr int P2M_OB = 3;   // upward pass of 32 orbitals x 1M points at 2, 3, 4: 18.3, 14.8, 25.0 ms (registers)
+template <int MAXN1, int OB>
+__global__ void __launch_bounds__(P2M_THREADS) p2m_mixed(const __grid_constant__ P2MArgs<float> a) {
+    constexpr int MH = (MAXN1 + 1) / 2, LP = 2 * MH;
     extern __shared__ double red[];  // [G][P]
-    __shared__ T sL[3][P2M_TILE][MAXN1];
-    __shared__ T sq[P2M_TILE];
+    __shared__ __align__(8) float sL[3][P2M_TILE][LP];
+    __shared__ float sq[OB][P2M_TILE];
+    const int item = blockIdx.x, orb0 = blockIdx.y * OB, no = min(OB, a.norb - orb0);
+    const int n1 = a.n1, pairs = n1 * n1, P = a.P;
+    const int G = P2M_THREADS / pairs;
+    const int tid = threadIdx.x;
+    const int g = tid / pairs, pr = tid % pairs;
+    const int k1 = pr / n1, k2 = pr % n1;
+    const bool active = g < G;
+    const int b = a.item_begin[item], e = a.item_end[item];
+    const double *gm = a.geom + 6L * a.item_slot[item];
+    const int axis = tid % 3;   // thread 3 p + d does source p along axis d
+    const double *xs = axis == 0 ? a.xs : (axis == 1 ? a.ys : a.zs);
+    const double center = gm[axis], inv = 1.0 / gm[3 + axis];
+    Sum3 acc[OB][MH];
+#pragma unroll
+    for (int o = 0; o < OB; o++)
+#pragma unroll
+        for (int m = 0; m < MH; m++) acc[o][m].hi = acc[o][m].mid = acc[o][m].lo = make_float2(0.f, 0.f);
+    for (int t0 = b; t0 < e; t0 += P2M_TILE) {
+        const int cnt = min(P2M_TILE, e - t0);
+        __syncthreads();   // the previous tile is no longer read
+        if (tid < 3 * cnt) {
+            float *L = sL[axis][tid / 3];
+            basis<float>(xs[t0 + tid / 3], center, inv, a.tn, n1, L);
+            if (n1 & 1) L[n1] = 0.f;   // the second lane of the last pair
+        }
+        for (int k = tid; k < OB * P2M_TILE; k += P2M_THREADS) {
+            const int o = k / P2M_TILE, p = k % P2M_TILE;
+            if (o < no && p < cnt) sq[o][p] = a.q[(long)(orb0 + o) * a.q_stride + t0 + p];
+        }
+        __syncthreads();
+        if (!active) continue;
+#pragma unroll
+        for (int o = 0; o < OB; o++) {
+            if (o >= no) break;
+            float2 t[MH];
+#pragma unroll
+            for (int m = 0; m < MH; m++) t[m] = make_float2(0.f, 0.f);
+            for (int p = g; p < cnt; p += G) {
+                const float axy = sL[0][p][k1] * sL[1][p][k2] * sq[o][p];
+                const float2 ax = make_float2(axy, axy);
+#pragma unroll
+                for (int m = 0; m < MH; m++)
+                    if (2 * m < n1) t[m] = __ffma2_rn(ax, *reinterpret_cast<const float2 *>(&sL[2][p][2 * m]), t[m]);
+            }
+#pragma unroll
+            for (int m = 0; m < MH; m++)
+                if (2 * m < n1) add(acc[o][m], t[m]);
+        }
+    }
+#pragma unroll
+    for (int o = 0; o < OB; o++) {
+        if (o >= no) break;
+        __syncthreads();   // red of the previous orbital is no longer read
+        if (active) {
+            double *r = red + (long)g * P + (long)pr * n1;
+#pragma unroll
+            for (int m = 0; m < MH; m++) {
+                const Sum3 &v = acc[o][m];
+                if (2 * m < n1) r[2 * m] = (double)v.hi.x + ((double)v.mid.x + (double)v.lo.x);
+                if (2 * m + 1 < n1) r[2 * m + 1] = (double)v.hi.y + ((double)v.mid.y + (double)v.lo.y);
+            }
+        }
+        __syncthreads();
+        double *out = a.part + ((long)(orb0 + o) * a.nitems + item) * P;
+        for (int k = tid; k < P; k += P2M_THREADS) {
+            double s = 0.0;
+            for (int gg = 0; gg < G; gg++) s += red[(long)gg * P + k];
+            out[k] = s;
+        }
+    }
+}
+
+template <int MAXN1>
+__global__ void __launch_bounds__(P2M_THREADS) p2m_f64(const __grid_constant__ P2MArgs<double> a) {
+    extern __shared__ double red[];  // [G][P]
+    __shared__ double sL[3][P2M_TILE][MAXN1];
+    __shared__ double sq[P2M_TILE];
     const int item = blockIdx.x, orb = blockIdx.y;
     const int n1 = a.n1, pairs = n1 * n1, P = a.P;
     const int G = P2M_THREADS / pairs;
@@ -54,7 +180,7 @@ __global__ void __launch_bounds__(P2M_THREADS) p2m_kernel(P2MArgs<T> a) {
     const int slot = a.item_slot[item];
     const int b = a.item_begin[item], e = a.item_end[item];
     const double *gm = a.geom + 6L * slot;
-    const T *q = a.q + (long)orb * a.q_stride;
+    const double *q = a.q + (long)orb * a.q_stride;
 
     double acc[MAXN1];
 #pragma unroll
@@ -65,36 +191,17 @@ __global__ void __launch_bounds__(P2M_THREADS) p2m_kernel(P2MArgs<T> a) {
         if (tid < 3 * cnt) {
             const int p = tid / 3, d = tid - 3 * (tid / 3);
             const double *src = d == 0 ? a.xs : (d == 1 ? a.ys : a.zs);
-            T u = (T)((src[t0 + p] - gm[d]) / gm[3 + d]);
-            int exact = -1;
-            for (int m = 0; m < n1; m++)
-                if (u - a.tn[m] == T(0)) exact = m;
-            if (exact >= 0) {
-                for (int m = 0; m < n1; m++) sL[d][p][m] = (m == exact) ? T(1) : T(0);
-            } else {
-                T s = T(0);
-                for (int m = 0; m < n1; m++) {
-                    T l = bary_weight<T>(m, n1) / (u - a.tn[m]);
-                    sL[d][p][m] = l;
-                    s += l;
-                }
-                for (int m = 0; m < n1; m++) sL[d][p][m] = sL[d][p][m] / s;
-            }
+            basis<double>(src[t0 + p], gm[d], gm[3 + d], a.tn, n1, sL[d][p]);
         }
         if (tid < cnt) sq[tid] = q[t0 + tid];
         __syncthreads();
         if (active) {
-            T tacc[MAXN1];
-#pragma unroll
-            for (int m = 0; m < MAXN1; m++) tacc[m] = T(0);
             for (int p = g; p < cnt; p += G) {
-                T axy = sL[0][p][k1] * sL[1][p][k2] * sq[p];
+                const double axy = sL[0][p][k1] * sL[1][p][k2] * sq[p];
 #pragma unroll
                 for (int m = 0; m < MAXN1; m++)
-                    if (m < n1) tacc[m] += axy * sL[2][p][m];
+                    if (m < n1) acc[m] += axy * sL[2][p][m];
             }
-#pragma unroll
-            for (int m = 0; m < MAXN1; m++) acc[m] += (double)tacc[m];
         }
         __syncthreads();
     }
@@ -145,16 +252,20 @@ int launch_p2m(Plan &p, const T *q, long q_stride, int norb, double *part, cudaS
     for (int m = 0; m <= MAX_DEGREE; m++) a.tn[m] = (T)(m <= p.degree ? p.cheb[m] : 0.0);
     const int G = P2M_THREADS / (p.n1 * p.n1);
     const size_t smem = sizeof(double) * (size_t)G * p.P;
-    dim3 grid(p.nitems, norb);
-    if (p.n1 <= 8) {
-        if (smem > 48 * 1024)
-            cudaFuncSetAttribute(p2m_kernel<T, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        launch(p2m_kernel<T, 8>, grid, P2M_THREADS, smem, s, a);
-    } else {
-        if (smem > 48 * 1024)
-            cudaFuncSetAttribute(p2m_kernel<T, MAX_DEGREE + 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)smem);
-        launch(p2m_kernel<T, MAX_DEGREE + 1>, grid, P2M_THREADS, smem, s, a);
+    a.norb = norb;
+    auto go = [&](auto kern, int ob) {
+        if (smem > 32 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        launch(kern, dim3(p.nitems, (norb + ob - 1) / ob), P2M_THREADS, smem, s, a);
+    };
+    if constexpr (sizeof(T) == 8) {
+        if (p.n1 <= 8) go(p2m_f64<8>, 1);
+        else go(p2m_f64<MAX_DEGREE + 1>, 1);
+    } else if (p.n1 <= 8) {
+        if (norb == 1) go(p2m_mixed<8, 1>, 1);
+        else go(p2m_mixed<8, P2M_OB>, P2M_OB);
+    } else {   // 11 sums of three words per orbital: two orbitals fill the registers
+        if (norb == 1) go(p2m_mixed<MAX_DEGREE + 1, 1>, 1);
+        else go(p2m_mixed<MAX_DEGREE + 1, 2>, 2);
     }
     TAGI_LAUNCH_CHECK();
     return TAGI_OK;
