@@ -784,15 +784,15 @@ __device__ __forceinline__ int q4_pos(int j, int o, int og) {   // float index o
 
 // Group tile rows: 0..2 negated coordinates (batch-relative, or hi parts of
 // the absolute splits), 3 weight, 4..6 negated lo parts (PRECISE).
-template <bool SS, bool MASK, bool PRECISE, int OG>
+template <bool SS, bool MASK, bool PRECISE, int OG, int N2 = OG / 2>
 __device__ __forceinline__ void group_chunk(const float (*__restrict__ s)[GTILE], const float4 *__restrict__ s_q4,
                                            int j0, int n, float2 tx, float2 ty, float2 tz, float2 lx, float2 ly,
                                            float2 lz, const float2 (&nfi)[OG], const float2 (&kc)[OG],
                                            float (&sum)[OG], float (&cmp)[OG]) {
     const int j1 = j0 + n;
-    float2 part[OG];
+    float2 part[2 * N2];
 #pragma unroll
-    for (int o = 0; o < OG; o++) part[o] = make_float2(0.f, 0.f);
+    for (int o = 0; o < 2 * N2; o++) part[o] = make_float2(0.f, 0.f);
 #pragma unroll 1   // measured: unrolling the source loop slows the group kernels
     for (int j = j0; j < j1; j += 2) {
         float2 dx = add2(tx, lds2(s[0] + j)), dy = add2(ty, lds2(s[1] + j)), dz = add2(tz, lds2(s[2] + j));
@@ -813,7 +813,7 @@ __device__ __forceinline__ void group_chunk(const float (*__restrict__ s)[GTILE]
         }
         const float2 r = mul2(r2, rinv);
 #pragma unroll
-        for (int o2 = 0; o2 < OG / 2; o2++) {
+        for (int o2 = 0; o2 < N2; o2++) {
             const float4 q4 = s_q4[(j >> 1) * (OG / 2) + o2];
 #pragma unroll
             for (int u = 0; u < 2; u++) {
@@ -826,8 +826,28 @@ __device__ __forceinline__ void group_chunk(const float (*__restrict__ s)[GTILE]
         }
     }
 #pragma unroll
-    for (int o = 0; o < OG; o++) kahan_add(sum[o], cmp[o], part[o].x + part[o].y);
+    for (int o = 0; o < 2 * N2; o++) kahan_add(sum[o], cmp[o], part[o].x + part[o].y);
 }
+
+// The chunk or proxy grid for the n2 pairs of orbitals that an item holds (its
+// last ones may be missing): FN<N2>(n2's value).
+template <int OG, typename FN>
+__device__ __forceinline__ void for_pairs(int n2, FN &&fn) {
+    if constexpr (OG == 8) {
+        switch (n2) {
+        case 1: fn(std::integral_constant<int, 1>()); return;
+        case 2: fn(std::integral_constant<int, 2>()); return;
+        case 3: fn(std::integral_constant<int, 3>()); return;
+        }
+    } else if (n2 == 1) {
+        fn(std::integral_constant<int, 1>());
+        return;
+    }
+    fn(std::integral_constant<int, OG / 2>());
+}
+// Pairs of orbitals of an item of OG that starts at g0.
+template <int OG>
+__device__ __forceinline__ int item_pairs(int norb, int g0) { return min(OG / 2, (norb - g0 + 1) >> 1); }
 
 template <bool SS, int OG, int PASS>
 __global__ void __launch_bounds__(GT, 4) near_group(const __grid_constant__ Work w) {
@@ -856,6 +876,7 @@ __global__ void __launch_bounds__(GT, 4) near_group(const __grid_constant__ Work
             kc[o] = dup2(orb < a.norb ? -a.kc32[orb] : 0.f);   // -k log2(e) as one FP32 constant
             if (orb < a.norb) kmin = fminf(kmin, a.kc32[orb]);
         }
+        const int n2 = item_pairs<OG>(a.norb, g0);
         const int r0 = a.rng_off[b], r1 = a.rng_off[b + 1];
         const int i = it.z + tid;
         const bool v = i < it.w;
@@ -935,8 +956,10 @@ __global__ void __launch_bounds__(GT, 4) near_group(const __grid_constant__ Work
                 for (int sl = 0; sl < GW; sl++) {
                     const int m = s_cnt[sl];
                     if (m == 0) break;
-                    group_chunk<SS, PASS == 1, PASS == 1, OG>(s_src, s_q4, sl * SLOT, m, tx, ty, tz, lx, ly, lz, nfi,
-                                                              kc, sum, cmp);
+                    for_pairs<OG>(n2, [&](auto c) {
+                        group_chunk<SS, PASS == 1, PASS == 1, OG, decltype(c)::value>(
+                            s_src, s_q4, sl * SLOT, m, tx, ty, tz, lx, ly, lz, nfi, kc, sum, cmp);
+                    });
                 }
             }
         }
@@ -951,7 +974,7 @@ __global__ void __launch_bounds__(GT, 4) near_group(const __grid_constant__ Work
 
 // One staged proxy grid against one target for a group of orbitals (see
 // far_cluster for the padded innermost axis).
-template <bool SS, int MAXN1, int OG, bool EXACT = false>
+template <bool SS, int MAXN1, int OG, bool EXACT = false, int N2 = OG / 2>
 __device__ __forceinline__ void far_group_cluster(const float4 *__restrict__ s_q4, const float *__restrict__ s_w,
                                                   const float (*s_p)[MAXN1], int n1_in,
                                                   float tx, float ty, float tz, const float2 (&nfi)[OG],
@@ -968,9 +991,9 @@ __device__ __forceinline__ void far_group_cluster(const float4 *__restrict__ s_q
     }
     int idx = 0;
     for (int k1 = 0; k1 < n1; k1++) {
-        float2 part[OG];
+        float2 part[2 * N2];
 #pragma unroll
-        for (int o = 0; o < OG; o++) part[o] = make_float2(0.f, 0.f);
+        for (int o = 0; o < 2 * N2; o++) part[o] = make_float2(0.f, 0.f);
         const float dx = tx - s_p[0][k1];
         const float dx2 = dx * dx;
         for (int k2 = 0; k2 < n1; k2++) {
@@ -984,7 +1007,7 @@ __device__ __forceinline__ void far_group_cluster(const float4 *__restrict__ s_q
                     const float2 nl = nlog2r2(r2);
                     const float2 wk = lds2(s_w + idx + 2 * m);
 #pragma unroll
-                    for (int o2 = 0; o2 < OG / 2; o2++) {
+                    for (int o2 = 0; o2 < N2; o2++) {
                         const float4 q4 = s_q4[((idx >> 1) + m) * (OG / 2) + o2];
 #pragma unroll
                         for (int u = 0; u < 2; u++) {
@@ -999,7 +1022,7 @@ __device__ __forceinline__ void far_group_cluster(const float4 *__restrict__ s_q
             idx += n1p;
         }
 #pragma unroll
-        for (int o = 0; o < OG; o++) kahan_add(sum[o], cmp[o], part[o].x + part[o].y);
+        for (int o = 0; o < 2 * N2; o++) kahan_add(sum[o], cmp[o], part[o].x + part[o].y);
     }
 }
 
@@ -1070,8 +1093,10 @@ __global__ void __launch_bounds__(GT, 4) far_group(const __grid_constant__ Work 
             }
             __syncthreads();
             if (!warp_busy) continue;
-            far_group_cluster<SS, MAXN1, OG, EXACT>(s_q4, s_w, s_p, n1, tx, ty, tz,
-                                                    nfi, kc, sum, cmp);
+            for_pairs<OG>(item_pairs<OG>(a.norb, g0), [&](auto c) {
+                far_group_cluster<SS, MAXN1, OG, EXACT, decltype(c)::value>(s_q4, s_w, s_p, n1, tx, ty, tz, nfi, kc,
+                                                                            sum, cmp);
+            });
         }
         if (v) {
 #pragma unroll
@@ -1170,8 +1195,11 @@ __global__ void __launch_bounds__(GT, 4) far_group_db(const __grid_constant__ Wo
             if (e + 1 < f1) stage(e + 1, cur ^ 1);
             if (!warp_busy) continue;
             const float *q = s_dyn + (size_t)cur * BUF;
-            far_group_cluster<SS, DB_N1, OG, true>(reinterpret_cast<const float4 *>(q), q + DB_P * OG, s_p[cur],
-                                                   DB_N1, tx, ty, tz, nfi, kc, sum, cmp);
+            for_pairs<OG>(item_pairs<OG>(a.norb, g0), [&](auto c) {
+                far_group_cluster<SS, DB_N1, OG, true, decltype(c)::value>(reinterpret_cast<const float4 *>(q),
+                                                                           q + DB_P * OG, s_p[cur], DB_N1, tx, ty, tz,
+                                                                           nfi, kc, sum, cmp);
+            });
         }
         if (v) {
 #pragma unroll
