@@ -709,16 +709,20 @@ __global__ void __launch_bounds__(FT, 2) far_mixed(const __grid_constant__ Work 
                     add_pending();
                     pending = nc * n1;
                 }
-                for (int cl = 0; cl < nc; cl++) {
-                    const int sl = s_slot[c0 + cl] >> 1;
-                    const float *qs = qh + (long)sl * P;
-                    const float *ws = a.what32 + (long)sl * P;
-                    for (int k = tid; k < Pp; k += FT) {
-                        const int row = k / n1p, k3 = k - row * n1p;
-                        const bool real = k3 < n1;
-                        const int src = row * n1 + (real ? k3 : 0);
-                        s_q[cl][k] = real ? qs[src] : 0.f;
-                        s_w[cl][k] = real ? ws[src] : 0.f;
+                for (int k = tid; k < Pp; k += FT) {   // the same grid point of all the tile's clusters at once
+                    const int row = k / n1p, k3 = k - row * n1p, src = row * n1 + k3;
+                    float vq[FAR_CL], vw[FAR_CL];
+#pragma unroll
+                    for (int cl = 0; cl < FAR_CL; cl++) {
+                        const bool real = cl < nc && k3 < n1;
+                        const long at = real ? (long)(s_slot[c0 + cl] >> 1) * P + src : 0;
+                        vq[cl] = real ? qh[at] : 0.f;
+                        vw[cl] = real ? a.what32[at] : 0.f;
+                    }
+#pragma unroll
+                    for (int cl = 0; cl < FAR_CL; cl++) {
+                        s_q[cl][k] = vq[cl];
+                        s_w[cl][k] = vw[cl];
                     }
                 }
                 for (int u = tid; u < 3 * n1 * nc; u += FT) {
@@ -1075,12 +1079,15 @@ __global__ void __launch_bounds__(GT, 4) far_group(const __grid_constant__ Work 
             const int slot = a.node_slot[a.far_list[e]];
             const double *gm = a.geom + 6L * slot;
             __syncthreads();
-            for (int k = tid; k < Pp * OG; k += GT) {   // orbital-major: coalesced global reads
-                const int o = k / Pp, kk = k - o * Pp;
+            for (int kk = tid; kk < Pp; kk += GT) {   // a point's charges of all orbitals at once
                 const int row = kk / n1p, k3 = kk - row * n1p;
-                const int orb = g0 + o;
-                reinterpret_cast<float *>(s_q4)[q4_pos(kk, o, OG)] =
-                    (k3 < n1 && orb < a.norb) ? a.qhat32[((long)orb * a.nslots + slot) * P + row * n1 + k3] : 0.f;
+                const float *q0 = a.qhat32 + ((long)g0 * a.nslots + slot) * P + row * n1 + k3;
+                float q[OG];
+#pragma unroll
+                for (int o = 0; o < OG; o++)
+                    q[o] = (k3 < n1 && g0 + o < a.norb) ? q0[(long)o * a.nslots * P] : 0.f;
+#pragma unroll
+                for (int o = 0; o < OG; o++) reinterpret_cast<float *>(s_q4)[q4_pos(kk, o, OG)] = q[o];
             }
             for (int k = tid; k < Pp; k += GT) {
                 const int row = k / n1p, k3 = k - row * n1p;
@@ -1464,15 +1471,22 @@ __global__ void __launch_bounds__(GT, 4) near_group16(const __grid_constant__ Wo
                     }
                     // a warp stages 8 sources x 4 orbitals at a time: 32-byte global
                     // segments, conflict-free shared writes with the QS16 stride
+                    // (all 32 loads of a lane are issued before the first is stored)
                     const int o4 = lane >> 3, j8 = lane & 7;
-                    for (int j = j8; j < cnt4; j += 8) {
+                    float q[8][4];
 #pragma unroll
-                        for (int o = o4; o < 16; o += 4) {
-                            const int orb = g0 + o;
-                            s_q[(wid * SLOT + j) * QS16 + o] =
-                                (j < cnt && orb < a.norb) ? a.q32[(long)orb * a.ns + t0 + j] : 0.f;
-                        }
+                    for (int i = 0; i < 4; i++) {
+                        const int orb = g0 + o4 + 4 * i;
+                        const float *qo = a.q32 + (long)orb * a.ns + t0;
+#pragma unroll
+                        for (int u = 0; u < 8; u++) q[u][i] = (j8 + 8 * u < cnt && orb < a.norb) ? qo[j8 + 8 * u] : 0.f;
                     }
+#pragma unroll
+                    for (int u = 0; u < 8; u++)
+                        if (j8 + 8 * u < cnt4) {
+#pragma unroll
+                            for (int i = 0; i < 4; i++) s_q[(wid * SLOT + j8 + 8 * u) * QS16 + o4 + 4 * i] = q[u][i];
+                        }
                 }
                 if (lane == 0) s_cnt[wid] = cnt4;
                 __syncthreads();
@@ -1625,20 +1639,27 @@ __global__ void __launch_bounds__(GT, 4) far_group16(const __grid_constant__ Wor
             sum[o] = 0.f;
             cmp[o] = 0.f;
         }
+        const int so = tid >> 3;   // the orbital whose charges this thread stages
+        const bool has = g0 + so < a.norb;
         for (int e = f0; e < f1; e++) {
             const int slot = a.node_slot[a.far_list[e]];
             const double *gm = a.geom + 6L * slot;
             __syncthreads();
-            // a warp stages 8 proxy points x 4 orbitals (see near_group16)
-            for (int k = tid; k < ((Pp + 7) & ~7) * 16; k += GT) {
-                const int kb = k >> 7, rem = k & 127;
-                const int o = rem >> 3, kk = (kb << 3) + (rem & 7);
-                if (kk >= Pp) continue;
-                const int row = kk / n1p, k3 = kk - row * n1p;
-                const int orb = g0 + o;
-                s_q[kk * QS16 + o] =
-                    (k3 < n1 && orb < a.norb) ? a.qhat32[((long)orb * a.nslots + slot) * P + row * n1 + k3] : 0.f;
+            // a warp stages 8 proxy points x 4 orbitals at a time (see near_group16), 16
+            // loads of a thread in flight
+            const float *qo = a.qhat32 + ((long)(has ? g0 + so : g0) * a.nslots + slot) * P;
+            for (int k0 = tid & 7; k0 < Pp; k0 += 8 * 16) {
+                float q[16];
+#pragma unroll
+                for (int u = 0; u < 16; u++) {
+                    const int kk = k0 + 8 * u, row = kk / n1p, k3 = kk - row * n1p;
+                    q[u] = (has && kk < Pp && k3 < n1) ? qo[row * n1 + k3] : 0.f;
+                }
+#pragma unroll
+                for (int u = 0; u < 16; u++)
+                    if (k0 + 8 * u < Pp) s_q[(k0 + 8 * u) * QS16 + so] = q[u];
             }
+#pragma unroll 4
             for (int k = tid; k < Pp; k += GT) {
                 const int row = k / n1p, k3 = k - row * n1p;
                 s_w[k] = k3 < n1 ? a.what32[(long)slot * P + row * n1 + k3] : 0.f;
