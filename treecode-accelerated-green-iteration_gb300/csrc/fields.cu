@@ -945,14 +945,23 @@ __global__ void __launch_bounds__(GT, 4) near_group(const __grid_constant__ Work
                             sts2(&s_src[2][d], neg_relative(hz, qz, ccz));
                         }
                         sts2(&s_src[3][d], make_float2(real0 ? a.w32[j0] : 0.f, real1 ? a.w32[j1] : 0.f));
-#pragma unroll
-                        for (int o = 0; o < OG; o++) {
-                            const float *qo = a.q32 + (long)(g0 + o) * a.ns;
-                            const bool has = g0 + o < a.norb;
-                            sts2(reinterpret_cast<float *>(s_q4) + q4_pos(d, o, OG),
-                                 make_float2(has && real0 ? qo[j0] : 0.f, has && real1 ? qo[j1] : 0.f));
-                        }
                     }
+                    // charges: lanes take the float4s of the staged layout in turn (pairs of
+                    // sources x pairs of orbitals), all loads before the first store
+                    constexpr int LP = 32 * 2 / OG;   // pairs of sources per turn of the warp
+                    const int o2 = lane % (OG / 2), oa = g0 + 2 * o2;
+                    const bool ha = oa < a.norb, hb = oa + 1 < a.norb;
+                    const float *qa = a.q32 + (long)(ha ? oa : g0) * a.ns + t0, *qb = qa + (hb ? a.ns : 0);
+                    float4 q[SLOT / 2 / LP];
+#pragma unroll
+                    for (int u = 0; u < SLOT / 2 / LP; u++) {
+                        const int ja = 2 * (u * LP + lane / (OG / 2));
+                        const bool r0v = ja < cnt, r1v = ja + 1 < cnt;
+                        q[u] = make_float4(ha && r0v ? qa[ja] : 0.f, ha && r1v ? qa[ja + 1] : 0.f,
+                                           hb && r0v ? qb[ja] : 0.f, hb && r1v ? qb[ja + 1] : 0.f);
+                    }
+#pragma unroll
+                    for (int u = 0; u < SLOT / 2 / LP; u++) s_q4[wid * (SLOT * OG / 4) + u * 32 + lane] = q[u];
                 }
                 if (lane == 0) s_cnt[wid] = cnt2;
                 __syncthreads();
