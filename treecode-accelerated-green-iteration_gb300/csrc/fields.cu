@@ -2,9 +2,9 @@
 //
 // One CTA works on one (target chunk of a batch, orbital) item at a time,
 // pulled from a global counter in heaviest-first order (persistent launch,
-// grid = resident CTAs).  In the single-orbital kernels the CTA's eight warps
-// form G groups of targets times S = 8 / G splits of each target's sources
-// (Fields::split, set per plan by field_split).  Each target's sum is formed in
+// grid = resident CTAs).  In the single-orbital kernels the CTA's warps form G
+// groups of targets times S splits of each target's sources (Fields::split, set
+// per plan by field_split).  Each target's sum is formed in
 // a fixed order (list order, then source order), so results do not depend on
 // scheduling; in mixed precision not on the split either: the splits' FP32
 // partials go through shared memory to one thread per target, which adds them
@@ -44,12 +44,9 @@ namespace tagi {
 
 namespace {
 
-constexpr int FT = 256;        // threads per field CTA
-constexpr int FW = FT / 32;    // warps per field CTA
-constexpr int NTILE = 512;     // sources per near-field tile
+constexpr int FT = 256;        // threads per CTA of the FP64 kernels
 constexpr int SLOT = 64;       // sources per slot of a tile: one FP32 run per lane pair
-constexpr int SLOTS = NTILE / SLOT;
-static_assert(SLOTS == FW, "warp w stages slot w of a tile");
+constexpr int NTILE = 4 * SLOT;  // sources per tile of the loop ceiling
 constexpr double LOG2E = 1.4426950408889634;
 
 __device__ __forceinline__ float rsqrt_mufu(float x) {
@@ -134,8 +131,8 @@ __device__ __forceinline__ void pass_end() {
 // The place of a warp in its CTA: target group g of G, source split sp of S.
 struct Place {
     int S, G, g, sp, lane, wid;
-    __device__ __forceinline__ explicit Place(int split)
-        : S(split), G(FW / split), lane(threadIdx.x & 31), wid(threadIdx.x >> 5) {
+    __device__ __forceinline__ Place(int split, int warps)
+        : S(split), G(warps / split), lane(threadIdx.x & 31), wid(threadIdx.x >> 5) {
         g = wid & (G - 1);
         sp = wid / G;
     }
@@ -331,8 +328,8 @@ __device__ __forceinline__ void sts2(float *p, float2 v) { *reinterpret_cast<flo
 // unscaled r^2 is multiplied by sc2 = sc^2, so the shortest pairs keep FP32
 // relative precision in r whatever the batch size.
 constexpr int NROWS_PRECISE = 8;
-template <int KERN, bool SS, bool MASK, bool PRECISE, int NT>
-__device__ __forceinline__ void near_chunk(const float (*__restrict__ s)[NTILE], int j0, int n, const float2 (&tx)[NT],
+template <int KERN, bool SS, bool MASK, bool PRECISE, int NT, int TILE>
+__device__ __forceinline__ void near_chunk(const float (*__restrict__ s)[TILE], int j0, int n, const float2 (&tx)[NT],
                                           const float2 (&ty)[NT], const float2 (&tz)[NT], const float2 (&lx)[NT],
                                           const float2 (&ly)[NT], const float2 (&lz)[NT], float2 sc2,
                                           const float2 (&nfi)[NT], float (&out)[NT]) {
@@ -384,16 +381,17 @@ __device__ __forceinline__ void near_chunk(const float (*__restrict__ s)[NTILE],
 // PASS 0 handles the ordinary near ranges, PASS 1 the close ones (double-float
 // coordinates, r = 0 mask) into a second output; two passes keep each
 // kernel's register footprint at one tile variant's.
-#ifndef TAGI_NEAR_MINB
-#define TAGI_NEAR_MINB 3   // resident CTAs per SM the near kernel is compiled for
-#endif
-template <int KERN, bool SS, int NT, int PASS>
-__global__ void __launch_bounds__(FT, TAGI_NEAR_MINB) near_mixed(const __grid_constant__ Work w) {
-    constexpr int NR = PASS == 1 ? NROWS_PRECISE : 5;
-    __shared__ __align__(16) float s_src[NR][NTILE];
-    __shared__ RangeTable<FT> s_rng;
-    __shared__ __align__(16) float s_part[SLOTS * FT];   // S > 1: partials [slot][target of the CTA]
-    __shared__ int s_cnt[SLOTS];   // sources of each slot, a multiple of 4; bit 30: leave the Gaussian out
+// SW warps per CTA: 8 where the mesh is small and eight splits share each target's
+// sources, 4 above, where more and smaller CTAs wait less at their barriers (24 warps
+// per SM either way).  near + far, ms, 8 and 4 warps: Coulomb 1.5M points 94.3 -> 92.2, 1.34M
+// points, degree 4, Yukawa 71.5 -> 66.7; Yukawa 50k points, whole call 1.11 and 1.31.
+template <int KERN, bool SS, int NT, int PASS, int SW>
+__global__ void __launch_bounds__(32 * SW, 24 / SW) near_mixed(const __grid_constant__ Work w) {
+    constexpr int NR = PASS == 1 ? NROWS_PRECISE : 5, ST = 32 * SW, TILE = SW * SLOT;   // warp w stages slot w of a tile
+    __shared__ __align__(16) float s_src[NR][TILE];
+    __shared__ RangeTable<ST> s_rng;
+    __shared__ __align__(16) float s_part[SW * ST];   // S > 1: partials [slot][target of the CTA]
+    __shared__ int s_cnt[SW];   // sources of each slot, a multiple of 4; bit 30: leave the Gaussian out
     __shared__ int s_item;
     constexpr int NOEXP = 1 << 30;
     const int tid = threadIdx.x;
@@ -403,7 +401,7 @@ __global__ void __launch_bounds__(FT, TAGI_NEAR_MINB) near_mixed(const __grid_co
         if (item >= w.nitems) break;
         const int4 it = w.items[item];
         const Fields &a = w.sys[it.y >> 16];
-        const Place pl(a.split);
+        const Place pl(a.split, SW);
         const int b = it.x, orb = it.y & 0xffff;
         const int bn = a.batch_node[b];
         const int te = it.w;
@@ -453,7 +451,7 @@ __global__ void __launch_bounds__(FT, TAGI_NEAR_MINB) near_mixed(const __grid_co
             sum[k] = 0.f;
             cmp[k] = 0.f;
         }
-        for (int e0 = r0; e0 < r1; e0 += FT) {
+        for (int e0 = r0; e0 < r1; e0 += ST) {
             // Ranges far enough away: Yukawa terms are exactly 0 in FP32
             // (2^{-r'} with r' > 127 flushes to zero) and the range is left out;
             // the Coulomb Gaussian correction is below 2^-40 of its term and is
@@ -466,11 +464,11 @@ __global__ void __launch_bounds__(FT, TAGI_NEAR_MINB) near_mixed(const __grid_co
                 r.x = range_begin(r) | (noexp ? (int)0x80000000u : 0);
                 return true;
             });
-            for (int c0 = 0; c0 < n.y; c0 += SLOTS) {
+            for (int c0 = 0; c0 < n.y; c0 += SW) {
                 __syncthreads();   // the previous tile is no longer read, its partials are written
                 if (pl.S > 1) {
                     add_pending();
-                    pending = min(SLOTS, n.y - c0);
+                    pending = min(SW, n.y - c0);
                 }
                 const int c = c0 + pl.wid;
                 int cnt4 = 0, flag = 0;
@@ -508,17 +506,17 @@ __global__ void __launch_bounds__(FT, TAGI_NEAR_MINB) near_mixed(const __grid_co
                 if (pl.lane == 0) s_cnt[pl.wid] = cnt4 | flag;
                 __syncthreads();
                 if (!warp_busy) continue;
-                for (int sl = pl.sp; sl < SLOTS; sl += pl.S) {
+                for (int sl = pl.sp; sl < SW; sl += pl.S) {
                     const int m = s_cnt[sl];
                     if (m == 0) break;
                     float part[NT];
                     if (PASS == 1)
-                        near_chunk<KERN, SS, true, true, NT>(s_src, sl * SLOT, m, tx, ty, tz, lx, ly, lz, sc2, nfi, part);
+                        near_chunk<KERN, SS, true, true, NT, TILE>(s_src, sl * SLOT, m, tx, ty, tz, lx, ly, lz, sc2, nfi, part);
                     else if (KERN == KERNEL_COULOMB && SS && (m & NOEXP))
-                        near_chunk<KERN, false, false, false, NT>(s_src, sl * SLOT, m & ~NOEXP, tx, ty, tz, lx, ly,
+                        near_chunk<KERN, false, false, false, NT, TILE>(s_src, sl * SLOT, m & ~NOEXP, tx, ty, tz, lx, ly,
                                                                   lz, sc2, nfi, part);
                     else
-                        near_chunk<KERN, SS, false, false, NT>(s_src, sl * SLOT, m, tx, ty, tz, lx, ly, lz, sc2, nfi,
+                        near_chunk<KERN, SS, false, false, NT, TILE>(s_src, sl * SLOT, m, tx, ty, tz, lx, ly, lz, sc2, nfi,
                                                                part);
 #pragma unroll
                     for (int k = 0; k < NT; k++) {
@@ -618,18 +616,20 @@ __device__ __forceinline__ int first_slab(int cl, int n1, const Place &pl) { ret
 // staged per pair of barriers.
 template <int MAXN1>
 __host__ __device__ constexpr int far_clusters() { return MAXN1 <= 4 ? 8 : (MAXN1 <= 8 ? 4 : 2); }
-constexpr int FAR_PART = 4096;   // partials of a far tile where a target's slabs are split (16 KB); 11 slabs of 256 targets fit
-static_assert(FAR_PART >= (MAX_DEGREE + 1) * FT, "one cluster's slabs of a CTA's targets");
+// Partials of a far tile where a target's slabs are split: at least one cluster's
+// slabs of the CTA's targets (two warps of targets with two targets per thread).
+__host__ __device__ constexpr int far_part(int warps) { return warps == 4 ? 2048 : 4096; }
+static_assert(far_part(4) >= (MAX_DEGREE + 1) * 128 && far_part(8) >= (MAX_DEGREE + 1) * 256, "slabs of one cluster");
 
-template <int KERN, bool SS, int MAXN1, int NT, bool EXACT = false>
-__global__ void __launch_bounds__(FT, 2) far_mixed(const __grid_constant__ Work w) {
+template <int KERN, bool SS, int MAXN1, int NT, int SW, bool EXACT = false>
+__global__ void __launch_bounds__(32 * SW, 16 / SW) far_mixed(const __grid_constant__ Work w) {
     constexpr int MAXPP = MAXN1 * MAXN1 * even_up<MAXN1>();
-    constexpr int FAR_CL = far_clusters<MAXN1>();
+    constexpr int FAR_CL = far_clusters<MAXN1>(), ST = 32 * SW, FAR_PART = far_part(SW);
     __shared__ __align__(16) float s_q[FAR_CL][MAXPP];
     __shared__ __align__(16) float s_w[FAR_CL][MAXPP];
     __shared__ float s_p[FAR_CL][3][MAXN1];
-    __shared__ int s_slot[FT];   // the item's next clusters that count: slot << 1 | leave the Gaussian out
-    __shared__ int s_kept[FW];
+    __shared__ int s_slot[ST];   // the item's next clusters that count: slot << 1 | leave the Gaussian out
+    __shared__ int s_kept[SW];
     __shared__ float s_part[FAR_PART];   // S > 1: partials [cluster of the tile, slab][target of the CTA]
     __shared__ int s_item;
     const int tid = threadIdx.x;
@@ -639,7 +639,7 @@ __global__ void __launch_bounds__(FT, 2) far_mixed(const __grid_constant__ Work 
         if (item >= w.nitems) break;
         const int4 it = w.items[item];
         const Fields &a = w.sys[it.y >> 16];
-        const Place pl(a.split);
+        const Place pl(a.split, SW);
         const int b = it.x, orb = it.y & 0xffff;
         const int n1 = EXACT ? MAXN1 : a.n1, P = EXACT ? MAXN1 * MAXN1 * MAXN1 : a.P;
         const int n1p = n1 + (n1 & 1), Pp = n1 * n1 * n1p;
@@ -677,7 +677,7 @@ __global__ void __launch_bounds__(FT, 2) far_mixed(const __grid_constant__ Work 
             sum[k] = 0.f;
             cmp[k] = 0.f;
         }
-        for (int e0 = f0; e0 < f1; e0 += FT) {
+        for (int e0 = f0; e0 < f1; e0 += ST) {
             int slot = 0, mode = 2;
             if (e0 + tid < f1) {
                 slot = a.node_slot[a.far_list[e0 + tid]];
@@ -697,7 +697,7 @@ __global__ void __launch_bounds__(FT, 2) far_mixed(const __grid_constant__ Work 
             __syncthreads();
             int pos = __popc(kept & ((1u << pl.lane) - 1u)), ne = 0;
 #pragma unroll
-            for (int v = 0; v < FW; v++) {
+            for (int v = 0; v < SW; v++) {
                 if (v < pl.wid) pos += s_kept[v];
                 ne += s_kept[v];
             }
@@ -709,7 +709,7 @@ __global__ void __launch_bounds__(FT, 2) far_mixed(const __grid_constant__ Work 
                     add_pending();
                     pending = nc * n1;
                 }
-                for (int k = tid; k < Pp; k += FT) {   // the same grid point of all the tile's clusters at once
+                for (int k = tid; k < Pp; k += ST) {   // the same grid point of all the tile's clusters at once
                     const int row = k / n1p, k3 = k - row * n1p, src = row * n1 + k3;
                     float vq[FAR_CL], vw[FAR_CL];
 #pragma unroll
@@ -725,7 +725,7 @@ __global__ void __launch_bounds__(FT, 2) far_mixed(const __grid_constant__ Work 
                         s_w[cl][k] = vw[cl];
                     }
                 }
-                for (int u = tid; u < 3 * n1 * nc; u += FT) {
+                for (int u = tid; u < 3 * n1 * nc; u += ST) {
                     const int cl = u / (3 * n1), v = u - cl * 3 * n1;
                     const int d = v / n1, m = v - d * n1;
                     const double *g = a.geom + 6L * (s_slot[c0 + cl] >> 1);
@@ -1876,7 +1876,7 @@ __global__ void __launch_bounds__(FT) near_f64(const __grid_constant__ Work w) {
         if (item >= w.nitems) break;
         const int4 it = w.items[item];
         const Fields &a = w.sys[it.y >> 16];
-        const Place pl(a.split);
+        const Place pl(a.split, FT / 32);
         const int b = it.x, orb = it.y & 0xffff;
         const double kp = a.kp64[orb];
         const ExpScale es = exp_scale(kp, KERN == KERNEL_COULOMB);
@@ -1932,7 +1932,7 @@ __global__ void __launch_bounds__(FT) far_f64(const __grid_constant__ Work w) {
         if (item >= w.nitems) break;
         const int4 it = w.items[item];
         const Fields &a = w.sys[it.y >> 16];
-        const Place pl(a.split);
+        const Place pl(a.split, FT / 32);
         const int b = it.x, orb = it.y & 0xffff;
         const int n1 = a.n1, P = a.P;
         const int f0 = a.far_off[b], f1 = a.far_off[b + 1];
@@ -2104,7 +2104,7 @@ __global__ void __launch_bounds__(FT) pair_peak_near(int reps, float *out) {
     for (int r = 0; r < reps; r++)
         for (int j0 = 0; j0 < NTILE; j0 += SLOT) {
             float part[2];
-            near_chunk<KERN, SS, false, false, 2>(s, j0, SLOT, tx, ty, tz, z2, z2, z2, dup2(1.f), nfi, part);
+            near_chunk<KERN, SS, false, false, 2, NTILE>(s, j0, SLOT, tx, ty, tz, z2, z2, z2, dup2(1.f), nfi, part);
             for (int k = 0; k < 2; k++) kahan_add(sum[k], cmp[k], part[k]);
         }
     out[blockIdx.x * FT + threadIdx.x] = sum[0] + sum[1] - cmp[0] - cmp[1];
@@ -2327,10 +2327,38 @@ int run_pair_peak(int variant, double *pairs_per_s, cudaStream_t s) {
 // Kernel shape shared by every system of one field launch.
 struct LaunchShape {
     int og = 1;     // orbitals per item (orbital-group kernels) or 1
-    int nt = 1;     // targets per thread (single-orbital mixed kernels)
+    int nt = 1;     // targets per thread and
+    int warps = 4;  // warps per CTA (single-orbital mixed kernels)
     int maxn1 = 1;        // largest proxy-grid edge n + 1
     int minn1 = 1 << 20;  // smallest proxy-grid edge n + 1
 };
+
+template <int KERN, bool SS, int SW>
+int launch_mixed(const Work &wn, const Work &wc, const Work &wf, const LaunchShape &sh, cudaStream_t s, bool *pdl) {
+    constexpr int ST = 32 * SW;
+    const bool one = sh.nt == 1, deg7 = sh.maxn1 == 8 && sh.minn1 == 8;
+    if (one) TAGI_TRY(launch_persistent(near_mixed<KERN, SS, 1, 0, SW>, wn, s, 0, ST, pdl));
+    else TAGI_TRY(launch_persistent(near_mixed<KERN, SS, 2, 0, SW>, wn, s, 0, ST, pdl));
+    phase_mark(PH_NEAR, false, s);
+    phase_mark(PH_NEAR_CLOSE, true, s);
+    if (one) TAGI_TRY(launch_persistent(near_mixed<KERN, SS, 1, 1, SW>, wc, s, 0, ST, pdl));
+    else TAGI_TRY(launch_persistent(near_mixed<KERN, SS, 2, 1, SW>, wc, s, 0, ST, pdl));
+    phase_mark(PH_NEAR_CLOSE, false, s);
+    phase_mark(PH_FAR, true, s);
+    if (one) {
+        if (sh.maxn1 <= 4) TAGI_TRY(launch_persistent(far_mixed<KERN, SS, 4, 1, SW>, wf, s, 0, ST, pdl));
+        else if (deg7) TAGI_TRY(launch_persistent(far_mixed<KERN, SS, 8, 1, SW, true>, wf, s, 0, ST, pdl));
+        else if (sh.maxn1 <= 8) TAGI_TRY(launch_persistent(far_mixed<KERN, SS, 8, 1, SW>, wf, s, 0, ST, pdl));
+        else TAGI_TRY(launch_persistent(far_mixed<KERN, SS, MAX_DEGREE + 1, 1, SW>, wf, s, 0, ST, pdl));
+    } else {
+        if (sh.maxn1 <= 4) TAGI_TRY(launch_persistent(far_mixed<KERN, SS, 4, 2, SW>, wf, s, 0, ST, pdl));
+        else if (deg7) TAGI_TRY(launch_persistent(far_mixed<KERN, SS, 8, 2, SW, true>, wf, s, 0, ST, pdl));
+        else if (sh.maxn1 <= 8) TAGI_TRY(launch_persistent(far_mixed<KERN, SS, 8, 2, SW>, wf, s, 0, ST, pdl));
+        else TAGI_TRY(launch_persistent(far_mixed<KERN, SS, MAX_DEGREE + 1, 2, SW>, wf, s, 0, ST, pdl));
+    }
+    phase_mark(PH_FAR, false, s);
+    return TAGI_OK;
+}
 
 template <int KERN, bool SS>
 int launch_fields(const SysCall *calls, const Fields *f, int nsys, const Schedule &sc, const LaunchShape &sh,
@@ -2356,7 +2384,6 @@ int launch_fields(const SysCall *calls, const Fields *f, int nsys, const Schedul
     wf.items = sc.items + sc.off[2];
     wf.nitems = sc.count[2];
     wf.queue = queue + 1;
-    const bool one = sh.nt == 1;
     phase_mark(PH_NEAR, true, s);
     bool pdl = false;   // no field pass of this call launched yet
     if (precision == PREC_MIXED && KERN == KERNEL_YUKAWA && sh.og == 16) {
@@ -2405,39 +2432,18 @@ int launch_fields(const SysCall *calls, const Fields *f, int nsys, const Schedul
         phase_mark(PH_FAR, false, s);
         return TAGI_OK;
     }
-    if (precision == PREC_MIXED) {
-        if (one) TAGI_TRY(launch_persistent(near_mixed<KERN, SS, 1, 0>, wn, s, 0, FT, &pdl));
-        else TAGI_TRY(launch_persistent(near_mixed<KERN, SS, 2, 0>, wn, s, 0, FT, &pdl));
-        phase_mark(PH_NEAR, false, s);
-        phase_mark(PH_NEAR_CLOSE, true, s);
-        if (one) TAGI_TRY(launch_persistent(near_mixed<KERN, SS, 1, 1>, wc, s, 0, FT, &pdl));
-        else TAGI_TRY(launch_persistent(near_mixed<KERN, SS, 2, 1>, wc, s, 0, FT, &pdl));
-        phase_mark(PH_NEAR_CLOSE, false, s);
-    } else {
+    if (precision == PREC_MIXED && sh.warps == 8) TAGI_TRY((launch_mixed<KERN, SS, 8>(wn, wc, wf, sh, s, &pdl)));
+    else if (precision == PREC_MIXED) TAGI_TRY((launch_mixed<KERN, SS, 4>(wn, wc, wf, sh, s, &pdl)));
+    if (precision != PREC_MIXED) {
         // one FP64 pass over all near ranges, close ones included
         TAGI_TRY(launch_persistent(near_f64<KERN, SS>, wn, s, f64_smem<KERN, SS>(), FT, &pdl));
         phase_mark(PH_NEAR, false, s);
-    }
-    phase_mark(PH_FAR, true, s);
-    if (precision == PREC_MIXED) {
-        const bool deg7 = sh.maxn1 == 8 && sh.minn1 == 8;
-        if (one) {
-            if (sh.maxn1 <= 4) TAGI_TRY(launch_persistent(far_mixed<KERN, SS, 4, 1>, wf, s, 0, FT, &pdl));
-            else if (deg7) TAGI_TRY(launch_persistent(far_mixed<KERN, SS, 8, 1, true>, wf, s, 0, FT, &pdl));
-            else if (sh.maxn1 <= 8) TAGI_TRY(launch_persistent(far_mixed<KERN, SS, 8, 1>, wf, s, 0, FT, &pdl));
-            else TAGI_TRY(launch_persistent(far_mixed<KERN, SS, MAX_DEGREE + 1, 1>, wf, s, 0, FT, &pdl));
-        } else {
-            if (sh.maxn1 <= 4) TAGI_TRY(launch_persistent(far_mixed<KERN, SS, 4, 2>, wf, s, 0, FT, &pdl));
-            else if (deg7) TAGI_TRY(launch_persistent(far_mixed<KERN, SS, 8, 2, true>, wf, s, 0, FT, &pdl));
-            else if (sh.maxn1 <= 8) TAGI_TRY(launch_persistent(far_mixed<KERN, SS, 8, 2>, wf, s, 0, FT, &pdl));
-            else TAGI_TRY(launch_persistent(far_mixed<KERN, SS, MAX_DEGREE + 1, 2>, wf, s, 0, FT, &pdl));
-        }
-    } else {
+        phase_mark(PH_FAR, true, s);
         if (sh.maxn1 <= 4) TAGI_TRY(launch_persistent(far_f64<KERN, SS, 4>, wf, s, f64_smem<KERN, SS>(), FT, &pdl));
         else if (sh.maxn1 <= 8) TAGI_TRY(launch_persistent(far_f64<KERN, SS, 8>, wf, s, f64_smem<KERN, SS>(), FT, &pdl));
         else TAGI_TRY(launch_persistent(far_f64<KERN, SS, MAX_DEGREE + 1>, wf, s, f64_smem<KERN, SS>(), FT, &pdl));
+        phase_mark(PH_FAR, false, s);
     }
-    phase_mark(PH_FAR, false, s);
     return TAGI_OK;
 }
 
@@ -2629,24 +2635,33 @@ bool schedule_matches(const Schedule &sc, const int *norb, int nsys, int og, int
 }
 
 // Warps that share a target's sources in the single-orbital kernels, by the
-// plan's targets: a CTA then holds 256 / split threads' targets, and a small
-// mesh still has items for every SM, while a large one stages each tile for as
-// many targets as fit.  Set by the plan and the precision, not by the launch, so
-// an FP64 sum's last bits are the same however calls are batched (mixed sums do
-// not depend on the split).
-// Measured, ms per call at split 1, 2, 4, 8 (the targets and sources in one piece
-// before: first figure): Yukawa, 50k points, plan kept 4.1 -> 4.2, 3.1, 2.0, 1.5;
-// FP64, 50k points, one shot 636 -> 333, 325, 204, 180; one shot, mixed: Coulomb, 913k
-// points, degree 6, 63.6 -> 60.3, 55.0, 45.9; 1.13M, degree 5, 61.0 -> 61.4, 68.0,
-// 60.3; 1.5M, degree 7, 114.4 -> 119.1, 115.1, 117.4, 121.2.
-int field_split(int nt, int precision) {
-    if (nt <= 131072) return 8;
-    return precision == PREC_FP64 || nt <= 1200000 ? 4 : 2;
+// plan's targets: a CTA then holds (warps / split) x 32 threads' targets, and a
+// small mesh still has items for every SM, while a large one stages each tile for
+// as many targets as fit.  An FP64 split follows from the plan alone, so the sums'
+// last bits are the same however calls are batched (mixed sums do not depend on
+// the split).  Measured, ms per call.  8 warps, split 1, 2, 4, 8 (targets and
+// sources in one piece before: first figure): Yukawa, 50k points, plan kept
+// 4.1 -> 4.2, 3.1, 2.0, 1.5; FP64, 50k points, one shot 636 -> 333, 325, 204, 180.
+// 4 warps, split 1, 2, 4, one shot: Coulomb, 913k points, degree 6 42.1, 38.9,
+// 38.6; 1.13M, degree 5 49.8, 48.1, 48.6; Yukawa, 1.34M, degree 4 73.0, 74.3, 76.7;
+// Coulomb, 1.5M, degree 7 104.1, 106.6, 106.9.
+int field_split(int nt, int warps, int precision) {
+    if (precision == PREC_FP64) return nt <= 131072 ? 8 : 4;
+    if (nt <= 131072) return warps;   // one warp of targets per CTA
+    return nt <= 1200000 ? 2 : 1;
+}
+
+// Warps per CTA of the single-orbital kernels: 8 if all systems are small.
+int field_warps(Plan *const *plans, int nsys, int precision) {
+    if (precision == PREC_FP64) return FT / 32;
+    for (int i = 0; i < nsys; i++)
+        if (plans[i]->tgt.n > 131072) return 4;
+    return 8;
 }
 
 // Targets that a CTA of the field kernels holds.
-int cta_targets(int nt, int og, int nt_per_thread, int precision) {
-    return og > 1 ? GT : FT / field_split(nt, precision) * nt_per_thread;
+int cta_targets(int nt, int og, int nt_per_thread, int warps, int precision) {
+    return og > 1 ? GT : 32 * warps / field_split(nt, warps, precision) * nt_per_thread;
 }
 
 // Targets per thread: the caller's request, else 2 where a batch holds more
@@ -2668,6 +2683,7 @@ int targets_per_thread(Plan *const *plans, int nsys, int precision, int og, int 
 int build_schedule(Plan *const *plans, const int *norb, int nsys, int og, int nt, int precision, Schedule &sc,
                    cudaStream_t s) {
     if (nsys < 1 || nsys > MAX_SYSTEMS) return set_error(TAGI_ERR_ARG, "%d systems (1..%d per launch)", nsys, MAX_SYSTEMS);
+    const int warps = field_warps(plans, nsys, precision);
     struct Batch {
         long long cost;   // pairs of one chunk
         int sys, b, begin, end, chunk;
@@ -2677,7 +2693,7 @@ int build_schedule(Plan *const *plans, const int *norb, int nsys, int og, int nt
         const Plan &p = *plans[i];
         if (norb[i] < 1 || norb[i] > 0xffff) return set_error(TAGI_ERR_ARG, "system %d: %d orbitals", i, norb[i]);
         if ((int)p.cost_near.size() != p.nbatch) return set_error(TAGI_ERR_STATE, "plan without batch costs");
-        const int warp = 32 * nt, most = cta_targets(p.tgt.n, og, nt, precision);
+        const int warp = 32 * nt, most = cta_targets(p.tgt.n, og, nt, warps, precision);
         for (int b = 0, at = 0; b < p.nbatch; at += p.batch_size[b++]) {
             const int n = p.batch_size[b], chunks = (n + most - 1) / most;
             const int chunk = ((n + chunks - 1) / chunks + warp - 1) / warp * warp;
@@ -2748,6 +2764,7 @@ int convolve_systems(SysCall *calls, int nsys, int kernel, int singularity, int 
     const bool ss = singularity == SING_SUBTRACTION;
     const bool capturing = stream_capturing(s);
     Fields f[MAX_SYSTEMS];
+    Plan *plans[MAX_SYSTEMS];
     LaunchShape sh;
     sh.og = sc.og;
     sh.nt = sc.nt;
@@ -2776,13 +2793,15 @@ int convolve_systems(SysCall *calls, int nsys, int kernel, int singularity, int 
         phase_mark(PH_UPWARD, false, s);
         if (!mixed && p.nslots && !p.what64) return set_error(TAGI_ERR_DEVICE, "FP64 weight charges missing");
         f[i] = make_fields(p, c.norb);
-        f[i].split = field_split(p.tgt.n, precision);
+        plans[i] = c.p;
         if (p.n1 > sh.maxn1) sh.maxn1 = p.n1;
         if (p.n1 < sh.minn1) sh.minn1 = p.n1;
         // the far and close-range passes write only the batches they visit
         TAGI_CUDA(cudaMemsetAsync(p.far_out, 0, sizeof(double) * (size_t)c.norb * nt, s));
         TAGI_CUDA(cudaMemsetAsync(p.near2_out, 0, sizeof(double) * (size_t)c.norb * nt, s));
     }
+    sh.warps = field_warps(plans, nsys, precision);
+    for (int i = 0; i < nsys; i++) f[i].split = field_split(plans[i]->tgt.n, sh.warps, precision);
     TAGI_CUDA(cudaMemsetAsync(queue, 0, 3 * sizeof(int), s));
     if (kernel == KERNEL_YUKAWA) {
         if (ss) TAGI_TRY((launch_fields<KERNEL_YUKAWA, true>(calls, f, nsys, sc, sh, precision, queue, s)));
