@@ -74,3 +74,13 @@ def test_lists_partition_sources(dev, small_mesh):
             c = lists["far_list"][e]
             cover[st["begin"][c]:st["end"][c]] += 1
         assert cover.min() == 1 and cover.max() == 1, f"batch {b}"
+
+
+@pytest.mark.parametrize("n", [1, 255, 257, 4099, 16384, 16385])
+def test_order_at_the_sort_switch(dev, oracle, n):
+    """Counting sort and radix passes meet at 16,384 points: order of equal codes
+    (points drawn from 1/4 as many places, on both sides of zero), boxes and lists."""
+    rng = np.random.default_rng(n)
+    pts = rng.uniform(-1, 1, ((n + 3) // 4, 3))[rng.integers(0, (n + 3) // 4, n)]
+    g, c = _plans(dev, oracle, pts, pts, np.ones(n), 0.8, 3, 300, 300)
+    _compare(g, c)

@@ -28,7 +28,7 @@
 // bit-identical to the reference's on the same 1-D node and weight tables.
 // Ring molecule, 5,104 cells, 16.9M points, build_mesh 2.38 -> 1.19 ms: the nearest corner
 // of a cell from the smallest square along each axis with one root per cell (eight
-// corners, a root each, per atom before: 92 us a level), leaves sorted by one block,
+// corners, a root each, per atom before: 92 us a level), leaves sorted in two launches,
 // scans of a level in one launch, and one refinement instead of a counting one first.
 #include "tagi_internal.h"
 
@@ -411,13 +411,12 @@ int tagi_mesh_refine(const double *baseCells, int numBase, const double *atomXYZ
     tmp.stream = s;
     int rc = TAGI_OK;
     do {
-        int *err = nullptr, *hcnt = nullptr;
+        int *err = nullptr;
         double *cells = nullptr;
         uint64_t *keys = nullptr;
         if ((rc = tmp.alloc(&err, 2)) || (rc = tmp.alloc(&cells, 6L * numBase)) ||
             (rc = tmp.alloc(&keys, numBase)))
             break;
-        (void)hcnt;
         if (cudaMemsetAsync(err, 0, 2 * sizeof(int), s) != cudaSuccess ||
             cudaMemcpyAsync(cells, baseCells, sizeof(double) * 6 * numBase, cudaMemcpyDeviceToDevice, s) !=
                 cudaSuccess) {
@@ -437,7 +436,8 @@ int tagi_mesh_refine(const double *baseCells, int numBase, const double *atomXYZ
             int *divide = nullptr, *fine = nullptr, *rank = nullptr;
             if ((rc = tmp.alloc(&divide, n)) || (rc = tmp.alloc(&fine, n)) || (rc = tmp.alloc(&rank, n + 1)))
                 break;
-            launch(mesh_classify, grid_for(n), MT, 0, s, cells, (int)n, depth, atomXYZ, numAtoms, p, divide,
+            // small blocks: a level has 500 to 5,000 cells, a chain of FP64 operations each
+            launch(mesh_classify, (unsigned)((n + 31) / 32), 32, 0, s, cells, (int)n, depth, atomXYZ, numAtoms, p, divide,
                    fine, err);
             if (cudaGetLastError() != cudaSuccess) {
                 rc = set_error(TAGI_ERR_CUDA, "mesh_classify launch failed");

@@ -159,6 +159,7 @@ constexpr int TC_M = 128, TC_N = 128, TC_K = 64, TC_STAGES = 3, TC_THREADS = 128
 constexpr int TC_TILE = 128 * TC_K * 2;                 // bytes of one operand's tile
 constexpr int TC_PITCH = TC_N + 4;                      // floats per staged row of C
 constexpr size_t TC_SMEM = 1024 + (size_t)TC_STAGES * 2 * TC_TILE;
+static_assert(TC_SMEM * 5 > 228 * 1024, "at most four blocks of 128 TMEM columns each may share an SM");
 static_assert((size_t)TC_M * TC_PITCH * 4 <= (size_t)TC_STAGES * 2 * TC_TILE, "C tile in the ring's memory");
 constexpr int TC_SPINS = 1 << 20;                       // tries of a barrier wait before it gives up
 
@@ -213,6 +214,10 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc(const __grid_constant__ CU
     __shared__ __align__(8) uint64_t s_full[TC_STAGES], s_empty[TC_STAGES], s_done;
     __shared__ unsigned s_tmem;
     __shared__ int s_fail;
+    // Early: this grid is resident as a whole by then, and the next kernel's blocks wait
+    // only for it.  A next gemm_tc takes its 128 TMEM columns before this one ends; shared
+    // memory allows at most two of these blocks on an SM, so all of them find columns.
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const GemmArgs &g = t.g;
     char *ring = s_raw + (1024 - (smem_u32(s_raw) & 1023)) % 1024;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -237,6 +242,7 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc(const __grid_constant__ CU
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const unsigned tmem = s_tmem;
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     if (tid == 0) {   // copies
         for (int i = 0; i < steps; i++) {
             const int st = i % TC_STAGES;
@@ -411,7 +417,7 @@ int run_gemm(GemmArgs g, int splits, int *used, cudaStream_t s) {
         t.g = g;
         TAGI_CUDA(cudaFuncSetAttribute(gemm_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM));
         dim3 grid((g.N + TC_N - 1) / TC_N, (g.M + TC_M - 1) / TC_M, *used);
-        launch(gemm_tc, grid, TC_THREADS, TC_SMEM, s, ma, mb, t);
+        TAGI_CUDA(launch_chained(gemm_tc, grid, TC_THREADS, TC_SMEM, s, ma, mb, t));
     } else {
         dim3 grid((g.N + BN - 1) / BN, (g.M + BM - 1) / BM, *used);
         launch(gemm_bf16, grid, GEMM_THREADS, 0, s, g);
@@ -422,6 +428,7 @@ int run_gemm(GemmArgs g, int splits, int *used, cudaStream_t s) {
 
 // out[m][n] = sum over splits of part[s][m][n] (fixed order)
 __global__ void splitk_reduce(const float *__restrict__ part, int splits, long mn, float *__restrict__ out) {
+    chain_begin();
     const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= mn) return;
     float s = 0.f;
@@ -534,6 +541,7 @@ __device__ __forceinline__ float to_f<__nv_bfloat16>(__nv_bfloat16 v) { return _
 template <typename T>
 __device__ __forceinline__ float column_sum(const T *__restrict__ G, long r0, long r1, int N, int j) {
     __shared__ float sh[COL_GROUPS][33];
+    chain_begin();
     float s = 0.f;
     if (j < N) {
 #pragma unroll 8
@@ -693,7 +701,7 @@ int tagi_mlp_gemm_splitk(const void *A, long long sAm, long long sAk, const void
     cudaStream_t s = (cudaStream_t)stream;
     TAGI_TRY(run_gemm(g, splits, &splits, s));
     const long mn = (long)M * N;
-    launch(splitk_reduce, (unsigned)((mn + 255) / 256), 256, 0, s, partial, splits, mn, C);
+    TAGI_CUDA(launch_chained(splitk_reduce, (unsigned)((mn + 255) / 256), 256, 0, s, partial, splits, mn, C));
     TAGI_LAUNCH_CHECK();
     return TAGI_OK;
 }
@@ -743,10 +751,11 @@ int tagi_mlp_colsum(const void *G, int isBf16, long long rows, int N, float *out
     const int chunks = (int)((rows + COL_ROWS - 1) / COL_ROWS);
     const dim3 g(chunks, (N + 31) / 32), t(32, COL_GROUPS);
     if (isBf16)
-        launch(colsum_partial<__nv_bfloat16>, g, t, 0, s, static_cast<const __nv_bfloat16 *>(G), (long)rows, N, work);
+        TAGI_CUDA(launch_chained(colsum_partial<__nv_bfloat16>, g, t, 0, s, static_cast<const __nv_bfloat16 *>(G),
+                                 (long)rows, N, work));
     else
-        launch(colsum_partial<float>, g, t, 0, s, static_cast<const float *>(G), (long)rows, N, work);
-    launch(colsum_final, (N + 31) / 32, t, 0, s, work, chunks, N, out);
+        TAGI_CUDA(launch_chained(colsum_partial<float>, g, t, 0, s, static_cast<const float *>(G), (long)rows, N, work));
+    TAGI_CUDA(launch_chained(colsum_final, (N + 31) / 32, t, 0, s, work, chunks, N, out));
     TAGI_LAUNCH_CHECK();
     return TAGI_OK;
 }

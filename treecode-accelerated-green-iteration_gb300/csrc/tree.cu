@@ -25,29 +25,44 @@ namespace tagi {
 
 namespace {
 
-__device__ __forceinline__ double dmin(double a, double b) { return a < b ? a : b; }
 __device__ __forceinline__ double dmax(double a, double b) { return a > b ? a : b; }
-
-__global__ void bbox_partial(const double *__restrict__ x, const double *__restrict__ y,
-                             const double *__restrict__ z, int n, double *__restrict__ part) {
-    double l[3] = {x[0], y[0], z[0]}, h[3] = {x[0], y[0], z[0]};
-    for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-         i += (long)gridDim.x * blockDim.x) {
-        double p[3] = {x[i], y[i], z[i]};
-#pragma unroll
-        for (int d = 0; d < 3; d++) {
-            l[d] = dmin(l[d], p[d]);
-            h[d] = dmax(h[d], p[d]);
-        }
-    }
+// FP64 comparisons go through the FP64 pipe (1/64 of the integer rate): smallest
+// and largest coordinates are taken on the bit patterns, mapped to integers of the
+// same order (-0 below +0).
+__device__ __forceinline__ long long ordered(double x) {
+    const long long v = __double_as_longlong(x);
+    return v ^ ((v >> 63) & 0x7fffffffffffffffLL);
+}
+__device__ __forceinline__ double from_ordered(long long v) {
+    return __longlong_as_double(v ^ ((v >> 63) & 0x7fffffffffffffffLL));
+}
+__device__ __forceinline__ void warp_minmax(long long (&l)[3], long long (&h)[3]) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1)
 #pragma unroll
         for (int d = 0; d < 3; d++) {
-            l[d] = dmin(l[d], __shfl_xor_sync(0xffffffffu, l[d], o));
-            h[d] = dmax(h[d], __shfl_xor_sync(0xffffffffu, h[d], o));
+            l[d] = min(l[d], __shfl_xor_sync(0xffffffffu, l[d], o));
+            h[d] = max(h[d], __shfl_xor_sync(0xffffffffu, h[d], o));
         }
-    __shared__ double sl[32][6];
+}
+
+__global__ void bbox_partial(const double *__restrict__ x, const double *__restrict__ y,
+                             const double *__restrict__ z, int n, long long *__restrict__ part) {
+    long long l[3], h[3];
+    l[0] = h[0] = ordered(x[0]);
+    l[1] = h[1] = ordered(y[0]);
+    l[2] = h[2] = ordered(z[0]);
+    for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
+         i += (long)gridDim.x * blockDim.x) {
+        const long long p[3] = {ordered(x[i]), ordered(y[i]), ordered(z[i])};
+#pragma unroll
+        for (int d = 0; d < 3; d++) {
+            l[d] = min(l[d], p[d]);
+            h[d] = max(h[d], p[d]);
+        }
+    }
+    warp_minmax(l, h);
+    __shared__ long long sl[32][6];
     int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     if (lane == 0)
         for (int d = 0; d < 3; d++) {
@@ -58,8 +73,8 @@ __global__ void bbox_partial(const double *__restrict__ x, const double *__restr
     if (threadIdx.x == 0) {
         for (int w = 1; w < (int)(blockDim.x >> 5); w++)
             for (int d = 0; d < 3; d++) {
-                sl[0][d] = dmin(sl[0][d], sl[w][d]);
-                sl[0][3 + d] = dmax(sl[0][3 + d], sl[w][3 + d]);
+                sl[0][d] = min(sl[0][d], sl[w][d]);
+                sl[0][3 + d] = max(sl[0][3 + d], sl[w][3 + d]);
             }
         for (int d = 0; d < 6; d++) part[blockIdx.x * 6 + d] = sl[0][d];
     }
@@ -67,35 +82,33 @@ __global__ void bbox_partial(const double *__restrict__ x, const double *__restr
 
 // params[0..2] = lower corner, params[3] = 2^21 / cube edge.  One block
 // reduces the per-block partials (min/max are exact in any order).
-__global__ void __launch_bounds__(256) bbox_final(const double *__restrict__ part, int nb,
+__global__ void __launch_bounds__(256) bbox_final(const long long *__restrict__ part, int nb,
                                                   double *__restrict__ params) {
-    double l[3] = {part[0], part[1], part[2]}, h[3] = {part[3], part[4], part[5]};
+    long long ol[3] = {part[0], part[1], part[2]}, oh[3] = {part[3], part[4], part[5]};
     for (int b = threadIdx.x; b < nb; b += blockDim.x)
         for (int d = 0; d < 3; d++) {
-            l[d] = dmin(l[d], part[b * 6 + d]);
-            h[d] = dmax(h[d], part[b * 6 + 3 + d]);
+            ol[d] = min(ol[d], part[b * 6 + d]);
+            oh[d] = max(oh[d], part[b * 6 + 3 + d]);
         }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-        for (int d = 0; d < 3; d++) {
-            l[d] = dmin(l[d], __shfl_xor_sync(0xffffffffu, l[d], o));
-            h[d] = dmax(h[d], __shfl_xor_sync(0xffffffffu, h[d], o));
-        }
-    __shared__ double sl[8][6];
+    warp_minmax(ol, oh);
+    __shared__ long long sl[8][6];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     if (lane == 0)
         for (int d = 0; d < 3; d++) {
-            sl[wid][d] = l[d];
-            sl[wid][3 + d] = h[d];
+            sl[wid][d] = ol[d];
+            sl[wid][3 + d] = oh[d];
         }
     __syncthreads();
     if (threadIdx.x != 0) return;
-    for (int w = 1; w < (int)(blockDim.x >> 5); w++)
-        for (int d = 0; d < 3; d++) {
-            l[d] = dmin(l[d], sl[w][d]);
-            h[d] = dmax(h[d], sl[w][3 + d]);
+    double l[3], h[3];
+    for (int d = 0; d < 3; d++) {
+        for (int w = 1; w < (int)(blockDim.x >> 5); w++) {
+            ol[d] = min(ol[d], sl[w][d]);
+            oh[d] = max(oh[d], sl[w][3 + d]);
         }
+        l[d] = from_ordered(ol[d]);
+        h[d] = from_ordered(oh[d]);
+    }
     double ext = __dsub_rn(h[0], l[0]);
     if (__dsub_rn(h[1], l[1]) > ext) ext = __dsub_rn(h[1], l[1]);
     if (__dsub_rn(h[2], l[2]) > ext) ext = __dsub_rn(h[2], l[2]);
@@ -303,43 +316,40 @@ __global__ void __launch_bounds__(256) node_boxes(const int *__restrict__ hdr, c
                                                   const int *__restrict__ end, const int *__restrict__ parent,
                                                   const int *__restrict__ first_child, const int *__restrict__ nchild,
                                                   const double *__restrict__ x, const double *__restrict__ y,
-                                                  const double *__restrict__ z, double *box, double *__restrict__ center,
+                                                  const double *__restrict__ z, long long *box, double *__restrict__ center,
                                                   double *__restrict__ half, double *__restrict__ radius, int *size,
                                                   int *leaves, int *done) {
     const int nn = hdr[0], lane = threadIdx.x & 31;
     for (int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < nn; w += (gridDim.x * blockDim.x) >> 5) {
         if (nchild[w]) continue;
-        double l[3] = {INFINITY, INFINITY, INFINITY}, h[3] = {-INFINITY, -INFINITY, -INFINITY};
+        const long long top = ordered(INFINITY), bottom = ordered(-INFINITY);
+        long long l[3] = {top, top, top}, h[3] = {bottom, bottom, bottom};
         int sz = 0, lv = 0;   // of the children (lane 0's own start below)
-        for (int i = begin[w] + lane; i < end[w]; i += 32) {
-            const double p[3] = {x[i], y[i], z[i]};
+        const int e = end[w];
+#pragma unroll 4
+        for (int i = begin[w] + lane; i < e; i += 32) {
+            const long long p[3] = {ordered(x[i]), ordered(y[i]), ordered(z[i])};
 #pragma unroll
             for (int d = 0; d < 3; d++) {
-                l[d] = dmin(l[d], p[d]);
-                h[d] = dmax(h[d], p[d]);
+                l[d] = min(l[d], p[d]);
+                h[d] = max(h[d], p[d]);
             }
         }
         for (int v = w;;) {
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-#pragma unroll
-                for (int d = 0; d < 3; d++) {
-                    l[d] = dmin(l[d], __shfl_xor_sync(0xffffffffu, l[d], o));
-                    h[d] = dmax(h[d], __shfl_xor_sync(0xffffffffu, h[d], o));
-                }
-                sz += __shfl_xor_sync(0xffffffffu, sz, o);
-                lv += __shfl_xor_sync(0xffffffffu, lv, o);
-            }
+            warp_minmax(l, h);
+            sz = __reduce_add_sync(0xffffffffu, sz);
+            lv = __reduce_add_sync(0xffffffffu, lv);
             int last = 0;
             const int pv = parent[v];
             if (lane == 0) {
                 double hh[3];
 #pragma unroll
                 for (int d = 0; d < 3; d++) {
+                    const double lo = from_ordered(l[d]), hi = from_ordered(h[d]);
                     __stcg(box + 6L * v + d, l[d]);
                     __stcg(box + 6L * v + 3 + d, h[d]);
-                    center[3L * v + d] = __dmul_rn(__dadd_rn(l[d], h[d]), 0.5);
-                    hh[d] = __dmul_rn(__dsub_rn(h[d], l[d]), 0.5);
+                    center[3L * v + d] = __dmul_rn(__dadd_rn(lo, hi), 0.5);
+                    hh[d] = __dmul_rn(__dsub_rn(hi, lo), 0.5);
                     half[3L * v + d] = hh[d];
                 }
                 double s = __dmul_rn(hh[0], hh[0]);
@@ -361,8 +371,8 @@ __global__ void __launch_bounds__(256) node_boxes(const int *__restrict__ hdr, c
             const bool has = lane < nchild[v];
 #pragma unroll
             for (int d = 0; d < 3; d++) {
-                l[d] = has ? __ldcg(box + 6L * c + d) : INFINITY;
-                h[d] = has ? __ldcg(box + 6L * c + 3 + d) : -INFINITY;
+                l[d] = has ? __ldcg(box + 6L * c + d) : top;
+                h[d] = has ? __ldcg(box + 6L * c + 3 + d) : bottom;
             }
             sz = has ? __ldcg(size + c) : 0;
             lv = has ? __ldcg(leaves + c) : 0;
@@ -422,7 +432,8 @@ int build_tree(Tree &t, const double *x, const double *y, const double *z, int n
     int rc = TAGI_OK;
     do {
         const int nbb = std::min(1024, (n + 255) / 256);
-        double *part = nullptr, *params = nullptr;
+        long long *part = nullptr;
+        double *params = nullptr;
         if ((rc = tmp.alloc(&part, 6L * nbb))) break;
         if ((rc = tmp.alloc(&params, 4))) break;
         launch(bbox_partial, nbb, 256, 0, s, x, y, z, n, part);
@@ -477,7 +488,7 @@ int build_tree(Tree &t, const double *x, const double *y, const double *z, int n
             launch(write_header, 1, 1, 0, s, hdr, t.nnodes);
         }
         const long nodes = small ? cap : t.nnodes;
-        double *box = nullptr;
+        long long *box = nullptr;   // lower and upper corners, ordered()
         int *work = nullptr;
         if ((rc = tmp.alloc(&box, 6 * nodes)) || (rc = tmp.alloc(&work, 3 * nodes)) ||
             (rc = ar.alloc(&t.center, 3 * nodes)) || (rc = ar.alloc(&t.half, 3 * nodes)) ||
