@@ -182,3 +182,38 @@ def test_tma_gemm_matches_numpy(L, native, mo, M, N, K, ta, tb):
     D = torch.zeros(M, N, dtype=torch.bfloat16, device="cuda")
     native.check(L.tagi_mlp_gemm(_p(At), sAm, sAk, _p(Bt), sBk, sBn, M, N, K, 2, None, _p(D), N, None, _p(mask), None))
     assert rel_l2(D.float().cpu().numpy(), ref * (mask.float().cpu().numpy() > 0)) <= 1e-2
+
+
+# Operands that TMA cannot read: odd rows, strides other than one on both axes, bases off
+# 16 bytes; one operand or both.
+@pytest.mark.parametrize("M,N,K", [(1, 1, 1), (125, 131, 65), (300, 343, 577), (129, 256, 125)])
+@pytest.mark.parametrize("a", ["rows", "columns", "strided"])
+@pytest.mark.parametrize("b", ["rows", "columns", "strided", "aligned"])
+def test_gemm_of_unaligned_operands(L, native, mo, M, N, K, a, b):
+    rng = np.random.default_rng(M + N + K)
+
+    def operand(x, kind):   # x[i, j]: device memory whose element (i, j) lies at i s0 + j s1
+        r, c = x.shape
+        ld = (c + 7) // 8 * 8 if kind == "aligned" else 2 * c + 1 if kind == "strided" else c + (c % 2 == 0)
+        if kind == "columns":
+            return operand(x.T, "rows")[:2] + operand(x.T, "rows")[:1:-1]
+        step = 2 if kind == "strided" else 1
+        off = 0 if kind == "aligned" else 1
+        buf = torch.full((off + r * ld,), float("nan"), dtype=torch.bfloat16, device="cuda")
+        buf[off:].view(r, ld)[:, :step * c:step] = _bf(x)
+        return buf, off, ld, step
+
+    A = mo.bf16(rng.standard_normal((M, K)).astype(np.float32))
+    B = mo.bf16(rng.standard_normal((K, N)).astype(np.float32))
+    Ab, ao, sAm, sAk = operand(A, a)
+    Bb, bo, sBk, sBn = operand(B, b)
+    ref = A.astype(np.float64) @ B.astype(np.float64)
+    C = torch.full((M, N), float("nan"), dtype=torch.float32, device="cuda")
+    native.check(L.tagi_mlp_gemm(_p(Ab[ao:]), sAm, sAk, _p(Bb[bo:]), sBk, sBn, M, N, K, 0, _p(C), None, N, None, None,
+                                 None))
+    assert rel_l2(C.cpu().numpy(), ref) <= 1e-5
+    part = torch.full((3 * M * N,), float("nan"), dtype=torch.float32, device="cuda")
+    C2 = torch.full_like(C, float("nan"))
+    native.check(L.tagi_mlp_gemm_splitk(_p(Ab[ao:]), sAm, sAk, _p(Bb[bo:]), sBk, sBn, M, N, K, 3, _p(part), _p(C2),
+                                        None))
+    assert rel_l2(C2.cpu().numpy(), ref) <= 1e-5

@@ -16,9 +16,9 @@
 // GEMMs run on the tensor cores, BF16 in, FP32 accumulate: C[M x N] =
 // A[M x K] B[K x N] with strides, so the transposes of the backward pass need
 // no copies.  Operands that TMA can read (one unit stride, the other a multiple
-// of 16 bytes, base 16-byte aligned) take gemm_tc (tcgen05, accumulators in
-// TMEM); others, such as rows of 125 or 343 patch points, take gemm_bf16
-// (warp-level mma.sync, element-wise staging).  Weight gradients split K across
+// of 16 bytes, base 16-byte aligned) are copied by TMA; others, such as rows of 125
+// or 343 patch points, by warps.  Both feed the same tcgen05 kernel (gemm_tc,
+// accumulators in TMEM).  Weight gradients split K across
 // blocks into partial sums that a second kernel adds in a fixed order: results
 // do not depend on scheduling.
 #include "tagi_internal.h"
@@ -29,9 +29,6 @@
 namespace tagi {
 
 namespace {
-
-constexpr int BM = 64, BN = 64, BK = 32;
-constexpr int GEMM_THREADS = 128;  // 4 warps, 2 x 2, 32 x 32 each
 
 enum { EPI_F32 = 0, EPI_BIAS_RELU_BF16 = 1, EPI_MASK_BF16 = 2, EPI_BIAS_F32 = 3 };
 
@@ -52,96 +49,6 @@ __device__ __forceinline__ unsigned pack2(__nv_bfloat16 lo, __nv_bfloat16 hi) {
     return (unsigned)__bfloat16_as_ushort(lo) | ((unsigned)__bfloat16_as_ushort(hi) << 16);
 }
 
-__device__ __forceinline__ void mma_bf16(float (&d)[4], unsigned a0, unsigned a1, unsigned a2, unsigned a3,
-                                         unsigned b0, unsigned b1) {
-    asm volatile(
-        "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
-        "{%0,%1,%2,%3};\n"
-        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-
-__global__ void __launch_bounds__(GEMM_THREADS) gemm_bf16(const GemmArgs g) {
-    __shared__ __nv_bfloat16 As[BM][BK + 8];
-    __shared__ __nv_bfloat16 Bs[BK][BN + 8];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int wm = (warp >> 1) * 32, wn = (warp & 1) * 32;
-    const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-    const int kb = blockIdx.z * g.k_per_split;
-    const int ke = min(g.K, kb + g.k_per_split);
-    const __nv_bfloat16 zero = __float2bfloat16(0.f);
-    float acc[2][4][4];
-#pragma unroll
-    for (int i = 0; i < 2; i++)
-#pragma unroll
-        for (int j = 0; j < 4; j++)
-#pragma unroll
-            for (int e = 0; e < 4; e++) acc[i][j][e] = 0.f;
-    for (int k0 = kb; k0 < ke; k0 += BK) {
-        // stage A[m0..m0+63][k0..k0+31] and B[k0..k0+31][n0..n0+63], zero outside
-        for (int e = tid; e < BM * BK; e += GEMM_THREADS) {
-            const int r = e / BK, c = e - r * BK;
-            const int m = m0 + r, k = k0 + c;
-            As[r][c] = (m < g.M && k < ke) ? g.A[(long)m * g.sAm + (long)k * g.sAk] : zero;
-        }
-        for (int e = tid; e < BK * BN; e += GEMM_THREADS) {
-            const int r = e / BN, c = e - r * BN;
-            const int k = k0 + r, n = n0 + c;
-            Bs[r][c] = (k < ke && n < g.N) ? g.B[(long)k * g.sBk + (long)n * g.sBn] : zero;
-        }
-        __syncthreads();
-#pragma unroll
-        for (int kk = 0; kk < BK; kk += 16) {
-            unsigned af[2][4], bfr[4][2];
-            const int ar = lane >> 2, ac = kk + 2 * (lane & 3);
-#pragma unroll
-            for (int i = 0; i < 2; i++) {
-                const int r = wm + i * 16 + ar;
-                af[i][0] = pack2(As[r][ac], As[r][ac + 1]);
-                af[i][1] = pack2(As[r + 8][ac], As[r + 8][ac + 1]);
-                af[i][2] = pack2(As[r][ac + 8], As[r][ac + 9]);
-                af[i][3] = pack2(As[r + 8][ac + 8], As[r + 8][ac + 9]);
-            }
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-                const int n = wn + j * 8 + (lane >> 2);
-                bfr[j][0] = pack2(Bs[ac][n], Bs[ac + 1][n]);
-                bfr[j][1] = pack2(Bs[ac + 8][n], Bs[ac + 9][n]);
-            }
-#pragma unroll
-            for (int i = 0; i < 2; i++)
-#pragma unroll
-                for (int j = 0; j < 4; j++)
-                    mma_bf16(acc[i][j], af[i][0], af[i][1], af[i][2], af[i][3], bfr[j][0], bfr[j][1]);
-        }
-        __syncthreads();
-    }
-    // epilogue: fragment element e -> row (lane/4) + 8 (e >= 2), col 2 (lane%4) + (e & 1)
-#pragma unroll
-    for (int i = 0; i < 2; i++)
-#pragma unroll
-        for (int j = 0; j < 4; j++)
-#pragma unroll
-            for (int e = 0; e < 4; e++) {
-                const int m = m0 + wm + i * 16 + (lane >> 2) + (e >= 2 ? 8 : 0);
-                const int n = n0 + wn + j * 8 + 2 * (lane & 3) + (e & 1);
-                if (m >= g.M || n >= g.N) continue;
-                float v = acc[i][j][e];
-                const long o = (long)m * g.sCm + n;
-                if (g.epi == EPI_F32) {
-                    g.C32[(long)blockIdx.z * g.M * g.sCm + o] = v;
-                } else if (g.epi == EPI_BIAS_F32) {
-                    g.C32[o] = v + g.bias[n];
-                } else if (g.epi == EPI_BIAS_RELU_BF16) {
-                    v += g.bias[n];
-                    g.C16[o] = __float2bfloat16_rn(v > 0.f ? v : 0.f);
-                } else {  // EPI_MASK_BF16
-                    const float keep = __bfloat162float(g.mask[o]) > 0.f ? 1.f : 0.f;
-                    g.C16[o] = __float2bfloat16_rn(v * keep);
-                }
-            }
-}
-
 // ---------------------------------------------------------------------------
 // gemm_tc: one 128 x 128 tile of C per CTA on the 5th-generation tensor cores.
 // Bound: at the extrapolator's sizes (10,752 rows, 256 wide) reading the
@@ -152,10 +59,14 @@ __global__ void __launch_bounds__(GEMM_THREADS) gemm_bf16(const GemmArgs g) {
 // through shared memory so that rows of C are written in whole sectors.  A tile
 // of either operand may lie K-major (rows of 64 k) or MN-major (rows of 64 m or n:
 // the weight gradients' transposes); TMA fills elements outside the matrix with 0.
-// 10,752 rows of 512-point patches, hidden width 256: five GEMMs and a column sum
-// 872 -> 157 us (mma.sync with element-wise staging before).
+// SA, SB: that operand's tiles come from eight more warps, which load 2 bytes per
+// element (a row may start at any of them) into registers while the previous stage is
+// read, and store them in the layout that TMA would have written.
+// Five GEMMs and a column sum, hidden width 256, before with mma.sync and element-wise
+// staging: 10,752 rows of 512-point patches 872 -> 110 us, 6,090 rows of 125 points
+// 480 -> 114 us (219 with mma.sync in the two products that TMA cannot read).
 // ---------------------------------------------------------------------------
-constexpr int TC_M = 128, TC_N = 128, TC_K = 64, TC_STAGES = 3, TC_THREADS = 128;
+constexpr int TC_M = 128, TC_N = 128, TC_K = 64, TC_STAGES = 3, TC_THREADS = 128, TC_LOADERS = 256;
 constexpr int TC_TILE = 128 * TC_K * 2;                 // bytes of one operand's tile
 constexpr int TC_PITCH = TC_N + 4;                      // floats per staged row of C
 constexpr size_t TC_SMEM = 1024 + (size_t)TC_STAGES * 2 * TC_TILE;
@@ -207,9 +118,35 @@ struct TcArgs {
 
 __device__ int g_tc_timeout;   // set by a CTA whose barrier wait gave up (its tile of C is NaN)
 
-__global__ void __launch_bounds__(TC_THREADS) gemm_tc(const __grid_constant__ CUtensorMap mapA,
-                                                      const __grid_constant__ CUtensorMap mapB,
-                                                      const __grid_constant__ TcArgs t) {
+// Rows of 64 consecutive k (K-major) or of 64 m of one k (MN-major) starting at row
+// `first` of a tile, `step` rows apart: the pair of elements at 2 lane, packed.
+template <int ROWS>
+__device__ __forceinline__ void load_rows(unsigned (&v)[ROWS], const __nv_bfloat16 *base, long smn, long sk, bool k_major,
+                                          int i0, int mn, int k0, int K, int first, int step, int lane) {
+    const unsigned short *p = reinterpret_cast<const unsigned short *>(base);
+#pragma unroll
+    for (int r = 0; r < ROWS; r++) {
+        const int row = first + r * step, c = 2 * lane;
+        const int i = k_major ? i0 + row : i0 + (row & 64) + c, k = k_major ? k0 + c : k0 + (row & 63);
+        const long o = i * smn + k * sk;
+        const bool in0 = i < mn && k < K, in1 = k_major ? i < mn && k + 1 < K : i + 1 < mn && k < K;
+        const unsigned lo = in0 ? __ldg(p + o) : 0, hi = in1 ? __ldg(p + o + (k_major ? sk : smn)) : 0;
+        v[r] = lo | hi << 16;
+    }
+}
+template <int ROWS>
+__device__ __forceinline__ void store_rows(const unsigned (&v)[ROWS], char *tile, int first, int step, int lane) {
+#pragma unroll
+    for (int r = 0; r < ROWS; r++) {
+        const int row = first + r * step;   // 128-byte swizzle: 16-byte piece c of row r lies at c ^ (r mod 8)
+        *reinterpret_cast<unsigned *>(tile + row * 128 + (((lane >> 2) ^ (row & 7)) << 4) + ((lane & 3) << 2)) = v[r];
+    }
+}
+
+template <bool SA, bool SB>
+__global__ void __launch_bounds__(TC_THREADS + (SA || SB ? TC_LOADERS : 0), 2) gemm_tc(
+    const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB, const __grid_constant__ TcArgs t) {
+    constexpr int WARPS = (TC_THREADS + (SA || SB ? TC_LOADERS : 0)) / 32, LW = TC_LOADERS / 32, ROWS = 128 / LW;
     extern __shared__ char s_raw[];
     __shared__ __align__(8) uint64_t s_full[TC_STAGES], s_empty[TC_STAGES], s_done;
     __shared__ unsigned s_tmem;
@@ -231,7 +168,7 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc(const __grid_constant__ CU
     }
     if (tid == 0) {
         for (int i = 0; i < TC_STAGES; i++) {
-            mbar_init(&s_full[i], 1);
+            mbar_init(&s_full[i], (SA && SB ? 0 : 1) + (SA || SB ? LW : 0));
             mbar_init(&s_empty[i], 1);
         }
         mbar_init(&s_done, 1);
@@ -243,7 +180,7 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc(const __grid_constant__ CU
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const unsigned tmem = s_tmem;
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    if (tid == 0) {   // copies
+    if ((!SA || !SB) && tid == 0) {   // copies
         for (int i = 0; i < steps; i++) {
             const int st = i % TC_STAGES;
             char *a = ring + st * 2 * TC_TILE, *b = a + TC_TILE;
@@ -252,14 +189,16 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc(const __grid_constant__ CU
                 break;
             }
             const int k = kb + i * TC_K;
-            mbar_expect(&s_full[st], 2 * TC_TILE);
-            if (t.a_kmajor) {
+            mbar_expect(&s_full[st], (SA || SB ? 1 : 2) * TC_TILE);
+            if (SA) {
+            } else if (t.a_kmajor) {
                 tma_load(a, &mapA, k, m0, &s_full[st]);
             } else {
                 tma_load(a, &mapA, m0, k, &s_full[st]);
                 tma_load(a + TC_TILE / 2, &mapA, m0 + 64, k, &s_full[st]);
             }
-            if (t.b_kmajor) {
+            if (SB) {
+            } else if (t.b_kmajor) {
                 tma_load(b, &mapB, k, n0, &s_full[st]);
             } else {
                 tma_load(b, &mapB, n0, k, &s_full[st]);
@@ -298,6 +237,26 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc(const __grid_constant__ CU
         asm volatile(
             "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(&s_done))
             : "memory");
+    } else if ((SA || SB) && warp >= TC_THREADS / 32) {   // loads by warps
+        const int w = warp - TC_THREADS / 32;
+        for (int i = 0; i < steps; i++) {
+            const int st = i % TC_STAGES, k = kb + i * TC_K;
+            char *a = ring + st * 2 * TC_TILE;
+            unsigned va[SA ? ROWS : 1], vb[SB ? ROWS : 1];
+            if (SA) load_rows(va, g.A, g.sAm, g.sAk, t.a_kmajor, m0, g.M, k, g.K, w, LW, lane);
+            if (SB) load_rows(vb, g.B, g.sBn, g.sBk, t.b_kmajor, n0, g.N, k, g.K, w, LW, lane);
+            const bool ready = i < TC_STAGES || mbar_wait(&s_empty[st], (i / TC_STAGES - 1) & 1);
+            if (!__all_sync(0xffffffffu, ready)) {
+                s_fail = 1;
+                break;
+            }
+            if (SA) store_rows(va, a, w, LW, lane);
+            if (SB) store_rows(vb, a + TC_TILE, w, LW, lane);
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the MMA reads through the async proxy
+            __syncwarp();
+            if (lane == 0)
+                asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&s_full[st])) : "memory");
+        }
     }
     __syncwarp();
     bool ok = mbar_wait(&s_done, 0);
@@ -314,7 +273,7 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc(const __grid_constant__ CU
     // accumulator: lane 32 warp + lane of TMEM is row m0 + 32 warp + lane
     float *crow = reinterpret_cast<float *>(ring) + (32 * warp + lane) * TC_PITCH;
 #pragma unroll
-    for (int c = 0; c < TC_N; c += 32) {
+    for (int c = 0; c < TC_N && warp < TC_THREADS / 32; c += 32) {
         unsigned v[32];
         asm volatile(
             "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
@@ -341,7 +300,7 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc(const __grid_constant__ CU
         float *C = g.C32 + (long)blockIdx.z * g.M * g.sCm + (long)m0 * g.sCm + n0;
         for (int c = lane; c < cols; c += 32) {
             const float bias = (g.epi == EPI_BIAS_F32 ? g.bias[n0 + c] : 0.f) + bad;
-            for (int r = warp; r < rows; r += TC_THREADS / 32) {
+            for (int r = warp; r < rows; r += WARPS) {
                 const float v = ct[r * TC_PITCH + c];
                 C[(long)r * g.sCm + c] = g.epi == EPI_BIAS_F32 ? v + bias : v + bad;
             }
@@ -357,7 +316,7 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc(const __grid_constant__ CU
         return __float2bfloat16_rn(v > 0.f ? v : (v != v ? v : 0.f));
     };
     const bool pairs = !(g.sCm & 1) && !(reinterpret_cast<uintptr_t>(C) & 3);
-    for (int r = warp; r < rows; r += TC_THREADS / 32) {
+    for (int r = warp; r < rows; r += WARPS) {
         if (pairs) {
             for (int c = 2 * lane; c < cols; c += 64) {
                 if (c + 1 < cols)
@@ -388,16 +347,17 @@ EncodeTiled encode_tiled() {
 }
 
 // Map of an operand with mn rows (or columns) and K: element (i, k) at
-// base[i smn + k sk].  false if TMA cannot read it.
+// base[i smn + k sk].  false if TMA cannot read it; *k_major says in which of the
+// two orders its tiles are read in either case.
 bool tc_map(CUtensorMap *map, const void *base, long smn, long sk, int mn, int K, int *k_major) {
     const bool km = sk == 1 && (smn > 1 || mn == 1), mm = !km && smn == 1;
+    *k_major = !mm;
     if (!km && !mm) return false;
     const long ld = km ? smn : sk;
     const int inner = km ? K : mn, outer = km ? mn : K;
     if (ld < inner || (ld * 2) % 16 || reinterpret_cast<uintptr_t>(base) % 16 || !encode_tiled()) return false;
     const cuuint64_t dims[2] = {(cuuint64_t)inner, (cuuint64_t)outer}, strides[1] = {(cuuint64_t)ld * 2};
     const cuuint32_t box[2] = {64, (cuuint32_t)(km ? 128 : 64)}, one[2] = {1, 1};
-    *k_major = km;
     return encode_tiled()(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void *>(base), dims, strides, box, one,
                           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
@@ -405,23 +365,19 @@ bool tc_map(CUtensorMap *map, const void *base, long smn, long sk, int mn, int K
 
 // One GEMM over `splits` ranges of K (g.k_per_split is set here).
 int run_gemm(GemmArgs g, int splits, int *used, cudaStream_t s) {
-    CUtensorMap ma, mb;
+    CUtensorMap ma{}, mb{};
     TcArgs t;
-    const bool tc = tc_map(&ma, g.A, g.sAm, g.sAk, g.M, g.K, &t.a_kmajor) &&
-                    tc_map(&mb, g.B, g.sBn, g.sBk, g.N, g.K, &t.b_kmajor);
-    const int step = tc ? TC_K : BK;
-    const int kps = ((g.K + splits - 1) / splits + step - 1) / step * step;
+    const bool sa = !tc_map(&ma, g.A, g.sAm, g.sAk, g.M, g.K, &t.a_kmajor),
+               sb = !tc_map(&mb, g.B, g.sBn, g.sBk, g.N, g.K, &t.b_kmajor);
+    const int kps = ((g.K + splits - 1) / splits + TC_K - 1) / TC_K * TC_K;
     g.k_per_split = kps;
     *used = (g.K + kps - 1) / kps;
-    if (tc) {
-        t.g = g;
-        TAGI_CUDA(cudaFuncSetAttribute(gemm_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM));
-        dim3 grid((g.N + TC_N - 1) / TC_N, (g.M + TC_M - 1) / TC_M, *used);
-        TAGI_CUDA(launch_chained(gemm_tc, grid, TC_THREADS, TC_SMEM, s, ma, mb, t));
-    } else {
-        dim3 grid((g.N + BN - 1) / BN, (g.M + BM - 1) / BM, *used);
-        launch(gemm_bf16, grid, GEMM_THREADS, 0, s, g);
-    }
+    t.g = g;
+    const auto kern = sa ? (sb ? gemm_tc<true, true> : gemm_tc<true, false>)
+                         : (sb ? gemm_tc<false, true> : gemm_tc<false, false>);
+    TAGI_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM));
+    const dim3 grid((g.N + TC_N - 1) / TC_N, (g.M + TC_M - 1) / TC_M, *used);
+    TAGI_CUDA(launch_chained(kern, grid, TC_THREADS + (sa || sb ? TC_LOADERS : 0), TC_SMEM, s, ma, mb, t));
     TAGI_LAUNCH_CHECK();
     return TAGI_OK;
 }
