@@ -512,8 +512,12 @@ int tagi_mesh_refine(const double *baseCells, int numBase, const double *atomXYZ
             break;
         }
         launch(mesh_iota, grid_for(total), MT, 0, s, idx, (int)total);
-        if ((rc = radix_sort_u64(all_keys, idx, (int)total, tmp, s))) break;
-        launch(mesh_cell_table, grid_for(total), MT, 0, s, idx, (int)total, all_cells, all_fine, p3, cellX, cellY,
+        uint64_t *keys_out = nullptr;
+        int *order_of = nullptr;
+        if ((rc = tmp.alloc(&keys_out, total)) || (rc = tmp.alloc(&order_of, total)) ||
+            (rc = radix_sort_u64(all_keys, idx, keys_out, order_of, (int)total, 64, tmp, s)))
+            break;
+        launch(mesh_cell_table, grid_for(total), MT, 0, s, order_of, (int)total, all_cells, all_fine, p3, cellX, cellY,
                cellZ, cellDX, cellDY, cellDZ, ptsPerCellCoarse, ptsPerCellFine);
         if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(s) != cudaSuccess)
             rc = set_error(TAGI_ERR_CUDA, "mesh cell table failed");

@@ -132,86 +132,128 @@ int exclusive_scan(const int *in, int *out, int n, int *d_total, Arena &ar, cuda
 
 namespace {
 
-constexpr int RS_THREADS = 256;
-constexpr int RS_ROUNDS = 8;
-constexpr int RS_TILE = RS_THREADS * RS_ROUNDS;
-constexpr int RS_WARPS = RS_THREADS / 32;
+// Radix passes: two chained launches per digit.  Bound: launch latency up to some
+// 200,000 keys, then L2 (12 bytes in, 12 out, scattered).  A block of the scatter adds up
+// where its tile's digits go from the tiles' counts, those of whole groups of tiles
+// first, so no scan runs between the two kernels: at 1.5M keys a block reads 27 rows
+// of 512 counts.  Nine-bit digits: 63-bit Morton codes take seven passes; 512 counters for
+// each of eight warps are 16 KB of shared memory.  Digits of eight bits with a scan
+// between took 24 launches (40 above 130,000 keys): @@
+constexpr int RS_THREADS = 256, RS_WARPS = RS_THREADS / 32, RS_BITS = 9, RS_DIGITS = 1 << RS_BITS;
 
-__global__ void __launch_bounds__(RS_THREADS) rs_histogram(const uint64_t *__restrict__ keys,
-                                                           int n, int shift,
-                                                           int *__restrict__ hist, int nblocks) {
-    __shared__ int cnt[256];
-    cnt[threadIdx.x] = 0;
+// counts[tile][digit], and their sums over groups of `group` tiles (zeroed before)
+template <int ROUNDS>
+__global__ void __launch_bounds__(RS_THREADS) rs_histogram(const uint64_t *__restrict__ keys, int n, int shift, int group,
+                                                           int *__restrict__ counts, int *__restrict__ sums) {
+    __shared__ int cnt[RS_DIGITS];
+    for (int d = threadIdx.x; d < RS_DIGITS; d += RS_THREADS) cnt[d] = 0;
+    chain_begin();
     __syncthreads();
-    const long base = (long)blockIdx.x * RS_TILE;
-    for (int r = 0; r < RS_ROUNDS; r++) {
-        long i = base + (long)r * RS_THREADS + threadIdx.x;
-        if (i < n) atomicAdd(&cnt[(int)((keys[i] >> shift) & 255u)], 1);
+    const long base = (long)blockIdx.x * ROUNDS * RS_THREADS;
+#pragma unroll
+    for (int r = 0; r < ROUNDS; r++) {
+        const long i = base + (long)r * RS_THREADS + threadIdx.x;
+        if (i < n) atomicAdd(&cnt[(int)(keys[i] >> shift) & (RS_DIGITS - 1)], 1);
     }
     __syncthreads();
-    hist[(long)threadIdx.x * nblocks + blockIdx.x] = cnt[threadIdx.x];
+    for (int d = threadIdx.x; d < RS_DIGITS; d += RS_THREADS) {
+        const int c = cnt[d];
+        counts[(long)blockIdx.x * RS_DIGITS + d] = c;
+        if (c) atomicAdd(sums + (long)(blockIdx.x / group) * RS_DIGITS + d, c);
+    }
 }
 
-// Stable scatter: elements of a tile are ranked in index order, warp by warp,
-// round by round; ties between tiles follow block order via the scanned
-// digit-major histogram.
-__global__ void __launch_bounds__(RS_THREADS) rs_scatter(const uint64_t *__restrict__ kin,
-                                                         const int *__restrict__ vin,
-                                                         uint64_t *__restrict__ kout,
-                                                         int *__restrict__ vout, int n, int shift,
-                                                         const int *__restrict__ offs,
-                                                         int nblocks) {
-    __shared__ int base[256];
-    __shared__ int wcnt[RS_WARPS][256];
-    base[threadIdx.x] = offs[(long)threadIdx.x * nblocks + blockIdx.x];
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const unsigned lt = (1u << lane) - 1u;
-    const long tile = (long)blockIdx.x * RS_TILE;
-    for (int r = 0; r < RS_ROUNDS; r++) {
-#pragma unroll
-        for (int w = 0; w < RS_WARPS; w++) wcnt[w][threadIdx.x] = 0;
-        __syncthreads();
-        long i = tile + (long)r * RS_THREADS + threadIdx.x;
-        bool valid = i < n;
-        uint64_t k = valid ? kin[i] : 0;
-        int v = valid ? vin[i] : 0;
-        int d = valid ? (int)((k >> shift) & 255u) : 256 + lane;  // invalid lanes stay alone
-        unsigned peers = __match_any_sync(0xffffffffu, d);
-        int rank = __popc(peers & lt);
-        if (valid && rank == 0) wcnt[wid][d] = __popc(peers);
-        __syncthreads();
-        {
-            int dd = threadIdx.x;
-            int run = base[dd];
-#pragma unroll
-            for (int w = 0; w < RS_WARPS; w++) {
-                int c = wcnt[w][dd];
-                wcnt[w][dd] = run;
-                run += c;
-            }
-            base[dd] = run;
-        }
-        __syncthreads();
-        if (valid) {
-            int pos = wcnt[wid][d] + rank;
-            kout[pos] = k;
-            vout[pos] = v;
-        }
-        __syncthreads();
+// Stable scatter.  Each warp owns 32 ROUNDS consecutive keys of the tile and ranks them
+// in order with its own counters; a column scan over the warps and the tile's start
+// of each digit turn the ranks into places.
+template <int ROUNDS>
+__global__ void __launch_bounds__(RS_THREADS) rs_scatter(const uint64_t *__restrict__ kin, const int *__restrict__ vin,
+                                                         uint64_t *__restrict__ kout, int *__restrict__ vout, int n,
+                                                         int shift, int group, int ngroups,
+                                                         const int *__restrict__ counts, const int *__restrict__ sums) {
+    __shared__ int wcnt[RS_WARPS][RS_DIGITS];
+    __shared__ int wtot[RS_WARPS];
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, tile = blockIdx.x;
+    for (int d = tid; d < RS_WARPS * RS_DIGITS; d += RS_THREADS) (&wcnt[0][0])[d] = 0;
+    chain_begin();
+    // digits 2 tid and 2 tid + 1: keys before this tile, and keys in all
+    int2 before = make_int2(0, 0), all = make_int2(0, 0);
+    const int mine = tile / group;
+#pragma unroll 8
+    for (int g = 0; g < ngroups; g++) {
+        const int2 c = reinterpret_cast<const int2 *>(sums + (long)g * RS_DIGITS)[tid];
+        all.x += c.x;
+        all.y += c.y;
+        if (g < mine) before.x += c.x, before.y += c.y;
     }
+#pragma unroll 8
+    for (int t = mine * group; t < tile; t++) {
+        const int2 c = reinterpret_cast<const int2 *>(counts + (long)t * RS_DIGITS)[tid];
+        before.x += c.x;
+        before.y += c.y;
+    }
+    const int incl = warp_incl_scan(all.x + all.y);
+    if (lane == 31) wtot[wid] = incl;
+    __syncthreads();
+    int first = incl - all.x - all.y;
+    for (int w = 0; w < wid; w++) first += wtot[w];
+    uint64_t k[ROUNDS];
+    int place[ROUNDS];
+    const long base = (long)tile * ROUNDS * RS_THREADS + (long)wid * ROUNDS * 32 + lane;
+#pragma unroll
+    for (int r = 0; r < ROUNDS; r++) k[r] = base + 32 * r < n ? kin[base + 32 * r] : 0;
+#pragma unroll
+    for (int r = 0; r < ROUNDS; r++) {
+        const bool valid = base + 32 * r < n;
+        const int d = (int)(k[r] >> shift) & (RS_DIGITS - 1);
+        const unsigned peers = __match_any_sync(0xffffffffu, valid ? d : RS_DIGITS + lane);   // invalid lanes stay alone
+        const int rank = __popc(peers & ((1u << lane) - 1u)), c = valid ? wcnt[wid][d] : 0;
+        place[r] = c + rank;
+        __syncwarp();
+        if (valid && rank == 0) wcnt[wid][d] = c + __popc(peers);
+        __syncwarp();
+    }
+    __syncthreads();
+    int2 run = make_int2(first + before.x, first + all.x + before.y);
+#pragma unroll
+    for (int w = 0; w < RS_WARPS; w++) {
+        int2 *p = reinterpret_cast<int2 *>(&wcnt[w][2 * tid]);
+        const int2 c = *p;
+        *p = run;
+        run.x += c.x;
+        run.y += c.y;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < ROUNDS; r++) {
+        const long i = base + 32 * r;
+        if (i < n) {
+            const int p = place[r] + wcnt[wid][(int)(k[r] >> shift) & (RS_DIGITS - 1)];
+            kout[p] = k[r];
+            vout[p] = vin[i];
+        }
+    }
+}
+
+template <int ROUNDS>
+int rs_pass(const uint64_t *kin, const int *vin, uint64_t *kout, int *vout, int n, int shift, int nb, int group,
+            int *counts, int *sums, cudaStream_t s) {
+    TAGI_CUDA(launch_chained(rs_histogram<ROUNDS>, nb, RS_THREADS, 0, s, kin, n, shift, group, counts, sums));
+    TAGI_CUDA(launch_chained(rs_scatter<ROUNDS>, nb, RS_THREADS, 0, s, kin, vin, kout, vout, n, shift, group,
+                             (nb + group - 1) / group, counts, sums));
+    return TAGI_OK;
 }
 
 // Up to SORT_SMALL pairs by counting: an element's place is the number of smaller
 // keys plus the equal keys before it.  n^2 comparisons over the whole chip take
-// 3 us at 6,000 keys and 25 at 16,384, where the radix passes are 40 launches (about
-// 100 us) and a bitonic network in one block took 124.  Counts are whole numbers:
+// 3 us at 6,000 keys and 25 at 16,384, the radix passes @@; a bitonic network in one
+// block took 124 at 6,000.  Counts are whole numbers:
 // the order of the atomic additions does not matter.
 constexpr int SORT_SMALL = 16384, CNT_THREADS = 256;
 __global__ void __launch_bounds__(CNT_THREADS) count_smaller(const uint64_t *__restrict__ keys,
-                                                             const int *__restrict__ vals, int n, int span,
-                                                             int *__restrict__ rank, uint64_t *__restrict__ kcopy,
-                                                             int *__restrict__ vcopy) {
+                                                             int n, int span, int *__restrict__ rank) {
     __shared__ uint64_t s_key[CNT_THREADS];
+    chain_begin();
     const int i = blockIdx.x * CNT_THREADS + threadIdx.x;
     const uint64_t k = i < n ? keys[i] : 0;
     const int j0 = blockIdx.y * span, j1 = min(j0 + span, n);
@@ -227,60 +269,53 @@ __global__ void __launch_bounds__(CNT_THREADS) count_smaller(const uint64_t *__r
             c += q < k || (q == k && t + j < i);
         }
     }
-    if (i >= n) return;
-    if (c) atomicAdd(rank + i, c);
-    if (blockIdx.y == 0) {
-        kcopy[i] = k;
-        vcopy[i] = vals[i];
-    }
+    if (i < n && c) atomicAdd(rank + i, c);
 }
-__global__ void place_sorted(const uint64_t *__restrict__ kcopy, const int *__restrict__ vcopy,
-                             const int *__restrict__ rank, int n, uint64_t *__restrict__ keys, int *__restrict__ vals) {
+__global__ void place_sorted(const uint64_t *__restrict__ kin, const int *__restrict__ vin, const int *__restrict__ rank,
+                             int n, uint64_t *__restrict__ kout, int *__restrict__ vout) {
+    chain_begin();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const int r = rank[i];
-    keys[r] = kcopy[i];
-    vals[r] = vcopy[i];
+    kout[r] = kin[i];
+    vout[r] = vin[i];
 }
 
 }  // namespace
 
-int radix_sort_u64(uint64_t *keys, int *vals, int n, Arena &ar, cudaStream_t s) {
-    if (n <= 1) return TAGI_OK;
+int radix_sort_u64(uint64_t *kin, int *vin, uint64_t *kout, int *vout, int n, int bits, Arena &ar, cudaStream_t s) {
+    if (n <= 0) return TAGI_OK;
     if (n <= SORT_SMALL) {
-        uint64_t *kc = nullptr;
-        int *vc = nullptr, *rank = nullptr;
-        TAGI_TRY(ar.alloc(&kc, n));
-        TAGI_TRY(ar.alloc(&vc, n));
+        int *rank = nullptr;
         TAGI_TRY(ar.alloc(&rank, n));
         TAGI_CUDA(cudaMemsetAsync(rank, 0, sizeof(int) * n, s));
         const int bx = (n + CNT_THREADS - 1) / CNT_THREADS;
         const int by = std::min(bx, (152 * 8 + bx - 1) / bx);   // about eight blocks per SM
         const int span = (n + by - 1) / by;
-        launch(count_smaller, dim3(bx, (n + span - 1) / span), CNT_THREADS, 0, s, keys, vals, n, span, rank, kc, vc);
-        launch(place_sorted, bx, CNT_THREADS, 0, s, kc, vc, rank, n, keys, vals);
+        launch(count_smaller, dim3(bx, (n + span - 1) / span), CNT_THREADS, 0, s, kin, n, span, rank);
+        TAGI_CUDA(launch_chained(place_sorted, bx, CNT_THREADS, 0, s, kin, vin, rank, n, kout, vout));
         TAGI_LAUNCH_CHECK();
         return TAGI_OK;
     }
-    int nb = (n + RS_TILE - 1) / RS_TILE;
-    uint64_t *k2 = nullptr;
-    int *v2 = nullptr, *hist = nullptr, *offs = nullptr;
-    TAGI_TRY(ar.alloc(&k2, n));
-    TAGI_TRY(ar.alloc(&v2, n));
-    TAGI_TRY(ar.alloc(&hist, 256L * nb));
-    TAGI_TRY(ar.alloc(&offs, 256L * nb));
-    uint64_t *ka = keys, *kb = k2;
-    int *va = vals, *vb = v2;
-    for (int shift = 0; shift < 64; shift += 8) {
-        launch(rs_histogram, nb, RS_THREADS, 0, s, ka, n, shift, hist, nb);
-        TAGI_LAUNCH_CHECK();
-        TAGI_TRY(exclusive_scan(hist, offs, 256 * nb, nullptr, ar, s));
-        launch(rs_scatter, nb, RS_THREADS, 0, s, ka, va, kb, vb, n, shift, offs, nb);
-        TAGI_LAUNCH_CHECK();
-        uint64_t *kt = ka; ka = kb; kb = kt;
-        int *vt = va; va = vb; vb = vt;
+    // one or two tiles per SM, so that the chain of one tile is short; larger ones mean fewer rows of counts
+    const int rounds = n > 1 << 18 ? 16 : n > 1 << 17 ? 8 : 2, tile = RS_THREADS * rounds;
+    const int nb = (int)(((long)n + tile - 1) / tile);
+    const int group = nb <= 1024 ? 16 : 64, ngroups = (nb + group - 1) / group, passes = (bits + RS_BITS - 1) / RS_BITS;
+    int *counts = nullptr, *sums = nullptr;
+    const long row = (long)ngroups * RS_DIGITS;
+    TAGI_TRY(ar.alloc(&counts, (long)nb * RS_DIGITS));
+    TAGI_TRY(ar.alloc(&sums, passes * row));
+    TAGI_CUDA(cudaMemsetAsync(sums, 0, sizeof(int) * passes * row, s));
+    for (int p = 0; p < passes; p++) {
+        const bool odd = p & 1;
+        TAGI_TRY((rounds == 16 ? rs_pass<16> : rounds == 8 ? rs_pass<8> : rs_pass<2>)(odd ? kout : kin, odd ? vout : vin, odd ? kin : kout, odd ? vin : vout, n,
+                                                    RS_BITS * p, nb, group, counts, sums + p * row, s));
     }
-    // 8 passes: the result is back in the caller's buffers.
+    TAGI_LAUNCH_CHECK();
+    if (passes % 2 == 0) {
+        TAGI_CUDA(cudaMemcpyAsync(kout, kin, sizeof(uint64_t) * n, cudaMemcpyDeviceToDevice, s));
+        TAGI_CUDA(cudaMemcpyAsync(vout, vin, sizeof(int) * n, cudaMemcpyDeviceToDevice, s));
+    }
     return TAGI_OK;
 }
 

@@ -263,7 +263,8 @@ void plan_destroy(Plan *p);
 
 // scan_sort.cu
 int exclusive_scan(const int *in, int *out, int n, int *d_total, Arena &ar, cudaStream_t s);
-int radix_sort_u64(uint64_t *keys, int *vals, int n, Arena &ar, cudaStream_t s);
+// Stable sort by the low `bits` bits of the keys into (kout, vout); (kin, vin) is overwritten.
+int radix_sort_u64(uint64_t *kin, int *vin, uint64_t *kout, int *vout, int n, int bits, Arena &ar, cudaStream_t s);
 
 // tree.cu
 int build_tree(Tree &t, const double *x, const double *y, const double *z, int n, int leaf,

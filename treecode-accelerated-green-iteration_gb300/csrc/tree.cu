@@ -84,6 +84,7 @@ __global__ void bbox_partial(const double *__restrict__ x, const double *__restr
 // reduces the per-block partials (min/max are exact in any order).
 __global__ void __launch_bounds__(256) bbox_final(const long long *__restrict__ part, int nb,
                                                   double *__restrict__ params) {
+    chain_begin();
     long long ol[3] = {part[0], part[1], part[2]}, oh[3] = {part[3], part[4], part[5]};
     for (int b = threadIdx.x; b < nb; b += blockDim.x)
         for (int d = 0; d < 3; d++) {
@@ -136,6 +137,7 @@ __global__ void morton_codes(const double *__restrict__ x, const double *__restr
                              const double *__restrict__ z, int n,
                              const double *__restrict__ params, uint64_t *__restrict__ codes,
                              int *__restrict__ idx) {
+    chain_begin();
     long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const double sc = params[3];
@@ -150,6 +152,7 @@ __global__ void gather3(const double *__restrict__ x, const double *__restrict__
                         const double *__restrict__ z, const int *__restrict__ perm, int n,
                         double *__restrict__ xs, double *__restrict__ ys,
                         double *__restrict__ zs) {
+    chain_begin();
     long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     int o = perm[i];
@@ -228,9 +231,12 @@ __global__ void fill_children(const uint64_t *__restrict__ codes, int *__restric
 constexpr int MAX_LEVELS = 23;   // 21 digits split at most
 constexpr int HDR = MAX_LEVELS + 3;
 
-// The whole octree by one block, a level at a time: eight threads per node find
-// the starts of its eight digits by binary search, so a round of 128 nodes is one
-// search deep, and nothing waits for the host between levels.  Meshes have a few
+// The whole octree by one block, a level at a time: a group of threads per node finds
+// the starts of its eight digits, so a round of nodes is one search deep, and
+// nothing waits for the host between levels.  A level of up to 32 nodes gives four
+// threads to a digit, which cut its range in five at a time (a chain of 7 loads
+// instead of 16 at 44,000 points), a wider one a thread: binary search, 128 nodes a
+// round.  44,000 points, leaves of 1834: 33 -> @@ us.  Meshes have a few
 // thousand nodes: 1.5M points, leaves of 2000: 8 levels, count + fill + scan
 // launches and a synchronisation each, 1.35 -> 0.78 ms for the tree and its sort.  Above
 // SMALL_TREE leaves' worth of points one launch per level is quicker.
@@ -241,7 +247,8 @@ __global__ void __launch_bounds__(BUILD_THREADS) build_nodes(const uint64_t *__r
                                                              int *__restrict__ parent, int *__restrict__ first_child,
                                                              int *__restrict__ nchild, int *__restrict__ hdr) {
     __shared__ int s_cnt[BUILD_THREADS / 32];
-    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, digit = tid & 7;
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    chain_begin();
     if (tid == 0) {
         begin[0] = 0;
         end[0] = n;
@@ -252,8 +259,10 @@ __global__ void __launch_bounds__(BUILD_THREADS) build_nodes(const uint64_t *__r
     for (;; level++) {
         if (tid == 0) hdr[2 + level] = ls;
         int next = le;
-        for (int base = ls; base < le; base += BUILD_THREADS / 8) {
-            const int v = base + (tid >> 3);
+        const int gb = le - ls <= BUILD_THREADS / 32 ? 2 : 0, probes = 1 << gb;   // threads per digit
+        const int digit = (tid >> gb) & 7, q = tid & (probes - 1);
+        for (int base = ls; base < le; base += BUILD_THREADS >> (3 + gb)) {
+            const int v = base + (tid >> (3 + gb));
             int b = 0, e = 0, sh = -1, lo = 0;
             if (v < le) {
                 b = begin[v];
@@ -264,15 +273,28 @@ __global__ void __launch_bounds__(BUILD_THREADS) build_nodes(const uint64_t *__r
                 const uint64_t key = ((codes[b] >> (sh + 3)) << 3) | (uint64_t)digit;
                 int hi = e;
                 lo = b;
-                while (lo < hi) {
-                    const int mid = lo + ((hi - lo) >> 1);
-                    if ((codes[mid] >> sh) >= key) hi = mid;
-                    else lo = mid + 1;
+                if (gb == 0) {
+                    while (lo < hi) {
+                        const int mid = lo + ((hi - lo) >> 1);
+                        if ((codes[mid] >> sh) >= key) hi = mid;
+                        else lo = mid + 1;
+                    }
+                } else {
+                    const unsigned group = 0xfu << (lane & 28);
+                    while (lo < hi) {
+                        const int w = hi - lo, mid = lo + (int)((long)w * (q + 1) / 5);
+                        const unsigned below = __ballot_sync(group, (codes[mid] >> sh) < key) & group;
+                        const int c = __popc(below);   // the first c probes lie before the digit
+                        const int left = __shfl_sync(group, mid, (lane & 28) + max(c - 1, 0));
+                        const int right = __shfl_sync(group, mid, (lane & 28) + min(c, 3));
+                        if (c > 0) lo = left + 1;
+                        if (c < 4) hi = right;
+                    }
                 }
             }
-            int to = __shfl_down_sync(0xffffffffu, lo, 1, 8);
+            int to = __shfl_down_sync(0xffffffffu, lo, probes, 8 << gb);
             if (digit == 7) to = e;
-            const bool child = sh >= 0 && to > lo;
+            const bool child = sh >= 0 && to > lo && q == 0;
             const unsigned m = __ballot_sync(0xffffffffu, child);
             __syncthreads();   // s_cnt of the previous round is no longer read
             if (lane == 0) s_cnt[wid] = __popc(m);
@@ -288,8 +310,8 @@ __global__ void __launch_bounds__(BUILD_THREADS) build_nodes(const uint64_t *__r
                 end[at] = to;
                 parent[at] = v;
             }
-            if (digit == 0 && v < le) {
-                const int c = __popc((m >> lane) & 0xffu);
+            if (digit == 0 && q == 0 && v < le) {
+                const int c = __popc((m >> lane) & (gb ? 0xffffffffu : 0xffu));
                 nchild[v] = c;
                 first_child[v] = c ? at : -1;
             }
@@ -310,24 +332,27 @@ __global__ void __launch_bounds__(BUILD_THREADS) build_nodes(const uint64_t *__r
 __global__ void write_header(int *hdr, int nnodes) { hdr[0] = nnodes; }
 
 // Boxes of all nodes in one launch, with the nodes and leaves of each subtree: a
-// warp does a leaf, and the warp that finishes a node's last child goes on with
-// the node.
-__global__ void __launch_bounds__(256) node_boxes(const int *__restrict__ hdr, const int *__restrict__ begin,
-                                                  const int *__restrict__ end, const int *__restrict__ parent,
-                                                  const int *__restrict__ first_child, const int *__restrict__ nchild,
-                                                  const double *__restrict__ x, const double *__restrict__ y,
-                                                  const double *__restrict__ z, long long *box, double *__restrict__ center,
-                                                  double *__restrict__ half, double *__restrict__ radius, int *size,
-                                                  int *leaves, int *done) {
-    const int nn = hdr[0], lane = threadIdx.x & 31;
-    for (int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < nn; w += (gridDim.x * blockDim.x) >> 5) {
+// block does a leaf, and the first warp of the one that finishes a node's last child
+// goes on with the node.  The chain of the climb holds only what the parent needs;
+// centers and radii (FP64) follow in preorder.  44,000 points, leaves of 1834, a warp
+// per leaf and all of a node's values in the climb before: 48 -> @@ us.
+constexpr int BOX_THREADS = 128;
+__global__ void __launch_bounds__(BOX_THREADS) node_boxes(const int *__restrict__ hdr, const int *__restrict__ begin,
+                                                          const int *__restrict__ end, const int *__restrict__ parent,
+                                                          const int *__restrict__ first_child,
+                                                          const int *__restrict__ nchild, const double *__restrict__ x,
+                                                          const double *__restrict__ y, const double *__restrict__ z,
+                                                          long long *box, int *size, int *leaves, int *done) {
+    __shared__ long long s_box[BOX_THREADS / 32][6];
+    chain_begin();
+    const int nn = hdr[0], tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const long long top = ordered(INFINITY), bottom = ordered(-INFINITY);
+    for (int w = blockIdx.x; w < nn; w += gridDim.x) {
         if (nchild[w]) continue;
-        const long long top = ordered(INFINITY), bottom = ordered(-INFINITY);
         long long l[3] = {top, top, top}, h[3] = {bottom, bottom, bottom};
-        int sz = 0, lv = 0;   // of the children (lane 0's own start below)
         const int e = end[w];
 #pragma unroll 4
-        for (int i = begin[w] + lane; i < e; i += 32) {
+        for (int i = begin[w] + tid; i < e; i += BOX_THREADS) {
             const long long p[3] = {ordered(x[i]), ordered(y[i]), ordered(z[i])};
 #pragma unroll
             for (int d = 0; d < 3; d++) {
@@ -335,27 +360,35 @@ __global__ void __launch_bounds__(256) node_boxes(const int *__restrict__ hdr, c
                 h[d] = max(h[d], p[d]);
             }
         }
+        warp_minmax(l, h);
+        __syncthreads();   // the previous leaf's corners are no longer read
+        if (lane == 0)
+#pragma unroll
+            for (int d = 0; d < 3; d++) {
+                s_box[wid][d] = l[d];
+                s_box[wid][3 + d] = h[d];
+            }
+        __syncthreads();
+        if (wid) continue;
+        const bool part = lane < BOX_THREADS / 32;
+#pragma unroll
+        for (int d = 0; d < 3; d++) {
+            l[d] = part ? s_box[lane][d] : top;
+            h[d] = part ? s_box[lane][3 + d] : bottom;
+        }
+        int sz = 0, lv = 0;   // of the children
         for (int v = w;;) {
+            const int pv = parent[v];
             warp_minmax(l, h);
             sz = __reduce_add_sync(0xffffffffu, sz);
             lv = __reduce_add_sync(0xffffffffu, lv);
             int last = 0;
-            const int pv = parent[v];
             if (lane == 0) {
-                double hh[3];
 #pragma unroll
                 for (int d = 0; d < 3; d++) {
-                    const double lo = from_ordered(l[d]), hi = from_ordered(h[d]);
                     __stcg(box + 6L * v + d, l[d]);
                     __stcg(box + 6L * v + 3 + d, h[d]);
-                    center[3L * v + d] = __dmul_rn(__dadd_rn(lo, hi), 0.5);
-                    hh[d] = __dmul_rn(__dsub_rn(hi, lo), 0.5);
-                    half[3L * v + d] = hh[d];
                 }
-                double s = __dmul_rn(hh[0], hh[0]);
-                s = __dadd_rn(s, __dmul_rn(hh[1], hh[1]));
-                s = __dadd_rn(s, __dmul_rn(hh[2], hh[2]));
-                radius[v] = __dsqrt_rn(s);
                 __stcg(size + v, sz + 1);
                 __stcg(leaves + v, v == w ? 1 : lv);
                 if (pv >= 0) {
@@ -380,16 +413,30 @@ __global__ void __launch_bounds__(256) node_boxes(const int *__restrict__ hdr, c
     }
 }
 
-// Each node's place in pre-order (children in digit order) and each leaf's among
-// the leaves, from the subtrees passed on the way to the root.
+// Each node's center, half edges and radius; its place in pre-order (children in digit
+// order) and each leaf's among the leaves, from the subtrees passed on the way to the
+// root.
 __global__ void preorder(const int *__restrict__ hdr, const int *__restrict__ begin, const int *__restrict__ end,
                          const int *__restrict__ parent, const int *__restrict__ first_child,
-                         const int *__restrict__ nchild, const double *__restrict__ center,
-                         const double *__restrict__ radius, const int *__restrict__ size,
+                         const int *__restrict__ nchild, const long long *__restrict__ box,
+                         double *__restrict__ center, double *__restrict__ half, double *__restrict__ radius,
+                         const int *__restrict__ size,
                          const int *__restrict__ leaves, PreNode *__restrict__ pre, int *__restrict__ leaf_node,
                          int *__restrict__ nleaves) {
+    chain_begin();
     const int nn = hdr[0];
     for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < nn; v += gridDim.x * blockDim.x) {
+        double cc[3], hh[3];
+#pragma unroll
+        for (int d = 0; d < 3; d++) {
+            const double lo = from_ordered(box[6L * v + d]), hi = from_ordered(box[6L * v + 3 + d]);
+            center[3L * v + d] = cc[d] = __dmul_rn(__dadd_rn(lo, hi), 0.5);
+            half[3L * v + d] = hh[d] = __dmul_rn(__dsub_rn(hi, lo), 0.5);
+        }
+        double s = __dmul_rn(hh[0], hh[0]);
+        s = __dadd_rn(s, __dmul_rn(hh[1], hh[1]));
+        s = __dadd_rn(s, __dmul_rn(hh[2], hh[2]));
+        radius[v] = s = __dsqrt_rn(s);
         int pos = 0, rank = 0;
         for (int c = v; c != 0;) {
             const int p = parent[c];
@@ -401,10 +448,10 @@ __global__ void preorder(const int *__restrict__ hdr, const int *__restrict__ be
             c = p;
         }
         PreNode q;
-        q.x = center[3L * v];
-        q.y = center[3L * v + 1];
-        q.z = center[3L * v + 2];
-        q.r = radius[v];
+        q.x = cc[0];
+        q.y = cc[1];
+        q.z = cc[2];
+        q.r = s;
         q.node = v;
         q.stop = pos + size[v];
         q.count = end[v] - begin[v];
@@ -437,14 +484,22 @@ int build_tree(Tree &t, const double *x, const double *y, const double *z, int n
         if ((rc = tmp.alloc(&part, 6L * nbb))) break;
         if ((rc = tmp.alloc(&params, 4))) break;
         launch(bbox_partial, nbb, 256, 0, s, x, y, z, n, part);
-        launch(bbox_final, 1, 256, 0, s, part, nbb, params);
+        if (launch_chained(bbox_final, 1, 256, 0, s, part, nbb, params) != cudaSuccess) {
+            rc = set_error(TAGI_ERR_CUDA, "bounding box launch");
+            break;
+        }
         if ((rc = ar.alloc(&t.codes, n))) break;
         if ((rc = ar.alloc(&t.perm, n))) break;
-        launch(morton_codes, (n + 255) / 256, 256, 0, s, x, y, z, n, params, t.codes, t.perm);
-        if (cudaGetLastError() != cudaSuccess) { rc = set_error(TAGI_ERR_CUDA, "morton launch"); break; }
-        if ((rc = radix_sort_u64(t.codes, t.perm, n, tmp, s))) break;
+        uint64_t *codes = nullptr;   // in the caller's order
+        int *idx = nullptr;
+        if ((rc = tmp.alloc(&codes, n)) || (rc = tmp.alloc(&idx, n))) break;
+        if (launch_chained(morton_codes, (n + 255) / 256, 256, 0, s, x, y, z, n, params, codes, idx) != cudaSuccess) { rc = set_error(TAGI_ERR_CUDA, "morton launch"); break; }
+        if ((rc = radix_sort_u64(codes, idx, t.codes, t.perm, n, 63, tmp, s))) break;
         if ((rc = ar.alloc(&t.x, n)) || (rc = ar.alloc(&t.y, n)) || (rc = ar.alloc(&t.z, n))) break;
-        launch(gather3, (n + 255) / 256, 256, 0, s, x, y, z, t.perm, n, t.x, t.y, t.z);
+        if (launch_chained(gather3, (n + 255) / 256, 256, 0, s, x, y, z, t.perm, n, t.x, t.y, t.z) != cudaSuccess) {
+            rc = set_error(TAGI_ERR_CUDA, "gather launch");
+            break;
+        }
 
         // internal nodes hold more than leaf points, n / leaf of them per level at most
         const bool small = n / leaf <= SMALL_TREE;
@@ -458,8 +513,11 @@ int build_tree(Tree &t, const double *x, const double *y, const double *z, int n
         nleaves = hdr + HDR;
         t.level_start.assign(1, 0);
         if (small) {
-            launch(build_nodes, 1, BUILD_THREADS, 0, s, t.codes, n, leaf, t.begin, t.end, t.parent, t.first_child,
-                   t.nchild, hdr);
+            if (launch_chained(build_nodes, 1, BUILD_THREADS, 0, s, t.codes, n, leaf, t.begin, t.end, t.parent,
+                               t.first_child, t.nchild, hdr) != cudaSuccess) {
+                rc = set_error(TAGI_ERR_CUDA, "tree launch");
+                break;
+            }
         } else {
             int *cc = nullptr, *off = nullptr, *total = nullptr;
             if ((rc = tmp.alloc(&cc, cap)) || (rc = tmp.alloc(&off, cap)) || (rc = tmp.alloc(&total, 1)))
@@ -499,11 +557,14 @@ int build_tree(Tree &t, const double *x, const double *y, const double *z, int n
             rc = set_error(TAGI_ERR_CUDA, "tree memset failed");
             break;
         }
-        const unsigned bw = (unsigned)std::min(152L * 8, (nodes + 7) / 8), bt = (unsigned)std::min(152L * 8, (nodes + 255) / 256);
-        launch(node_boxes, bw, 256, 0, s, hdr, t.begin, t.end, t.parent, t.first_child, t.nchild, t.x, t.y, t.z, box,
-               t.center, t.half, t.radius, size, leaves, done);
-        launch(preorder, bt, 256, 0, s, hdr, t.begin, t.end, t.parent, t.first_child, t.nchild, t.center, t.radius, size,
-               leaves, t.pre, t.leaf_node, nleaves);
+        const unsigned bw = (unsigned)std::min(152L * 16, nodes), bt = (unsigned)std::min(152L * 8, (nodes + 127) / 128);
+        if (launch_chained(node_boxes, bw, BOX_THREADS, 0, s, hdr, t.begin, t.end, t.parent, t.first_child, t.nchild, t.x,
+                           t.y, t.z, box, size, leaves, done) != cudaSuccess ||
+            launch_chained(preorder, bt, 128, 0, s, hdr, t.begin, t.end, t.parent, t.first_child, t.nchild, box, t.center,
+                           t.half, t.radius, size, leaves, t.pre, t.leaf_node, nleaves) != cudaSuccess) {
+            rc = set_error(TAGI_ERR_CUDA, "node box launch");
+            break;
+        }
         int h[HDR + 1] = {};
         if (cudaMemcpyAsync(h, hdr, sizeof(h), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
             cudaStreamSynchronize(s) != cudaSuccess) {
