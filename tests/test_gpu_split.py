@@ -73,3 +73,32 @@ def test_fp64_pairs_over_the_distance_range(BT, dev, scale, name, k, sing):
     got = dev.TreecodePlan.for_mesh(*to_cuda(*p, w), theta=0.7, degree=2, source_leaf=200, target_leaf=200).convolve(
         *to_cuda(f, f), getattr(BT.Kernel, name), [k], getattr(BT.Singularity, sing), precision="fp64").cpu().numpy()
     assert np.all(np.abs(got - (t.sum(1) + own)) <= 1e-12 * (np.abs(t).sum(1) + np.abs(own)) + 1e-300)
+
+
+@pytest.mark.parametrize("degree", range(1, 11))
+def test_rows_of_every_degree(BT, dev, oracle, degree):
+    """Odd and even proxy rows, alone and beside another degree in one launch, one
+    orbital per item and groups: the far kernels' loops of each length."""
+    x, y, z, w, _ = cloud(9001, degree)
+    leaf = 130
+    F = np.random.default_rng(degree).standard_normal((5, 9001))
+    k = np.linspace(0.6, 1.4, 5)
+    plan = dev.TreecodePlan.for_mesh(*to_cuda(x, y, z, w), theta=0.8, degree=degree, source_leaf=leaf, target_leaf=leaf,
+                                     size_check=0.05)
+    assert plan.info()["far_entries"] > 0
+    c = oracle.Plan(x, y, z, x, y, z, w, 0.8, degree, leaf, leaf, 0.05)
+    (Ft,) = to_cuda(F)
+    ref = np.stack([c.convolve(F[o], F[o], w, BT.Kernel.YUKAWA, [k[o]], BT.Singularity.SUBTRACTION) for o in range(5)])
+    for og in (1, 4, 8, 16):
+        got = plan.convolve(Ft, Ft, BT.Kernel.YUKAWA, k, BT.Singularity.SUBTRACTION, precision="mixed",
+                            orbitals_per_item=og)
+        assert rel_l2(got.cpu().numpy(), ref) <= 1e-6
+    other = dev.TreecodePlan.for_mesh(*to_cuda(x, y, z, w), theta=0.8, degree=11 - degree, source_leaf=leaf,
+                                      target_leaf=leaf, size_check=0.05)
+    for og in (1, 4):
+        S = dev.Systems([plan, other], (5, 5), BT.Kernel.YUKAWA, orbitals_per_item=og)
+        got = S.convolve([Ft, Ft], [Ft, Ft], [k, k], BT.Singularity.SUBTRACTION)[0]
+        assert rel_l2(got.cpu().numpy(), ref) <= 1e-6
+        S.close()
+    other.close()
+    plan.close()

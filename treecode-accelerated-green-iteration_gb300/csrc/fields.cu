@@ -554,16 +554,23 @@ __global__ void __launch_bounds__(32 * SW, 24 / SW) near_mixed(const __grid_cons
 // ---------------------------------------------------------------------------
 template <int MAXN1>
 __host__ __device__ constexpr int even_up() { return MAXN1 + (MAXN1 & 1); }
+// How much of the loops over a proxy grid is known at compile time (far_loops
+// chooses).  FAR_ANY: n + 1 <= MAXN1.  FAR_ROWS: n + 1 = MAXN1 - 1 or MAXN1 (even), so a
+// row is MAXN1 / 2 pairs of points without tests.  FAR_FIXED: n + 1 = MAXN1.  Whole calls,
+// FAR_ANY -> FAR_ROWS: ring sweep, 150k points, 10 orbitals, degree 5 22.9 -> 21.0 ms; Yukawa,
+// 657k points, degree 5 67.3 -> 63.7; two-mesh, 5 Coulomb fields, degree 10 261 -> 247; 10
+// orbitals, degree 8 51.6 -> 49.3; Coulomb, 144k points, degree 4 3.70 -> 3.34.
+enum { FAR_ANY, FAR_ROWS, FAR_FIXED };
 
-template <int KERN, bool SS, bool EXPTERM, int MAXN1, int NT, bool EXACT, typename Add>
+template <int KERN, bool SS, bool EXPTERM, int MAXN1, int NT, int LOOPS, typename Add>
 __device__ __forceinline__ void far_cluster(const float *__restrict__ s_q, const float *__restrict__ s_w,
                                             const float (*s_p)[MAXN1], int n1_in, int slab0, int slab_step,
                                             const float (&tx)[NT], const float (&ty)[NT], const float (&tz)[NT],
                                             const float2 (&nfi)[NT], Add add) {
     constexpr int MH = even_up<MAXN1>() / 2;
     constexpr bool PSS = KERN == KERNEL_YUKAWA ? SS : (SS && EXPTERM);
-    const int n1 = EXACT ? MAXN1 : n1_in;   // EXACT: every loop bound known at compile time
-    const int n1p = n1 + (n1 & 1);
+    const int n1 = LOOPS == FAR_FIXED ? MAXN1 : n1_in;
+    const int n1p = LOOPS ? even_up<MAXN1>() : n1 + (n1 & 1);
     float2 dz2[NT][MH];
 #pragma unroll
     for (int k = 0; k < NT; k++)
@@ -592,7 +599,7 @@ __device__ __forceinline__ void far_cluster(const float *__restrict__ s_q, const
             }
 #pragma unroll
             for (int m = 0; m < MH; m++) {
-                if (2 * m < n1) {
+                if (LOOPS || 2 * m < n1) {
                     const float2 q = lds2(s_q + idx + 2 * m), wv = lds2(s_w + idx + 2 * m);
 #pragma unroll
                     for (int k = 0; k < NT; k++)
@@ -611,9 +618,7 @@ __device__ __forceinline__ void far_cluster(const float *__restrict__ s_q, const
 // whole tile.
 __device__ __forceinline__ int first_slab(int cl, int n1, const Place &pl) { return (pl.sp - cl * n1) & (pl.S - 1); }
 
-// EXACT: every system of the launch has n + 1 = MAXN1 (the loops over the
-// proxy grid are then fully known at compile time).  FAR_CL clusters are
-// staged per pair of barriers.
+// FAR_CL clusters are staged per pair of barriers.
 template <int MAXN1>
 __host__ __device__ constexpr int far_clusters() { return MAXN1 <= 4 ? 8 : (MAXN1 <= 8 ? 4 : 2); }
 // Partials of a far tile where a target's slabs are split: at least one cluster's
@@ -621,7 +626,7 @@ __host__ __device__ constexpr int far_clusters() { return MAXN1 <= 4 ? 8 : (MAXN
 __host__ __device__ constexpr int far_part(int warps) { return warps == 4 ? 2048 : 4096; }
 static_assert(far_part(4) >= (MAX_DEGREE + 1) * 128 && far_part(8) >= (MAX_DEGREE + 1) * 256, "slabs of one cluster");
 
-template <int KERN, bool SS, int MAXN1, int NT, int SW, bool EXACT = false>
+template <int KERN, bool SS, int MAXN1, int NT, int SW, int LOOPS = FAR_ANY>
 __global__ void __launch_bounds__(32 * SW, 16 / SW) far_mixed(const __grid_constant__ Work w) {
     constexpr int MAXPP = MAXN1 * MAXN1 * even_up<MAXN1>();
     constexpr int FAR_CL = far_clusters<MAXN1>(), ST = 32 * SW, FAR_PART = far_part(SW);
@@ -641,8 +646,8 @@ __global__ void __launch_bounds__(32 * SW, 16 / SW) far_mixed(const __grid_const
         const Fields &a = w.sys[it.y >> 16];
         const Place pl(a.split, SW);
         const int b = it.x, orb = it.y & 0xffff;
-        const int n1 = EXACT ? MAXN1 : a.n1, P = EXACT ? MAXN1 * MAXN1 * MAXN1 : a.P;
-        const int n1p = n1 + (n1 & 1), Pp = n1 * n1 * n1p;
+        const int n1 = LOOPS == FAR_FIXED ? MAXN1 : a.n1, P = LOOPS == FAR_FIXED ? MAXN1 * MAXN1 * MAXN1 : a.P;
+        const int n1p = LOOPS ? even_up<MAXN1>() : n1 + (n1 & 1), Pp = n1 * n1 * n1p;
         const int f0 = a.far_off[b], f1 = a.far_off[b + 1];
         const int bn = a.batch_node[b];
         const int te = it.w;
@@ -741,10 +746,10 @@ __global__ void __launch_bounds__(32 * SW, 16 / SW) far_mixed(const __grid_const
                     };
                     const int slab = first_slab(cl, n1, pl);
                     if (s_slot[c0 + cl] & 1)
-                        far_cluster<KERN, SS, false, MAXN1, NT, EXACT>(s_q[cl], s_w[cl], s_p[cl], n1, slab, pl.S, tx,
+                        far_cluster<KERN, SS, false, MAXN1, NT, LOOPS>(s_q[cl], s_w[cl], s_p[cl], n1, slab, pl.S, tx,
                                                                        ty, tz, nfi, add);
                     else
-                        far_cluster<KERN, SS, true, MAXN1, NT, EXACT>(s_q[cl], s_w[cl], s_p[cl], n1, slab, pl.S, tx,
+                        far_cluster<KERN, SS, true, MAXN1, NT, LOOPS>(s_q[cl], s_w[cl], s_p[cl], n1, slab, pl.S, tx,
                                                                       ty, tz, nfi, add);
                 }
             }
@@ -987,14 +992,14 @@ __global__ void __launch_bounds__(GT, 4) near_group(const __grid_constant__ Work
 
 // One staged proxy grid against one target for a group of orbitals (see
 // far_cluster for the padded innermost axis).
-template <bool SS, int MAXN1, int OG, bool EXACT = false, int N2 = OG / 2>
+template <bool SS, int MAXN1, int OG, int LOOPS = FAR_ANY, int N2 = OG / 2>
 __device__ __forceinline__ void far_group_cluster(const float4 *__restrict__ s_q4, const float *__restrict__ s_w,
                                                   const float (*s_p)[MAXN1], int n1_in,
                                                   float tx, float ty, float tz, const float2 (&nfi)[OG],
                                                   const float2 (&kc)[OG], float (&sum)[OG], float (&cmp)[OG]) {
     constexpr int MH = even_up<MAXN1>() / 2;
-    const int n1 = EXACT ? MAXN1 : n1_in;
-    const int n1p = n1 + (n1 & 1);
+    const int n1 = LOOPS == FAR_FIXED ? MAXN1 : n1_in;
+    const int n1p = LOOPS ? even_up<MAXN1>() : n1 + (n1 & 1);
     float2 dz2[MH];
 #pragma unroll
     for (int m = 0; m < MH; m++) {
@@ -1014,7 +1019,7 @@ __device__ __forceinline__ void far_group_cluster(const float4 *__restrict__ s_q
             const float2 rxy = dup2(fmaf(dy, dy, dx2));
 #pragma unroll
             for (int m = 0; m < MH; m++) {
-                if (2 * m < n1) {
+                if (LOOPS || 2 * m < n1) {
                     const float2 r2 = add2(rxy, dz2[m]);
                     const float2 rr = mul2(r2, rsqrt2(r2));
                     const float2 nl = nlog2r2(r2);
@@ -1046,7 +1051,7 @@ __host__ __device__ constexpr size_t far_group_smem(int n1, int og) {
     return sizeof(float) * (size_t)n1 * n1 * (n1 + (n1 & 1)) * (og + 1);
 }
 
-template <bool SS, int MAXN1, int OG, bool EXACT = false>
+template <bool SS, int MAXN1, int OG, int LOOPS = FAR_ANY>
 __global__ void __launch_bounds__(GT, 4) far_group(const __grid_constant__ Work w) {
     extern __shared__ __align__(16) float s_dyn[];
     __shared__ float s_p[3][MAXN1];
@@ -1060,8 +1065,8 @@ __global__ void __launch_bounds__(GT, 4) far_group(const __grid_constant__ Work 
         const int4 it = w.items[item];
         const Fields &a = w.sys[it.y >> 16];
         const int b = it.x, g0 = it.y & 0xffff;
-        const int n1 = EXACT ? MAXN1 : a.n1, P = EXACT ? MAXN1 * MAXN1 * MAXN1 : a.P;
-        const int n1p = n1 + (n1 & 1), Pp = n1 * n1 * n1p;
+        const int n1 = LOOPS == FAR_FIXED ? MAXN1 : a.n1, P = LOOPS == FAR_FIXED ? MAXN1 * MAXN1 * MAXN1 : a.P;
+        const int n1p = LOOPS ? even_up<MAXN1>() : n1 + (n1 & 1), Pp = n1 * n1 * n1p;
         const float *s_w = s_dyn + (size_t)Pp * OG;   // Pp * OG is a multiple of 4: float4 aligned
         const int f0 = a.far_off[b], f1 = a.far_off[b + 1];
         const int bn = a.batch_node[b];
@@ -1110,7 +1115,7 @@ __global__ void __launch_bounds__(GT, 4) far_group(const __grid_constant__ Work 
             __syncthreads();
             if (!warp_busy) continue;
             for_pairs<OG>(item_pairs<OG>(a.norb, g0), [&](auto c) {
-                far_group_cluster<SS, MAXN1, OG, EXACT, decltype(c)::value>(s_q4, s_w, s_p, n1, tx, ty, tz, nfi, kc,
+                far_group_cluster<SS, MAXN1, OG, LOOPS, decltype(c)::value>(s_q4, s_w, s_p, n1, tx, ty, tz, nfi, kc,
                                                                             sum, cmp);
             });
         }
@@ -1212,7 +1217,7 @@ __global__ void __launch_bounds__(GT, 4) far_group_db(const __grid_constant__ Wo
             if (!warp_busy) continue;
             const float *q = s_dyn + (size_t)cur * BUF;
             for_pairs<OG>(item_pairs<OG>(a.norb, g0), [&](auto c) {
-                far_group_cluster<SS, DB_N1, OG, true, decltype(c)::value>(reinterpret_cast<const float4 *>(q),
+                far_group_cluster<SS, DB_N1, OG, FAR_FIXED, decltype(c)::value>(reinterpret_cast<const float4 *>(q),
                                                                            q + DB_P * OG, s_p[cur], DB_N1, tx, ty, tz,
                                                                            nfi, kc, sum, cmp);
             });
@@ -1517,14 +1522,14 @@ __global__ void __launch_bounds__(GT, 4) near_group16(const __grid_constant__ Wo
 // One staged proxy grid against one target for 16 orbitals (see far_cluster
 // for the padded innermost axis; charges staged QS16 floats per proxy point).
 // NP: filled orbital pairs, as in group16_tile.
-template <bool SS, int MAXN1, bool EXACT, int NP = 8>
+template <bool SS, int MAXN1, int LOOPS, int NP = 8>
 __device__ __forceinline__ void far_group16_cluster(const float *__restrict__ s_q, const float *__restrict__ s_w,
                                                     const float (*s_p)[MAXN1], int n1_in,
                                                     float tx, float ty, float tz, const float2 (&nfi)[8],
                                                     const float2 (&kc)[8], float (&sum)[16], float (&cmp)[16]) {
     constexpr int MH = even_up<MAXN1>() / 2;
-    const int n1 = EXACT ? MAXN1 : n1_in;
-    const int n1p = n1 + (n1 & 1);
+    const int n1 = LOOPS == FAR_FIXED ? MAXN1 : n1_in;
+    const int n1p = LOOPS ? even_up<MAXN1>() : n1 + (n1 & 1);
     float2 dz2[MH];
 #pragma unroll
     for (int m = 0; m < MH; m++) {
@@ -1544,7 +1549,7 @@ __device__ __forceinline__ void far_group16_cluster(const float *__restrict__ s_
             const float2 rxy = dup2(fmaf(dy, dy, dx2));
 #pragma unroll
             for (int m = 0; m < MH; m++) {
-                if (2 * m < n1) {
+                if (LOOPS || 2 * m < n1) {
                     const float2 r2 = add2(rxy, dz2[m]);
                     const float2 rr = mul2(r2, rsqrt2(r2));
                     const float2 nl = nlog2r2(r2);
@@ -1580,14 +1585,14 @@ __device__ __forceinline__ void far_group16_cluster(const float *__restrict__ s_
     }
 }
 
-template <bool SS, int MAXN1, bool EXACT>
+template <bool SS, int MAXN1, int LOOPS>
 __device__ __forceinline__ void far_group16_cluster_np(int np, const float *__restrict__ s_q,
                                                        const float *__restrict__ s_w, const float (*s_p)[MAXN1],
                                                        int n1, float tx, float ty,
                                                        float tz, const float2 (&nfi)[8], const float2 (&kc)[8],
                                                        float (&sum)[16], float (&cmp)[16]) {
 #define TAGI_F16(N) \
-    far_group16_cluster<SS, MAXN1, EXACT, N>(s_q, s_w, s_p, n1, tx, ty, tz, nfi, kc, sum, cmp)
+    far_group16_cluster<SS, MAXN1, LOOPS, N>(s_q, s_w, s_p, n1, tx, ty, tz, nfi, kc, sum, cmp)
     switch (np) {
     case 1: TAGI_F16(1); break;
     case 2: TAGI_F16(2); break;
@@ -1607,7 +1612,7 @@ __host__ __device__ constexpr size_t far_group16_smem(int n1) {
     return sizeof(float) * (size_t)n1 * n1 * (n1 + (n1 & 1)) * (QS16 + 1);
 }
 
-template <bool SS, int MAXN1, bool EXACT>
+template <bool SS, int MAXN1, int LOOPS>
 __global__ void __launch_bounds__(GT, 4) far_group16(const __grid_constant__ Work w) {
     extern __shared__ __align__(16) float s_dyn[];
     __shared__ float s_p[3][MAXN1];
@@ -1620,8 +1625,8 @@ __global__ void __launch_bounds__(GT, 4) far_group16(const __grid_constant__ Wor
         const int4 it = w.items[item];
         const Fields &a = w.sys[it.y >> 16];
         const int b = it.x, g0 = it.y & 0xffff;
-        const int n1 = EXACT ? MAXN1 : a.n1, P = EXACT ? MAXN1 * MAXN1 * MAXN1 : a.P;
-        const int n1p = n1 + (n1 & 1), Pp = n1 * n1 * n1p;
+        const int n1 = LOOPS == FAR_FIXED ? MAXN1 : a.n1, P = LOOPS == FAR_FIXED ? MAXN1 * MAXN1 * MAXN1 : a.P;
+        const int n1p = LOOPS ? even_up<MAXN1>() : n1 + (n1 & 1), Pp = n1 * n1 * n1p;
         float *s_q = s_dyn;
         float *s_w = s_dyn + (size_t)Pp * QS16;
         const int f0 = a.far_off[b], f1 = a.far_off[b + 1];
@@ -1680,7 +1685,7 @@ __global__ void __launch_bounds__(GT, 4) far_group16(const __grid_constant__ Wor
             }
             __syncthreads();
             if (!warp_busy) continue;
-            far_group16_cluster_np<SS, MAXN1, EXACT>(group16_pairs(a.norb, g0), s_q, s_w, s_p, n1,
+            far_group16_cluster_np<SS, MAXN1, LOOPS>(group16_pairs(a.norb, g0), s_q, s_w, s_p, n1,
                                                      tx, ty, tz,                                                      nfi, kc, sum, cmp);
         }
         if (v) {
@@ -2131,7 +2136,7 @@ __global__ void __launch_bounds__(FT) pair_peak_far(int reps, float *out) {
         nfi[k] = dup2(-0.3f);
     }
     for (int r = 0; r < reps; r++)
-        far_cluster<KERN, SS, true, N1, 2, true>(s_q, s_w, s_p, N1, 0, 1, tx, ty, tz, nfi,
+        far_cluster<KERN, SS, true, N1, 2, FAR_FIXED>(s_q, s_w, s_p, N1, 0, 1, tx, ty, tz, nfi,
                                                  [&](int, int k, float part) { kahan_add(sum[k], cmp[k], part); });
     out[blockIdx.x * FT + threadIdx.x] = sum[0] + sum[1] - cmp[0] - cmp[1];
 }
@@ -2191,7 +2196,7 @@ __global__ void __launch_bounds__(GT, 4) pair_peak_far_group(int reps, float *ou
         sum[o] = cmp[o] = 0.f;
     }
     for (int r = 0; r < reps; r++)
-        far_group_cluster<SS, N1, OG, true>(s_q4, s_w, s_p, N1, tx, ty, tz, nfi, kc, sum, cmp);
+        far_group_cluster<SS, N1, OG, FAR_FIXED>(s_q4, s_w, s_p, N1, tx, ty, tz, nfi, kc, sum, cmp);
     float acc = 0.f;
 #pragma unroll
     for (int o = 0; o < OG; o++) acc += sum[o] - cmp[o];
@@ -2255,7 +2260,7 @@ __global__ void __launch_bounds__(GT, 4) pair_peak_far_group16(int reps, float *
 #pragma unroll
     for (int o = 0; o < 16; o++) sum[o] = cmp[o] = 0.f;
     for (int r = 0; r < reps; r++)
-        far_group16_cluster<SS, N1, true>(s_q, s_w, s_p, N1, tx, ty, tz, nfi, kc, sum, cmp);
+        far_group16_cluster<SS, N1, FAR_FIXED>(s_q, s_w, s_p, N1, tx, ty, tz, nfi, kc, sum, cmp);
     float acc = 0.f;
 #pragma unroll
     for (int o = 0; o < 16; o++) acc += sum[o] - cmp[o];
@@ -2333,10 +2338,30 @@ struct LaunchShape {
     int minn1 = 1 << 20;  // smallest proxy-grid edge n + 1
 };
 
+// fn(MAXN1, loops) for the far kernel of a launch: rows of a known length where all its
+// systems have one, everything known at degree 7, the usual one.
+template <int N, int LOOPS, typename FN>
+int far_call(FN &&fn) { return fn(std::integral_constant<int, N>(), std::integral_constant<int, LOOPS>()); }
+template <typename FN>
+int far_loops(const LaunchShape &sh, FN &&fn) {
+    const int row = sh.maxn1 + (sh.maxn1 & 1);
+    if (sh.maxn1 <= 4) return far_call<4, FAR_ANY>(fn);
+    if (sh.minn1 == 8 && sh.maxn1 == 8) return far_call<8, FAR_FIXED>(fn);
+    if (sh.minn1 >= row - 1) {
+        if (row == 6) return far_call<6, FAR_ROWS>(fn);
+        if (row == 8) return far_call<8, FAR_ROWS>(fn);
+        if (row == 10) return far_call<10, FAR_ROWS>(fn);
+        return far_call<12, FAR_ROWS>(fn);
+    }
+    if (sh.maxn1 <= 8) return far_call<8, FAR_ANY>(fn);
+    return far_call<MAX_DEGREE + 1, FAR_ANY>(fn);
+}
+static_assert(MAX_DEGREE == 10, "far_loops lists the row lengths");
+
 template <int KERN, bool SS, int SW>
 int launch_mixed(const Work &wn, const Work &wc, const Work &wf, const LaunchShape &sh, cudaStream_t s, bool *pdl) {
     constexpr int ST = 32 * SW;
-    const bool one = sh.nt == 1, deg7 = sh.maxn1 == 8 && sh.minn1 == 8;
+    const bool one = sh.nt == 1;
     if (one) TAGI_TRY(launch_persistent(near_mixed<KERN, SS, 1, 0, SW>, wn, s, 0, ST, pdl));
     else TAGI_TRY(launch_persistent(near_mixed<KERN, SS, 2, 0, SW>, wn, s, 0, ST, pdl));
     phase_mark(PH_NEAR, false, s);
@@ -2345,17 +2370,10 @@ int launch_mixed(const Work &wn, const Work &wc, const Work &wf, const LaunchSha
     else TAGI_TRY(launch_persistent(near_mixed<KERN, SS, 2, 1, SW>, wc, s, 0, ST, pdl));
     phase_mark(PH_NEAR_CLOSE, false, s);
     phase_mark(PH_FAR, true, s);
-    if (one) {
-        if (sh.maxn1 <= 4) TAGI_TRY(launch_persistent(far_mixed<KERN, SS, 4, 1, SW>, wf, s, 0, ST, pdl));
-        else if (deg7) TAGI_TRY(launch_persistent(far_mixed<KERN, SS, 8, 1, SW, true>, wf, s, 0, ST, pdl));
-        else if (sh.maxn1 <= 8) TAGI_TRY(launch_persistent(far_mixed<KERN, SS, 8, 1, SW>, wf, s, 0, ST, pdl));
-        else TAGI_TRY(launch_persistent(far_mixed<KERN, SS, MAX_DEGREE + 1, 1, SW>, wf, s, 0, ST, pdl));
-    } else {
-        if (sh.maxn1 <= 4) TAGI_TRY(launch_persistent(far_mixed<KERN, SS, 4, 2, SW>, wf, s, 0, ST, pdl));
-        else if (deg7) TAGI_TRY(launch_persistent(far_mixed<KERN, SS, 8, 2, SW, true>, wf, s, 0, ST, pdl));
-        else if (sh.maxn1 <= 8) TAGI_TRY(launch_persistent(far_mixed<KERN, SS, 8, 2, SW>, wf, s, 0, ST, pdl));
-        else TAGI_TRY(launch_persistent(far_mixed<KERN, SS, MAX_DEGREE + 1, 2, SW>, wf, s, 0, ST, pdl));
-    }
+    TAGI_TRY(far_loops(sh, [&](auto maxn1, auto loops) {
+        if (one) return launch_persistent(far_mixed<KERN, SS, maxn1(), 1, SW, loops()>, wf, s, 0, ST, pdl);
+        return launch_persistent(far_mixed<KERN, SS, maxn1(), 2, SW, loops()>, wf, s, 0, ST, pdl);
+    }));
     phase_mark(PH_FAR, false, s);
     return TAGI_OK;
 }
@@ -2393,14 +2411,9 @@ int launch_fields(const SysCall *calls, const Fields *f, int nsys, const Schedul
         TAGI_TRY(launch_persistent(near_group16<SS, 1>, wc, s, near_group16_smem(1), GT, &pdl));
         phase_mark(PH_NEAR_CLOSE, false, s);
         phase_mark(PH_FAR, true, s);
-        if (sh.maxn1 <= 4)
-            TAGI_TRY(launch_persistent(far_group16<SS, 4, false>, wf, s, far_group16_smem(sh.maxn1), GT, &pdl));
-        else if (sh.maxn1 == 8 && sh.minn1 == 8)   // degree 7 everywhere: fixed loops
-            TAGI_TRY(launch_persistent(far_group16<SS, 8, true>, wf, s, far_group16_smem(8), GT, &pdl));
-        else if (sh.maxn1 <= 8)
-            TAGI_TRY(launch_persistent(far_group16<SS, 8, false>, wf, s, far_group16_smem(sh.maxn1), GT, &pdl));
-        else
-            TAGI_TRY(launch_persistent(far_group16<SS, MAX_DEGREE + 1, false>, wf, s, far_group16_smem(sh.maxn1), GT, &pdl));
+        TAGI_TRY(far_loops(sh, [&](auto maxn1, auto loops) {
+            return launch_persistent(far_group16<SS, maxn1(), loops()>, wf, s, far_group16_smem(sh.maxn1), GT, &pdl);
+        }));
         phase_mark(PH_FAR, false, s);
         return TAGI_OK;
     }
@@ -2415,20 +2428,16 @@ int launch_fields(const SysCall *calls, const Fields *f, int nsys, const Schedul
         else TAGI_TRY(launch_persistent(near_group<SS, 4, 1>, wc, s, 0, GT, &pdl));
         phase_mark(PH_NEAR_CLOSE, false, s);
         phase_mark(PH_FAR, true, s);
-        const size_t fsm = far_group_smem(sh.maxn1, sh.og);
-        if (sh.maxn1 <= 4) {
-            if (g8) TAGI_TRY(launch_persistent(far_group<SS, 4, 8>, wf, s, fsm, GT, &pdl));
-            else TAGI_TRY(launch_persistent(far_group<SS, 4, 4>, wf, s, fsm, GT, &pdl));
-        } else if (sh.maxn1 == 8 && sh.minn1 == 8) {   // degree 7 everywhere: pipelined staging, fixed loops
-            if (g8) TAGI_TRY(launch_persistent(far_group_db<SS, 8>, wf, s, far_group_db_smem(8), GT, &pdl));
-            else TAGI_TRY(launch_persistent(far_group_db<SS, 4>, wf, s, far_group_db_smem(4), GT, &pdl));
-        } else if (sh.maxn1 <= 8) {
-            if (g8) TAGI_TRY(launch_persistent(far_group<SS, 8, 8>, wf, s, fsm, GT, &pdl));
-            else TAGI_TRY(launch_persistent(far_group<SS, 8, 4>, wf, s, fsm, GT, &pdl));
-        } else {
-            if (g8) TAGI_TRY(launch_persistent(far_group<SS, MAX_DEGREE + 1, 8>, wf, s, fsm, GT, &pdl));
-            else TAGI_TRY(launch_persistent(far_group<SS, MAX_DEGREE + 1, 4>, wf, s, fsm, GT, &pdl));
-        }
+        TAGI_TRY(far_loops(sh, [&](auto maxn1, auto loops) {
+            if constexpr (loops() == FAR_FIXED) {   // pipelined staging
+                if (g8) return launch_persistent(far_group_db<SS, 8>, wf, s, far_group_db_smem(8), GT, &pdl);
+                return launch_persistent(far_group_db<SS, 4>, wf, s, far_group_db_smem(4), GT, &pdl);
+            } else {
+                const size_t fsm = far_group_smem(sh.maxn1, sh.og);
+                if (g8) return launch_persistent(far_group<SS, maxn1(), 8, loops()>, wf, s, fsm, GT, &pdl);
+                return launch_persistent(far_group<SS, maxn1(), 4, loops()>, wf, s, fsm, GT, &pdl);
+            }
+        }));
         phase_mark(PH_FAR, false, s);
         return TAGI_OK;
     }
