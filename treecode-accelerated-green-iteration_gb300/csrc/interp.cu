@@ -106,7 +106,7 @@ __global__ void __launch_bounds__(IT, 10) interp_cells(
     __shared__ double s_t[2][p3];                // contracted over x; over x and y
     __shared__ double s_f0[2][p1];               // the x and y coordinates that they belong to
     __shared__ double s_L[3][p2];        // Lx, Ly, Lz: [fine index][node]
-    __shared__ double s_inv[3][p1];                 // reciprocal sums of their rows
+    __shared__ double s_sum[3][p1], s_inv[3][p1];   // sums of their rows, reciprocals
     __shared__ double s_f[3][p1];                // the block's 1-D fine coordinates
     __shared__ double s_nx[p1], s_ny[p1], s_nz[p1], s_w[p1];
     // the cells' points must fit the arrays: nothing is read or written otherwise
@@ -193,6 +193,7 @@ __global__ void __launch_bounds__(IT, 10) interp_cells(
                 double sum = 0.0;
 #pragma unroll
                 for (int k = 0; k < p1; k++) sum += s_L[d][m * p1 + k];
+                s_sum[d][m] = sum;
                 s_inv[d][m] = 1.0 / sum;
                 if (d < 2) s_f0[d][m] = s_f[d][m];
             }
@@ -201,7 +202,14 @@ __global__ void __launch_bounds__(IT, 10) interp_cells(
 #pragma unroll 1
         for (int q = tid; q < 3 * p2; q += IT) {
             const int d = q / p2, mk = q - d * p2;
-            if (d == 2 || (d == 0 ? newx : newy)) s_L[d][mk] *= s_inv[d][mk / p1];
+            if (d == 2 || (d == 0 ? newx : newy)) {
+                // a quotient from the reciprocal and its remainder: a product alone would give
+                // a whole row the reciprocal's rounding error (4.3e-16 instead of 4.2e-16
+                // from 64-bit results in the largest case)
+                const int m = mk / p1;
+                const double v = s_L[d][mk], inv = s_inv[d][m], qt = v * inv;
+                s_L[d][mk] = fma(fma(-qt, s_sum[d][m], v), inv, qt);
+            }
         }
         __syncthreads();
         if (newx) {   // T1[a][j][k] = sum_i Lx[a][i] F[i][j][k]
