@@ -93,7 +93,7 @@ __device__ __noinline__ double interp_point(double tx, double ty, double tz, con
 // children instead of 24, 39 instead of 81 per 27 points of 27.  The rows of 1-D
 // weights are divided out by all threads: in one thread per row the divisions of a
 // single warp held up the block as long as its contractions.  Ring molecule, 14.3M fine
-// points, order 7: 1184 -> 556 us a call.
+// points, order 7: 1184 -> 571 us a call.
 template <int p1>
 __global__ void __launch_bounds__(IT, 10) interp_cells(
     const double *__restrict__ cX, const double *__restrict__ cY, const double *__restrict__ cZ,

@@ -15,10 +15,9 @@
 //   coarse points   utilities/mpiMeshBuilding.py:725-752
 //   fine points     utilities/mpiMeshBuilding.py:755-840
 //
-// GPU layout.  Refinement is level-synchronous: one thread per cell of the
-// current level decides divide / leaf; an exclusive scan of the divide flags
-// places the 8 children of each dividing cell in the next level and each leaf
-// in this level's leaf list.  Every cell carries a 64-bit path key (base cell
+// GPU layout.  Refinement is level-synchronous, one launch per level: eight lanes per
+// cell of the current level decide divide / leaf and write its children into the next
+// level or the leaf into the list of leaves.  Every cell carries a 64-bit path key (base cell
 // index in bits 48-63, then 3 bits per level, child digit 4i+2j+k), so one
 // radix sort of the leaf keys gives the depth-first order.  Point generation
 // is one thread per output point (32 bytes written: x, y, z, w); fine points
@@ -26,13 +25,15 @@
 // is FP64 with explicit round-to-nearest intrinsics in the order the
 // reference's numpy expressions evaluate, so the cells and points are
 // bit-identical to the reference's on the same 1-D node and weight tables.
-// Ring molecule, 5,104 cells, 16.9M points, build_mesh 2.38 -> 1.19 ms: the nearest corner
+// Ring molecule, 5,104 cells, 16.9M points, build_mesh 2.37 -> 0.58 ms: the nearest corner
 // of a cell from the smallest square along each axis with one root per cell (eight
-// corners, a root each, per atom before: 92 us a level), leaves sorted in two launches,
-// scans of a level in one launch, and one refinement instead of a counting one first.
+// corners, a root each, per atom before: 92 us a level), no counts read back between levels,
+// leaves sorted in two launches, and one refinement instead of a counting one first.
 #include "tagi_internal.h"
 
+#include <algorithm>
 #include <cmath>
+#include <type_traits>
 
 namespace tagi {
 namespace {
@@ -48,6 +49,8 @@ struct Rule {
     int ge2, ge1, fine;  // level >= 2, level >= 1, level < -1
     int nsub;            // -int(level): fine children per side
     int min_depth, max_depth;
+    // distances and sides of the cascade, each rounded as the reference's expression
+    double far, r4, r2, h4th, h2th, h2, h4, h8, a1, a2, a3, r15;
 };
 
 struct Tables {
@@ -57,121 +60,144 @@ struct Tables {
 
 __device__ __forceinline__ double half_of(double a) { return __dmul_rn(a, 0.5); }
 
-// divide flag and fine children of one cell (CellStruct_CC.py:2344-2439).
-__global__ void __launch_bounds__(MT) mesh_classify(const double *__restrict__ cells, int n, int depth,
-                                                    const double *__restrict__ atoms, int natoms,
-                                                    Rule p, int *__restrict__ divide,
-                                                    int *__restrict__ fine, int *__restrict__ err) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const double *c = cells + 6L * i;
-    const double xmin = c[0], xmax = c[1], ymin = c[2], ymax = c[3], zmin = c[4], zmax = c[5];
-    int div = 0, nf = 1;
-    if (depth < p.min_depth) {
-        div = 1;
-    } else {
-        // The distance to the nearest corner: rounded squares, sums and roots are
-        // monotone, so the smallest square along each axis gives the smallest
-        // rounded distance of the eight corners, and one root serves all atoms.
-        double d2 = __longlong_as_double(0x7ff0000000000000LL);
-        bool inside = false;
-        for (int a = 0; a < natoms; a++) {
-            const double ax = atoms[3 * a], ay = atoms[3 * a + 1], az = atoms[3 * a + 2];
-            if (ax < xmax && ay < ymax && az < zmax && ax > xmin && ay > ymin && az > zmin) {
-                inside = true;
+// Counters of a refinement, on the device.
+struct Progress {
+    unsigned long long fine;            // children (or 1) per leaf, summed
+    int err;                            // 1: refines below maxDepth; 2: a level or the leaves do not fit
+    int leaves;
+    int count[MESH_MAX_DEPTH + 2];      // cells of each level
+};
+
+__global__ void mesh_start(Progress *p, int nbase) {
+    const int i = threadIdx.x;
+    if (i < MESH_MAX_DEPTH + 2) p->count[i] = i ? 0 : nbase;
+    if (i == 0) {
+        p->fine = 0;
+        p->err = p->leaves = 0;
+    }
+}
+
+// One level: divide flag and fine children of each cell (CellStruct_CC.py:2344-2439), the
+// children of a dividing cell into the next level, a leaf into the leaf list.  Eight lanes a
+// cell: they share the atoms, then a lane writes a child.  Places are taken from the
+// counters as warps come, one addition a warp and counter: the leaves are sorted by their
+// keys afterwards, so the order within a level does not matter, and the host reads no
+// count between levels.  A level was a classification of one thread per cell (14 us: 12
+// atoms in turn on the FP64 pipe), a scan, a copy to the host and eight allocations, 85 us in all.
+constexpr int CELL_LANES = 8, LEVEL_THREADS = 128;
+__global__ void __launch_bounds__(LEVEL_THREADS) mesh_level(
+    const double *__restrict__ cells, const uint64_t *__restrict__ keys, int depth, const double *__restrict__ atoms,
+    int natoms, const __grid_constant__ Rule p, Progress *prog, double *__restrict__ next_cells,
+    uint64_t *__restrict__ next_keys, int next_cap, double *__restrict__ leaf_cells, uint64_t *__restrict__ leaf_keys,
+    int *__restrict__ leaf_fine, int leaf_cap) {
+    chain_begin();
+    const int n = prog->count[depth];
+    if (prog->err & 2) return;
+    const int lane = threadIdx.x & 31, q = lane & (CELL_LANES - 1);
+    const int group = (blockIdx.x * LEVEL_THREADS + threadIdx.x) / CELL_LANES, groups = gridDim.x * LEVEL_THREADS / CELL_LANES;
+    const int warp_first = group - lane / CELL_LANES;
+    for (int base = warp_first; base < n; base += groups) {   // the same for all of a warp
+        const int i = base + lane / CELL_LANES;
+        const bool valid = i < n;
+        const double *c = cells + 6L * (valid ? i : 0);
+        const double xmin = c[0], xmax = c[1], ymin = c[2], ymax = c[3], zmin = c[4], zmax = c[5];
+        int div = 0, nf = 1;
+        if (depth < p.min_depth) {
+            div = 1;
+        } else {
+            // The distance to the nearest corner: rounded squares, sums and roots are
+            // monotone, so the smallest square along each axis gives the smallest
+            // rounded distance of the eight corners, and one root serves all atoms.
+            double d2 = __longlong_as_double(0x7ff0000000000000LL);
+            int inside = 0;
+            for (int a = q; a < natoms; a += CELL_LANES) {
+                const double ax = atoms[3 * a], ay = atoms[3 * a + 1], az = atoms[3 * a + 2];
+                if (ax < xmax && ay < ymax && az < zmax && ax > xmin && ay > ymin && az > zmin) {
+                    inside = 1;
+                    continue;
+                }
+                const double x0 = __dsub_rn(xmin, ax), x1 = __dsub_rn(xmax, ax), y0 = __dsub_rn(ymin, ay),
+                             y1 = __dsub_rn(ymax, ay), z0 = __dsub_rn(zmin, az), z1 = __dsub_rn(zmax, az);
+                const double x = fmin(fabs(x0), fabs(x1)), y = fmin(fabs(y0), fabs(y1)), z = fmin(fabs(z0), fabs(z1));
+                const double s = __dadd_rn(__dadd_rn(__dmul_rn(x, x), __dmul_rn(y, y)), __dmul_rn(z, z));
+                if (s < d2) d2 = s;
+            }
+            // d2 >= +0 and no NaN got in: its bit pattern orders as an integer does
+            long long b2 = __double_as_longlong(d2);
+#pragma unroll
+            for (int o = CELL_LANES / 2; o > 0; o >>= 1) {
+                b2 = min(b2, __shfl_xor_sync(0xffffffffu, b2, o));
+                inside |= __shfl_xor_sync(0xffffffffu, inside, o);
+            }
+            double dist = p.far;
+            const double dc = __dsqrt_rn(__longlong_as_double(b2));
+            if (dc < dist) dist = dc;
+            if (inside) dist = 0.0;
+            const double sz = __dsub_rn(zmax, zmin), sx = __dsub_rn(xmax, xmin), sy = __dsub_rn(ymax, ymin);
+            double side = sz;
+            if (sx > side) side = sx;
+            if (sy > side) side = sy;
+            if (side > p.H)
+                div = 1;
+            else if (p.ge2 && dist < p.r4)
+                div = side > p.h4th;
+            else if (p.ge1 && dist < p.r2)
+                div = side > p.h2th;
+            else if (dist < p.r)
+                div = side > p.h;
+            else if (dist < p.a1)
+                div = side > p.h2;
+            else if (dist < p.a2)
+                div = side > p.h4;
+            else if (dist < p.a3)
+                div = side > p.h8;
+            if (!div && p.fine && dist < p.r15) nf = p.nsub * p.nsub * p.nsub;
+        }
+        if (div && depth >= p.max_depth) {
+            if (valid && q == 0) atomicOr(&prog->err, 1);
+            div = 0;
+        }
+        // places: one bit per cell in each mask
+        const unsigned first = 0x01010101u;
+        const unsigned md = __ballot_sync(0xffffffffu, valid && div) & first, ml = __ballot_sync(0xffffffffu, valid && !div) & first;
+        const int fine = __reduce_add_sync(0xffffffffu, valid && !div && q == 0 ? nf : 0);
+        int at_d = 0, at_l = 0;
+        if (lane == 0) {
+            if (md) at_d = atomicAdd(&prog->count[depth + 1], 8 * __popc(md));
+            if (ml) {
+                at_l = atomicAdd(&prog->leaves, __popc(ml));
+                atomicAdd(&prog->fine, (unsigned long long)fine);
+            }
+        }
+        const unsigned before = (1u << (lane & ~(CELL_LANES - 1))) - 1u;
+        at_d = __shfl_sync(0xffffffffu, at_d, 0) + 8 * __popc(md & before);
+        at_l = __shfl_sync(0xffffffffu, at_l, 0) + __popc(ml & before);
+        if (!valid) continue;
+        const uint64_t key = keys ? keys[i] : (uint64_t)i << 48;
+        if (div) {
+            if (at_d > next_cap - 8) {
+                if (q == 0) atomicOr(&prog->err, 2);
                 continue;
             }
-            const double x0 = __dsub_rn(xmin, ax), x1 = __dsub_rn(xmax, ax), y0 = __dsub_rn(ymin, ay),
-                         y1 = __dsub_rn(ymax, ay), z0 = __dsub_rn(zmin, az), z1 = __dsub_rn(zmax, az);
-            const double x = fmin(fabs(x0), fabs(x1)), y = fmin(fabs(y0), fabs(y1)), z = fmin(fabs(z0), fabs(z1));
-            const double s = __dadd_rn(__dadd_rn(__dmul_rn(x, x), __dmul_rn(y, y)), __dmul_rn(z, z));
-            if (s < d2) d2 = s;
+            // child q = 4 ii + 2 jj + kk; xdiv = (xmax + xmin)/2 (TreeStruct_CC.py:1129-1131)
+            const double xm = half_of(__dadd_rn(xmax, xmin)), ym = half_of(__dadd_rn(ymax, ymin)),
+                         zm = half_of(__dadd_rn(zmax, zmin));
+            double *o = next_cells + 6L * (at_d + q);
+            o[0] = q & 4 ? xm : xmin;
+            o[1] = q & 4 ? xmax : xm;
+            o[2] = q & 2 ? ym : ymin;
+            o[3] = q & 2 ? ymax : ym;
+            o[4] = q & 1 ? zm : zmin;
+            o[5] = q & 1 ? zmax : zm;
+            next_keys[at_d + q] = key | ((uint64_t)q << (3 * (MESH_MAX_DEPTH - 1 - depth)));
+        } else if (at_l >= leaf_cap) {
+            if (q == 0) atomicOr(&prog->err, 2);
+        } else {
+            if (q < 6) leaf_cells[6L * at_l + q] = c[q];
+            if (q == 6) leaf_keys[at_l] = key;
+            if (q == 7) leaf_fine[at_l] = nf;
         }
-        double dist = __dadd_rn(10.0, p.H);
-        const double dc = __dsqrt_rn(d2);
-        if (dc < dist) dist = dc;
-        if (inside) dist = 0.0;
-        const double sz = __dsub_rn(zmax, zmin), sx = __dsub_rn(xmax, xmin), sy = __dsub_rn(ymax, ymin);
-        double side = sz;
-        if (sx > side) side = sx;
-        if (sy > side) side = sy;
-        const double h = p.h, r = p.r;
-        const double h2 = __dmul_rn(2.0, h), h4 = __dmul_rn(4.0, h), h8 = __dmul_rn(8.0, h);
-        const double a1 = __dadd_rn(r, __dmul_rn(h2, 1.0));
-        const double a2 = __dadd_rn(r, __dmul_rn(__dadd_rn(h2, h4), 1.0));
-        const double a3 = __dadd_rn(r, __dmul_rn(__dadd_rn(__dadd_rn(h2, h4), h8), 1.0));
-        if (side > p.H)
-            div = 1;
-        else if (p.ge2 && dist < __ddiv_rn(r, 4.0))
-            div = side > __ddiv_rn(h, 4.0);
-        else if (p.ge1 && dist < __ddiv_rn(r, 2.0))
-            div = side > __ddiv_rn(h, 2.0);
-        else if (dist < r)
-            div = side > h;
-        else if (dist < a1)
-            div = side > h2;
-        else if (dist < a2)
-            div = side > h4;
-        else if (dist < a3)
-            div = side > h8;
-        if (!div && p.fine && dist < __dmul_rn(r, 1.5)) nf = p.nsub * p.nsub * p.nsub;
     }
-    if (div && depth >= p.max_depth) {
-        atomicOr(err, 1);
-        div = 0;
-    }
-    divide[i] = div;
-    fine[i] = nf;
-}
-
-// Children of dividing cells into the next level; leaves into this level's
-// leaf list.  rank = exclusive scan of divide.
-__global__ void __launch_bounds__(MT) mesh_emit(const double *__restrict__ cells,
-                                                const uint64_t *__restrict__ keys, int n, int depth,
-                                                const int *__restrict__ divide,
-                                                const int *__restrict__ fine,
-                                                const int *__restrict__ rank,
-                                                double *__restrict__ next_cells,
-                                                uint64_t *__restrict__ next_keys,
-                                                double *__restrict__ leaf_cells,
-                                                uint64_t *__restrict__ leaf_keys,
-                                                int *__restrict__ leaf_fine) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const double *c = cells + 6L * i;
-    const uint64_t key = keys[i];
-    const int rk = rank[i];
-    if (divide[i]) {
-        // xdiv = (xmax + xmin)/2 (TreeStruct_CC.py:1129-1131)
-        const double xb[3] = {c[0], half_of(__dadd_rn(c[1], c[0])), c[1]};
-        const double yb[3] = {c[2], half_of(__dadd_rn(c[3], c[2])), c[3]};
-        const double zb[3] = {c[4], half_of(__dadd_rn(c[5], c[4])), c[5]};
-        const int shift = 3 * (MESH_MAX_DEPTH - 1 - depth);
-#pragma unroll
-        for (int q = 0; q < 8; q++) {
-            const int ii = q >> 2, jj = (q >> 1) & 1, kk = q & 1;
-            double *o = next_cells + 6L * (8L * rk + q);
-            o[0] = xb[ii];
-            o[1] = xb[ii + 1];
-            o[2] = yb[jj];
-            o[3] = yb[jj + 1];
-            o[4] = zb[kk];
-            o[5] = zb[kk + 1];
-            next_keys[8L * rk + q] = key | ((uint64_t)q << shift);
-        }
-    } else {
-        const long l = (long)i - rk;
-        double *o = leaf_cells + 6L * l;
-#pragma unroll
-        for (int k = 0; k < 6; k++) o[k] = c[k];
-        leaf_keys[l] = key;
-        leaf_fine[l] = fine[i];
-    }
-}
-
-__global__ void mesh_base_keys(uint64_t *__restrict__ keys, int n) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) keys[i] = (uint64_t)i << 48;
 }
 
 __global__ void mesh_iota(int *__restrict__ v, int n) {
@@ -405,119 +431,106 @@ int tagi_mesh_refine(const double *baseCells, int numBase, const double *atomXYZ
     if (p.fine && p.nsub > 4)
         return set_error(TAGI_ERR_UNSUPPORTED, "fine mesh of %d^3 children per cell (1, 8, 27 or 64 supported)",
                          p.nsub);
+    // host and device round these alike: the factors are powers of two but for r 1.5
+    p.far = 10.0 + H;
+    p.r4 = r / 4.0;
+    p.r2 = r / 2.0;
+    p.h4th = h / 4.0;
+    p.h2th = h / 2.0;
+    p.h2 = 2.0 * h;
+    p.h4 = 4.0 * h;
+    p.h8 = 8.0 * h;
+    p.a1 = r + p.h2;
+    p.a2 = r + (p.h2 + p.h4);
+    p.a3 = r + ((p.h2 + p.h4) + p.h8);
+    p.r15 = r * 1.5;
     const int p1 = order + 1, p3 = p1 * p1 * p1;
     cudaStream_t s = (cudaStream_t)stream;
     Arena tmp;
     tmp.stream = s;
     int rc = TAGI_OK;
     do {
-        int *err = nullptr;
-        double *cells = nullptr;
-        uint64_t *keys = nullptr;
-        if ((rc = tmp.alloc(&err, 2)) || (rc = tmp.alloc(&cells, 6L * numBase)) ||
-            (rc = tmp.alloc(&keys, numBase)))
-            break;
-        if (cudaMemsetAsync(err, 0, 2 * sizeof(int), s) != cudaSuccess ||
-            cudaMemcpyAsync(cells, baseCells, sizeof(double) * 6 * numBase, cudaMemcpyDeviceToDevice, s) !=
-                cudaSuccess) {
-            rc = set_error(TAGI_ERR_CUDA, "mesh setup copy failed");
-            break;
-        }
-        launch(mesh_base_keys, grid_for(numBase), MT, 0, s, keys, numBase);
-        struct Level {
-            double *cells;
-            uint64_t *keys;
-            int *fine;
-            long n;
-        };
-        std::vector<Level> leaves;
-        long n = numBase, total = 0;
-        for (int depth = 0; n > 0; depth++) {
-            int *divide = nullptr, *fine = nullptr, *rank = nullptr;
-            if ((rc = tmp.alloc(&divide, n)) || (rc = tmp.alloc(&fine, n)) || (rc = tmp.alloc(&rank, n + 1)))
-                break;
-            // small blocks: a level has 500 to 5,000 cells, a chain of FP64 operations each
-            launch(mesh_classify, (unsigned)((n + 31) / 32), 32, 0, s, cells, (int)n, depth, atomXYZ, numAtoms, p, divide,
-                   fine, err);
-            if (cudaGetLastError() != cudaSuccess) {
-                rc = set_error(TAGI_ERR_CUDA, "mesh_classify launch failed");
-                break;
+        Progress *prog = nullptr, h_prog;
+        double *cells[2] = {}, *leaf_cells = nullptr;
+        uint64_t *keys[2] = {}, *leaf_keys = nullptr;
+        int *leaf_fine = nullptr;
+        if ((rc = tmp.alloc(&prog, 1))) break;
+        // Room for the usual counts; a mesh that needs more starts again with more.
+        long level_cap = std::max(32768L, 16L * numBase), leaf_cap = std::max(16384L, 16L * numBase);
+        long total = 0;
+        for (;;) {
+            char *block = nullptr;   // two levels and the leaves
+            const long cell = 6 * sizeof(double) + sizeof(uint64_t);
+            if ((rc = tmp.alloc(&block, 2 * level_cap * cell + leaf_cap * (cell + (long)sizeof(int))))) break;
+            char *at = block;
+            auto take = [&](auto *&ptr, long count) {
+                ptr = reinterpret_cast<std::remove_reference_t<decltype(ptr)>>(at);
+                at += count * sizeof(*ptr);
+            };
+            for (int k = 0; k < 2; k++) take(cells[k], 6 * level_cap);
+            take(leaf_cells, 6 * leaf_cap);
+            for (int k = 0; k < 2; k++) take(keys[k], level_cap);
+            take(leaf_keys, leaf_cap);
+            take(leaf_fine, leaf_cap);
+            launch(mesh_start, 1, 32, 0, s, prog, numBase);
+            // LEVELS levels are launched at a time: one more costs 2 us where it has no cells
+            constexpr int LEVELS = 6;
+            for (int depth = 0; !rc;) {
+                for (int k = 0; k < LEVELS && depth <= MESH_MAX_DEPTH && !rc; k++, depth++) {
+                    const int from = depth & 1, to = from ^ 1;
+                    // a level holds at most 8 times the cells of the one before
+                    const long most = std::min(level_cap, depth < 10 ? (long)numBase << (3 * depth) : level_cap);
+                    const int grid = (int)std::min(152L * 8, (most * CELL_LANES + LEVEL_THREADS - 1) / LEVEL_THREADS);
+                    if (launch_chained(mesh_level, grid, LEVEL_THREADS, 0, s, depth ? cells[from] : baseCells,
+                                       depth ? keys[from] : (const uint64_t *)nullptr, depth, atomXYZ, numAtoms, p, prog,
+                                       cells[to], keys[to], (int)level_cap, leaf_cells, leaf_keys, leaf_fine,
+                                       (int)leaf_cap) != cudaSuccess)
+                        rc = set_error(TAGI_ERR_CUDA, "mesh_level launch failed");
+                }
+                if (rc) break;
+                if (cudaMemcpyAsync(&h_prog, prog, sizeof(Progress), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+                    cudaStreamSynchronize(s) != cudaSuccess) {
+                    rc = set_error(TAGI_ERR_CUDA, "mesh refinement failed: %s", cudaGetErrorString(cudaGetLastError()));
+                    break;
+                }
+                if (h_prog.err & 2 || depth > MESH_MAX_DEPTH || h_prog.count[depth] == 0) break;
             }
-            if ((rc = exclusive_scan(divide, rank, (int)n, rank + n, tmp, s))) break;
-            int h_div = 0;
-            if ((rc = read_ints(rank + n, &h_div, 1, s))) break;
-            const long nleaf = n - h_div, nnext = 8L * h_div;
-            if (total + nleaf > MESH_MAX_CELLS || nnext > MESH_MAX_CELLS) {
+            if (rc || !(h_prog.err & 2)) break;
+            long most = 0;
+            for (int d = 1; d <= MESH_MAX_DEPTH + 1; d++) most = std::max(most, (long)h_prog.count[d]);
+            // blocks that start after the overflow count nothing more: the next try may need still more room
+            if (most > MESH_MAX_CELLS || h_prog.leaves > MESH_MAX_CELLS) {
                 rc = set_error(TAGI_ERR_ARG, "refinement exceeds %ld cells", MESH_MAX_CELLS);
                 break;
             }
-            Level L{nullptr, nullptr, nullptr, nleaf};
-            double *ncells = nullptr;
-            uint64_t *nkeys = nullptr;
-            if ((rc = tmp.alloc(&L.cells, 6 * nleaf)) || (rc = tmp.alloc(&L.keys, nleaf)) ||
-                (rc = tmp.alloc(&L.fine, nleaf)) || (rc = tmp.alloc(&ncells, 6 * nnext)) ||
-                (rc = tmp.alloc(&nkeys, nnext)))
-                break;
-            launch(mesh_emit, grid_for(n), MT, 0, s, cells, keys, (int)n, depth, divide, fine, rank, ncells,
-                   nkeys, L.cells, L.keys, L.fine);
-            if (cudaGetLastError() != cudaSuccess) {
-                rc = set_error(TAGI_ERR_CUDA, "mesh_emit launch failed");
-                break;
-            }
-            leaves.push_back(L);
-            total += nleaf;
-            cells = ncells;
-            keys = nkeys;
-            n = nnext;
+            if (most > level_cap) level_cap = std::min(MESH_MAX_CELLS, std::max(2 * most, 4 * level_cap));
+            else leaf_cap = std::min(MESH_MAX_CELLS, std::max(2L * h_prog.leaves, 4 * leaf_cap));
+            tmp.release();
+            if ((rc = tmp.alloc(&prog, 1))) break;
         }
         if (rc) break;
-        int h_err[2] = {0, 0};
-        if ((rc = read_ints(err, h_err, 2, s))) break;
-        if (h_err[0]) {
+        if (h_prog.err) {
             rc = set_error(TAGI_ERR_ARG, "the divide rule refines below maxDepth %d", maxDepth);
             break;
         }
+        total = h_prog.leaves;
         *numCells = (int)total;
         if (numCoarsePoints) *numCoarsePoints = (long long)total * p3;
-        // gather every level's leaves, then sort by path key (depth-first order)
-        double *all_cells = nullptr;
-        uint64_t *all_keys = nullptr;
-        int *all_fine = nullptr, *idx = nullptr, *fsum = nullptr;
-        if ((rc = tmp.alloc(&all_cells, 6 * total)) || (rc = tmp.alloc(&all_keys, total)) ||
-            (rc = tmp.alloc(&all_fine, total)) || (rc = tmp.alloc(&idx, total)) ||
-            (rc = tmp.alloc(&fsum, total + 1)))
-            break;
-        long at = 0;
-        for (const Level &L : leaves) {
-            if (L.n == 0) continue;
-            if (cudaMemcpyAsync(all_cells + 6 * at, L.cells, sizeof(double) * 6 * L.n, cudaMemcpyDeviceToDevice,
-                                s) != cudaSuccess ||
-                cudaMemcpyAsync(all_keys + at, L.keys, sizeof(uint64_t) * L.n, cudaMemcpyDeviceToDevice, s) !=
-                    cudaSuccess ||
-                cudaMemcpyAsync(all_fine + at, L.fine, sizeof(int) * L.n, cudaMemcpyDeviceToDevice, s) !=
-                    cudaSuccess) {
-                rc = set_error(TAGI_ERR_CUDA, "mesh leaf gather failed");
-                break;
-            }
-            at += L.n;
-        }
-        if (rc) break;
-        if ((rc = exclusive_scan(all_fine, fsum, (int)total, fsum + total, tmp, s))) break;
-        int h_fine = 0;
-        if ((rc = read_ints(fsum + total, &h_fine, 1, s))) break;
-        if (numFinePoints) *numFinePoints = (long long)h_fine * p3;
+        if (numFinePoints) *numFinePoints = (long long)h_prog.fine * p3;
         if (query) break;
         if (capacity < total) {
             rc = set_error(TAGI_ERR_ARG, "capacity %d < %ld cells (numCells holds the count)", capacity, total);
             break;
         }
+        int *idx = nullptr;
+        if ((rc = tmp.alloc(&idx, total))) break;
         launch(mesh_iota, grid_for(total), MT, 0, s, idx, (int)total);
         uint64_t *keys_out = nullptr;
         int *order_of = nullptr;
         if ((rc = tmp.alloc(&keys_out, total)) || (rc = tmp.alloc(&order_of, total)) ||
-            (rc = radix_sort_u64(all_keys, idx, keys_out, order_of, (int)total, 64, tmp, s)))
+            (rc = radix_sort_u64(leaf_keys, idx, keys_out, order_of, (int)total, 64, tmp, s)))
             break;
-        launch(mesh_cell_table, grid_for(total), MT, 0, s, order_of, (int)total, all_cells, all_fine, p3, cellX, cellY,
+        launch(mesh_cell_table, grid_for(total), MT, 0, s, order_of, (int)total, leaf_cells, leaf_fine, p3, cellX, cellY,
                cellZ, cellDX, cellDY, cellDZ, ptsPerCellCoarse, ptsPerCellFine);
         if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(s) != cudaSuccess)
             rc = set_error(TAGI_ERR_CUDA, "mesh cell table failed");
