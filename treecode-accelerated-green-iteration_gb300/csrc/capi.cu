@@ -222,7 +222,7 @@ int plan_create(Plan **out, int nt, const double *tx, const double *ty, const do
             launch(split_points, (nt + 255) / 256, 256, 0, s, p->tgt.x, p->tgt.y, p->tgt.z, nt, p->tgt_hi, p->tgt_lo);
         }
         if ((rc = build_lists(*p, s))) break;
-        if ((rc = build_weight_charges(*p, s))) break;
+        if (!one_shot && (rc = build_weight_charges(*p, s))) break;   // modified_charges makes a one-shot plan's
         phase_mark(PH_LISTS, false, s);
         if (one_shot) break;   // the convolution follows on the same stream
         cudaError_t e = cudaStreamSynchronize(s);

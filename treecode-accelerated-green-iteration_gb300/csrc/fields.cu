@@ -1997,6 +1997,7 @@ template <bool MIXED>
 __global__ void prep_sources(const double *__restrict__ sv, const int *__restrict__ perm,
                              const double *__restrict__ w, int ns, float *__restrict__ q32,
                              double *__restrict__ q64, double *__restrict__ f64) {
+    chain_begin();
     long j = (long)blockIdx.x * blockDim.x + threadIdx.x;
     int orb = blockIdx.y;
     if (j >= ns) return;
@@ -2013,13 +2014,18 @@ __global__ void prep_sources(const double *__restrict__ sv, const int *__restric
 
 template <bool MIXED>
 __global__ void prep_targets(const double *__restrict__ tv, const int *__restrict__ perm, int nt,
-                             float *__restrict__ f32, double *__restrict__ f64) {
+                             float *__restrict__ f32, double *__restrict__ f64, double *__restrict__ close_out,
+                             double *__restrict__ far_out) {
+    chain_begin();
     long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
     int orb = blockIdx.y;
     if (i >= nt) return;
     double f = tv[(long)orb * nt + perm[i]];
     if (MIXED) f32[(long)orb * nt + i] = (float)f;
     else f64[(long)orb * nt + i] = f;
+    // the far and close-range passes write only the batches they visit
+    close_out[(long)orb * nt + i] = 0.0;
+    far_out[(long)orb * nt + i] = 0.0;
 }
 
 // phi_i = near + far + f_i * SS factor, scattered back to caller order.  The
@@ -2467,12 +2473,20 @@ int launch_fields(const SysCall *calls, const Fields *f, int nsys, const Schedul
 // subtraction term then belong to one kernel parameter, k' = k (1 + O(2^-24)),
 // and the rounding of k moves the result by about twice that, smoothly,
 // instead of entering the cancellation of the subtraction.
-__global__ void orbital_constants(const double *__restrict__ kp, int nkp, int norb, int kernel, int sing,
-                                  int mixed, double *__restrict__ kpo, float *__restrict__ kc,
-                                  double *__restrict__ ss, int *__restrict__ err) {
+// Kernel parameters given on the host ride along as arguments (a copy of eight bytes from
+// pageable memory takes 15 us), up to HOST_KP orbitals of them.
+constexpr int HOST_KP = 64;
+struct HostParams {
+    double k[HOST_KP];
+};
+__global__ void orbital_constants(const double *__restrict__ kp, int nkp, const __grid_constant__ HostParams h, int norb,
+                                  int kernel, int sing, int mixed, double *__restrict__ kpo, float *__restrict__ kc,
+                                  double *__restrict__ ss, int *__restrict__ err, int *__restrict__ queue) {
+    chain_begin();
     const int o = blockIdx.x * blockDim.x + threadIdx.x;
+    if (queue && o < 3) queue[o] = 0;   // the field passes' work counters
     if (o >= norb) return;
-    const double k = kp[(long)o * nkp];
+    const double k = kp ? kp[(long)o * nkp] : h.k[o];
     const bool used = kernel == KERNEL_YUKAWA || sing == SING_SUBTRACTION;
     const bool bad = !isfinite(k) || (used && !(k > 0.0));
     if (bad) atomicOr(err, 1);
@@ -2565,7 +2579,7 @@ int ensure_scratch(Plan &p, int norb, int precision) {
         take(&p.q64, no * ns, fp64);
         take(&p.f64s, no * ns, fp64);
         take(&p.ft64, no * nt, fp64);
-        take(&p.part, no * p.nitems * p.P);
+        take(&p.part, (no + (p.one_shot ? 1 : 0)) * p.nitems * p.P);
         take(&p.qhat32, no * p.nslots * p.P, mixed);
         take(&p.qhat64, no * p.nslots * p.P, fp64);
         take(&p.exp_table, EXP_N, fp64);
@@ -2744,19 +2758,22 @@ int build_schedule(Plan *const *plans, const int *norb, int nsys, int og, int nt
 }
 
 // Per-orbital constants of one system into p.d_kp / d_kc / d_ss.
-static int orbital_setup(Plan &p, const SysCall &c, int kernel, int singularity, int mixed, cudaStream_t s) {
+static int orbital_setup(Plan &p, const SysCall &c, int kernel, int singularity, int mixed, int *queue, cudaStream_t s) {
     const double *src = c.kp;
     int stride = c.nkp;
-    if (!c.kp_device) {
+    HostParams h{};
+    if (!c.kp_device && c.norb <= HOST_KP) {
+        for (int o = 0; o < c.norb; o++) h.k[o] = c.kp[(long)o * c.nkp];
+        src = nullptr;
+    } else if (!c.kp_device) {
         p.h_kp.resize(c.norb);
         for (int o = 0; o < c.norb; o++) p.h_kp[o] = c.kp[(long)o * c.nkp];
         TAGI_CUDA(cudaMemcpyAsync(p.d_kp, p.h_kp.data(), sizeof(double) * c.norb, cudaMemcpyHostToDevice, s));
         src = p.d_kp;
         stride = 1;
     }
-    launch(orbital_constants, (c.norb + 127) / 128, 128, 0, s, src, stride, c.norb, kernel, singularity, mixed,
-           p.d_kp, p.d_kc, p.d_ss, p.err_flag + 1);
-    TAGI_LAUNCH_CHECK();
+    TAGI_CUDA(launch_chained(orbital_constants, (c.norb + 127) / 128, 128, 0, s, src, stride, h, c.norb, kernel,
+                             singularity, mixed, p.d_kp, p.d_kc, p.d_ss, p.err_flag + 1, queue));
     return TAGI_OK;
 }
 
@@ -2787,31 +2804,27 @@ int convolve_systems(SysCall *calls, int nsys, int kernel, int singularity, int 
                                  "precision, and kernel parameters on the device");
         }
         TAGI_TRY(ensure_scratch(p, c.norb, precision));
-        TAGI_TRY(orbital_setup(p, c, kernel, singularity, mixed ? 1 : 0, s));
+        TAGI_TRY(orbital_setup(p, c, kernel, singularity, mixed ? 1 : 0, i == 0 ? queue : nullptr, s));
         const int ns = p.src.n, nt = p.tgt.n;
         dim3 gs((ns + 255) / 256, c.norb), gt((nt + 255) / 256, c.norb);
         phase_mark(PH_GLUE, true, s);
-        launch(mixed ? prep_sources<true> : prep_sources<false>, gs, 256, 0, s, c.sv, p.src.perm, p.sw64, ns, p.q32,
-               p.q64, p.f64s);
-        launch(mixed ? prep_targets<true> : prep_targets<false>, gt, 256, 0, s, c.tv, p.tgt.perm, nt, p.ft32, p.ft64);
+        TAGI_CUDA(launch_chained(mixed ? prep_sources<true> : prep_sources<false>, gs, 256, 0, s, c.sv, p.src.perm,
+                                 p.sw64, ns, p.q32, p.q64, p.f64s));
+        TAGI_CUDA(launch_chained(mixed ? prep_targets<true> : prep_targets<false>, gt, 256, 0, s, c.tv, p.tgt.perm, nt,
+                                 p.ft32, p.ft64, p.near2_out, p.far_out));
         phase_mark(PH_GLUE, false, s);
-        TAGI_LAUNCH_CHECK();
         phase_mark(PH_UPWARD, true, s);
         TAGI_TRY(modified_charges(p, mixed ? PREC_MIXED : PREC_FP64, c.norb, s));
-        if (!mixed) TAGI_TRY(ensure_weight_charges64(p, s));  // before what64 is read below
+        if (!mixed && !p.one_shot) TAGI_TRY(ensure_weight_charges64(p, s));  // before what64 is read below
         phase_mark(PH_UPWARD, false, s);
         if (!mixed && p.nslots && !p.what64) return set_error(TAGI_ERR_DEVICE, "FP64 weight charges missing");
         f[i] = make_fields(p, c.norb);
         plans[i] = c.p;
         if (p.n1 > sh.maxn1) sh.maxn1 = p.n1;
         if (p.n1 < sh.minn1) sh.minn1 = p.n1;
-        // the far and close-range passes write only the batches they visit
-        TAGI_CUDA(cudaMemsetAsync(p.far_out, 0, sizeof(double) * (size_t)c.norb * nt, s));
-        TAGI_CUDA(cudaMemsetAsync(p.near2_out, 0, sizeof(double) * (size_t)c.norb * nt, s));
     }
     sh.warps = field_warps(plans, nsys, precision);
     for (int i = 0; i < nsys; i++) f[i].split = field_split(plans[i]->tgt.n, sh.warps, precision);
-    TAGI_CUDA(cudaMemsetAsync(queue, 0, 3 * sizeof(int), s));
     if (kernel == KERNEL_YUKAWA) {
         if (ss) TAGI_TRY((launch_fields<KERNEL_YUKAWA, true>(calls, f, nsys, sc, sh, precision, queue, s)));
         else TAGI_TRY((launch_fields<KERNEL_YUKAWA, false>(calls, f, nsys, sc, sh, precision, queue, s)));

@@ -252,9 +252,9 @@ int rs_pass(const uint64_t *kin, const int *vin, uint64_t *kout, int *vout, int 
 constexpr int SORT_SMALL = 16384, CNT_THREADS = 256;
 __global__ void __launch_bounds__(CNT_THREADS) count_smaller(const uint64_t *__restrict__ keys,
                                                              int n, int span, int *__restrict__ rank) {
-    __shared__ uint64_t s_key[CNT_THREADS];
+    __shared__ __align__(16) uint64_t s_key[CNT_THREADS];
     chain_begin();
-    const int i = blockIdx.x * CNT_THREADS + threadIdx.x;
+    const int i0 = blockIdx.x * CNT_THREADS, i = i0 + threadIdx.x;
     const uint64_t k = i < n ? keys[i] : 0;
     const int j0 = blockIdx.y * span, j1 = min(j0 + span, n);
     int c = 0;
@@ -263,10 +263,20 @@ __global__ void __launch_bounds__(CNT_THREADS) count_smaller(const uint64_t *__r
         __syncthreads();
         if (threadIdx.x < m) s_key[threadIdx.x] = keys[t + threadIdx.x];
         __syncthreads();
+        // equal keys count where they lie before this one: all or none of a tile that lies
+        // before or after the block's keys, which leaves one comparison
+        if (t + m <= i0) {
 #pragma unroll 8
-        for (int j = 0; j < m; j++) {
-            const uint64_t q = s_key[j];
-            c += q < k || (q == k && t + j < i);
+            for (int j = 0; j < m; j++) c += s_key[j] <= k;
+        } else if (t >= i0 + CNT_THREADS) {
+#pragma unroll 8
+            for (int j = 0; j < m; j++) c += s_key[j] < k;
+        } else {
+#pragma unroll 4
+            for (int j = 0; j < m; j++) {
+                const uint64_t q = s_key[j];
+                c += q < k || (q == k && t + j < i);
+            }
         }
     }
     if (i < n && c) atomicAdd(rank + i, c);

@@ -35,10 +35,16 @@ struct P2MArgs {
     const double *xs, *ys, *zs;  // sorted sources
     const T *q;                  // [norb][ns] sorted charges
     long q_stride;
+    const T *w;                  // the last vector, if it lies elsewhere (weights)
     double *part;                // [norb][nitems][P]
     int n1, P, norb;
     T tn[MAX_DEGREE + 1];
 };
+
+template <typename T>
+__device__ __forceinline__ const T *charges(const P2MArgs<T> &a, int orb) {
+    return a.w && orb == a.norb - 1 ? a.w : a.q + (long)orb * a.q_stride;
+}
 
 template <typename T>
 __device__ __forceinline__ T bary_weight(int m, int n1) {
@@ -100,6 +106,7 @@ __global__ void __launch_bounds__(P2M_THREADS) p2m_mixed(const __grid_constant__
     const int g = tid / pairs, pr = tid % pairs;
     const int k1 = pr / n1, k2 = pr % n1;
     const bool active = g < G;
+    chain_begin();
     const int b = a.item_begin[item], e = a.item_end[item];
     const double *gm = a.geom + 6L * a.item_slot[item];
     const int axis = tid % 3;   // thread 3 p + d does source p along axis d
@@ -120,7 +127,7 @@ __global__ void __launch_bounds__(P2M_THREADS) p2m_mixed(const __grid_constant__
         }
         for (int k = tid; k < OB * P2M_TILE; k += P2M_THREADS) {
             const int o = k / P2M_TILE, p = k % P2M_TILE;
-            if (o < no && p < cnt) sq[o][p] = a.q[(long)(orb0 + o) * a.q_stride + t0 + p];
+            if (o < no && p < cnt) sq[o][p] = charges(a, orb0 + o)[t0 + p];
         }
         __syncthreads();
         if (!active) continue;
@@ -177,10 +184,11 @@ __global__ void __launch_bounds__(P2M_THREADS) p2m_f64(const __grid_constant__ P
     const int g = tid / pairs, pr = tid % pairs;
     const int k1 = pr / n1, k2 = pr % n1;
     const bool active = g < G;
+    chain_begin();
     const int slot = a.item_slot[item];
     const int b = a.item_begin[item], e = a.item_end[item];
     const double *gm = a.geom + 6L * slot;
-    const double *q = a.q + (long)orb * a.q_stride;
+    const double *q = charges(a, orb);
 
     double acc[MAXN1];
 #pragma unroll
@@ -221,20 +229,22 @@ __global__ void __launch_bounds__(P2M_THREADS) p2m_f64(const __grid_constant__ P
 
 template <typename TO>
 __global__ void p2m_reduce(const double *__restrict__ part, const int *__restrict__ slot_item_off,
-                           int nslots, int nitems, int P, TO *__restrict__ out) {
+                           int nslots, int nitems, int P, TO *__restrict__ out, TO *__restrict__ wout) {
     const int slot = blockIdx.x, orb = blockIdx.y;
+    chain_begin();
     const int i0 = slot_item_off[slot], i1 = slot_item_off[slot + 1];
     const double *pp = part + (long)orb * nitems * P;
-    TO *o = out + ((long)orb * nslots + slot) * P;
+    TO *o = wout && orb == (int)gridDim.y - 1 ? wout + (long)slot * P : out + ((long)orb * nslots + slot) * P;
     for (int k = threadIdx.x; k < P; k += blockDim.x) {
         double s = 0.0;
+#pragma unroll 8
         for (int it = i0; it < i1; it++) s += pp[(long)it * P + k];
         o[k] = (TO)s;
     }
 }
 
 template <typename T>
-int launch_p2m(Plan &p, const T *q, long q_stride, int norb, double *part, cudaStream_t s) {
+int launch_p2m(Plan &p, const T *q, long q_stride, int norb, double *part, cudaStream_t s, const T *w = nullptr) {
     P2MArgs<T> a;
     a.item_slot = p.item_slot;
     a.item_begin = p.item_begin;
@@ -246,6 +256,7 @@ int launch_p2m(Plan &p, const T *q, long q_stride, int norb, double *part, cudaS
     a.zs = p.src.z;
     a.q = q;
     a.q_stride = q_stride;
+    a.w = w;
     a.part = part;
     a.n1 = p.n1;
     a.P = p.P;
@@ -255,20 +266,27 @@ int launch_p2m(Plan &p, const T *q, long q_stride, int norb, double *part, cudaS
     a.norb = norb;
     auto go = [&](auto kern, int ob) {
         if (smem > 32 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        launch(kern, dim3(p.nitems, (norb + ob - 1) / ob), P2M_THREADS, smem, s, a);
+        return launch_chained(kern, dim3(p.nitems, (norb + ob - 1) / ob), P2M_THREADS, smem, s, a);
     };
+    cudaError_t e;
     if constexpr (sizeof(T) == 8) {
-        if (p.n1 <= 8) go(p2m_f64<8>, 1);
-        else go(p2m_f64<MAX_DEGREE + 1>, 1);
+        if (p.n1 <= 8) e = go(p2m_f64<8>, 1);
+        else e = go(p2m_f64<MAX_DEGREE + 1>, 1);
     } else if (p.n1 <= 8) {
-        if (norb == 1) go(p2m_mixed<8, 1>, 1);
-        else go(p2m_mixed<8, P2M_OB>, P2M_OB);
+        if (norb == 1) e = go(p2m_mixed<8, 1>, 1);
+        else e = go(p2m_mixed<8, P2M_OB>, P2M_OB);
     } else {   // 11 sums of three words per orbital: two orbitals fill the registers
-        if (norb == 1) go(p2m_mixed<MAX_DEGREE + 1, 1>, 1);
-        else go(p2m_mixed<MAX_DEGREE + 1, 2>, 2);
+        if (norb == 1) e = go(p2m_mixed<MAX_DEGREE + 1, 1>, 1);
+        else e = go(p2m_mixed<MAX_DEGREE + 1, 2>, 2);
     }
-    TAGI_LAUNCH_CHECK();
+    TAGI_CUDA(e);
     return TAGI_OK;
+}
+
+template <typename TO>
+cudaError_t launch_reduce(const Plan &p, int rows, const double *part, TO *out, TO *wout, cudaStream_t s) {
+    return launch_chained(p2m_reduce<TO>, dim3(p.nslots, rows), 256, 0, s, part, p.slot_item_off, p.nslots, p.nitems, p.P,
+                          out, wout);
 }
 
 }  // namespace
@@ -286,9 +304,7 @@ int build_weight_charges(Plan &p, cudaStream_t s) {
     int rc = tmp.alloc(&part, (size_t)p.nitems * p.P);
     if (!rc) rc = launch_p2m<float>(p, p.sw32, p.src.n, 1, part, s);
     if (!rc) {
-        launch(p2m_reduce<float>, dim3(p.nslots, 1), 256, 0, s, part, p.slot_item_off, p.nslots, p.nitems, p.P,
-               p.what32);
-        if (cudaGetLastError() != cudaSuccess) rc = set_error(TAGI_ERR_CUDA, "weight charge kernels");
+        if (launch_reduce<float>(p, 1, part, p.what32, nullptr, s) != cudaSuccess) rc = set_error(TAGI_ERR_CUDA, "weight charge kernels");
     }
     tmp.release();
     return rc;
@@ -298,15 +314,11 @@ int ensure_weight_charges64(Plan &p, cudaStream_t s) {
     if (p.what64_ready) return TAGI_OK;
     if (!p.what64) {
         const size_t count = (size_t)p.nslots * p.P + 1;
-        if (p.one_shot) {
-            TAGI_TRY(p.arena.alloc(&p.what64, count));
-        } else {
-            // plain cudaMalloc: the first FP64 call may run on another stream than the plan's
-            void *v = nullptr;
-            TAGI_CUDA(cudaMalloc(&v, sizeof(double) * count));
-            p.arena.ptrs.push_back(v);
-            p.what64 = static_cast<double *>(v);
-        }
+        // plain cudaMalloc: the first FP64 call may run on another stream than the plan's
+        void *v = nullptr;
+        TAGI_CUDA(cudaMalloc(&v, sizeof(double) * count));
+        p.arena.ptrs.push_back(v);
+        p.what64 = static_cast<double *>(v);
     }
     if (p.nslots) {
         Arena tmp;
@@ -315,9 +327,7 @@ int ensure_weight_charges64(Plan &p, cudaStream_t s) {
         int rc = tmp.alloc(&part, (size_t)p.nitems * p.P);
         if (!rc) rc = launch_p2m<double>(p, p.sw64, p.src.n, 1, part, s);
         if (!rc) {
-            launch(p2m_reduce<double>, dim3(p.nslots, 1), 256, 0, s, part, p.slot_item_off, p.nslots, p.nitems,
-                   p.P, p.what64);
-            if (cudaGetLastError() != cudaSuccess) rc = set_error(TAGI_ERR_CUDA, "weight charge kernels");
+            if (launch_reduce<double>(p, 1, part, p.what64, nullptr, s) != cudaSuccess) rc = set_error(TAGI_ERR_CUDA, "weight charge kernels");
         }
         tmp.release();
         if (rc) return rc;
@@ -326,19 +336,24 @@ int ensure_weight_charges64(Plan &p, cudaStream_t s) {
     return TAGI_OK;
 }
 
-// Charges for norb sorted charge vectors already in p.q32 / p.q64.
+// Charges for norb sorted charge vectors already in p.q32 / p.q64.  A one-shot plan has
+// no weight charges yet: they ride along as one more vector (two launches and a chain of
+// 23 us less at 6,000 points).
+template <typename T>
+static int charges_with_weights(Plan &p, const T *q, const T *w, int norb, T *qhat, T **what, cudaStream_t s) {
+    if (p.one_shot && !*what) TAGI_TRY(p.arena.alloc(what, (size_t)p.nslots * p.P));
+    T *const wout = p.one_shot ? *what : nullptr;
+    const int rows = norb + (wout ? 1 : 0);
+    TAGI_TRY(launch_p2m<T>(p, q, p.src.n, rows, p.part, s, wout ? w : nullptr));
+    TAGI_CUDA(launch_reduce<T>(p, rows, p.part, qhat, wout, s));
+    return TAGI_OK;
+}
+
 int modified_charges(Plan &p, int precision, int norb, cudaStream_t s) {
     if (p.nslots == 0) return TAGI_OK;
-    if (precision == PREC_MIXED) {
-        TAGI_TRY(launch_p2m<float>(p, p.q32, p.src.n, norb, p.part, s));
-        launch(p2m_reduce<float>, dim3(p.nslots, norb), 256, 0, s, p.part, p.slot_item_off, p.nslots,
-                                                               p.nitems, p.P, p.qhat32);
-    } else {
-        TAGI_TRY(launch_p2m<double>(p, p.q64, p.src.n, norb, p.part, s));
-        launch(p2m_reduce<double>, dim3(p.nslots, norb), 256, 0, s, p.part, p.slot_item_off, p.nslots,
-                                                                p.nitems, p.P, p.qhat64);
-    }
-    TAGI_LAUNCH_CHECK();
+    if (precision == PREC_MIXED) return charges_with_weights<float>(p, p.q32, p.sw32, norb, p.qhat32, &p.what32, s);
+    TAGI_TRY(charges_with_weights<double>(p, p.q64, p.sw64, norb, p.qhat64, &p.what64, s));
+    if (p.one_shot) p.what64_ready = true;
     return TAGI_OK;
 }
 
