@@ -138,7 +138,7 @@ namespace {
 // first, so no scan runs between the two kernels: at 1.5M keys a block reads 27 rows
 // of 512 counts.  Nine-bit digits: 63-bit Morton codes take seven passes; 512 counters for
 // each of eight warps are 16 KB of shared memory.  Digits of eight bits with a scan
-// between took 24 launches (40 above 130,000 keys): @@
+// between took 24 launches (40 above 130,000 keys).  44,000 keys: 60 us.
 constexpr int RS_THREADS = 256, RS_WARPS = RS_THREADS / 32, RS_BITS = 9, RS_DIGITS = 1 << RS_BITS;
 
 // counts[tile][digit], and their sums over groups of `group` tiles (zeroed before)
@@ -245,9 +245,9 @@ int rs_pass(const uint64_t *kin, const int *vin, uint64_t *kout, int *vout, int 
 }
 
 // Up to SORT_SMALL pairs by counting: an element's place is the number of smaller
-// keys plus the equal keys before it.  n^2 comparisons over the whole chip take
-// 3 us at 6,000 keys and 25 at 16,384, the radix passes @@; a bitonic network in one
-// block took 124 at 6,000.  Counts are whole numbers:
+// keys plus the equal keys before it.  n^2 comparisons over the whole chip: 16 us at
+// 6,022 keys, 47 at 15,336 (the radix passes 60 at 44,000; at 16,384 they are even); a
+// bitonic network in one block took 124 at 6,022.  Counts are whole numbers:
 // the order of the atomic additions does not matter.
 constexpr int SORT_SMALL = 16384, CNT_THREADS = 256;
 __global__ void __launch_bounds__(CNT_THREADS) count_smaller(const uint64_t *__restrict__ keys,

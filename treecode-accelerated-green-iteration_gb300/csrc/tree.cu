@@ -236,7 +236,7 @@ constexpr int HDR = MAX_LEVELS + 3;
 // nothing waits for the host between levels.  A level of up to 32 nodes gives four
 // threads to a digit, which cut its range in five at a time (a chain of 7 loads
 // instead of 16 at 44,000 points), a wider one a thread: binary search, 128 nodes a
-// round.  44,000 points, leaves of 1834: 33 -> @@ us.  Meshes have a few
+// round.  44,000 points, leaves of 1834: 33 -> 25 us.  Meshes have a few
 // thousand nodes: 1.5M points, leaves of 2000: 8 levels, count + fill + scan
 // launches and a synchronisation each, 1.35 -> 0.78 ms for the tree and its sort.  Above
 // SMALL_TREE leaves' worth of points one launch per level is quicker.
@@ -335,7 +335,7 @@ __global__ void write_header(int *hdr, int nnodes) { hdr[0] = nnodes; }
 // block does a leaf, and the first warp of the one that finishes a node's last child
 // goes on with the node.  The chain of the climb holds only what the parent needs;
 // centers and radii (FP64) follow in preorder.  44,000 points, leaves of 1834, a warp
-// per leaf and all of a node's values in the climb before: 48 -> @@ us.
+// per leaf and all of a node's values in the climb before: 48 -> 15 us.
 constexpr int BOX_THREADS = 128;
 __global__ void __launch_bounds__(BOX_THREADS) node_boxes(const int *__restrict__ hdr, const int *__restrict__ begin,
                                                           const int *__restrict__ end, const int *__restrict__ parent,
