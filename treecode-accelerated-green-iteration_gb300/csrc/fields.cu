@@ -38,6 +38,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <functional>
 #include <type_traits>
 
 namespace tagi {
@@ -2783,8 +2784,10 @@ static int orbital_setup(Plan &p, const SysCall &c, int kernel, int singularity,
 // epilogues.  Under stream capture nothing may allocate or copy from host
 // memory: scratch, schedule and FP64 weight charges must exist already, and
 // kernel parameters must be on the device.
-int convolve_systems(SysCall *calls, int nsys, int kernel, int singularity, int precision, const Schedule &sc,
-                     int *queue, cudaStream_t s) {
+// later: makes the schedule while the set-up kernels and the upward pass run, where the
+// caller has none yet.
+static int convolve_with(SysCall *calls, int nsys, int kernel, int singularity, int precision, const Schedule *ready,
+                         const std::function<int(const Schedule **)> &later, int *queue, cudaStream_t s) {
     if (nsys < 1 || nsys > MAX_SYSTEMS) return set_error(TAGI_ERR_ARG, "%d systems (1..%d per launch)", nsys, MAX_SYSTEMS);
     const bool mixed = precision == PREC_MIXED;
     const bool ss = singularity == SING_SUBTRACTION;
@@ -2792,8 +2795,6 @@ int convolve_systems(SysCall *calls, int nsys, int kernel, int singularity, int 
     Fields f[MAX_SYSTEMS];
     Plan *plans[MAX_SYSTEMS];
     LaunchShape sh;
-    sh.og = sc.og;
-    sh.nt = sc.nt;
     for (int i = 0; i < nsys; i++) {
         SysCall &c = calls[i];
         Plan &p = *c.p;
@@ -2823,6 +2824,10 @@ int convolve_systems(SysCall *calls, int nsys, int kernel, int singularity, int 
         if (p.n1 > sh.maxn1) sh.maxn1 = p.n1;
         if (p.n1 < sh.minn1) sh.minn1 = p.n1;
     }
+    if (!ready) TAGI_TRY(later(&ready));
+    const Schedule &sc = *ready;
+    sh.og = sc.og;
+    sh.nt = sc.nt;
     sh.warps = field_warps(plans, nsys, precision);
     for (int i = 0; i < nsys; i++) f[i].split = field_split(plans[i]->tgt.n, sh.warps, precision);
     if (kernel == KERNEL_YUKAWA) {
@@ -2850,6 +2855,11 @@ int convolve_systems(SysCall *calls, int nsys, int kernel, int singularity, int 
     return TAGI_OK;
 }
 
+int convolve_systems(SysCall *calls, int nsys, int kernel, int singularity, int precision, const Schedule &sc, int *queue,
+                     cudaStream_t s) {
+    return convolve_with(calls, nsys, kernel, singularity, precision, &sc, nullptr, queue, s);
+}
+
 // Single-plan call (norb orbitals over one mesh) with the plan's cached
 // work list.
 int convolve(Plan &p, const double *tv, const double *sv, double *out, int norb, int kernel,
@@ -2861,9 +2871,10 @@ int convolve(Plan &p, const double *tv, const double *sv, double *out, int norb,
     const Schedule *sc = nullptr;
     for (const Schedule &c : p.scheds)
         if (schedule_matches(c, &norb, 1, og, nt, precision)) sc = &c;
-    if (!sc) {
-        if (stream_capturing(s))
-            return set_error(TAGI_ERR_STATE, "graph capture needs a prior uncaptured call with the same orbital count");
+    if (!sc && stream_capturing(s))
+        return set_error(TAGI_ERR_STATE, "graph capture needs a prior uncaptured call with the same orbital count");
+    if (norb < 1 || norb > 0xffff) return set_error(TAGI_ERR_ARG, "system 0: %d orbitals", norb);
+    auto make_schedule = [&](const Schedule **out) -> int {
         constexpr size_t KEEP = 4;  // work lists kept per plan (e.g. Hartree + orbital batch)
         if (p.scheds.size() >= KEEP) {
             TAGI_CUDA(cudaDeviceSynchronize());
@@ -2877,8 +2888,9 @@ int convolve(Plan &p, const double *tv, const double *sv, double *out, int norb,
             p.scheds.pop_back();
             return rc;
         }
-        sc = &p.scheds.back();
-    }
+        *out = &p.scheds.back();
+        return TAGI_OK;
+    };
     SysCall c;
     c.p = &p;
     c.tv = tv;
@@ -2888,7 +2900,7 @@ int convolve(Plan &p, const double *tv, const double *sv, double *out, int norb,
     c.kp = kparams;
     c.nkp = nkp;
     c.kp_device = kp_device;
-    return convolve_systems(&c, 1, kernel, singularity, precision, *sc, p.queue, s);
+    return convolve_with(&c, 1, kernel, singularity, precision, sc, make_schedule, p.queue, s);
 }
 
 int pair_peak(int kernel, int singularity, int variant, double kp, double *pairs_per_s, cudaStream_t s) {

@@ -26,6 +26,8 @@
 #include <cuda.h>
 #include <cuda_bf16.h>
 
+#include <algorithm>
+
 namespace tagi {
 
 namespace {
@@ -66,12 +68,16 @@ __device__ __forceinline__ unsigned pack2(__nv_bfloat16 lo, __nv_bfloat16 hi) {
 // staging: 10,752 rows of 512-point patches 872 -> 78 us, 6,090 rows of 125 points
 // 480 -> 114 us (219 with mma.sync in the two products that TMA cannot read).
 // ---------------------------------------------------------------------------
-constexpr int TC_M = 128, TC_N = 128, TC_K = 64, TC_STAGES = 3, TC_THREADS = 128, TC_LOADERS = 256;
+constexpr int TC_M = 128, TC_N = 128, TC_K = 64, TC_THREADS = 128, TC_LOADERS = 256;
+// Stages of the ring: 3 (two CTAs per SM), or 6 where the grid leaves an SM to each CTA and
+// TMA feeds both operands: a K loop runs at the stages in flight over a load's latency.  Six
+// calls at 10,752 rows, 78.5 -> 75.8 us; tiles that warps load gained nothing (343 points).
 constexpr int TC_TILE = 128 * TC_K * 2;                 // bytes of one operand's tile
 constexpr int TC_PITCH = TC_N + 4;                      // floats per staged row of C
-constexpr size_t TC_SMEM = 1024 + (size_t)TC_STAGES * 2 * TC_TILE;
-static_assert(TC_SMEM * 5 > 228 * 1024, "at most four blocks of 128 TMEM columns each may share an SM");
-static_assert((size_t)TC_M * TC_PITCH * 4 <= (size_t)TC_STAGES * 2 * TC_TILE, "C tile in the ring's memory");
+__host__ __device__ constexpr size_t tc_smem(int stages) { return 1024 + (size_t)stages * 2 * TC_TILE; }
+static_assert(tc_smem(3) * 5 > 228 * 1024, "at most four blocks of 128 TMEM columns each may share an SM");
+static_assert((size_t)TC_M * TC_PITCH * 4 <= (size_t)3 * 2 * TC_TILE, "C tile in the ring's memory");
+static_assert(tc_smem(6) <= 227 * 1024, "one block's shared memory");
 constexpr int TC_SPINS = 1 << 20;                       // tries of a barrier wait before it gives up
 
 __device__ __forceinline__ unsigned smem_u32(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
@@ -143,12 +149,12 @@ __device__ __forceinline__ void store_rows(const unsigned (&v)[ROWS], char *tile
     }
 }
 
-template <bool SA, bool SB>
-__global__ void __launch_bounds__(TC_THREADS + (SA || SB ? TC_LOADERS : 0), 2) gemm_tc(
+template <bool SA, bool SB, int STAGES>
+__global__ void __launch_bounds__(TC_THREADS + (SA || SB ? TC_LOADERS : 0), STAGES == 3 ? 2 : 1) gemm_tc(
     const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB, const __grid_constant__ TcArgs t) {
     constexpr int WARPS = (TC_THREADS + (SA || SB ? TC_LOADERS : 0)) / 32, LW = TC_LOADERS / 32, ROWS = 128 / LW;
     extern __shared__ char s_raw[];
-    __shared__ __align__(8) uint64_t s_full[TC_STAGES], s_empty[TC_STAGES], s_done;
+    __shared__ __align__(8) uint64_t s_full[STAGES], s_empty[STAGES], s_done;
     __shared__ unsigned s_tmem;
     __shared__ int s_fail;
     // Early: this grid is resident as a whole by then, and the next kernel's blocks wait
@@ -167,7 +173,7 @@ __global__ void __launch_bounds__(TC_THREADS + (SA || SB ? TC_LOADERS : 0), 2) g
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
     if (tid == 0) {
-        for (int i = 0; i < TC_STAGES; i++) {
+        for (int i = 0; i < STAGES; i++) {
             mbar_init(&s_full[i], (SA && SB ? 0 : 1) + (SA || SB ? LW : 0));
             mbar_init(&s_empty[i], 1);
         }
@@ -182,9 +188,9 @@ __global__ void __launch_bounds__(TC_THREADS + (SA || SB ? TC_LOADERS : 0), 2) g
     asm volatile("griddepcontrol.wait;" ::: "memory");
     if ((!SA || !SB) && tid == 0) {   // copies
         for (int i = 0; i < steps; i++) {
-            const int st = i % TC_STAGES;
+            const int st = i % STAGES;
             char *a = ring + st * 2 * TC_TILE, *b = a + TC_TILE;
-            if (i >= TC_STAGES && !mbar_wait(&s_empty[st], (i / TC_STAGES - 1) & 1)) {
+            if (i >= STAGES && !mbar_wait(&s_empty[st], (i / STAGES - 1) & 1)) {
                 s_fail = 1;
                 break;
             }
@@ -211,8 +217,8 @@ __global__ void __launch_bounds__(TC_THREADS + (SA || SB ? TC_LOADERS : 0), 2) g
                                (t.b_kmajor ? 0u : 1u << 16) | (unsigned)(TC_N / 8) << 17 | (unsigned)(TC_M / 16) << 24;
         const unsigned stepA = t.a_kmajor ? 32 >> 4 : 2048 >> 4, stepB = t.b_kmajor ? 32 >> 4 : 2048 >> 4;
         for (int i = 0; i < steps; i++) {
-            const int st = i % TC_STAGES;
-            if (!mbar_wait(&s_full[st], (i / TC_STAGES) & 1)) {
+            const int st = i % STAGES;
+            if (!mbar_wait(&s_full[st], (i / STAGES) & 1)) {
                 s_fail = 1;
                 break;
             }
@@ -240,12 +246,12 @@ __global__ void __launch_bounds__(TC_THREADS + (SA || SB ? TC_LOADERS : 0), 2) g
     } else if ((SA || SB) && warp >= TC_THREADS / 32) {   // loads by warps
         const int w = warp - TC_THREADS / 32;
         for (int i = 0; i < steps; i++) {
-            const int st = i % TC_STAGES, k = kb + i * TC_K;
+            const int st = i % STAGES, k = kb + i * TC_K;
             char *a = ring + st * 2 * TC_TILE;
             unsigned va[SA ? ROWS : 1], vb[SB ? ROWS : 1];
             if (SA) load_rows(va, g.A, g.sAm, g.sAk, t.a_kmajor, m0, g.M, k, g.K, w, LW, lane);
             if (SB) load_rows(vb, g.B, g.sBn, g.sBk, t.b_kmajor, n0, g.N, k, g.K, w, LW, lane);
-            const bool ready = i < TC_STAGES || mbar_wait(&s_empty[st], (i / TC_STAGES - 1) & 1);
+            const bool ready = i < STAGES || mbar_wait(&s_empty[st], (i / STAGES - 1) & 1);
             if (!__all_sync(0xffffffffu, ready)) {
                 s_fail = 1;
                 break;
@@ -266,7 +272,7 @@ __global__ void __launch_bounds__(TC_THREADS + (SA || SB ? TC_LOADERS : 0), 2) g
     if (!ok) {   // give the copies in flight time to land before the memory is reused or left
         if (tid == 0) {
             g_tc_timeout = 1;
-            for (int st = 0; st < TC_STAGES; st++) mbar_wait(&s_full[st], 0), mbar_wait(&s_full[st], 1);
+            for (int st = 0; st < STAGES; st++) mbar_wait(&s_full[st], 0), mbar_wait(&s_full[st], 1);
         }
         __syncthreads();
     }
@@ -436,11 +442,16 @@ int run_gemm(GemmArgs g, int splits, int *used, cudaStream_t s) {
     g.k_per_split = kps;
     *used = (g.K + kps - 1) / kps;
     t.g = g;
-    const auto kern = sa ? (sb ? gemm_tc<true, true> : gemm_tc<true, false>)
-                         : (sb ? gemm_tc<false, true> : gemm_tc<false, false>);
-    TAGI_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM));
     const dim3 grid((g.N + TC_N - 1) / TC_N, (g.M + TC_M - 1) / TC_M, *used);
-    TAGI_CUDA(launch_chained(kern, grid, TC_THREADS + (sa || sb ? TC_LOADERS : 0), TC_SMEM, s, ma, mb, t));
+    int dev = 0, sms = 0;
+    TAGI_CUDA(cudaGetDevice(&dev));
+    TAGI_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    const bool deep = !sa && !sb && (long)grid.x * grid.y * grid.z <= sms && std::min(kps, g.K) > 3 * TC_K;
+    const auto kern = sa ? (sb ? gemm_tc<true, true, 3> : gemm_tc<true, false, 3>)
+                         : (sb ? gemm_tc<false, true, 3> : deep ? gemm_tc<false, false, 6> : gemm_tc<false, false, 3>);
+    const size_t smem = tc_smem(deep ? 6 : 3);
+    TAGI_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    TAGI_CUDA(launch_chained(kern, grid, TC_THREADS + (sa || sb ? TC_LOADERS : 0), smem, s, ma, mb, t));
     TAGI_LAUNCH_CHECK();
     return TAGI_OK;
 }

@@ -267,8 +267,17 @@ int exclusive_scan(const int *in, int *out, int n, int *d_total, Arena &ar, cuda
 int radix_sort_u64(uint64_t *kin, int *vin, uint64_t *kout, int *vout, int n, int bits, Arena &ar, cudaStream_t s);
 
 // tree.cu
-int build_tree(Tree &t, const double *x, const double *y, const double *z, int n, int leaf,
-               Arena &ar, int *err_flag, cudaStream_t s);
+// build_tree enqueues a tree; finish_trees reads the headers of one or two of them back (one
+// wait) and gives their work memory back.  Whatever needs only the sorted points may be
+// enqueued in between.
+struct TreeBuild {
+    Arena tmp;
+    int *hdr = nullptr;      // device: node and level counts
+    bool small = false;
+};
+int build_tree(TreeBuild &w, Tree &t, const double *x, const double *y, const double *z, int n, int leaf, Arena &ar,
+               cudaStream_t s);
+int finish_trees(TreeBuild *const *w, Tree *const *t, int count, cudaStream_t s);
 int build_lists(Plan &p, cudaStream_t s);
 
 // upward.cu

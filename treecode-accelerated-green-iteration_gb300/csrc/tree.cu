@@ -470,11 +470,10 @@ __global__ void init_root(int *begin, int *end, int *parent, int n) {
 
 }  // namespace
 
-int build_tree(Tree &t, const double *x, const double *y, const double *z, int n, int leaf,
-               Arena &ar, int *err_flag, cudaStream_t s) {
-    (void)err_flag;
+int build_tree(TreeBuild &w, Tree &t, const double *x, const double *y, const double *z, int n, int leaf, Arena &ar,
+               cudaStream_t s) {
     t.n = n;
-    Arena tmp;
+    Arena &tmp = w.tmp;
     tmp.stream = s;
     int rc = TAGI_OK;
     do {
@@ -502,7 +501,7 @@ int build_tree(Tree &t, const double *x, const double *y, const double *z, int n
         }
 
         // internal nodes hold more than leaf points, n / leaf of them per level at most
-        const bool small = n / leaf <= SMALL_TREE;
+        const bool small = w.small = n / leaf <= SMALL_TREE;
         const long cap = std::min(2L * n + 1, small ? 8L * 21 * (n / leaf) + 9 : 2L * n + 1);
         if ((rc = ar.alloc(&t.begin, cap)) || (rc = ar.alloc(&t.end, cap)) ||
             (rc = ar.alloc(&t.parent, cap)) || (rc = ar.alloc(&t.first_child, cap)) ||
@@ -510,6 +509,7 @@ int build_tree(Tree &t, const double *x, const double *y, const double *z, int n
             break;
         int *hdr = nullptr, *nleaves = nullptr;
         if ((rc = tmp.alloc(&hdr, HDR + 1))) break;
+        w.hdr = hdr;
         nleaves = hdr + HDR;
         t.level_start.assign(1, 0);
         if (small) {
@@ -565,21 +565,30 @@ int build_tree(Tree &t, const double *x, const double *y, const double *z, int n
             rc = set_error(TAGI_ERR_CUDA, "node box launch");
             break;
         }
-        int h[HDR + 1] = {};
-        if (cudaMemcpyAsync(h, hdr, sizeof(h), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
-            cudaStreamSynchronize(s) != cudaSuccess) {
-            rc = set_error(TAGI_ERR_CUDA, "tree build: %s", cudaGetErrorString(cudaGetLastError()));
-            break;
-        }
-        t.nleaves = h[HDR];
-        if (small) {
-            t.nnodes = h[0];
-            t.level_start.assign(h + 2, h + 3 + h[1]);
-        }
-        t.nlevels = (int)t.level_start.size() - 1;
         if (cudaGetLastError() != cudaSuccess) { rc = set_error(TAGI_ERR_CUDA, "node box launch"); break; }
     } while (0);
-    tmp.release();
+    return rc;
+}
+
+int finish_trees(TreeBuild *const *w, Tree *const *t, int count, cudaStream_t s) {
+    int h[2][HDR + 1] = {};
+    int rc = TAGI_OK;
+    for (int k = 0; k < count && !rc; k++)
+        if (cudaMemcpyAsync(h[k], w[k]->hdr, sizeof(h[k]), cudaMemcpyDeviceToHost, s) != cudaSuccess)
+            rc = set_error(TAGI_ERR_CUDA, "tree build: %s", cudaGetErrorString(cudaGetLastError()));
+    if (!rc && cudaStreamSynchronize(s) != cudaSuccess)
+        rc = set_error(TAGI_ERR_CUDA, "tree build: %s", cudaGetErrorString(cudaGetLastError()));
+    for (int k = 0; k < count; k++) {
+        w[k]->tmp.release();
+        if (rc) continue;
+        Tree &q = *t[k];
+        q.nleaves = h[k][HDR];
+        if (w[k]->small) {
+            q.nnodes = h[k][0];
+            q.level_start.assign(h[k] + 2, h[k] + 3 + h[k][1]);
+        }
+        q.nlevels = (int)q.level_start.size() - 1;
+    }
     return rc;
 }
 
@@ -858,7 +867,8 @@ int build_lists(Plan &p, cudaStream_t s) {
         const int nb = p.nbatch;
         int *ncnt = nullptr, *fcnt = nullptr;
         if ((rc = tmp.alloc(&ncnt, nb)) || (rc = tmp.alloc(&fcnt, nb))) break;
-        if ((rc = ar.alloc(&p.near_off, nb + 1)) || (rc = ar.alloc(&p.far_off, nb + 1))) break;
+        if ((rc = ar.alloc(&p.near_off, 2 * (nb + 1)))) break;   // both offsets: one copy brings both totals back
+        p.far_off = p.near_off + nb + 1;
         int *node_flag = nullptr;
         if ((rc = tmp.alloc(&node_flag, nns))) break;
         cudaMemsetAsync(node_flag, 0, sizeof(int) * nns, s);
@@ -882,22 +892,27 @@ int build_lists(Plan &p, cudaStream_t s) {
         launch(traverse<false>, bw, 256, 0, s, ta);
         if ((rc = exclusive_scan(ncnt, p.near_off, nb, p.near_off + nb, tmp, s))) break;
         if ((rc = exclusive_scan(fcnt, p.far_off, nb, p.far_off + nb, tmp, s))) break;
-        if (cudaMemcpyAsync(&p.near_total, p.near_off + nb, sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
-            cudaMemcpyAsync(&p.far_total, p.far_off + nb, sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+        // Room that does not depend on the counts is taken while the walk runs: at most nns slots;
+        // items: a slot's last chunk is partial
+        const long most = nns + (long)p.src.nlevels * (p.src.n / p2m_chunk(p.src.n) + 1);
+        long long *costs = nullptr;   // 4 per batch, then the range, slot and item counts
+        if ((rc = ar.alloc(&p.rng_off, nb + 1)) || (rc = ar.alloc(&p.node_slot, nns)) || (rc = ar.alloc(&p.slot_node, nns)) ||
+            (rc = ar.alloc(&p.slot_geom, 6L * nns)) || (rc = ar.alloc(&p.slot_item_off, nns + 1)) ||
+            (rc = ar.alloc(&p.item_slot, most)) || (rc = ar.alloc(&p.item_begin, most)) ||
+            (rc = ar.alloc(&p.item_end, most)) || (rc = tmp.alloc(&costs, 4L * nb + 2)))
+            break;
+        int totals[2] = {0, 0};
+        if (cudaMemcpy2DAsync(totals, sizeof(int), p.near_off + nb, sizeof(int) * (nb + 1), sizeof(int), 2,
+                              cudaMemcpyDeviceToHost, s) != cudaSuccess ||
             cudaStreamSynchronize(s) != cudaSuccess) {
             rc = set_error(TAGI_ERR_CUDA, "list build: %s", cudaGetErrorString(cudaGetLastError()));
             break;
         }
-        // at most near_total ranges and nns slots; items: a slot's last chunk is partial
-        const long most = nns + (long)p.src.nlevels * (p.src.n / p2m_chunk(p.src.n) + 1);
-        long long *costs = nullptr;   // 4 per batch, then the range, slot and item counts
+        p.near_total = totals[0];
+        p.far_total = totals[1];
+        // at most near_total ranges
         if ((rc = ar.alloc(&p.near_list, p.near_total)) || (rc = ar.alloc(&p.far_list, p.far_total)) ||
-            (rc = ar.alloc(&p.rng_off, nb + 1)) || (rc = ar.alloc(&p.rng, p.near_total)) ||
-            (rc = ar.alloc(&p.rng_dmin, p.near_total)) || (rc = ar.alloc(&p.node_slot, nns)) ||
-            (rc = ar.alloc(&p.slot_node, nns)) || (rc = ar.alloc(&p.slot_geom, 6L * nns)) ||
-            (rc = ar.alloc(&p.slot_item_off, nns + 1)) || (rc = ar.alloc(&p.item_slot, most)) ||
-            (rc = ar.alloc(&p.item_begin, most)) || (rc = ar.alloc(&p.item_end, most)) ||
-            (rc = tmp.alloc(&costs, 4L * nb + 2)))
+            (rc = ar.alloc(&p.rng, p.near_total)) || (rc = ar.alloc(&p.rng_dmin, p.near_total)))
             break;
         int *counts = reinterpret_cast<int *>(costs + 4L * nb);
         ta.near_list = p.near_list;
