@@ -416,9 +416,12 @@ __global__ void __launch_bounds__(32 * SW, 24 / SW) near_mixed(const __grid_cons
         const float *ft = a.ft32 + (long)orb * a.nt;
         const int r0 = a.rng_off[b], r1 = a.rng_off[b + 1];
         // consecutive targets per thread: the threads with targets form a
-        // prefix of the groups, so whole warps past it skip the pair loops
-        const int i0 = it.z + NT * (32 * pl.g + pl.lane);
-        const bool warp_busy = it.z + NT * 32 * pl.g < te;
+        // prefix of the groups, so whole warps past it skip the pair loops.  A warp with
+        // at most 32 targets left takes one per lane, at half the cost of two
+        const int first = NT * 32 * pl.g;   // of the warp's targets in the item
+        const bool warp_busy = it.z + first < te;
+        const bool single = NT == 2 && it.z + first + 32 >= te;
+        const int place = first + (single ? pl.lane : NT * pl.lane), i0 = it.z + place;
         float2 tx[NT], ty[NT], tz[NT], lx[NT], ly[NT], lz[NT], nfi[NT];
         // S == 1: the Kahan sums of this thread's own targets; S > 1: sum[0], cmp[0]
         // are those of target it.z + tid
@@ -432,7 +435,7 @@ __global__ void __launch_bounds__(32 * SW, 24 / SW) near_mixed(const __grid_cons
 #pragma unroll
         for (int k = 0; k < NT; k++) {
             const int i = i0 + k;
-            const bool v = i < te;
+            const bool v = i < te && !(single && k > 0);
             if (PASS == 1) {
                 const float4 h = v ? a.thi[i] : make_float4(0.f, 0.f, 0.f, 0.f);
                 const float4 l = v ? a.tlo[i] : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -511,18 +514,28 @@ __global__ void __launch_bounds__(32 * SW, 24 / SW) near_mixed(const __grid_cons
                     const int m = s_cnt[sl];
                     if (m == 0) break;
                     float part[NT];
-                    if (PASS == 1)
-                        near_chunk<KERN, SS, true, true, NT, TILE>(s_src, sl * SLOT, m, tx, ty, tz, lx, ly, lz, sc2, nfi, part);
-                    else if (KERN == KERNEL_COULOMB && SS && (m & NOEXP))
-                        near_chunk<KERN, false, false, false, NT, TILE>(s_src, sl * SLOT, m & ~NOEXP, tx, ty, tz, lx, ly,
-                                                                  lz, sc2, nfi, part);
-                    else
-                        near_chunk<KERN, SS, false, false, NT, TILE>(s_src, sl * SLOT, m, tx, ty, tz, lx, ly, lz, sc2, nfi,
-                                                               part);
+                    auto chunk = [&](auto nt) {
+                        constexpr int N = decltype(nt)::value;
+                        const float2(&x)[N] = reinterpret_cast<const float2(&)[N]>(tx), (&y)[N] = reinterpret_cast<const float2(&)[N]>(ty),
+                                    (&z)[N] = reinterpret_cast<const float2(&)[N]>(tz), (&u)[N] = reinterpret_cast<const float2(&)[N]>(lx),
+                                    (&v)[N] = reinterpret_cast<const float2(&)[N]>(ly), (&w)[N] = reinterpret_cast<const float2(&)[N]>(lz),
+                                    (&f)[N] = reinterpret_cast<const float2(&)[N]>(nfi);
+                        float(&o)[N] = reinterpret_cast<float(&)[N]>(part);
+                        if (PASS == 1)
+                            near_chunk<KERN, SS, true, true, N, TILE>(s_src, sl * SLOT, m, x, y, z, u, v, w, sc2, f, o);
+                        else if (KERN == KERNEL_COULOMB && SS && (m & NOEXP))
+                            near_chunk<KERN, false, false, false, N, TILE>(s_src, sl * SLOT, m & ~NOEXP, x, y, z, u, v, w,
+                                                                           sc2, f, o);
+                        else
+                            near_chunk<KERN, SS, false, false, N, TILE>(s_src, sl * SLOT, m, x, y, z, u, v, w, sc2, f, o);
+                    };
+                    if (single) chunk(std::integral_constant<int, 1>());
+                    else chunk(std::integral_constant<int, NT>());
 #pragma unroll
                     for (int k = 0; k < NT; k++) {
+                        if (single && k > 0) break;
                         if (pl.S == 1) kahan_add(sum[k], cmp[k], part[k]);
-                        else s_part[sl * T + NT * (32 * pl.g + pl.lane) + k] = part[k];
+                        else s_part[sl * T + place + k] = part[k];
                     }
                 }
             }
@@ -536,7 +549,7 @@ __global__ void __launch_bounds__(32 * SW, 24 / SW) near_mixed(const __grid_cons
         }
 #pragma unroll
         for (int k = 0; k < NT; k++)
-            if (i0 + k < te) a.out[(long)orb * a.nt + i0 + k] = ((double)sum[k] - (double)cmp[k]) * sc;
+            if (i0 + k < te && !(single && k > 0)) a.out[(long)orb * a.nt + i0 + k] = ((double)sum[k] - (double)cmp[k]) * sc;
     }
     pass_end();
 }
@@ -658,8 +671,10 @@ __global__ void __launch_bounds__(32 * SW, 16 / SW) far_mixed(const __grid_const
         const double sc = (double)scf;
         const float *ft = a.ft32 + (long)orb * a.nt;
         const float *qh = a.qhat32 + (long)orb * a.nslots * P;
-        const int i0 = it.z + NT * (32 * pl.g + pl.lane);
-        const bool warp_busy = it.z + NT * 32 * pl.g < te;
+        const int first = NT * 32 * pl.g;   // as in near_mixed
+        const bool warp_busy = it.z + first < te;
+        const bool single = NT == 2 && it.z + first + 32 >= te;
+        const int place = first + (single ? pl.lane : NT * pl.lane), i0 = it.z + place;
         float tx[NT], ty[NT], tz[NT];
         // S == 1: the Kahan sums of this thread's own targets; S > 1: sum[0], cmp[0]
         // are those of target it.z + tid
@@ -675,7 +690,7 @@ __global__ void __launch_bounds__(32 * SW, 16 / SW) far_mixed(const __grid_const
 #pragma unroll
         for (int k = 0; k < NT; k++) {
             const int i = i0 + k;
-            const bool v = i < te;
+            const bool v = i < te && !(single && k > 0);
             tx[k] = v ? (float)(a.tx[i] - cb[0]) * scf : 0.f;
             ty[k] = v ? (float)(a.ty[i] - cb[1]) * scf : 0.f;
             tz[k] = v ? (float)(a.tz[i] - cb[2]) * scf : 0.f;
@@ -743,15 +758,23 @@ __global__ void __launch_bounds__(32 * SW, 16 / SW) far_mixed(const __grid_const
                 for (int cl = 0; cl < nc; cl++) {
                     auto add = [&](int k1, int k, float part) {
                         if (pl.S == 1) kahan_add(sum[k], cmp[k], part);
-                        else s_part[(cl * n1 + k1) * T + NT * (32 * pl.g + pl.lane) + k] = part;
+                        else s_part[(cl * n1 + k1) * T + place + k] = part;
                     };
                     const int slab = first_slab(cl, n1, pl);
-                    if (s_slot[c0 + cl] & 1)
-                        far_cluster<KERN, SS, false, MAXN1, NT, LOOPS>(s_q[cl], s_w[cl], s_p[cl], n1, slab, pl.S, tx,
-                                                                       ty, tz, nfi, add);
-                    else
-                        far_cluster<KERN, SS, true, MAXN1, NT, LOOPS>(s_q[cl], s_w[cl], s_p[cl], n1, slab, pl.S, tx,
-                                                                      ty, tz, nfi, add);
+                    auto cluster = [&](auto nt) {
+                        constexpr int N = decltype(nt)::value;
+                        const float(&x)[N] = reinterpret_cast<const float(&)[N]>(tx), (&y)[N] = reinterpret_cast<const float(&)[N]>(ty),
+                                   (&z)[N] = reinterpret_cast<const float(&)[N]>(tz);
+                        const float2(&f)[N] = reinterpret_cast<const float2(&)[N]>(nfi);
+                        if (s_slot[c0 + cl] & 1)
+                            far_cluster<KERN, SS, false, MAXN1, N, LOOPS>(s_q[cl], s_w[cl], s_p[cl], n1, slab, pl.S, x, y,
+                                                                          z, f, add);
+                        else
+                            far_cluster<KERN, SS, true, MAXN1, N, LOOPS>(s_q[cl], s_w[cl], s_p[cl], n1, slab, pl.S, x, y,
+                                                                         z, f, add);
+                    };
+                    if (single) cluster(std::integral_constant<int, 1>());
+                    else cluster(std::integral_constant<int, NT>());
                 }
             }
         }
@@ -764,7 +787,7 @@ __global__ void __launch_bounds__(32 * SW, 16 / SW) far_mixed(const __grid_const
         }
 #pragma unroll
         for (int k = 0; k < NT; k++)
-            if (i0 + k < te) a.out[(long)orb * a.nt + i0 + k] = ((double)sum[k] - (double)cmp[k]) * sc;
+            if (i0 + k < te && !(single && k > 0)) a.out[(long)orb * a.nt + i0 + k] = ((double)sum[k] - (double)cmp[k]) * sc;
     }
     pass_end();
 }
