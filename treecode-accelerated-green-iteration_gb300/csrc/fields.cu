@@ -220,6 +220,16 @@ __device__ __forceinline__ int range_of_chunk(const RangeTable<THREADS> &t, int 
     }
     return lo;
 }
+// The same from range e on: a warp's chunks follow one another, so it is the last range or
+// one of the next, where the search is a chain of five reads of shared memory ahead of a
+// tile's loads.  Single-orbital kernels, Yukawa, 50k points, one orbital 1032 -> 995 us; the
+// orbital groups, whose registers are full, keep the search (32 orbitals x 1M points 1001
+// and 1026 ms).
+template <int THREADS>
+__device__ __forceinline__ int next_range(const RangeTable<THREADS> &t, int nr, int c, int e) {
+    while (e + 1 < nr && t.first[e + 1] <= c) e++;
+    return e;
+}
 
 // Packed FP32 pairs.  On the sm_100 family one FADD2 / FMUL2 / FFMA2
 // instruction applies the same round-to-nearest IEEE operation to two lanes
@@ -468,6 +478,7 @@ __global__ void __launch_bounds__(32 * SW, 24 / SW) near_mixed(const __grid_cons
                 r.x = range_begin(r) | (noexp ? (int)0x80000000u : 0);
                 return true;
             });
+            int range = 0;
             for (int c0 = 0; c0 < n.y; c0 += SW) {
                 __syncthreads();   // the previous tile is no longer read, its partials are written
                 if (pl.S > 1) {
@@ -477,7 +488,7 @@ __global__ void __launch_bounds__(32 * SW, 24 / SW) near_mixed(const __grid_cons
                 const int c = c0 + pl.wid;
                 int cnt4 = 0, flag = 0;
                 if (c < n.y) {
-                    const int e = range_of_chunk(s_rng, n.x, c);
+                    const int e = range = next_range(s_rng, n.x, c, range);
                     const int rb = s_rng.begin[e];
                     const int t0 = (rb & 0x7fffffff) + (c - s_rng.first[e]) * SLOT;
                     const int cnt = min(SLOT, s_rng.end[e] - t0);

@@ -235,7 +235,10 @@ __global__ void p2m_reduce(const double *__restrict__ part, const int *__restric
     const int i0 = slot_item_off[slot], i1 = slot_item_off[slot + 1];
     const double *pp = part + (long)orb * nitems * P;
     TO *o = wout && orb == (int)gridDim.y - 1 ? wout + (long)slot * P : out + ((long)orb * nslots + slot) * P;
-    for (int k = threadIdx.x; k < P; k += blockDim.x) {
+    // a thread per grid point: its sum over the items is a chain, whose loads go out eight at
+    // a time (50k points, degree 7: 19 us behind the sums with 256 threads per slot, now 5)
+    const int k = blockIdx.z * blockDim.x + threadIdx.x;
+    if (k < P) {
         double s = 0.0;
 #pragma unroll 8
         for (int it = i0; it < i1; it++) s += pp[(long)it * P + k];
@@ -285,7 +288,7 @@ int launch_p2m(Plan &p, const T *q, long q_stride, int norb, double *part, cudaS
 
 template <typename TO>
 cudaError_t launch_reduce(const Plan &p, int rows, const double *part, TO *out, TO *wout, cudaStream_t s) {
-    return launch_chained(p2m_reduce<TO>, dim3(p.nslots, rows), 256, 0, s, part, p.slot_item_off, p.nslots, p.nitems, p.P,
+    return launch_chained(p2m_reduce<TO>, dim3(p.nslots, rows, (p.P + 63) / 64), 64, 0, s, part, p.slot_item_off, p.nslots, p.nitems, p.P,
                           out, wout);
 }
 
