@@ -150,7 +150,7 @@ int tagi_plan_convolve(tagi_plan *plan, int numOrbitals, const double *targetVal
  * gives NaN output and sets a flag that tagi_plan_check_parameters returns.
  * orbitalsPerItem: 0 = automatic, 1, 4, 8 or 16 (Yukawa mixed precision
  * shares each pair's geometry across a group of orbitals; other cases use 1).
- * targetsPerThread: 0 = automatic (2 when a batch exceeds 256 targets), 1 or
+ * targetsPerThread: 0 = automatic (by the number of targets), 1 or
  * 2 (mixed single-orbital field kernels; a tuning knob, results unchanged).
  * Extends callTreedriver (BaryTreeInterface.py:88-158), which has neither. */
 int tagi_plan_convolve_ex(tagi_plan *plan, int numOrbitals, const double *targetValues,

@@ -2722,11 +2722,21 @@ int cta_targets(int nt, int og, int nt_per_thread, int warps, int precision) {
     return og > 1 ? GT : 32 * warps / field_split(nt, warps, precision) * nt_per_thread;
 }
 
-// Targets per thread: the caller's request, else 2 where a batch holds more
-// than FT targets (single-orbital mixed kernels only).
-int targets_per_thread(Plan *const *plans, int nsys, int precision, int og, int requested) {
+// Targets per thread (single-orbital mixed kernels only): the caller's request, else 2
+// where that leaves some 380 items of 64 targets.  Meshes whose CTAs hold one warp of targets
+// (field_split): two targets per thread read each staged source once for both, but halve
+// the items, and the chip holds 456 of these CTAs.  One against two, us, Yukawa, one orbital,
+// leaves of 500: 9k targets 108, 140; 15k 186, 215; 21k 289, 294; 26k 382, 358; 40k 766, 643;
+// 50k 1158, 963 (leaves of 300 and 1000 and Coulomb change sides at the same size).  Larger
+// meshes: 2 where a batch fills a CTA, which holds the targets of up to eight warps.
+int targets_per_thread(Plan *const *plans, const int *norb, int nsys, int precision, int og, int requested) {
     if (precision != PREC_MIXED || og != 1) return 1;
     if (requested == 1 || requested == 2) return requested;
+    if (field_warps(plans, nsys, precision) == 8) {
+        long targets = 0;
+        for (int i = 0; i < nsys; i++) targets += (long)plans[i]->tgt.n * norb[i];
+        return targets > 24000 ? 2 : 1;
+    }
     for (int i = 0; i < nsys; i++)
         if (plans[i]->max_batch > FT) return 2;
     return 1;
@@ -2901,7 +2911,7 @@ int convolve(Plan &p, const double *tv, const double *sv, double *out, int norb,
              int og_request, int nt_request) {
     const int og = orbitals_per_item(kernel, precision, &norb, nullptr, 1, og_request, p.n1);
     Plan *pp = &p;
-    const int nt = targets_per_thread(&pp, 1, precision, og, nt_request);
+    const int nt = targets_per_thread(&pp, &norb, 1, precision, og, nt_request);
     const Schedule *sc = nullptr;
     for (const Schedule &c : p.scheds)
         if (schedule_matches(c, &norb, 1, og, nt, precision)) sc = &c;

@@ -123,7 +123,7 @@ int tagi_systems_create(tagi_systems **systems, int numSystems, tagi_plan *const
         wt.push_back((double)q->src.n);
     }
     const int og = orbitals_per_item(kernel, precision, y->norb.data(), wt.data(), numSystems, orbitalsPerItem, maxn1);
-    const int nt = targets_per_thread(y->plans.data(), numSystems, precision, og, targetsPerThread);
+    const int nt = targets_per_thread(y->plans.data(), y->norb.data(), numSystems, precision, og, targetsPerThread);
     int rc = build_schedule(y->plans.data(), y->norb.data(), numSystems, og, nt, precision, y->sched,
                             y->stream);
     if (!rc) {

@@ -290,7 +290,7 @@ constexpr int MAX_SYSTEMS = 8;  // systems per field launch
 int ensure_scratch(Plan &p, int norb, int precision);
 int orbitals_per_item(int kernel, int precision, const int *norb, const double *weight, int nsys, int requested,
                       int max_n1);
-int targets_per_thread(Plan *const *plans, int nsys, int precision, int og, int requested);
+int targets_per_thread(Plan *const *plans, const int *norb, int nsys, int precision, int og, int requested);
 int build_schedule(Plan *const *plans, const int *norb, int nsys, int og, int nt, int precision, Schedule &sc,
                    cudaStream_t s);
 bool schedule_matches(const Schedule &sc, const int *norb, int nsys, int og, int nt, int precision);
