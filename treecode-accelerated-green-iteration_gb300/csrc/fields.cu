@@ -26,7 +26,8 @@
 //     (far) and the runs are added with Kahan compensation;
 //   * the singularity-subtraction term f_i * 4pi/k^2 (Yukawa) or
 //     f_i * 2pi/a^2 (Coulomb) is added in FP64 in the epilogue.
-// FP64 mode: identical structure, FP64 everywhere (exp, sqrt, division).
+// FP64 mode: identical structure, FP64 results: 1/r by a Newton step from the FP32 estimate,
+// the exponential from a table and a short polynomial (inv_root, exp_root).
 //
 // Pair terms (targets i, sources j, r = |x_i - y_j| > 0):
 //   Yukawa  SS  w_j (f_j - f_i) e^{-k r}/r        skip  w_j f_j e^{-k r}/r
