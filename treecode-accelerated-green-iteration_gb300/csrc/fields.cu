@@ -2030,9 +2030,9 @@ __global__ void __launch_bounds__(FT) far_f64(const __grid_constant__ Work w) {
 // Per-call glue: sorted charges, epilogue.
 // ---------------------------------------------------------------------------
 template <bool MIXED>
-__global__ void prep_sources(const double *__restrict__ sv, const int *__restrict__ perm,
-                             const double *__restrict__ w, int ns, float *__restrict__ q32,
-                             double *__restrict__ q64, double *__restrict__ f64) {
+__global__ void prep_sources(const double *sv, const int *perm,
+                             const double *w, int ns, float *q32,
+                             double *q64, double *f64) {
     chain_begin();
     long j = (long)blockIdx.x * blockDim.x + threadIdx.x;
     int orb = blockIdx.y;
@@ -2049,9 +2049,9 @@ __global__ void prep_sources(const double *__restrict__ sv, const int *__restric
 }
 
 template <bool MIXED>
-__global__ void prep_targets(const double *__restrict__ tv, const int *__restrict__ perm, int nt,
-                             float *__restrict__ f32, double *__restrict__ f64, double *__restrict__ close_out,
-                             double *__restrict__ far_out) {
+__global__ void prep_targets(const double *tv, const int *perm, int nt,
+                             float *f32, double *f64, double *close_out,
+                             double *far_out) {
     chain_begin();
     long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
     int orb = blockIdx.y;
@@ -2515,9 +2515,9 @@ constexpr int HOST_KP = 64;
 struct HostParams {
     double k[HOST_KP];
 };
-__global__ void orbital_constants(const double *__restrict__ kp, int nkp, const __grid_constant__ HostParams h, int norb,
-                                  int kernel, int sing, int mixed, double *__restrict__ kpo, float *__restrict__ kc,
-                                  double *__restrict__ ss, int *__restrict__ err, int *__restrict__ queue) {
+__global__ void orbital_constants(const double *kp, int nkp, const __grid_constant__ HostParams h, int norb,
+                                  int kernel, int sing, int mixed, double *kpo, float *kc,
+                                  double *ss, int *err, int *queue) {
     chain_begin();
     const int o = blockIdx.x * blockDim.x + threadIdx.x;
     if (queue && o < 3) queue[o] = 0;   // the field passes' work counters

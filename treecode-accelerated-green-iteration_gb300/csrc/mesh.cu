@@ -86,10 +86,10 @@ __global__ void mesh_start(Progress *p, int nbase) {
 // atoms in turn on the FP64 pipe), a scan, a copy to the host and eight allocations, 85 us in all.
 constexpr int CELL_LANES = 8, LEVEL_THREADS = 128;
 __global__ void __launch_bounds__(LEVEL_THREADS) mesh_level(
-    const double *__restrict__ cells, const uint64_t *__restrict__ keys, int depth, const double *__restrict__ atoms,
-    int natoms, const __grid_constant__ Rule p, Progress *prog, double *__restrict__ next_cells,
-    uint64_t *__restrict__ next_keys, int next_cap, double *__restrict__ leaf_cells, uint64_t *__restrict__ leaf_keys,
-    int *__restrict__ leaf_fine, int leaf_cap) {
+    const double *cells, const uint64_t *keys, int depth, const double *atoms,
+    int natoms, const __grid_constant__ Rule p, Progress *prog, double *next_cells,
+    uint64_t *next_keys, int next_cap, double *leaf_cells, uint64_t *leaf_keys,
+    int *leaf_fine, int leaf_cap) {
     chain_begin();
     const int n = prog->count[depth];
     if (prog->err & 2) return;

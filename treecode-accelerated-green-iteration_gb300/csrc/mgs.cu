@@ -65,9 +65,9 @@ __device__ __forceinline__ double warp_sum(double v) {
 // partial[row][block] for the rows of this block's row group.  n: points (VEC:
 // pairs of points), chunk: of them per block.
 template <bool VEC>
-__global__ void __launch_bounds__(MT) mgs_dots(const double *__restrict__ V, const double *__restrict__ U,
-                                               const double *__restrict__ W, int target, long npts, long n, long chunk,
-                                               double *__restrict__ partial) {
+__global__ void __launch_bounds__(MT) mgs_dots(const double *V, const double *U,
+                                               const double *W, int target, long npts, long n, long chunk,
+                                               double *partial) {
     typedef Pts<VEC> P;
     __shared__ double sh[RB][MW];
     chain_begin();
@@ -121,10 +121,10 @@ __global__ void __launch_bounds__(MT) mgs_dots(const double *__restrict__ V, con
 // U -= sum_i r_i V_i with r_i from the dot kernel's partials; norm partials.
 constexpr int SROWS = 128;   // projections held in shared memory at a time
 template <bool VEC>
-__global__ void __launch_bounds__(MT) mgs_subtract(const double *__restrict__ V, double *__restrict__ U,
-                                                   const double *__restrict__ W, const double *__restrict__ partial,
+__global__ void __launch_bounds__(MT) mgs_subtract(const double *V, double *U,
+                                                   const double *W, const double *partial,
                                                    int nblk, int target, long npts, long n, long chunk,
-                                                   double *__restrict__ npart) {
+                                                   double *npart) {
     typedef Pts<VEC> P;
     __shared__ double s_r[SROWS], sh[MW];
     chain_begin();
@@ -179,8 +179,8 @@ __device__ __forceinline__ double divide(double u, double norm, double inv) {
 }
 
 template <bool VEC>
-__global__ void __launch_bounds__(MT) mgs_normalize(double *__restrict__ V, double *__restrict__ U,
-                                                    const double *__restrict__ npart, int nblk, int target, long npts,
+__global__ void __launch_bounds__(MT) mgs_normalize(double *V, double *U,
+                                                    const double *npart, int nblk, int target, long npts,
                                                     long n, long chunk) {
     typedef Pts<VEC> P;
     __shared__ double s_norm;

@@ -136,7 +136,7 @@ __device__ __forceinline__ void load_rows(unsigned (&v)[ROWS], const __nv_bfloat
         const int i = k_major ? i0 + row : i0 + (row & 64) + c, k = k_major ? k0 + c : k0 + (row & 63);
         const long o = i * smn + k * sk;
         const bool in0 = i < mn && k < K, in1 = k_major ? i < mn && k + 1 < K : i + 1 < mn && k < K;
-        const unsigned lo = in0 ? __ldg(p + o) : 0, hi = in1 ? __ldg(p + o + (k_major ? sk : smn)) : 0;
+        const unsigned lo = in0 ? p[o] : 0, hi = in1 ? p[o + (k_major ? sk : smn)] : 0;
         v[r] = lo | hi << 16;
     }
 }
@@ -457,7 +457,7 @@ int run_gemm(GemmArgs g, int splits, int *used, cudaStream_t s) {
 }
 
 // out[m][n] = sum over splits of part[s][m][n] (fixed order)
-__global__ void splitk_reduce(const float *__restrict__ part, int splits, long mn, float *__restrict__ out) {
+__global__ void splitk_reduce(const float *part, int splits, long mn, float *out) {
     chain_begin();
     const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= mn) return;
@@ -569,7 +569,7 @@ __device__ __forceinline__ float to_f<__nv_bfloat16>(__nv_bfloat16 v) { return _
 // Sums rows r0 + g, r0 + g + COL_GROUPS, ... of column j for this thread's group g,
 // then the groups; valid in group 0.
 template <typename T>
-__device__ __forceinline__ float column_sum(const T *__restrict__ G, long r0, long r1, int N, int j) {
+__device__ __forceinline__ float column_sum(const T *G, long r0, long r1, int N, int j) {
     __shared__ float sh[COL_GROUPS][33];
     chain_begin();
     float s = 0.f;
@@ -585,16 +585,16 @@ __device__ __forceinline__ float column_sum(const T *__restrict__ G, long r0, lo
 }
 
 template <typename T>
-__global__ void __launch_bounds__(32 * COL_GROUPS) colsum_partial(const T *__restrict__ G, long rows, int N,
-                                                                  float *__restrict__ part) {
+__global__ void __launch_bounds__(32 * COL_GROUPS) colsum_partial(const T *G, long rows, int N,
+                                                                  float *part) {
     const int j = blockIdx.y * 32 + threadIdx.x;
     const long r0 = (long)blockIdx.x * COL_ROWS;
     const float s = column_sum(G, r0, min(rows, r0 + COL_ROWS), N, j);
     if (threadIdx.y == 0 && j < N) part[(long)blockIdx.x * N + j] = s;
 }
 
-__global__ void __launch_bounds__(32 * COL_GROUPS) colsum_final(const float *__restrict__ part, int chunks, int N,
-                                                                float *__restrict__ out) {
+__global__ void __launch_bounds__(32 * COL_GROUPS) colsum_final(const float *part, int chunks, int N,
+                                                                float *out) {
     const int j = blockIdx.x * 32 + threadIdx.x;
     const float s = column_sum(part, 0, chunks, N, j);
     if (threadIdx.y == 0 && j < N) out[j] = s;

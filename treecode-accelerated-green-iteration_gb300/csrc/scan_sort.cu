@@ -143,8 +143,8 @@ constexpr int RS_THREADS = 256, RS_WARPS = RS_THREADS / 32, RS_BITS = 9, RS_DIGI
 
 // counts[tile][digit], and their sums over groups of `group` tiles (zeroed before)
 template <int ROUNDS>
-__global__ void __launch_bounds__(RS_THREADS) rs_histogram(const uint64_t *__restrict__ keys, int n, int shift, int group,
-                                                           int *__restrict__ counts, int *__restrict__ sums) {
+__global__ void __launch_bounds__(RS_THREADS) rs_histogram(const uint64_t *keys, int n, int shift, int group,
+                                                           int *counts, int *sums) {
     __shared__ int cnt[RS_DIGITS];
     for (int d = threadIdx.x; d < RS_DIGITS; d += RS_THREADS) cnt[d] = 0;
     chain_begin();
@@ -167,10 +167,10 @@ __global__ void __launch_bounds__(RS_THREADS) rs_histogram(const uint64_t *__res
 // in order with its own counters; a column scan over the warps and the tile's start
 // of each digit turn the ranks into places.
 template <int ROUNDS>
-__global__ void __launch_bounds__(RS_THREADS) rs_scatter(const uint64_t *__restrict__ kin, const int *__restrict__ vin,
-                                                         uint64_t *__restrict__ kout, int *__restrict__ vout, int n,
+__global__ void __launch_bounds__(RS_THREADS) rs_scatter(const uint64_t *kin, const int *vin,
+                                                         uint64_t *kout, int *vout, int n,
                                                          int shift, int group, int ngroups,
-                                                         const int *__restrict__ counts, const int *__restrict__ sums) {
+                                                         const int *counts, const int *sums) {
     __shared__ int wcnt[RS_WARPS][RS_DIGITS];
     __shared__ int wtot[RS_WARPS];
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, tile = blockIdx.x;
@@ -250,8 +250,8 @@ int rs_pass(const uint64_t *kin, const int *vin, uint64_t *kout, int *vout, int 
 // bitonic network in one block took 124 at 6,022.  Counts are whole numbers:
 // the order of the atomic additions does not matter.
 constexpr int SORT_SMALL = 16384, CNT_THREADS = 256;
-__global__ void __launch_bounds__(CNT_THREADS) count_smaller(const uint64_t *__restrict__ keys,
-                                                             int n, int span, int *__restrict__ rank) {
+__global__ void __launch_bounds__(CNT_THREADS) count_smaller(const uint64_t *keys,
+                                                             int n, int span, int *rank) {
     __shared__ __align__(16) uint64_t s_key[CNT_THREADS];
     chain_begin();
     const int i0 = blockIdx.x * CNT_THREADS, i = i0 + threadIdx.x;
@@ -281,8 +281,8 @@ __global__ void __launch_bounds__(CNT_THREADS) count_smaller(const uint64_t *__r
     }
     if (i < n && c) atomicAdd(rank + i, c);
 }
-__global__ void place_sorted(const uint64_t *__restrict__ kin, const int *__restrict__ vin, const int *__restrict__ rank,
-                             int n, uint64_t *__restrict__ kout, int *__restrict__ vout) {
+__global__ void place_sorted(const uint64_t *kin, const int *vin, const int *rank,
+                             int n, uint64_t *kout, int *vout) {
     chain_begin();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;

@@ -68,6 +68,14 @@ inline void launch(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, c
 // has ended (programmatic dependent launch): it calls chain_begin() before it
 // touches anything an earlier kernel wrote or reads, which waits for that kernel
 // and its writes, so only its launch latency overlaps.
+//
+// Such a kernel is resident while earlier kernels of its chain still write the memory that it
+// reads afterwards.  A `const T *__restrict__` parameter (or __ldg) tells the compiler that this
+// memory does not change as long as the kernel runs: it may then read ahead of chain_begin(),
+// whose memory clobber says nothing about a pointer that no one else holds, and through the
+// read-only path, which need not see writes of that time.  So no kernel that calls
+// chain_begin(), and no function that it calls, takes __restrict__ pointers or uses __ldg: plain
+// loads stay behind the wait, which makes the earlier kernels' writes visible to them.
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_chained(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
                                   Args &&...args) {

@@ -82,8 +82,8 @@ __global__ void bbox_partial(const double *__restrict__ x, const double *__restr
 
 // params[0..2] = lower corner, params[3] = 2^21 / cube edge.  One block
 // reduces the per-block partials (min/max are exact in any order).
-__global__ void __launch_bounds__(256) bbox_final(const long long *__restrict__ part, int nb,
-                                                  double *__restrict__ params) {
+__global__ void __launch_bounds__(256) bbox_final(const long long *part, int nb,
+                                                  double *params) {
     chain_begin();
     long long ol[3] = {part[0], part[1], part[2]}, oh[3] = {part[3], part[4], part[5]};
     for (int b = threadIdx.x; b < nb; b += blockDim.x)
@@ -133,10 +133,10 @@ __device__ __forceinline__ uint32_t quantize(double p, double lo, double scale) 
     return v > 2097151u ? 2097151u : v;
 }
 
-__global__ void morton_codes(const double *__restrict__ x, const double *__restrict__ y,
-                             const double *__restrict__ z, int n,
-                             const double *__restrict__ params, uint64_t *__restrict__ codes,
-                             int *__restrict__ idx) {
+__global__ void morton_codes(const double *x, const double *y,
+                             const double *z, int n,
+                             const double *params, uint64_t *codes,
+                             int *idx) {
     chain_begin();
     long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -148,10 +148,10 @@ __global__ void morton_codes(const double *__restrict__ x, const double *__restr
     idx[i] = (int)i;
 }
 
-__global__ void gather3(const double *__restrict__ x, const double *__restrict__ y,
-                        const double *__restrict__ z, const int *__restrict__ perm, int n,
-                        double *__restrict__ xs, double *__restrict__ ys,
-                        double *__restrict__ zs) {
+__global__ void gather3(const double *x, const double *y,
+                        const double *z, const int *perm, int n,
+                        double *xs, double *ys,
+                        double *zs) {
     chain_begin();
     long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -172,7 +172,7 @@ __device__ __forceinline__ int run_end(const uint64_t *__restrict__ codes, int l
     return lo;
 }
 
-__device__ __forceinline__ int split_shift(const uint64_t *__restrict__ codes, int b, int e) {
+__device__ __forceinline__ int split_shift(const uint64_t *codes, int b, int e) {
     uint64_t x = codes[b] ^ codes[e - 1];
     if (x == 0) return -1;
     int hb = 63 - __clzll((long long)x);
@@ -242,10 +242,10 @@ constexpr int HDR = MAX_LEVELS + 3;
 // SMALL_TREE leaves' worth of points one launch per level is quicker.
 constexpr int SMALL_TREE = 4096;
 constexpr int BUILD_THREADS = 1024;
-__global__ void __launch_bounds__(BUILD_THREADS) build_nodes(const uint64_t *__restrict__ codes, int n, int leaf,
-                                                             int *__restrict__ begin, int *__restrict__ end,
-                                                             int *__restrict__ parent, int *__restrict__ first_child,
-                                                             int *__restrict__ nchild, int *__restrict__ hdr) {
+__global__ void __launch_bounds__(BUILD_THREADS) build_nodes(const uint64_t *codes, int n, int leaf,
+                                                             int *begin, int *end,
+                                                             int *parent, int *first_child,
+                                                             int *nchild, int *hdr) {
     __shared__ int s_cnt[BUILD_THREADS / 32];
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     chain_begin();
@@ -337,11 +337,11 @@ __global__ void write_header(int *hdr, int nnodes) { hdr[0] = nnodes; }
 // centers and radii (FP64) follow in preorder.  44,000 points, leaves of 1834, a warp
 // per leaf and all of a node's values in the climb before: 48 -> 15 us.
 constexpr int BOX_THREADS = 128;
-__global__ void __launch_bounds__(BOX_THREADS) node_boxes(const int *__restrict__ hdr, const int *__restrict__ begin,
-                                                          const int *__restrict__ end, const int *__restrict__ parent,
-                                                          const int *__restrict__ first_child,
-                                                          const int *__restrict__ nchild, const double *__restrict__ x,
-                                                          const double *__restrict__ y, const double *__restrict__ z,
+__global__ void __launch_bounds__(BOX_THREADS) node_boxes(const int *hdr, const int *begin,
+                                                          const int *end, const int *parent,
+                                                          const int *first_child,
+                                                          const int *nchild, const double *x,
+                                                          const double *y, const double *z,
                                                           long long *box, int *size, int *leaves, int *done) {
     __shared__ long long s_box[BOX_THREADS / 32][6];
     chain_begin();
@@ -416,13 +416,13 @@ __global__ void __launch_bounds__(BOX_THREADS) node_boxes(const int *__restrict_
 // Each node's center, half edges and radius; its place in pre-order (children in digit
 // order) and each leaf's among the leaves, from the subtrees passed on the way to the
 // root.
-__global__ void preorder(const int *__restrict__ hdr, const int *__restrict__ begin, const int *__restrict__ end,
-                         const int *__restrict__ parent, const int *__restrict__ first_child,
-                         const int *__restrict__ nchild, const long long *__restrict__ box,
-                         double *__restrict__ center, double *__restrict__ half, double *__restrict__ radius,
-                         const int *__restrict__ size,
-                         const int *__restrict__ leaves, PreNode *__restrict__ pre, int *__restrict__ leaf_node,
-                         int *__restrict__ nleaves) {
+__global__ void preorder(const int *hdr, const int *begin, const int *end,
+                         const int *parent, const int *first_child,
+                         const int *nchild, const long long *box,
+                         double *center, double *half, double *radius,
+                         const int *size,
+                         const int *leaves, PreNode *pre, int *leaf_node,
+                         int *nleaves) {
     chain_begin();
     const int nn = hdr[0];
     for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < nn; v += gridDim.x * blockDim.x) {

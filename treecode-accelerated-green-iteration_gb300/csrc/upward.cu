@@ -228,8 +228,8 @@ __global__ void __launch_bounds__(P2M_THREADS) p2m_f64(const __grid_constant__ P
 }
 
 template <typename TO>
-__global__ void p2m_reduce(const double *__restrict__ part, const int *__restrict__ slot_item_off,
-                           int nslots, int nitems, int P, TO *__restrict__ out, TO *__restrict__ wout) {
+__global__ void p2m_reduce(const double *part, const int *slot_item_off,
+                           int nslots, int nitems, int P, TO *out, TO *wout) {
     const int slot = blockIdx.x, orb = blockIdx.y;
     chain_begin();
     const int i0 = slot_item_off[slot], i1 = slot_item_off[slot + 1];
