@@ -106,6 +106,7 @@ struct Work {
     const int4 *items;            // {batch, sys << 16 | first orbital, target begin, end}, heaviest first
     int nitems;
     int *queue;                   // this pass's work counter
+    int turn;                     // FP64: which of an item's CTAs' worth of targets
     const double *exp_table;      // FP64 passes: 2^{i / EXP_N}
     Fields sys[MAX_SYSTEMS];
 };
@@ -1924,9 +1925,9 @@ __global__ void __launch_bounds__(FT) near_f64(const __grid_constant__ Work w) {
         const double *f = a.f64 + (long)orb * a.ns;
         const double *ft = a.ft64 + (long)orb * a.nt;
         const int r0 = a.rng_off[b], r1 = a.rng_off[b + 1];
-        const int i = it.z + 32 * pl.g + pl.lane;
+        const int first = it.z + 32 * (w.turn * pl.G + pl.g), i = first + pl.lane;
         const bool v = i < it.w;
-        const bool warp_busy = it.z + 32 * pl.g < it.w;
+        const bool warp_busy = first < it.w;
         const double xi = v ? a.tx[i] : 0.0, yi = v ? a.ty[i] : 0.0, zi = v ? a.tz[i] : 0.0;
         const double fi = v ? ft[i] : 0.0;
         double acc = 0.0;
@@ -1981,9 +1982,9 @@ __global__ void __launch_bounds__(FT) far_f64(const __grid_constant__ Work w) {
         const ExpScale es = exp_scale(kp, KERN == KERNEL_COULOMB);
         const double *ft = a.ft64 + (long)orb * a.nt;
         const double *qh = a.qhat64 + (long)orb * a.nslots * P;
-        const int i = it.z + 32 * pl.g + pl.lane;
+        const int first = it.z + 32 * (w.turn * pl.G + pl.g), i = first + pl.lane;
         const bool v = i < it.w;
-        const bool warp_busy = it.z + 32 * pl.g < it.w;
+        const bool warp_busy = first < it.w;
         const double xi = v ? a.tx[i] : 0.0, yi = v ? a.ty[i] : 0.0, zi = v ? a.tz[i] : 0.0;
         const double fi = v ? ft[i] : 0.0;
         double acc = 0.0;
@@ -2486,14 +2487,25 @@ int launch_fields(const SysCall *calls, const Fields *f, int nsys, const Schedul
     if (precision == PREC_MIXED && sh.warps == 8) TAGI_TRY((launch_mixed<KERN, SS, 8>(wn, wc, wf, sh, s, &pdl)));
     else if (precision == PREC_MIXED) TAGI_TRY((launch_mixed<KERN, SS, 4>(wn, wc, wf, sh, s, &pdl)));
     if (precision != PREC_MIXED) {
-        // one FP64 pass over all near ranges, close ones included
-        TAGI_TRY(launch_persistent(near_f64<KERN, SS>, wn, s, f64_smem<KERN, SS>(), FT, &pdl));
-        phase_mark(PH_NEAR, false, s);
-        phase_mark(PH_FAR, true, s);
-        if (sh.maxn1 <= 4) TAGI_TRY(launch_persistent(far_f64<KERN, SS, 4>, wf, s, f64_smem<KERN, SS>(), FT, &pdl));
-        else if (sh.maxn1 <= 8) TAGI_TRY(launch_persistent(far_f64<KERN, SS, 8>, wf, s, f64_smem<KERN, SS>(), FT, &pdl));
-        else TAGI_TRY(launch_persistent(far_f64<KERN, SS, MAX_DEGREE + 1>, wf, s, f64_smem<KERN, SS>(), FT, &pdl));
-        phase_mark(PH_FAR, false, s);
+        // one FP64 pass over all near ranges, close ones included.  A list made for mixed precision
+        // (schedule_for_capture) may hold more targets per item than a CTA: the passes are then
+        // repeated for the next ones
+        const int cta = FT / f[0].split, turns = sc.precision == PREC_FP64 ? 1 : (sc.most + cta - 1) / cta;
+        for (int turn = 0; turn < turns; turn++) {
+            if (turn) {
+                TAGI_CUDA(cudaMemsetAsync(queue, 0, 3 * sizeof(int), s));
+                pdl = false;
+            }
+            wn.turn = wf.turn = turn;
+            if (turn) phase_mark(PH_NEAR, true, s);
+            TAGI_TRY(launch_persistent(near_f64<KERN, SS>, wn, s, f64_smem<KERN, SS>(), FT, &pdl));
+            phase_mark(PH_NEAR, false, s);
+            phase_mark(PH_FAR, true, s);
+            if (sh.maxn1 <= 4) TAGI_TRY(launch_persistent(far_f64<KERN, SS, 4>, wf, s, f64_smem<KERN, SS>(), FT, &pdl));
+            else if (sh.maxn1 <= 8) TAGI_TRY(launch_persistent(far_f64<KERN, SS, 8>, wf, s, f64_smem<KERN, SS>(), FT, &pdl));
+            else TAGI_TRY(launch_persistent(far_f64<KERN, SS, MAX_DEGREE + 1>, wf, s, f64_smem<KERN, SS>(), FT, &pdl));
+            phase_mark(PH_FAR, false, s);
+        }
     }
     return TAGI_OK;
 }
@@ -2693,6 +2705,21 @@ bool schedule_matches(const Schedule &sc, const int *norb, int nsys, int og, int
     return true;
 }
 
+// Of a plan's work lists the one for this call under stream capture, where none can be made: the
+// call's own, or one that another targets-per-thread setting or precision made for these orbitals
+// and this group size.  Mixed results do not depend on how a list cuts the batches; FP64 passes
+// run once more for the targets that a CTA does not hold; an FP64 item's targets fit one thread
+// each of a mixed kernel's CTA (cta_targets: 32 and 32 up to 131,072 targets, 64 and 64 or 128 above).
+const Schedule *schedule_for_capture(const std::vector<Schedule> &scheds, int norb, int og, int nt, int precision) {
+    const Schedule *best = nullptr;
+    for (const Schedule &c : scheds) {
+        if (!schedule_matches(c, &norb, 1, og, c.nt, c.precision)) continue;
+        if (c.nt == nt && c.precision == precision) return &c;
+        if (!best || c.precision == precision) best = &c;
+    }
+    return best;
+}
+
 // Warps that share a target's sources in the single-orbital kernels, by the
 // plan's targets: a CTA then holds (warps / split) x 32 threads' targets, and a
 // small mesh still has items for every SM, while a large one stages each tile for
@@ -2753,6 +2780,7 @@ int build_schedule(Plan *const *plans, const int *norb, int nsys, int og, int nt
                    cudaStream_t s) {
     if (nsys < 1 || nsys > MAX_SYSTEMS) return set_error(TAGI_ERR_ARG, "%d systems (1..%d per launch)", nsys, MAX_SYSTEMS);
     const int warps = field_warps(plans, nsys, precision);
+    sc.most = 0;
     struct Batch {
         long long cost;   // pairs of one chunk
         int sys, b, begin, end, chunk;
@@ -2763,6 +2791,7 @@ int build_schedule(Plan *const *plans, const int *norb, int nsys, int og, int nt
         if (norb[i] < 1 || norb[i] > 0xffff) return set_error(TAGI_ERR_ARG, "system %d: %d orbitals", i, norb[i]);
         if ((int)p.cost_near.size() != p.nbatch) return set_error(TAGI_ERR_STATE, "plan without batch costs");
         const int warp = 32 * nt, most = cta_targets(p.tgt.n, og, nt, warps, precision);
+        sc.most = std::max(sc.most, most);
         for (int b = 0, at = 0; b < p.nbatch; at += p.batch_size[b++]) {
             const int n = p.batch_size[b], chunks = (n + most - 1) / most;
             const int chunk = ((n + chunks - 1) / chunks + warp - 1) / warp * warp;
@@ -2914,10 +2943,14 @@ int convolve(Plan &p, const double *tv, const double *sv, double *out, int norb,
     Plan *pp = &p;
     const int nt = targets_per_thread(&pp, &norb, 1, precision, og, nt_request);
     const Schedule *sc = nullptr;
-    for (const Schedule &c : p.scheds)
-        if (schedule_matches(c, &norb, 1, og, nt, precision)) sc = &c;
-    if (!sc && stream_capturing(s))
-        return set_error(TAGI_ERR_STATE, "graph capture needs a prior uncaptured call with the same orbital count");
+    if (stream_capturing(s)) {
+        sc = schedule_for_capture(p.scheds, norb, og, nt, precision);
+        if (!sc)
+            return set_error(TAGI_ERR_STATE, "graph capture needs a prior uncaptured call with the same orbital count");
+    } else {
+        for (const Schedule &c : p.scheds)
+            if (schedule_matches(c, &norb, 1, og, nt, precision)) sc = &c;
+    }
     if (norb < 1 || norb > 0xffff) return set_error(TAGI_ERR_ARG, "system 0: %d orbitals", norb);
     auto make_schedule = [&](const Schedule **out) -> int {
         constexpr size_t KEEP = 4;  // work lists kept per plan (e.g. Hartree + orbital batch)

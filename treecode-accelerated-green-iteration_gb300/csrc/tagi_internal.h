@@ -177,6 +177,7 @@ struct Schedule {
     int og = 0;                 // 0 = not built
     int nt = 1;
     int precision = PREC_MIXED;
+    int most = 0;               // targets of an item at most
     std::vector<int> norb;      // orbitals per system the schedule was built for
     int4 *items = nullptr;      // device, owned unless borrowed
     bool borrowed = false;      // items belong to the plan's arena (one-shot calls)
