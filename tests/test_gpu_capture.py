@@ -47,3 +47,32 @@ def test_lists_of_other_settings_serve(BT, dev, n, leaf, before, then):
     assert torch.isfinite(got).all() and torch.equal(got, call(F, k, **then))
     g.close()
     plan.close()
+
+
+def test_calls_in_other_forms_leave_a_captured_list_alone(BT, dev):
+    """A plan keeps the lists of four orbital counts whatever forms each is called in: a graph over
+    one of them stays valid while the other three are called in both precisions and with one and
+    two targets per thread, and gives the captured call's result on new values."""
+    x, y, z, w, _ = cloud(2001, 7)
+    plan = dev.TreecodePlan.for_mesh(*to_cuda(x, y, z, w), theta=0.8, degree=3, source_leaf=130, target_leaf=130)
+    gen = torch.Generator().manual_seed(7)
+    F = torch.randn((4, 2001), generator=gen, dtype=torch.float64).cuda()
+    k = torch.tensor([0.7, 0.9, 1.1, 1.3], dtype=torch.float64, device="cuda")
+    SS = BT.Singularity.SUBTRACTION
+    s = torch.cuda.Stream()
+    G, out = F.clone(), torch.zeros_like(F)
+    plan.convolve(G, G, BT.Kernel.COULOMB, k, SS, precision="mixed", out=out)
+    torch.cuda.synchronize()
+    with dev.Graph.capture(s) as g:
+        plan.convolve(G, G, BT.Kernel.COULOMB, k, SS, precision="mixed", out=out, stream=s)
+    for norb in (1, 2, 3, 4):
+        for kw in (dict(precision="fp64"), dict(precision="mixed", targets_per_thread=1),
+                   dict(precision="mixed", targets_per_thread=2)):
+            plan.convolve(F[:norb], F[:norb], BT.Kernel.COULOMB, k[:norb], SS, **kw)
+    G.copy_(2.0 * F)
+    torch.cuda.synchronize()
+    g.replay(s)
+    torch.cuda.synchronize()
+    assert torch.equal(out, plan.convolve(2.0 * F, 2.0 * F, BT.Kernel.COULOMB, k, SS, precision="mixed"))
+    g.close()
+    plan.close()

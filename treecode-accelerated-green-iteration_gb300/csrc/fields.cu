@@ -2953,11 +2953,30 @@ int convolve(Plan &p, const double *tv, const double *sv, double *out, int norb,
     }
     if (norb < 1 || norb > 0xffff) return set_error(TAGI_ERR_ARG, "system 0: %d orbitals", norb);
     auto make_schedule = [&](const Schedule **out) -> int {
-        constexpr size_t KEEP = 4;  // work lists kept per plan (e.g. Hartree + orbital batch)
-        if (p.scheds.size() >= KEEP) {
+        // Lists of KEEP orbital counts and group sizes are kept (e.g. Hartree + orbital batch), each
+        // in up to three forms (precision, targets per thread): a captured graph reads its list from
+        // here, and calls on the same orbitals in another form must not take it away.
+        constexpr int KEEP = 4;
+        auto same_orbitals = [](const Schedule &a, const Schedule &b) { return a.og == b.og && a.norb == b.norb; };
+        int kinds = 0;
+        bool known = false;
+        for (size_t i = 0; i < p.scheds.size(); i++) {
+            bool first = true;
+            for (size_t j = 0; j < i; j++) first = first && !same_orbitals(p.scheds[i], p.scheds[j]);
+            kinds += first;
+            known = known || schedule_matches(p.scheds[i], &norb, 1, og, p.scheds[i].nt, p.scheds[i].precision);
+        }
+        if (!known && kinds >= KEEP) {   // the oldest orbital count's lists go
             TAGI_CUDA(cudaDeviceSynchronize());
-            p.scheds.front().release();
-            p.scheds.erase(p.scheds.begin());
+            const Schedule oldest = p.scheds.front();
+            for (size_t i = 0; i < p.scheds.size();) {
+                if (same_orbitals(p.scheds[i], oldest)) {
+                    p.scheds[i].release();
+                    p.scheds.erase(p.scheds.begin() + i);
+                } else {
+                    i++;
+                }
+            }
         }
         p.scheds.emplace_back();
         const int rc = build_schedule(&pp, &norb, 1, og, nt, precision, p.scheds.back(), s);
