@@ -11,10 +11,10 @@
 // in list order.
 //
 // Mixed precision (default fast path):
-//   * coordinates are translated to the batch center in FP64, then rounded to
-//     FP32 (targets once per batch, sources/proxy points while staging into
-//     shared memory), so pair distances keep FP32 precision relative to the
-//     batch size rather than to the domain size;
+//   * coordinates are taken relative to the batch center, then rounded to FP32: targets (and
+//     proxy points) in FP64; sources from FP32 hi/lo splits, to 2^-49 of their distance from
+//     the the origin (neg_relative), or in FP64 too in plans so far from the origin that this would
+//     show (WIDE kernels).  Close ranges use the splits themselves;
 //   * coordinates are also multiplied by a per-orbital scale sc, so that with
 //     r' = sc r the kernels need no multiply for the exp2 argument:
 //       Yukawa       sc = k log2(e):          e^{-k r}/r     = sc 2^{-r'} / r'
@@ -319,6 +319,11 @@ __device__ __forceinline__ float2 neg_relative(float2 xh, float2 xl, const Split
     const float2 p = mul2(d, sc);
     return add2(p, fma2(e, sc, fma2(d, sc, neg2(p))));
 }
+// -(x - c) sc in FP64, rounded once (WIDE kernels, for plans whose batches lie so far from the
+// origin that the splits' 48 bits would show: Plan::wide)
+__device__ __forceinline__ float2 neg_relative64(const double *__restrict__ x, int j0, int j1, double c, double sc) {
+    return make_float2(-(float)((x[j0] - c) * sc), -(float)((x[j1] - c) * sc));
+}
 __device__ __forceinline__ void sts2(float *p, float2 v) { *reinterpret_cast<float2 *>(p) = v; }
 
 // Near-field source tile in shared memory, structure of arrays, NEGATED
@@ -398,7 +403,7 @@ __device__ __forceinline__ void near_chunk(const float (*__restrict__ s)[TILE], 
 // sources, 4 above, where more and smaller CTAs wait less at their barriers (24 warps
 // per SM either way).  near + far, ms, 8 and 4 warps: Coulomb 1.5M points 94.3 -> 92.2, 1.34M
 // points, degree 4, Yukawa 71.5 -> 66.7; Yukawa 50k points, whole call 1.11 and 1.31.
-template <int KERN, bool SS, int NT, int PASS, int SW>
+template <int KERN, bool SS, int NT, int PASS, int SW, bool WIDE = false>
 __global__ void __launch_bounds__(32 * SW, 24 / SW) near_mixed(const __grid_constant__ Work w) {
     constexpr int NR = PASS == 1 ? NROWS_PRECISE : 5, ST = 32 * SW, TILE = SW * SLOT;   // warp w stages slot w of a tile
     __shared__ __align__(16) float s_src[NR][TILE];
@@ -500,21 +505,27 @@ __global__ void __launch_bounds__(32 * SW, 24 / SW) near_mixed(const __grid_cons
                     if (j < cnt4) {
                         const bool real0 = j < cnt, real1 = j + 1 < cnt;
                         const int j0 = t0 + (real0 ? j : 0), j1 = t0 + (real1 ? j + 1 : 0);   // padding: the first source
-                        const float4 h0 = a.shi[j0], h1 = a.shi[j1], l0 = a.slo[j0], l1 = a.slo[j1];
-                        const float2 hx = make_float2(h0.x, h1.x), hy = make_float2(h0.y, h1.y),
-                                     hz = make_float2(h0.z, h1.z), qx = make_float2(l0.x, l1.x),
-                                     qy = make_float2(l0.y, l1.y), qz = make_float2(l0.z, l1.z);
-                        if constexpr (PASS == 1) {
-                            sts2(&s_src[0][d], neg2(hx));
-                            sts2(&s_src[1][d], neg2(hy));
-                            sts2(&s_src[2][d], neg2(hz));
-                            sts2(&s_src[5][d], neg2(qx));
-                            sts2(&s_src[6][d], neg2(qy));
-                            sts2(&s_src[7][d], neg2(qz));
+                        if constexpr (WIDE) {
+                            sts2(&s_src[0][d], neg_relative64(a.sx, j0, j1, cbx, sc));
+                            sts2(&s_src[1][d], neg_relative64(a.sy, j0, j1, cby, sc));
+                            sts2(&s_src[2][d], neg_relative64(a.sz, j0, j1, cbz, sc));
                         } else {
-                            sts2(&s_src[0][d], neg_relative(hx, qx, ccx, dup2(scf)));
-                            sts2(&s_src[1][d], neg_relative(hy, qy, ccy, dup2(scf)));
-                            sts2(&s_src[2][d], neg_relative(hz, qz, ccz, dup2(scf)));
+                            const float4 h0 = a.shi[j0], h1 = a.shi[j1], l0 = a.slo[j0], l1 = a.slo[j1];
+                            const float2 hx = make_float2(h0.x, h1.x), hy = make_float2(h0.y, h1.y),
+                                         hz = make_float2(h0.z, h1.z), qx = make_float2(l0.x, l1.x),
+                                         qy = make_float2(l0.y, l1.y), qz = make_float2(l0.z, l1.z);
+                            if constexpr (PASS == 1) {
+                                sts2(&s_src[0][d], neg2(hx));
+                                sts2(&s_src[1][d], neg2(hy));
+                                sts2(&s_src[2][d], neg2(hz));
+                                sts2(&s_src[5][d], neg2(qx));
+                                sts2(&s_src[6][d], neg2(qy));
+                                sts2(&s_src[7][d], neg2(qz));
+                            } else {
+                                sts2(&s_src[0][d], neg_relative(hx, qx, ccx, dup2(scf)));
+                                sts2(&s_src[1][d], neg_relative(hy, qy, ccy, dup2(scf)));
+                                sts2(&s_src[2][d], neg_relative(hz, qz, ccz, dup2(scf)));
+                            }
                         }
                         sts2(&s_src[3][d], make_float2(real0 ? q[j0] : 0.f, real1 ? q[j1] : 0.f));
                         sts2(&s_src[4][d], make_float2(real0 ? a.w32[j0] : 0.f, real1 ? a.w32[j1] : 0.f));
@@ -895,7 +906,7 @@ __device__ __forceinline__ void for_pairs(int n2, FN &&fn) {
 template <int OG>
 __device__ __forceinline__ int item_pairs(int norb, int g0) { return min(OG / 2, (norb - g0 + 1) >> 1); }
 
-template <bool SS, int OG, int PASS>
+template <bool SS, int OG, int PASS, bool WIDE = false>
 __global__ void __launch_bounds__(GT, 4) near_group(const __grid_constant__ Work w) {
     constexpr int NR = PASS == 1 ? 7 : 4;
     __shared__ __align__(16) float s_src[NR][GTILE];
@@ -970,21 +981,27 @@ __global__ void __launch_bounds__(GT, 4) near_group(const __grid_constant__ Work
                     if (j < cnt2) {
                         const bool real0 = j < cnt, real1 = j + 1 < cnt;
                         const int j0 = t0 + (real0 ? j : 0), j1 = t0 + (real1 ? j + 1 : 0);   // padding: the first source
-                        const float4 h0 = a.shi[j0], h1 = a.shi[j1], l0 = a.slo[j0], l1 = a.slo[j1];
-                        const float2 hx = make_float2(h0.x, h1.x), hy = make_float2(h0.y, h1.y),
-                                     hz = make_float2(h0.z, h1.z), qx = make_float2(l0.x, l1.x),
-                                     qy = make_float2(l0.y, l1.y), qz = make_float2(l0.z, l1.z);
-                        if constexpr (PASS == 1) {
-                            sts2(&s_src[0][d], neg2(hx));
-                            sts2(&s_src[1][d], neg2(hy));
-                            sts2(&s_src[2][d], neg2(hz));
-                            sts2(&s_src[4][d], neg2(qx));
-                            sts2(&s_src[5][d], neg2(qy));
-                            sts2(&s_src[6][d], neg2(qz));
+                        if constexpr (WIDE) {
+                            sts2(&s_src[0][d], neg_relative64(a.sx, j0, j1, cbx, 1.0));
+                            sts2(&s_src[1][d], neg_relative64(a.sy, j0, j1, cby, 1.0));
+                            sts2(&s_src[2][d], neg_relative64(a.sz, j0, j1, cbz, 1.0));
                         } else {
-                            sts2(&s_src[0][d], neg_relative(hx, qx, ccx));
-                            sts2(&s_src[1][d], neg_relative(hy, qy, ccy));
-                            sts2(&s_src[2][d], neg_relative(hz, qz, ccz));
+                            const float4 h0 = a.shi[j0], h1 = a.shi[j1], l0 = a.slo[j0], l1 = a.slo[j1];
+                            const float2 hx = make_float2(h0.x, h1.x), hy = make_float2(h0.y, h1.y),
+                                         hz = make_float2(h0.z, h1.z), qx = make_float2(l0.x, l1.x),
+                                         qy = make_float2(l0.y, l1.y), qz = make_float2(l0.z, l1.z);
+                            if constexpr (PASS == 1) {
+                                sts2(&s_src[0][d], neg2(hx));
+                                sts2(&s_src[1][d], neg2(hy));
+                                sts2(&s_src[2][d], neg2(hz));
+                                sts2(&s_src[4][d], neg2(qx));
+                                sts2(&s_src[5][d], neg2(qy));
+                                sts2(&s_src[6][d], neg2(qz));
+                            } else {
+                                sts2(&s_src[0][d], neg_relative(hx, qx, ccx));
+                                sts2(&s_src[1][d], neg_relative(hy, qy, ccy));
+                                sts2(&s_src[2][d], neg_relative(hz, qz, ccz));
+                            }
                         }
                         sts2(&s_src[3][d], make_float2(real0 ? a.w32[j0] : 0.f, real1 ? a.w32[j1] : 0.f));
                     }
@@ -1431,7 +1448,7 @@ __host__ __device__ constexpr size_t near_group16_smem(int pass) {
     return sizeof(float) * ((size_t)GTILE * ((pass == 1 ? 7 : 4) + QS16) + 32 * GT);
 }
 
-template <bool SS, int PASS>
+template <bool SS, int PASS, bool WIDE = false>
 __global__ void __launch_bounds__(GT, 4) near_group16(const __grid_constant__ Work w) {
     constexpr int NR = PASS == 1 ? 7 : 4;
     extern __shared__ __align__(16) float s_dyn[];
@@ -1502,21 +1519,27 @@ __global__ void __launch_bounds__(GT, 4) near_group16(const __grid_constant__ Wo
                     if (j < cnt4) {
                         const bool real0 = j < cnt, real1 = j + 1 < cnt;
                         const int j0 = t0 + (real0 ? j : 0), j1 = t0 + (real1 ? j + 1 : 0);   // padding: the first source
-                        const float4 h0 = a.shi[j0], h1 = a.shi[j1], l0 = a.slo[j0], l1 = a.slo[j1];
-                        const float2 hx = make_float2(h0.x, h1.x), hy = make_float2(h0.y, h1.y),
-                                     hz = make_float2(h0.z, h1.z), qx = make_float2(l0.x, l1.x),
-                                     qy = make_float2(l0.y, l1.y), qz = make_float2(l0.z, l1.z);
-                        if constexpr (PASS == 1) {
-                            sts2(&s_src[0][d], neg2(hx));
-                            sts2(&s_src[1][d], neg2(hy));
-                            sts2(&s_src[2][d], neg2(hz));
-                            sts2(&s_src[4][d], neg2(qx));
-                            sts2(&s_src[5][d], neg2(qy));
-                            sts2(&s_src[6][d], neg2(qz));
+                        if constexpr (WIDE) {
+                            sts2(&s_src[0][d], neg_relative64(a.sx, j0, j1, cbx, 1.0));
+                            sts2(&s_src[1][d], neg_relative64(a.sy, j0, j1, cby, 1.0));
+                            sts2(&s_src[2][d], neg_relative64(a.sz, j0, j1, cbz, 1.0));
                         } else {
-                            sts2(&s_src[0][d], neg_relative(hx, qx, ccx));
-                            sts2(&s_src[1][d], neg_relative(hy, qy, ccy));
-                            sts2(&s_src[2][d], neg_relative(hz, qz, ccz));
+                            const float4 h0 = a.shi[j0], h1 = a.shi[j1], l0 = a.slo[j0], l1 = a.slo[j1];
+                            const float2 hx = make_float2(h0.x, h1.x), hy = make_float2(h0.y, h1.y),
+                                         hz = make_float2(h0.z, h1.z), qx = make_float2(l0.x, l1.x),
+                                         qy = make_float2(l0.y, l1.y), qz = make_float2(l0.z, l1.z);
+                            if constexpr (PASS == 1) {
+                                sts2(&s_src[0][d], neg2(hx));
+                                sts2(&s_src[1][d], neg2(hy));
+                                sts2(&s_src[2][d], neg2(hz));
+                                sts2(&s_src[4][d], neg2(qx));
+                                sts2(&s_src[5][d], neg2(qy));
+                                sts2(&s_src[6][d], neg2(qz));
+                            } else {
+                                sts2(&s_src[0][d], neg_relative(hx, qx, ccx));
+                                sts2(&s_src[1][d], neg_relative(hy, qy, ccy));
+                                sts2(&s_src[2][d], neg_relative(hz, qz, ccz));
+                            }
                         }
                         sts2(&s_src[3][d], make_float2(real0 ? a.w32[j0] : 0.f, real1 ? a.w32[j1] : 0.f));
                     }
@@ -2379,7 +2402,14 @@ struct LaunchShape {
     int warps = 4;  // warps per CTA (single-orbital mixed kernels)
     int maxn1 = 1;        // largest proxy-grid edge n + 1
     int minn1 = 1 << 20;  // smallest proxy-grid edge n + 1
+    bool wide = false;    // some plan's sources are staged from FP64 coordinates (Plan::wide)
 };
+
+// fn(WIDE) for the ordinary near pass.
+template <typename FN>
+int near_call(const LaunchShape &sh, FN &&fn) {
+    return sh.wide ? fn(std::integral_constant<bool, true>()) : fn(std::integral_constant<bool, false>());
+}
 
 // fn(MAXN1, loops) for the far kernel of a launch: rows of a known length where all its
 // systems have one, everything known at degree 7, the usual one.
@@ -2405,8 +2435,12 @@ template <int KERN, bool SS, int SW>
 int launch_mixed(const Work &wn, const Work &wc, const Work &wf, const LaunchShape &sh, cudaStream_t s, bool *pdl) {
     constexpr int ST = 32 * SW;
     const bool one = sh.nt == 1;
-    if (one) TAGI_TRY(launch_persistent(near_mixed<KERN, SS, 1, 0, SW>, wn, s, 0, ST, pdl));
-    else TAGI_TRY(launch_persistent(near_mixed<KERN, SS, 2, 0, SW>, wn, s, 0, ST, pdl));
+    TAGI_TRY(near_call(sh, [&](auto wide) {
+        // two targets per thread hold an item cut for one as well
+        if constexpr (!wide())
+            if (one) return launch_persistent(near_mixed<KERN, SS, 1, 0, SW>, wn, s, 0, ST, pdl);
+        return launch_persistent(near_mixed<KERN, SS, 2, 0, SW, wide()>, wn, s, 0, ST, pdl);
+    }));
     phase_mark(PH_NEAR, false, s);
     phase_mark(PH_NEAR_CLOSE, true, s);
     if (one) TAGI_TRY(launch_persistent(near_mixed<KERN, SS, 1, 1, SW>, wc, s, 0, ST, pdl));
@@ -2448,7 +2482,9 @@ int launch_fields(const SysCall *calls, const Fields *f, int nsys, const Schedul
     phase_mark(PH_NEAR, true, s);
     bool pdl = false;   // no field pass of this call launched yet
     if (precision == PREC_MIXED && KERN == KERNEL_YUKAWA && sh.og == 16) {
-        TAGI_TRY(launch_persistent(near_group16<SS, 0>, wn, s, near_group16_smem(0), GT, &pdl));
+        TAGI_TRY(near_call(sh, [&](auto wide) {
+            return launch_persistent(near_group16<SS, 0, wide()>, wn, s, near_group16_smem(0), GT, &pdl);
+        }));
         phase_mark(PH_NEAR, false, s);
         phase_mark(PH_NEAR_CLOSE, true, s);
         TAGI_TRY(launch_persistent(near_group16<SS, 1>, wc, s, near_group16_smem(1), GT, &pdl));
@@ -2463,8 +2499,10 @@ int launch_fields(const SysCall *calls, const Fields *f, int nsys, const Schedul
     if (precision == PREC_MIXED && KERN == KERNEL_YUKAWA && sh.og > 1) {
         // orbital groups share the geometry of each pair across og orbitals
         const bool g8 = sh.og == 8;
-        if (g8) TAGI_TRY(launch_persistent(near_group<SS, 8, 0>, wn, s, 0, GT, &pdl));
-        else TAGI_TRY(launch_persistent(near_group<SS, 4, 0>, wn, s, 0, GT, &pdl));
+        TAGI_TRY(near_call(sh, [&](auto wide) {
+            if (g8) return launch_persistent(near_group<SS, 8, 0, wide()>, wn, s, 0, GT, &pdl);
+            return launch_persistent(near_group<SS, 4, 0, wide()>, wn, s, 0, GT, &pdl);
+        }));
         phase_mark(PH_NEAR, false, s);
         phase_mark(PH_NEAR_CLOSE, true, s);
         if (g8) TAGI_TRY(launch_persistent(near_group<SS, 8, 1>, wc, s, 0, GT, &pdl));
@@ -2895,6 +2933,7 @@ static int convolve_with(SysCall *calls, int nsys, int kernel, int singularity, 
         if (!mixed && p.nslots && !p.what64) return set_error(TAGI_ERR_DEVICE, "FP64 weight charges missing");
         f[i] = make_fields(p, c.norb);
         plans[i] = c.p;
+        sh.wide = sh.wide || p.wide;
         if (p.n1 > sh.maxn1) sh.maxn1 = p.n1;
         if (p.n1 < sh.minn1) sh.minn1 = p.n1;
     }

@@ -107,6 +107,7 @@ __device__ __forceinline__ void chain_begin() {
 __host__ __device__ __forceinline__ int range_begin(int2 r) { return r.x & 0x7fffffff; }
 __host__ __device__ __forceinline__ bool range_is_close(int2 r) { return r.x < 0; }
 constexpr double CLOSE_RANGE_FRACTION = 0.1;
+constexpr double WIDE_GAP = 1.0 / 65536;   // of a batch center's largest coordinate (Plan::wide)
 
 // Optional per-phase timing with CUDA events on the launching stream
 // (tagi_profile / tagi_profile_read); no-ops unless enabled.
@@ -244,6 +245,11 @@ struct Plan {
     std::vector<double> h_kp, h_ss;
     std::vector<void *> scratch;           // freed on regrow / destroy
     // statistics (host)
+    // Some batch center lies so far from the origin that the sources' FP32 hi/lo splits, whose error
+    // is 2^-49 |c|, could add more than 2^-8 to the rounding of a relative coordinate in an ordinary
+    // near range: one nearer to its batch than WIDE_GAP |c|.  Meshes around the origin have none (|c|
+    // is some hundred batch radii, an ordinary range a tenth of one or more away).
+    bool wide = false;
     double near_pairs = 0, far_pairs = 0;  // pair interactions per orbital
     double near_close_pairs = 0;           // part of near_pairs in close ranges
     // per-batch pair counts (host) for work ordering: ordinary near ranges,

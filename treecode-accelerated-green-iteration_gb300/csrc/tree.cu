@@ -736,7 +736,8 @@ __device__ __forceinline__ double box_gap(const double *cb, const double *hb, co
 // Close ranges are stored with bit 31 of their begin set (range_is_close).
 // rng_dmin = smallest node gap of the range, rounded down: a lower bound of
 // every pair distance in it.  One warp per batch, 32 entries at a time; the fill
-// also writes the batch's pair counts: near, far (clusters), size, close.
+// also writes the batch's pair counts: near, close, far (clusters), and its size with bit 32 set if an
+// ordinary range is too near for its distance from the origin (Plan::wide).
 template <bool FILL>
 __global__ void __launch_bounds__(256) merge_ranges(int nbatch, const int *__restrict__ near_off,
                                                     const int *__restrict__ near_list, const int *__restrict__ sbegin,
@@ -755,6 +756,8 @@ __global__ void __launch_bounds__(256) merge_ranges(int nbatch, const int *__res
     const double cb[3] = {tcenter[3L * bn], tcenter[3L * bn + 1], tcenter[3L * bn + 2]};
     const double hb[3] = {thalf[3L * bn], thalf[3L * bn + 1], thalf[3L * bn + 2]};
     const double close_gap = CLOSE_RANGE_FRACTION * tradius[bn];
+    const double wide_gap = WIDE_GAP * dmax(dmax(fabs(cb[0]), fabs(cb[1])), fabs(cb[2]));
+    bool wide = false;
     const int e0 = near_off[b], e1 = near_off[b + 1];
     int k = 0, prev_end = -1, prev_close = 0;   // ranges begun; the last entry's end and class
     double carry = INFINITY;                    // smallest gap of the range in progress
@@ -774,6 +777,7 @@ __global__ void __launch_bounds__(256) merge_ranges(int nbatch, const int *__res
             nclose = gap <= close_gap;
             all += ne - nb;
             if (nclose) close_all += ne - nb;
+            else wide = wide || !(gap >= wide_gap);
         }
         int pe = __shfl_up_sync(0xffffffffu, ne, 1), pc = __shfl_up_sync(0xffffffffu, nclose, 1);
         if (lane == 0) {
@@ -807,6 +811,7 @@ __global__ void __launch_bounds__(256) merge_ranges(int nbatch, const int *__res
         k += __popc(m);
     }
     if constexpr (FILL) {
+        const bool any_wide = __any_sync(0xffffffffu, wide);
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
             all += __shfl_xor_sync(0xffffffffu, all, o);
@@ -817,7 +822,7 @@ __global__ void __launch_bounds__(256) merge_ranges(int nbatch, const int *__res
             costs[4L * b] = nt * all;
             costs[4L * b + 1] = nt * close_all;
             costs[4L * b + 2] = nt * (long long)(far_off[b + 1] - far_off[b]);
-            costs[4L * b + 3] = nt;
+            costs[4L * b + 3] = nt | (long long)any_wide << 32;
         }
     } else if (lane == 0) {
         cnt[b] = k;
@@ -1001,7 +1006,8 @@ int build_lists(Plan &p, cudaStream_t s) {
             p.near_pairs += (double)c[0];
             p.near_close_pairs += (double)c[1];
             p.far_pairs += (double)c[2] * p.P;
-            p.batch_size[b] = (int)c[3];
+            p.batch_size[b] = (int)(c[3] & 0xffffffffLL);
+            p.wide = p.wide || c[3] >> 32;
             p.max_batch = std::max(p.max_batch, p.batch_size[b]);
             p.cost_near[b] = c[0] - c[1];
             p.cost_close[b] = c[1];
