@@ -1770,13 +1770,15 @@ __global__ void __launch_bounds__(GT, 4) far_group16(const __grid_constant__ Wor
 //   * 2^{-t/EXP_N} with t = K r, K = k EXP_N / ln 2 in two doubles: n = rint(t)
 //     from FP32, the remainder f = n - t by fused multiply-adds on z and z d (r
 //     itself is not rounded), and a table of 2^{i/EXP_N}, i < EXP_N, times a cubic
-//     in f, |f| < 0.6 (table lookup and short polynomial: P. T. P. Tang, ACM TOMS
-//     15, 1989); the cubic's upper terms are below 2^-30 and go to FP32;
+//     in f (table lookup and short polynomial: P. T. P. Tang, ACM TOMS 15, 1989), whose upper
+//     terms go to FP32.  t's FP32 error grows with it: |f| < 0.56 up to kr = 16, 0.7 at 50, 1.9
+//     at 300, 3.7 at 707, where the upper terms are 2^-24 and FP32 leaves 26 units of 2^-53;
 //   * conversions between FP32 and FP64 are shifts of the bit patterns.
-// Against 128-bit arithmetic e^{-kr}/r is off by 0.45 ulp rms at kr <= 1 and 1.2
-// at kr <= 16 (sqrt, exp and a division: 0.45 and 2.8).  A squared distance
-// outside FP32's range (zero: a coincident pair; NaN) takes the library
-// functions; e^{-kr} below 2^-1021 counts as 0.
+// Against 128-bit arithmetic (estimates of 1/r up to 2 FP32 ulp off) e^{-kr}/r has an rms error of
+// 0.83, 1.8, 6.9, 47, 128 units of 2^-53 for kr up to 1, 16, 50, 300, 707; sqrt, exp and a division
+// have 0.62, 3.1, 14, 98, 280, and one more rounding in the sum.  A squared distance
+// outside FP32's range (zero: a coincident pair; NaN) and an exponential that is a
+// subnormal number (EXP_LIMIT) take the library functions.
 // Near field, 50k points, split 8: 167 -> 79 ms; the whole one-shot call 177 -> 84 ms.
 // ---------------------------------------------------------------------------
 constexpr int EXP_BITS = 13, EXP_N = 1 << EXP_BITS;
@@ -1854,20 +1856,21 @@ __device__ __forceinline__ InvRoot inv_root(double r2) {
     return q;
 }
 
-constexpr float EXP_LIMIT = 1021.f * EXP_N;
+// t from which the exponential is not a normal number (pair_f64_any then), and from which it is 0
+// to the last bit.
+constexpr float EXP_LIMIT = 1021.f * EXP_N, EXP_NONE = 1080.f * EXP_N;
 // 2^{(n - t)/EXP_N} 2^{-n/EXP_N}: tf = t in FP32; the caller forms f = n - t from nd = n.
 __device__ __forceinline__ double exp_n(float tf, int &n) {
-    n = __float2int_rn(fminf(tf, EXP_LIMIT));
+    n = __float2int_rn(tf);
     return bits_f2d((float)n);
 }
-__device__ __forceinline__ double exp_finish(double f, int n, float tf, const double *__restrict__ tab) {
+__device__ __forceinline__ double exp_finish(double f, int n, const double *__restrict__ tab) {
     constexpr double C1 = 0x1.62e42fefa39efp-14;                       // ln 2 / EXP_N
     constexpr float C2 = 0x1.ebfbdff82c58fp-29, C3 = 0x1.c6b08d704a0c0p-44;   // C1^2 / 2, C1^3 / 6
     const double q = __fma_rn(f, bits_f2d(__fmaf_rn(bits_d2f(f), C3, C2)), C1);
     const double t = tab[-n & (EXP_N - 1)];
     const double ts = __hiloint2double(__double2hiint(t) + (((-n) >> EXP_BITS) << 20), __double2loint(t));
-    const double v = __fma_rn(ts, __dmul_rn(f, q), ts);
-    return tf < EXP_LIMIT ? v : 0.0;
+    return __fma_rn(ts, __dmul_rn(f, q), ts);
 }
 // e^{-k r}
 __device__ __forceinline__ double exp_root(const InvRoot &q, const ExpScale &s, const double *__restrict__ tab) {
@@ -1876,7 +1879,7 @@ __device__ __forceinline__ double exp_root(const InvRoot &q, const ExpScale &s, 
     double f = __fma_rn(-s.kh, q.z, exp_n(tf, n));
     f = __fma_rn(-s.kh, __dmul_rn(q.z, q.d), f);
     f = __fma_rn(-s.kl, q.z, f);
-    return exp_finish(f, n, tf, tab);
+    return exp_finish(f, n, tab);
 }
 // e^{-a^2 x}
 __device__ __forceinline__ double exp_square(double x, const ExpScale &s, const double *__restrict__ tab) {
@@ -1884,27 +1887,32 @@ __device__ __forceinline__ double exp_square(double x, const ExpScale &s, const 
     int n;
     double f = __fma_rn(-s.kh, x, exp_n(tf, n));
     f = __fma_rn(-s.kl, x, f);
-    return exp_finish(f, n, tf, tab);
+    return exp_finish(f, n, tab);
 }
 
-// One pair with the library's functions: r2 outside FP32's range.  q and w are the
-// charge f w and the weight; the near field passes f and w (near: true).
+// One pair with the library's functions: r2 outside FP32's range, or t = tf from EXP_LIMIT on.  q and w
+// are the charge f w and the weight; the near field passes f and w (near: true).
 template <int KERN, bool SS, bool NEAR>
-__device__ __noinline__ double pair_f64_any(double r2, double q, double w, double fi, double kp) {
+__device__ __noinline__ double pair_f64_any(double r2, float tf, double q, double w, double fi, double kp) {
     if (NEAR && !(r2 > 0.0)) return 0.0;
+    const bool none = tf >= EXP_NONE && in_fp32_range(r2);   // no exponential to form
     const double r = sqrt(r2);
     if (KERN == KERNEL_YUKAWA) {
-        const double g = exp(-kp * r) / r;
+        const double g = none ? 0.0 : exp(-kp * r) / r;
         return SS ? (NEAR ? w * (q - fi) : q - fi * w) * g : q * g;
     }
-    if (SS) return (NEAR ? w * (q - fi * exp(-kp * kp * r2)) : q - fi * w * exp(-kp * kp * r2)) / r;
+    if (SS) {
+        const double e = none ? 0.0 : exp(-kp * kp * r2);
+        return (NEAR ? w * (q - fi * e) : q - fi * w * e) / r;
+    }
     return q / r;
 }
 template <int KERN, bool SS, bool NEAR>
 __device__ __forceinline__ double pair_f64(double r2, double q, double w, double fi, double kp, const ExpScale &es,
                                            const double *__restrict__ tab, double acc) {
-    if (!in_fp32_range(r2)) return acc + pair_f64_any<KERN, SS, NEAR>(r2, q, w, fi, kp);
     const InvRoot v = inv_root(r2);
+    const float tf = KERN == KERNEL_YUKAWA ? v.zf * es.kf : (SS ? bits_d2f(r2) * es.kf : 0.f);
+    if (!in_fp32_range(r2) || tf >= EXP_LIMIT) return acc + pair_f64_any<KERN, SS, NEAR>(r2, tf, q, w, fi, kp);
     const double rinv = __fma_rn(v.y, v.d, v.y);
     if (KERN == KERNEL_YUKAWA) {
         const double c = SS ? (NEAR ? w * (q - fi) : __fma_rn(-fi, w, q)) : q;
