@@ -68,12 +68,19 @@ __device__ __forceinline__ void add(Sum3 &a, float2 v) {
     a.lo = __fadd2_rn(a.lo, two_sum(a.mid, two_sum(a.hi, v)));
 }
 
-// Barycentric basis values of coordinate src in the slot's box along one axis, into
-// L[0..n1-1].
+// a / h from inv = 1 / h: the product corrected by its exact remainder, which gives the rounded
+// quotient (P. W. Markstein, IBM J. Res. Dev. 34, 1990).  The product alone can fall on the other
+// side of a tie when it is rounded to FP32.
+__device__ __forceinline__ double quotient(double a, double h, double inv) {
+    if (!(h > 1e-290 && h < 1e290)) return a / h;
+    const double q = __dmul_rn(a, inv);
+    return __fma_rn(__fma_rn(-q, h, a), inv, q);
+}
+
+// Barycentric basis values of the coordinate that lies at u in the slot's box ([-1, 1]) along one
+// axis, into L[0..n1-1].
 template <typename T>
-__device__ __forceinline__ void basis(double src, double c, double h, const T *tn, int n1, T *L) {
-    // FP32 basis: the FP64 quotient is only rounded to FP32, so a product serves
-    const T u = sizeof(T) == 4 ? (T)((src - c) * h) : (T)((src - c) / h);
+__device__ __forceinline__ void basis(T u, const T *tn, int n1, T *L) {
     int exact = -1;
     for (int m = 0; m < n1; m++)
         if (u - tn[m] == T(0)) exact = m;
@@ -111,7 +118,7 @@ __global__ void __launch_bounds__(P2M_THREADS) p2m_mixed(const __grid_constant__
     const double *gm = a.geom + 6L * a.item_slot[item];
     const int axis = tid % 3;   // thread 3 p + d does source p along axis d
     const double *xs = axis == 0 ? a.xs : (axis == 1 ? a.ys : a.zs);
-    const double center = gm[axis], inv = 1.0 / gm[3 + axis];
+    const double center = gm[axis], width = gm[3 + axis], inv = 1.0 / width;
     Sum3 acc[OB][MH];
 #pragma unroll
     for (int o = 0; o < OB; o++)
@@ -122,7 +129,7 @@ __global__ void __launch_bounds__(P2M_THREADS) p2m_mixed(const __grid_constant__
         __syncthreads();   // the previous tile is no longer read
         if (tid < 3 * cnt) {
             float *L = sL[axis][tid / 3];
-            basis<float>(xs[t0 + tid / 3], center, inv, a.tn, n1, L);
+            basis<float>((float)quotient(xs[t0 + tid / 3] - center, width, inv), a.tn, n1, L);
             if (n1 & 1) L[n1] = 0.f;   // the second lane of the last pair
         }
         for (int k = tid; k < OB * P2M_TILE; k += P2M_THREADS) {
@@ -199,7 +206,7 @@ __global__ void __launch_bounds__(P2M_THREADS) p2m_f64(const __grid_constant__ P
         if (tid < 3 * cnt) {
             const int p = tid / 3, d = tid - 3 * (tid / 3);
             const double *src = d == 0 ? a.xs : (d == 1 ? a.ys : a.zs);
-            basis<double>(src[t0 + p], gm[d], gm[3 + d], a.tn, n1, sL[d][p]);
+            basis<double>((src[t0 + p] - gm[d]) / gm[3 + d], a.tn, n1, sL[d][p]);
         }
         if (tid < cnt) sq[tid] = q[t0 + tid];
         __syncthreads();
