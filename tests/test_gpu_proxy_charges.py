@@ -36,3 +36,18 @@ def test_coordinates_are_rounded_quotients(dev):
         got = plan.charges(3)[0, 0].astype(np.float32)
         plan.close()
         assert np.array_equal(got, ref), (h, t, got, ref)
+
+
+@pytest.mark.parametrize("norb", [1, 3])
+@pytest.mark.parametrize("big", [np.inf, -np.inf, 3e38])
+def test_infinite_sums_stay_infinite(BT, dev, norb, big):
+    """One infinite charge, or finite ones whose sum is beyond FP32, among positive basis values."""
+    n = 70
+    x = np.linspace(-1.0, 1.0, n) + 1e-3      # no source on a node but the outermost two
+    plan = far_plan(dev, x, np.ones(n))
+    f = np.full((norb, n), 1.0 if np.isinf(big) else big)
+    f[:, 0] = f[:, -1] = 1.0
+    f[:, 31] = big
+    plan.convolve(*to_cuda(np.zeros((norb, 1)), f), BT.Kernel.COULOMB, [1.0], BT.Singularity.SKIPPING, precision="mixed")
+    assert np.array_equal(plan.charges(2, norb)[:, 0], np.full((norb, 8), np.copysign(np.inf, big)))
+    plan.close()

@@ -67,6 +67,10 @@ __device__ __forceinline__ float2 two_sum(float2 &s, float2 v) {   // s += v; re
 __device__ __forceinline__ void add(Sum3 &a, float2 v) {
     a.lo = __fadd2_rn(a.lo, two_sum(a.mid, two_sum(a.hi, v)));
 }
+// The words' sum.  An infinite first word has NaN errors: it is the sum, as in FP64.
+__device__ __forceinline__ double total(float hi, float mid, float lo) {
+    return fabsf(hi) < INFINITY ? (double)hi + ((double)mid + (double)lo) : (double)hi;
+}
 
 // a / h from inv = 1 / h: the product corrected by its exact remainder, which gives the rounded
 // quotient (P. W. Markstein, IBM J. Res. Dev. 34, 1990).  The product alone can fall on the other
@@ -100,8 +104,10 @@ __device__ __forceinline__ void basis(T u, const T *tn, int n1, T *L) {
 // Mixed: OB orbitals of one item.  Thread (g, k1, k2) sums the sources g, g + G, ...
 // of each tile for its row of the grid.
 constexpr int P2M_OB = 3;   // upward pass of 32 orbitals x 1M points at 2, 3, 4: 18.3, 14.8, 25.0 ms (registers)
+// Resident CTAs per SM: one orbital needs few registers, and 50k points are 6 us quicker with four CTAs
+// than with three.
 template <int MAXN1, int OB>
-__global__ void __launch_bounds__(P2M_THREADS) p2m_mixed(const __grid_constant__ P2MArgs<float> a) {
+__global__ void __launch_bounds__(P2M_THREADS, OB > 1 ? 2 : (MAXN1 <= 8 ? 4 : 3)) p2m_mixed(const __grid_constant__ P2MArgs<float> a) {
     constexpr int MH = (MAXN1 + 1) / 2, LP = 2 * MH;
     extern __shared__ double red[];  // [G][P]
     __shared__ __align__(8) float sL[3][P2M_TILE][LP];
@@ -165,8 +171,8 @@ __global__ void __launch_bounds__(P2M_THREADS) p2m_mixed(const __grid_constant__
 #pragma unroll
             for (int m = 0; m < MH; m++) {
                 const Sum3 &v = acc[o][m];
-                if (2 * m < n1) r[2 * m] = (double)v.hi.x + ((double)v.mid.x + (double)v.lo.x);
-                if (2 * m + 1 < n1) r[2 * m + 1] = (double)v.hi.y + ((double)v.mid.y + (double)v.lo.y);
+                if (2 * m < n1) r[2 * m] = total(v.hi.x, v.mid.x, v.lo.x);
+                if (2 * m + 1 < n1) r[2 * m + 1] = total(v.hi.y, v.mid.y, v.lo.y);
             }
         }
         __syncthreads();
