@@ -336,6 +336,12 @@ int tagi_mlp_gemm_splitk(const void *A, long long sAm, long long sAk, const void
 /* Rows (orbital, cell) of features [psi/s_psi, d/s_d, eps, 0...] (bf16, row
  * stride ldx >= 2P+1), the patch scales s_d (floored by dfloor[orbital]) and
  * d/s_d in f32.  The mesh stores each cell's P points contiguously. */
+/* Waits for the stream and says whether a GEMM on this device gave up a wait inside its
+ * pipeline since the last check (its tile of the result is NaN then): TAGI_ERR_DEVICE, and the
+ * mark is cleared.  Such waits end after a bounded number of tries.
+ * tagi_mlp_wait_probe makes one run out after `tries`, for tests of this path. */
+int tagi_mlp_check(void *stream);
+int tagi_mlp_wait_probe(int tries, void *stream);
 int tagi_mlp_patch_features(const double *psi, const double *d, const double *eps,
                             const double *dfloor, int numOrbitals, int numCells, int P,
                             long long numPoints, int ldx, void *X, float *scale, float *dn,

@@ -64,6 +64,8 @@ SIGNATURES = {
                            _i, _i, _i, _i, _vp, _vp, ctypes.c_longlong, _vp, _vp, _vp]),
     "tagi_mlp_gemm_splitk": (_i, [_vp, ctypes.c_longlong, ctypes.c_longlong, _vp, ctypes.c_longlong,
                                   ctypes.c_longlong, _i, _i, _i, _i, _vp, _vp, _vp]),
+    "tagi_mlp_check": (_i, [_vp]),
+    "tagi_mlp_wait_probe": (_i, [_i, _vp]),
     "tagi_mlp_patch_features": (_i, [_vp, _vp, _vp, _vp, _i, _i, _i, ctypes.c_longlong, _i, _vp, _vp, _vp, _vp]),
     "tagi_mlp_patch_target": (_i, [_vp, _vp, _i, _i, _i, ctypes.c_longlong, _vp, _vp]),
     "tagi_mlp_mse_grad": (_i, [_vp, _vp, _vp, _vp, _i, _i, _vp, _vp, _vp, _vp, _vp]),

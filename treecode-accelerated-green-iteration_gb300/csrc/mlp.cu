@@ -78,7 +78,9 @@ __host__ __device__ constexpr size_t tc_smem(int stages) { return 1024 + (size_t
 static_assert(tc_smem(3) * 5 > 228 * 1024, "at most four blocks of 128 TMEM columns each may share an SM");
 static_assert((size_t)TC_M * TC_PITCH * 4 <= (size_t)3 * 2 * TC_TILE, "C tile in the ring's memory");
 static_assert(tc_smem(6) <= 227 * 1024, "one block's shared memory");
-constexpr int TC_SPINS = 1 << 20;                       // tries of a barrier wait before it gives up
+// Tries of a barrier wait before it gives up, 3.8 us each where nothing comes: one second; a sixteenth for
+// each stage's copies after a wait gave up.
+constexpr int TC_SPINS = 1 << 18, TC_DRAIN = TC_SPINS / 16;
 
 __device__ __forceinline__ unsigned smem_u32(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void mbar_init(uint64_t *b, unsigned n) {
@@ -87,9 +89,9 @@ __device__ __forceinline__ void mbar_init(uint64_t *b, unsigned n) {
 __device__ __forceinline__ void mbar_expect(uint64_t *b, unsigned bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(b)), "r"(bytes) : "memory");
 }
-// false if the phase did not complete within TC_SPINS tries
-__device__ __forceinline__ bool mbar_wait(uint64_t *b, unsigned parity) {
-    for (int i = 0; i < TC_SPINS; i++) {
+// false if the phase did not complete within `tries` tries
+__device__ __forceinline__ bool mbar_wait(uint64_t *b, unsigned parity, int tries = TC_SPINS) {
+    for (int i = 0; i < tries; i++) {
         unsigned ok;
         asm volatile(
             "{\n.reg .pred p;\n"
@@ -122,7 +124,16 @@ struct TcArgs {
     int a_kmajor, b_kmajor;
 };
 
-__device__ int g_tc_timeout;   // set by a CTA whose barrier wait gave up (its tile of C is NaN)
+__device__ int g_tc_timeout;   // set by a CTA whose barrier wait gave up (its tile of C is NaN); tagi_mlp_check
+
+__global__ void take_timeout(int *out) { *out = atomicExch(&g_tc_timeout, 0); }
+
+// A wait that nothing ends, as in gemm_tc.
+__global__ void wait_probe(int tries) {
+    __shared__ __align__(8) uint64_t bar;
+    mbar_init(&bar, 1);
+    if (!mbar_wait(&bar, 0, tries)) g_tc_timeout = 1;
+}
 
 // Rows of 64 consecutive k (K-major) or of 64 m of one k (MN-major) starting at row
 // `first` of a tile, `step` rows apart: the pair of elements at 2 lane, packed.
@@ -265,14 +276,14 @@ __global__ void __launch_bounds__(TC_THREADS + (SA || SB ? TC_LOADERS : 0), STAG
         }
     }
     __syncwarp();
-    bool ok = mbar_wait(&s_done, 0);
+    bool ok = mbar_wait(&s_done, 0, TC_SPINS + steps);   // the whole K loop
     __syncthreads();
     ok = ok && !s_fail;
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     if (!ok) {   // give the copies in flight time to land before the memory is reused or left
         if (tid == 0) {
             g_tc_timeout = 1;
-            for (int st = 0; st < STAGES; st++) mbar_wait(&s_full[st], 0), mbar_wait(&s_full[st], 1);
+            for (int st = 0; st < STAGES; st++) mbar_wait(&s_full[st], 0, TC_DRAIN), mbar_wait(&s_full[st], 1, TC_DRAIN);
         }
         __syncthreads();
     }
@@ -732,6 +743,28 @@ int tagi_mlp_gemm_splitk(const void *A, long long sAm, long long sAk, const void
     TAGI_TRY(run_gemm(g, splits, &splits, s));
     const long mn = (long)M * N;
     TAGI_CUDA(launch_chained(splitk_reduce, (unsigned)((mn + 255) / 256), 256, 0, s, partial, splits, mn, C));
+    TAGI_LAUNCH_CHECK();
+    return TAGI_OK;
+}
+
+int tagi_mlp_check(void *stream) {
+    cudaStream_t s = (cudaStream_t)stream;
+    Arena tmp;
+    tmp.stream = s;
+    int *flag = nullptr, h = 0;
+    TAGI_TRY(tmp.alloc(&flag, 1));
+    launch(take_timeout, 1, 1, 0, s, flag);
+    const cudaError_t e = cudaMemcpyAsync(&h, flag, sizeof(int), cudaMemcpyDeviceToHost, s);
+    tmp.release();
+    if (e != cudaSuccess || cudaStreamSynchronize(s) != cudaSuccess)
+        return set_error(TAGI_ERR_CUDA, "GEMM status: %s", cudaGetErrorString(cudaGetLastError()));
+    if (h) return set_error(TAGI_ERR_DEVICE, "a GEMM's barrier wait ran out: its tile of the result is NaN");
+    return TAGI_OK;
+}
+
+int tagi_mlp_wait_probe(int tries, void *stream) {
+    if (tries < 0 || tries > TC_SPINS) return set_error(TAGI_ERR_ARG, "%d tries outside [0, %d]", tries, TC_SPINS);
+    launch(wait_probe, 1, 1, 0, (cudaStream_t)stream, tries);
     TAGI_LAUNCH_CHECK();
     return TAGI_OK;
 }

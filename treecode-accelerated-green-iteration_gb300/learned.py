@@ -125,6 +125,11 @@ class MLP:
         _native.check(L.tagi_mlp_colsum(_p(self.dH1), 1, rows, H, _p(g["b1"]), _p(self.cwork), cw, s))
         return self._lossbuf[0]
 
+    def check(self):
+        """Wait for the stream; TagiError if a GEMM gave up a wait since the last check (NaN results
+        that no input explains)."""
+        _native.check(_native.lib().tagi_mlp_check(self._s()))
+
     def adam_step(self, beta1=0.9, beta2=0.999, eps=1e-8):
         self.t += 1
         L, s = _native.lib(), self._s()
@@ -320,5 +325,5 @@ class LearnedExtrapolator:
                     self._propose(gi)
             if self.cool > 0:
                 self.cool -= 1
-            gi.stream.synchronize()
+            self.net.check()   # waits for the stream
         return res
