@@ -76,6 +76,16 @@ cudaMemPool_t pool_of(int dev) {
 }
 }  // namespace
 
+cudaError_t device_malloc(void **p, size_t bytes) {
+    cudaError_t e = cudaMalloc(p, bytes);
+    int dev = -1;
+    if (e != cudaErrorMemoryAllocation || cudaGetDevice(&dev) != cudaSuccess) return e;
+    cudaGetLastError();
+    cudaMemPool_t pool = pool_of(dev);
+    if (!pool || cudaDeviceSynchronize() != cudaSuccess || cudaMemPoolTrimTo(pool, 0) != cudaSuccess) return e;
+    return cudaMalloc(p, bytes);
+}
+
 // Under stream capture the allocation becomes a node of the caller's graph, which
 // the default pool's call does.
 cudaError_t pool_alloc(void **p, size_t bytes, cudaStream_t s) {

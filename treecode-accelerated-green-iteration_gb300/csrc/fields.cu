@@ -2694,7 +2694,7 @@ int ensure_scratch(Plan &p, int norb, int precision) {
         for (void *v : p.scratch) cudaFree(v);
         p.scratch.clear();
         p.scratch_orbitals = 0;
-        const cudaError_t e = cudaMalloc(reinterpret_cast<void **>(&block), bytes);
+        const cudaError_t e = device_malloc(reinterpret_cast<void **>(&block), bytes);
         if (e != cudaSuccess)
             return set_error(TAGI_ERR_CUDA, "device allocation of %zu bytes failed: %s", bytes, cudaGetErrorString(e));
         p.scratch.push_back(block);
@@ -2866,7 +2866,7 @@ int build_schedule(Plan *const *plans, const int *norb, int nsys, int og, int nt
         TAGI_CUDA(cudaDeviceSynchronize());
         sc.release();
         void *v = nullptr;
-        TAGI_CUDA(cudaMalloc(&v, sizeof(int4) * all.size()));
+        TAGI_CUDA(device_malloc(&v, sizeof(int4) * all.size()));
         sc.items = static_cast<int4 *>(v);
     }
     // pageable source: the copy has read it when the call returns

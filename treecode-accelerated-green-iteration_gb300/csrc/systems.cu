@@ -128,7 +128,7 @@ int tagi_systems_create(tagi_systems **systems, int numSystems, tagi_plan *const
                             y->stream);
     if (!rc) {
         void *v = nullptr;
-        if (cudaMalloc(&v, 3 * sizeof(int)) != cudaSuccess)
+        if (device_malloc(&v, 3 * sizeof(int)) != cudaSuccess)
             rc = set_error(TAGI_ERR_CUDA, "work counter allocation failed");
         y->queue = static_cast<int *>(v);
     }

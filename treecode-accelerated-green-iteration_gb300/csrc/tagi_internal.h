@@ -121,6 +121,8 @@ void phase_mark(int phase, bool begin, cudaStream_t s);
 // calls (0.4% of this GPU's memory); tagi_release_memory gives those back too.
 constexpr unsigned long long POOL_KEEP = 1ULL << 30;
 cudaError_t pool_alloc(void **p, size_t bytes, cudaStream_t s);
+// cudaMalloc for memory that is valid on every stream; what the pool keeps unused makes room for it.
+cudaError_t device_malloc(void **p, size_t bytes);
 
 // Stream-ordered device allocations owned by a plan (freed on destroy).
 struct Arena {

@@ -332,7 +332,7 @@ int ensure_weight_charges64(Plan &p, cudaStream_t s) {
         const size_t count = (size_t)p.nslots * p.P + 1;
         // plain cudaMalloc: the first FP64 call may run on another stream than the plan's
         void *v = nullptr;
-        TAGI_CUDA(cudaMalloc(&v, sizeof(double) * count));
+        TAGI_CUDA(device_malloc(&v, sizeof(double) * count));
         p.arena.ptrs.push_back(v);
         p.what64 = static_cast<double *>(v);
     }

@@ -187,6 +187,12 @@ def treecode(tx, ty, tz, tv, sx, sy, sz, sv, sw, kernel, kernel_params, singular
     return out
 
 
+def release_memory():
+    """Give the device memory that the library keeps between calls (at most 1 GiB on the current
+    device, tagi_release_memory) back to the driver; later calls take it anew."""
+    _native.check(_native.lib().tagi_release_memory())
+
+
 def direct(tx, ty, tz, tv, sx, sy, sz, sv, sw, kernel, kernel_params, singularity, subset=None,
            stream=None):
     """Exact FP64 direct sum at the targets in ``subset`` (int32 CUDA tensor) or all."""
