@@ -115,6 +115,7 @@ def refine_cells(base, atoms, order, h, H, r, level, min_depth=0, max_depth=16, 
         rc = L.tagi_mesh_refine(*args, *outs, room, ctypes.byref(ncell), ctypes.byref(ncp), ctypes.byref(nfp), s)
         n = ncell.value
         if rc and n > room:
+            L.tagi_clear_error()   # the count is the answer; the next call fills the table
             room = n
             continue
         _native.check(rc)
