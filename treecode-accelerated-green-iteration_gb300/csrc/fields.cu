@@ -70,10 +70,9 @@ __device__ __forceinline__ float lg2_mufu(float x) {
 struct Fields {
     // target side (sorted order)
     const double *tx, *ty, *tz;
-    const int *tbegin, *tend;
     const double *tcenter, *tradius;
     const int *batch_node;
-    int nbatch, nt, norb;
+    int nt, norb;
     // near side
     const int *rng_off;
     const int2 *rng;
@@ -2602,12 +2601,9 @@ Fields make_fields(const Plan &p, int norb) {
     a.tx = p.tgt.x;
     a.ty = p.tgt.y;
     a.tz = p.tgt.z;
-    a.tbegin = p.tgt.begin;
-    a.tend = p.tgt.end;
     a.tcenter = p.tgt.center;
     a.tradius = p.tgt.radius;
     a.batch_node = p.batch_node;
-    a.nbatch = p.nbatch;
     a.nt = p.tgt.n;
     a.norb = norb;
     a.rng_off = p.rng_off;

@@ -480,7 +480,7 @@ int tagi_mesh_refine(const double *baseCells, int numBase, const double *atomXYZ
                     const int from = depth & 1, to = from ^ 1;
                     // a level holds at most 8 times the cells of the one before
                     const long most = std::min(level_cap, depth < 10 ? (long)numBase << (3 * depth) : level_cap);
-                    const int grid = (int)std::min(152L * 8, (most * CELL_LANES + LEVEL_THREADS - 1) / LEVEL_THREADS);
+                    const int grid = (int)std::min(GPU_SMS * 8, (most * CELL_LANES + LEVEL_THREADS - 1) / LEVEL_THREADS);
                     if (launch_chained(mesh_level, grid, LEVEL_THREADS, 0, s, depth ? cells[from] : baseCells,
                                        depth ? keys[from] : (const uint64_t *)nullptr, depth, atomXYZ, numAtoms, p, prog,
                                        cells[to], keys[to], (int)level_cap, leaf_cells, leaf_keys, leaf_fine,
@@ -578,7 +578,7 @@ int tagi_mesh_points(const double *cellX, const double *cellY, const double *cel
     const unsigned m2 = p2 > 1 ? (unsigned)((0x100000000ULL + p2 - 1) / p2) : 0u;
     auto warp_grid = [](long nsubcells) {
         long g = (nsubcells + PW - 1) / PW;
-        return (int)(g < 1 ? 1 : (g > 152L * 32 ? 152L * 32 : g));
+        return (int)(g < 1 ? 1 : (g > GPU_SMS * 32 ? GPU_SMS * 32 : g));
     };
     launch(mesh_points_warp, warp_grid(numCells), PW * 32, 0, s, cellX, cellY, cellZ, cellDX, cellDY, cellDZ,
            (const int *)nullptr, (const int *)nullptr, numCells, (long)numCells, p1, m1, m2, t, X, Y, Z, W);

@@ -300,7 +300,7 @@ int radix_sort_u64(uint64_t *kin, int *vin, uint64_t *kout, int *vout, int n, in
         TAGI_TRY(ar.alloc(&rank, n));
         TAGI_CUDA(cudaMemsetAsync(rank, 0, sizeof(int) * n, s));
         const int bx = (n + CNT_THREADS - 1) / CNT_THREADS;
-        const int by = std::min(bx, (152 * 8 + bx - 1) / bx);   // about eight blocks per SM
+        const int by = std::min(bx, ((int)GPU_SMS * 8 + bx - 1) / bx);   // about eight blocks per SM
         const int span = (n + by - 1) / by;
         launch(count_smaller, dim3(bx, (n + span - 1) / span), CNT_THREADS, 0, s, kin, n, span, rank);
         TAGI_CUDA(launch_chained(place_sorted, bx, CNT_THREADS, 0, s, kin, vin, rank, n, kout, vout));

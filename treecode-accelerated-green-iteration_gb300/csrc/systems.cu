@@ -192,7 +192,7 @@ int tagi_systems_destroy(tagi_systems *systems) {
     if (!systems) return TAGI_OK;
     Systems *y = reinterpret_cast<Systems *>(systems);
     cudaDeviceSynchronize();
-    if (y->sched.items) cudaFree(y->sched.items);
+    y->sched.release();
     if (y->queue) cudaFree(y->queue);
     delete y;
     return TAGI_OK;

@@ -29,6 +29,7 @@ enum { APPROX_LAGRANGE = 1 };
 enum { COMPUTE_PARTICLE_CLUSTER = 1 };
 enum { PREC_MIXED = 0, PREC_FP64 = 1 };
 
+constexpr long GPU_SMS = 152;         // of a GB300: grids of kernels whose blocks take work in turns
 constexpr int MAX_DEGREE = 10;        // far-field kernels are instantiated for 1..10
 
 int set_error(int code, const char *fmt, ...);

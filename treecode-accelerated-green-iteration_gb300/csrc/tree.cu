@@ -557,7 +557,7 @@ int build_tree(TreeBuild &w, Tree &t, const double *x, const double *y, const do
             rc = set_error(TAGI_ERR_CUDA, "tree memset failed");
             break;
         }
-        const unsigned bw = (unsigned)std::min(152L * 16, nodes), bt = (unsigned)std::min(152L * 8, (nodes + 127) / 128);
+        const unsigned bw = (unsigned)std::min(GPU_SMS * 16, nodes), bt = (unsigned)std::min(GPU_SMS * 8, (nodes + 127) / 128);
         if (launch_chained(node_boxes, bw, BOX_THREADS, 0, s, hdr, t.begin, t.end, t.parent, t.first_child, t.nchild, t.x,
                            t.y, t.z, box, size, leaves, done) != cudaSuccess ||
             launch_chained(preorder, bt, 128, 0, s, hdr, t.begin, t.end, t.parent, t.first_child, t.nchild, box, t.center,
