@@ -11,8 +11,8 @@
 //  * first-kind weights (-1)^i sin((2i+1) pi / (2p+2))                 :49-51
 //  * exact-node guard |t - node| < DBL_MIN; as in the reference, the x and z
 //    exact-node tests compare against the z and x loop indices (:127,:139)
-// One CTA per interpolated cell, coarse values staged in shared memory; fine
-// points on tensor grids (the mesh builders' layout) take a sum-factorised
+// Two to eight CTAs per cell share its children, each with the coarse values in shared
+// memory; fine points on tensor grids (the mesh builders' layout) take a sum-factorised
 // path, any other point the reference's per-point formula (see interp_cells).
 #include "tagi_internal.h"
 
@@ -75,8 +75,8 @@ __device__ __noinline__ double interp_point(double tx, double ty, double tz, con
     return temp * den;
 }
 
-// One CTA per interpolated cell.  A cell's fine points come in blocks of
-// (p+1)^3 (one block per child cell).  When a block is a tensor grid in
+// Two to eight CTAs per cell.  A cell's fine points come in blocks of (p+1)^3 (one block
+// per child cell), each CTA's following one another.  When a block is a tensor grid in
 // x-major order (x depends on the block index i only, y on j, z on k -- the
 // layout the mesh builders write) and none of its 1-D coordinates sits on a
 // coarse node, the interpolant is the sum-factorised product
@@ -203,7 +203,7 @@ __global__ void __launch_bounds__(IT, 10) interp_cells(
         for (int q = tid; q < 3 * p2; q += IT) {
             const int d = q / p2, mk = q - d * p2;
             if (d == 2 || (d == 0 ? newx : newy)) {
-                // a quotient from the reciprocal and its remainder: a product alone would give
+                // a quotient from the reciprocal and its remainder (Markstein, 1990): a product alone would give
                 // a whole row the reciprocal's rounding error (4.3e-16 instead of 4.2e-16
                 // from 64-bit results in the largest case)
                 const int m = mk / p1;
@@ -287,8 +287,13 @@ int interp_device(const double *cX, const double *cY, const double *cZ, const do
         cudaMemsetAsync(err, 0, sizeof(int), s);
         if ((rc = exclusive_scan(ppc_c, off_c, ncells, off_c + ncells, tmp, s))) break;
         if ((rc = exclusive_scan(ppc_f, off_f, ncells, off_f + ncells, tmp, s))) break;
-        // a cell's blocks go to several CTAs where the cells alone would not fill the
-        // chip; 624 cells (112 of them with children), order 6, 1 -> 8 parts: 131 -> 118 us a call
+        // A cell's children go to several CTAs where the cells alone would not fill the chip; each
+        // CTA stages the cell and forms its own contractions.  Us a call for 1, 2, 4, 8 parts, a
+        // fifth of the cells with 8 children of order 7: 624 cells 127, 99, 91, 89; 1,400 180, 136,
+        // 118, 121; 3,900 257, 199, 200, 240; 8,000 357, 323, 336, 435; 12,000 457, 436, 462, 612;
+        // order 3: 624 cells 76, 64, 58, 57; 12,000 139, 130, 143, 164.  Points off the tensor
+        // grid or on a node would take 4 parts above 4,000 cells as well (20,000 cells, order 5: 2
+        // parts 2196 us, 4 parts 2007, 8 parts 1899).
         const dim3 grid(ncells, ncells < 1500 ? 8 : (ncells < 4000 ? 4 : 2));
         switch (p1) {   // every loop over nodes known at compile time
 #define TAGI_INTERP(N)                                                                                             \

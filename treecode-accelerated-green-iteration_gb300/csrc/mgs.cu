@@ -171,7 +171,7 @@ __global__ void __launch_bounds__(MT) mgs_subtract(const double *V, double *U,
 }
 
 // u / norm to the last place from the reciprocal: q = u inv, then one correction by
-// the exact remainder (q itself where it is not finite).
+// the exact remainder (P. W. Markstein, IBM J. Res. Dev. 34, 1990; q itself where it is not finite).
 __device__ __forceinline__ double divide(double u, double norm, double inv) {
     const double q = __dmul_rn(u, inv);
     const double c = __fma_rn(__fma_rn(-q, norm, u), inv, q);

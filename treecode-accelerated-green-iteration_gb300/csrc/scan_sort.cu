@@ -135,8 +135,8 @@ namespace {
 // Radix passes: two chained launches per digit.  Bound: launch latency up to some
 // 200,000 keys, then L2 (12 bytes in, 12 out, scattered).  A block of the scatter adds up
 // where its tile's digits go from the tiles' counts, those of whole groups of tiles
-// first, so no scan runs between the two kernels: at 1.5M keys a block reads 27 rows
-// of 512 counts.  Nine-bit digits: 63-bit Morton codes take seven passes; 512 counters for
+// first, so no scan runs between the two kernels: at 1.5M keys (367 tiles) a block reads
+// 23 rows of group sums and up to 15 rows of its group's tiles, 512 counts each.  Nine-bit digits: 63-bit Morton codes take seven passes; 512 counters for
 // each of eight warps are 16 KB of shared memory.  Digits of eight bits with a scan
 // between took 24 launches (40 above 130,000 keys).  44,000 keys: 60 us.
 constexpr int RS_THREADS = 256, RS_WARPS = RS_THREADS / 32, RS_BITS = 9, RS_DIGITS = 1 << RS_BITS;

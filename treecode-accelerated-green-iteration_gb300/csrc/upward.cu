@@ -9,7 +9,7 @@
 // sums and a second kernel adds the partials of a slot in item order, so results
 // do not depend on scheduling.  The weight charges (q = w) are built once per plan;
 // charge vectors are done per call, in FP32 products summed over a tile of 64
-// sources, the tiles' sums then accumulated without error (mixed), or all in
+// sources, the tiles' sums then accumulated to about 72 bits (mixed), or all in
 // FP64.
 //
 // Bound (mixed): FP32 issue.  A tile's sums were added in FP64, whose pipe (1/64 of
