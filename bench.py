@@ -1383,7 +1383,8 @@ def interp_arm(args):
     value = fine points interpolated per second, coarse values and both meshes
     resident in HBM; e2e = the same through the host-pointer drop-in
     InterpolateBetweenTwoMeshes with every array on the host.  Roofline: the
-    FP64 pipe (three 1-D contractions, 3(p+1) multiply-adds per fine point);
+    FP64 pipe (three 1-D contractions shared by the children of a cell, 14 (p+1) / 8
+    multiply-adds per interpolated point);
     the algorithmic bytes (coarseN + 4 fineN) x 8 are reported beside it
     against the measured HBM rate."""
     import torch
@@ -1434,11 +1435,13 @@ def interp_arm(args):
     interp_err = float(torch.linalg.norm(out - Ff) / torch.linalg.norm(Ff))
     rates = pipe_rates(L, nat, stream)
     p1 = order + 1
-    # the mesh's fine points lie on tensor grids per child cell, so the kernel takes its
-    # sum-factorised path: three 1-D contractions, 3 (p+1) multiply-adds per fine point
-    # (plus 3 (p+1)^2 divisions per block of (p+1)^3 points, left out of the count)
-    dfma_per_point = 3 * p1
-    ach_fp64 = nf * dfma_per_point / (ms * 1e-3)
+    # The mesh's fine points lie on tensor grids per child cell, so the kernel takes its
+    # sum-factorised path, in which children share contractions: of the 8 children of a cell
+    # 2 contractions over x, 4 over y and 8 over z of p + 1 multiply-adds per grid point (plus
+    # the rows of weights, left out of the count).  Cells without children are copied.
+    dfma_per_point = (2 + 4 + 8) * p1 / 8.0
+    interpolated = int(m.PtsPerCellFine[m.PtsPerCellFine > p1 ** 3].sum())
+    ach_fp64 = interpolated * dfma_per_point / (ms * 1e-3)
     alg_bytes = 8.0 * (nc + 4 * nf)
     peaks = {}
     try:
@@ -1447,9 +1450,10 @@ def interp_arm(args):
     except OSError:
         pass
     hbm = peaks.get("hbm_gbs") or 6800.0
-    roof = {"bound": "fp64", "kernel": "interp_cells (one CTA per cell, sum-factorised tensor-grid path)",
+    roof = {"bound": "fp64", "kernel": "interp_cells (sum-factorised tensor-grid path)",
             "achieved": ach_fp64 / 1e9, "peak": rates["dfma"] / 1e9, "unit": "G DFMA/s",
-            "frac": ach_fp64 / rates["dfma"], "ops_per_fine_point": dfma_per_point, "traffic": None,
+            "frac": ach_fp64 / rates["dfma"], "ops_per_fine_point": dfma_per_point,
+            "interpolated_points": interpolated, "traffic": None,
             "peak_source": "FP64 DFMA rate measured live on this GPU (tagi_pipe_rates)",
             "hbm_view": {"algorithmic_bytes": alg_bytes, "achieved_gbs": alg_bytes / (ms * 1e-3) / 1e9,
                          "peak_gbs": hbm, "frac": alg_bytes / (ms * 1e-3) / 1e9 / hbm,
